@@ -504,11 +504,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                     b0 = Bits{in[2 * (kBM + pt) + sw], in[2 * (kBM + pt) + (sw ^ 1)]};
                     if (two_b)
                         b1 = Bits{in[2 * (kBM + pt + 128) + sw], in[2 * (kBM + pt + 128) + (sw ^ 1)]};
-                    mbar_arrive(&in_empty[islot]);
-                    if (++islot == kIn) {
-                        islot = 0;
-                        iph ^= 1u;
-                    }
                 } else if (kb + 1 < G.kb) {  // next block's bits load while this one expands
                     xa = load_bits(P.r, ra, P.n_r, P.n_words, kb + 1, vec);
                     xb0 = load_bits(P.q, qb0, P.n_q, P.n_words, kb + 1, vec);
@@ -528,6 +523,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                 cb1 += popc_bits(b1);
                 fence_proxy_async_smem();
                 mbar_arrive(&full[stage]);
+                if (use_in) {
+                    // the slot is given back only here, after its words have
+                    // been used and the proxy fence: an arrive directly after
+                    // the reads let the next tensor load land before queued
+                    // reads had returned (seen when the epilogue's per-lane
+                    // stores filled the load/store queue)
+                    mbar_arrive(&in_empty[islot]);
+                    if (++islot == kIn) {
+                        islot = 0;
+                        iph ^= 1u;
+                    }
+                }
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1u;

@@ -233,3 +233,26 @@ def test_output_pitch(cuda_device, measure, ld):
     host = buf.cpu().numpy()
     _bits_equal(host[:, :nq], oracle.fingerprint(measure, a, va, b, None, n_words, np.nan))
     assert (host[:, nq:] == 7.0).all()
+
+
+@pytest.mark.parametrize("n_bits", [512, 2048, 4096])
+@pytest.mark.parametrize("nq,ld", [(2047, 2047), (2046, 2048), (4001, 4004)])
+def test_many_tiles_odd_columns(cuda_device, nq, ld, n_bits):
+    """Many tiles per CTA while the epilogue stores lane by lane (unaligned rows,
+    or the last columns of aligned ones): every value equal to the oracle, twice."""
+    import torch
+
+    from cudams import kernels, synthetic
+
+    dev = torch.device("cuda", torch.cuda.current_device())
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(dev)  # noqa: E731
+    nr, n_words = 9001, n_bits // 32
+    a = synthetic.fingerprints(nr, n_bits=n_bits, seed=31)
+    b = synthetic.fingerprints(nq, n_bits=n_bits, seed=32)
+    want = oracle.fingerprint("jaccard", a, None, b, None, n_words, np.nan)
+    ta, tb = t(a), t(b)
+    for _ in range(2):
+        out = torch.full((nr, ld), 7.0, dtype=torch.float32, device=dev)[:, :nq]
+        kernels.fingerprint_matrix("jaccard", ta, None, tb, None, n_words, np.nan, out=out,
+                                   check_errors=True)
+        _bits_equal(out.cpu().numpy(), want)
