@@ -7,16 +7,19 @@
 // ordered differs.
 //
 // Pipeline of one call (all on one stream, no host synchronisation):
-//   1. validate_kernel   offsets sane, spectra <= CMS_MAX_PEAKS; else every
-//                        later kernel exits at once and the error word is set
-//   2. norms_kernel      sqrt(sum (a*b)^2) per spectrum, sequential float64
-//   3. order kernels     reference spectra ordered by peak count, largest
+//   1. prep_kernel       both sets: offsets sane, spectra <= CMS_MAX_PEAKS
+//                        (else every later kernel exits at once and the error
+//                        word is set); sqrt(sum (a*b)^2) per spectrum,
+//                        sequential float64; the reference spectra's length
+//                        classes and the query peaks' bucket counts
+//   2. order_scatter     reference spectra ordered by peak count, largest
 //                        first (log2 length classes), for load balance
-//   4. index kernels     query spectra are cut into tiles of tile_spectra;
+//   3. index kernels     query spectra are cut into tiles of tile_spectra;
 //                        each tile's peaks are bucketed by m/z (bucket width
-//                        tol by default, buckets hashed modulo n_buckets) into a
-//                        CSR "tile stream" of (m/z, query<<16 | peak)
-//   5. join_kernel       persistent warps; one work item = (reference
+//                        tol by default, buckets hashed modulo n_buckets;
+//                        two-launch scan of the counts, then scatter) into a
+//                        CSR "tile stream" of (m/z, query<<16 | peak, weight)
+//   4. join_kernel       persistent warps; one work item = (reference
 //                        spectrum, query tile).  Lanes take reference peaks,
 //                        jump through the bucket table to the tile-stream
 //                        entries inside the tolerance window (the
@@ -37,13 +40,13 @@
 //                        stores just before, and each run stores its result
 //                        over its zeros.  Pairs with longer runs (or >=
 //                        match_limit candidates) go to a spill list.
-//   6. pair_kernel       one CTA per spilled pair (or per pair of the whole
+//   5. pair_kernel       one CTA per spilled pair (or per pair of the whole
 //                        matrix in mode 2): exact generation-order sweep with
 //                        match_limit truncation, bitonic sort of (key, gen)
 //                        (in registers when there are eight candidates a
 //                        thread, else in shared memory), warp greedy with
 //                        per-chunk conflict masks and used-peak bitmasks.
-//   7. mirror_kernel     (symmetric dense calls, csrc/mirror.cu) lower
+//   6. mirror_kernel     (symmetric dense calls, csrc/mirror.cu) lower
 //                        triangle copied from the upper one.
 #include <algorithm>
 #include <cmath>
@@ -67,78 +70,14 @@ constexpr int kModifiedMaxPeaks = 32767;  // modified cosine: reference peak ind
 
 __device__ __forceinline__ double peak_a(const double* a, int64_t i) { return a ? a[i] : 1.0; }
 
-// ---------------------------------------------------------------------------
-// 1. validation
-// ---------------------------------------------------------------------------
-__global__ void validate_kernel(SpecSet S, uint32_t* bad, uint32_t* err,
-                                int max_peaks = CMS_MAX_PEAKS) {
-    const int64_t n = S.n;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t lo = S.off[s], hi = S.off[s + 1];
-        uint32_t e = 0;
-        if (lo < 0 || hi < lo || hi > S.n_peaks) e |= kErrBadOffsets;
-        if (hi - lo > max_peaks) e |= kErrSpectrumTooLong;
-        if (e) {
-            atomicOr(err, e);
-            atomicOr(bad, 1u);
-        }
-    }
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
 
 // ---------------------------------------------------------------------------
-// 2. norms: sn[s] = sqrt(sum_k (a_k*b_k)^2), summed in peak order
-// ---------------------------------------------------------------------------
-__global__ void norms_kernel(SpecSet S, double* sn, const uint32_t* bad) {
-    if (*bad) return;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < S.n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t lo = S.off[s], hi = S.off[s + 1];
-        double acc = 0.0;
-        for (int64_t k = lo; k < hi; ++k) {
-            const double w = __dmul_rn(peak_a(S.a, k), S.b[k]);
-            acc = __dadd_rn(acc, __dmul_rn(w, w));
-        }
-        sn[s] = sqrt(acc);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// 3. reference order: largest length class first
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int length_class(int64_t len) {
-    return len <= 0 ? 0 : min(kOrderClasses - 1, 64 - __clzll((unsigned long long)len));
-}
-
-__global__ void order_count_kernel(SpecSet S, uint32_t* cls_count, const uint32_t* bad) {
-    if (*bad) return;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < S.n;
-         s += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&cls_count[length_class(S.off[s + 1] - S.off[s])], 1u);
-}
-
-__global__ void order_scatter_kernel(SpecSet S, const uint32_t* cls_count, uint32_t* cls_cursor,
-                                     int32_t* order, const uint32_t* bad) {
-    if (*bad) return;
-    __shared__ uint32_t base[kOrderClasses];
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (int c = kOrderClasses - 1; c >= 0; --c) {
-            base[c] = acc;
-            acc += cls_count[c];
-        }
-    }
-    __syncthreads();
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < S.n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int c = length_class(S.off[s + 1] - S.off[s]);
-        const uint32_t pos = base[c] + atomicAdd(&cls_cursor[c], 1u);
-        order[pos] = (int32_t)s;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// 4. tile index over the query side
+// tile index over the query side
 // ---------------------------------------------------------------------------
 // tile-stream entry: m/z, (query within tile << 16 | peak), intensity weight b
 struct __align__(16) Entry {
@@ -166,77 +105,225 @@ __device__ __forceinline__ long long bucket_of(float x, double inv_w) {
 // of modified cosine (NL) its m/z minus its spectrum's precursor m/z, computed
 // in float64 and rounded to float32 (the join widens its windows by a margin
 // that covers this rounding and confirms each candidate exactly).
+__device__ __forceinline__ float loss_value(float mz, double prec) {
+    return __double2float_rn(__dsub_rn((double)mz, prec));
+}
 template <bool NL>
 __device__ __forceinline__ float index_value(const SpecSet& B, int64_t s, int64_t k) {
-    if (!NL) return B.mz[k];
-    return __double2float_rn(__dsub_rn((double)B.mz[k], B.prec[s]));
+    return NL ? loss_value(B.mz[k], B.prec[s]) : B.mz[k];
 }
 
-// warp per spectrum: histogram of (tile, bucket)
-template <bool NL>
-__global__ void index_count_kernel(SpecSet B, IndexGeom g, uint32_t* cnt, const uint32_t* bad) {
-    if (*bad) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const unsigned mask = (unsigned)(g.nb - 1);
-    for (int64_t s = warp; s < B.n; s += nwarps) {
-        const int64_t t = s / g.tile;
-        const int64_t lo = B.off[s], hi = B.off[s + 1];
-        uint32_t* c = cnt + t * (int64_t)g.nb;
-        for (int64_t k = lo + lane; k < hi; k += 32) {
-            const unsigned bk = (unsigned)bucket_of(index_value<NL>(B, s, k), g.inv_w) & mask;
-            atomicAdd(&c[bk], 1u);
-        }
-    }
+// ---------------------------------------------------------------------------
+// 1. preparation of a spectrum set: validation, norms, length classes and
+//    bucket counts in one launch
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int length_class(int64_t len) {
+    return len <= 0 ? 0 : min(kOrderClasses - 1, 64 - __clzll((unsigned long long)len));
 }
 
-// CTA per tile: exclusive scan of the bucket counts into tab[t][0..nb], and
-// reset the counters to the bucket starts (scatter cursors).
-__global__ void index_scan_kernel(IndexGeom g, uint32_t* cnt_cur, uint32_t* tab,
-                                  const uint32_t* bad) {
-    if (*bad) return;
-    const int t = blockIdx.x;
-    uint32_t* c = cnt_cur + (int64_t)t * g.nb;
-    uint32_t* out = tab + (int64_t)t * (g.nb + 1);
-    const int per = (g.nb + blockDim.x - 1) / blockDim.x;
-    const int begin = min(g.nb, (int)threadIdx.x * per);
-    const int end = min(g.nb, begin + per);
-    uint32_t local = 0;
-    for (int k = begin; k < end; ++k) local += c[k];
-    // block exclusive scan of `local`
-    __shared__ uint32_t warp_sums[32];
+struct PrepSide {
+    SpecSet S;
+    double* sn;           // sqrt(sum_k (a_k * b_k)^2), summed in peak order
+    uint32_t* cls_count;  // spectra per length class (null: not wanted)
+    uint32_t* cnt;        // peaks per (tile, bucket) of the m/z index (null: not wanted)
+    uint32_t* cnt2;       // the same of the neutral-loss index (null: not wanted)
+};
+
+// cnt / cnt2 have geometry g.  Offsets out of order or range and spectra above
+// max_peaks raise the error word and *bad, which stops every later kernel of
+// the call; such a spectrum is skipped here.
+//
+// A norm is one float64 sum in peak order, a serial chain, so a warp takes
+// kPrepSpectra spectra at once: their peaks come 32 at a time with coalesced
+// loads through a shared-memory tile, and lane j adds up spectrum j while the
+// next 32 peaks of each are in flight.  One thread a spectrum, reading its
+// peaks one after the other, took 24 us for 1024 spectra of up to 200 peaks,
+// 84 us for 50000 of up to 1000 and 445 us for 900 of up to 2000, for each
+// side; this takes 10, 52 and 60 us (17 and 84 us with the bucket counts, which
+// took 7 and 47 us in a launch of their own).
+constexpr int kPrepSpectra = 8;
+constexpr int kPrepThreads = 128;
+__global__ void __launch_bounds__(kPrepThreads)
+prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks) {
+    __shared__ double s_tile[kPrepThreads / 32][kPrepSpectra][33];
+    __shared__ uint32_t s_cls[kOrderClasses];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t incl = local;
+    const unsigned full = 0xffffffffu;
+    double(*tile)[33] = s_tile[wid];
+    if (threadIdx.x < kOrderClasses) s_cls[threadIdx.x] = 0u;
+    __syncthreads();
+    const unsigned mask = (unsigned)(g.nb - 1);
+    const int64_t warps = (int64_t)gridDim.x * (kPrepThreads / 32);
+    const int64_t n = P.S.n;
+    for (int64_t s0 = ((int64_t)blockIdx.x * (kPrepThreads / 32) + wid) * kPrepSpectra; s0 < n;
+         s0 += warps * kPrepSpectra) {
+        int64_t lo = 0;
+        int len = 0;
+        if (lane < kPrepSpectra && s0 + lane < n) {
+            lo = P.S.off[s0 + lane];
+            const int64_t hi = P.S.off[s0 + lane + 1];
+            uint32_t e = 0;
+            if (lo < 0 || hi < lo || hi > P.S.n_peaks) e |= kErrBadOffsets;
+            if (hi - lo > max_peaks) e |= kErrSpectrumTooLong;
+            if (e) {
+                atomicOr(err, e);
+                atomicOr(bad, 1u);
+                lo = 0;
+            } else {
+                len = (int)(hi - lo);
+                if (P.cls_count) atomicAdd(&s_cls[length_class(len)], 1u);
+            }
+        }
+        const int longest = __reduce_max_sync(full, len);
+        // the loads of all spectra are issued before the first is used
+        double v[kPrepSpectra], w[kPrepSpectra];
+        float z[kPrepSpectra];
+        auto load = [&](int c) {
+#pragma unroll
+            for (int j = 0; j < kPrepSpectra; ++j) {
+                const int64_t k = __shfl_sync(full, lo, j) + c + lane;
+                const bool in = c + lane < __shfl_sync(full, len, j);
+                v[j] = in ? P.S.b[k] : 0.0;
+                w[j] = (in && P.S.a) ? P.S.a[k] : 1.0;
+                z[j] = (in && P.cnt) ? P.S.mz[k] : 0.f;
+            }
+        };
+        auto count = [&](int c) {
+            if (!P.cnt) return;
+#pragma unroll
+            for (int j = 0; j < kPrepSpectra; ++j) {
+                if (c + lane >= __shfl_sync(full, len, j)) continue;
+                const int64_t t = (s0 + j) / g.tile * (int64_t)g.nb;
+                atomicAdd(&P.cnt[t + ((unsigned)bucket_of(z[j], g.inv_w) & mask)], 1u);
+                if (P.cnt2) {
+                    const float d = loss_value(z[j], P.S.prec[s0 + j]);
+                    atomicAdd(&P.cnt2[t + ((unsigned)bucket_of(d, g.inv_w) & mask)], 1u);
+                }
+            }
+        };
+        double acc = 0.0;
+        load(0);
+        for (int c = 0; c < longest; c += 32) {
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < kPrepSpectra; ++j) {
+                const double x = __dmul_rn(w[j], v[j]);
+                tile[j][lane] = __dmul_rn(x, x);
+            }
+            count(c);
+            __syncwarp();
+            if (c + 32 < longest) load(c + 32);
+            // past a spectrum's end the tile holds +0.0, which leaves the sum as it is
+            if (lane < kPrepSpectra) {
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) acc = __dadd_rn(acc, tile[lane][k]);
+            }
+        }
+        if (lane < kPrepSpectra && s0 + lane < n) P.sn[s0 + lane] = sqrt(acc);
+        __syncwarp();
+    }
+    __syncthreads();
+    if (P.cls_count && threadIdx.x < kOrderClasses && s_cls[threadIdx.x])
+        atomicAdd(&P.cls_count[threadIdx.x], s_cls[threadIdx.x]);
+}
+
+// Exclusive scan of the bucket counts into tab[t][0..nb], and the counters to
+// the bucket starts (scatter cursors), in two launches of one CTA per chunk of
+// kScanChunk buckets: the chunks' sums, then each chunk's own scan on top of
+// the sums of its tile's earlier chunks.  Coalesced both ways: 25 us for 25
+// tiles of 2^18 buckets (one CTA a tile, each thread walking its own run of
+// buckets: 636 us).
+constexpr int kScanThreads = 256;
+constexpr int kScanPer = 16;
+constexpr int kScanChunk = kScanThreads * kScanPer;
+__host__ __device__ constexpr int scan_chunks(int nb) { return (nb + kScanChunk - 1) / kScanChunk; }
+
+__device__ __forceinline__ uint32_t block_sum(uint32_t x, uint32_t* s_warp) {
+    x = __reduce_add_sync(0xffffffffu, x);
+    __syncthreads();  // s_warp free from an earlier use
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = x;
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) total += s_warp[w];
+    return total;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+index_sums_kernel(IndexGeom g, const uint32_t* cnt, uint32_t* sums, const uint32_t* bad) {
+    if (*bad) return;
+    __shared__ uint32_t s_warp[kScanThreads / 32];
+    const int per_tile = scan_chunks(g.nb);
+    const int t = (int)blockIdx.x / per_tile, ch = (int)blockIdx.x % per_tile;
+    const uint32_t* c = cnt + (int64_t)t * g.nb + (int64_t)ch * kScanChunk;
+    const int m = min(kScanChunk, g.nb - ch * kScanChunk);
+    uint32_t x = 0;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+        const int k = i * kScanThreads + (int)threadIdx.x;
+        if (k < m) x += c[k];
+    }
+    x = block_sum(x, s_warp);
+    if (threadIdx.x == 0) sums[blockIdx.x] = x;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+index_scan_kernel(IndexGeom g, uint32_t* cnt_cur, uint32_t* tab, const uint32_t* sums,
+                  const uint32_t* bad) {
+    if (*bad) return;
+    __shared__ uint32_t s_val[kScanChunk + kScanChunk / kScanPer];
+    __shared__ uint32_t s_warp[kScanThreads / 32], s_incl[kScanThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int per_tile = scan_chunks(g.nb);
+    const int t = (int)blockIdx.x / per_tile, ch = (int)blockIdx.x % per_tile;
+    uint32_t* c = cnt_cur + (int64_t)t * g.nb + (int64_t)ch * kScanChunk;
+    uint32_t* out = tab + (int64_t)t * (g.nb + 1) + (int64_t)ch * kScanChunk;
+    const int m = min(kScanChunk, g.nb - ch * kScanChunk);
+    // coalesced in, kScanPer consecutive buckets a thread out of shared memory
+    // (one word of padding per kScanPer, so that neither side has conflicts)
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+        const int k = i * kScanThreads + tid;
+        s_val[k + k / kScanPer] = k < m ? c[k] : 0u;
+    }
+    uint32_t prev = 0;  // the tile's earlier chunks
+    for (int i = tid; i < ch; i += kScanThreads) prev += sums[t * per_tile + i];
+    prev = block_sum(prev, s_warp);
+    uint32_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) sum += s_val[tid * (kScanPer + 1) + i];
+    uint32_t incl = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += v;
     }
-    if (lane == 31) warp_sums[wid] = incl;
+    if (lane == 31) s_incl[wid] = incl;
     __syncthreads();
-    if (wid == 0) {
-        const int nw = blockDim.x >> 5;
-        uint32_t v = lane < nw ? warp_sums[lane] : 0u;
+    uint32_t run = prev + incl - sum;
+    for (int w = 0; w < wid; ++w) run += s_incl[w];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
-            if (lane >= d) v += u;
-        }
-        if (lane < nw) warp_sums[lane] = v;
-    }
-    __syncthreads();
-    uint32_t run = incl - local + (wid > 0 ? warp_sums[wid - 1] : 0u);
-    for (int k = begin; k < end; ++k) {
-        const uint32_t v = c[k];
-        out[k] = run;
-        c[k] = run;
+    for (int i = 0; i < kScanPer; ++i) {
+        const uint32_t v = s_val[tid * (kScanPer + 1) + i];
+        s_val[tid * (kScanPer + 1) + i] = run;
         run += v;
     }
-    if (threadIdx.x == blockDim.x - 1) out[g.nb] = run;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+        const int k = i * kScanThreads + tid;
+        if (k < m) {
+            const uint32_t v = s_val[k + k / kScanPer];
+            out[k] = v;
+            c[k] = v;
+        }
+    }
+    if (ch == per_tile - 1 && tid == kScanThreads - 1) out[m] = run;
 }
 
-// warp per spectrum: scatter (value, q_local<<16 | peak) into the tile stream
+// Warp per spectrum: its peaks (value, q_local<<16 | peak) into the tile
+// stream, four chunks of 32 with their cursor atomics in flight at a time
+// (4.7 M peaks: 110 us; one chunk at a time 135 us).
 template <bool NL>
 __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entry* ent,
                                      const uint32_t* bad) {
@@ -245,22 +332,74 @@ __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entr
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned mask = (unsigned)(g.nb - 1);
+    constexpr int kU = 4;
     for (int64_t s = warp; s < B.n; s += nwarps) {
         const int64_t t = s / g.tile;
         const int64_t base = B.off[t * g.tile];
         const uint32_t ql = (uint32_t)(s - t * g.tile);
         const int64_t lo = B.off[s], hi = B.off[s + 1];
         uint32_t* c = cur + t * (int64_t)g.nb;
-        for (int64_t k = lo + lane; k < hi; k += 32) {
-            const float mz = index_value<NL>(B, s, k);
-            const unsigned bk = (unsigned)bucket_of(mz, g.inv_w) & mask;
-            const uint32_t pos = atomicAdd(&c[bk], 1u);
-            Entry en;
-            en.mz = mz;
-            en.id = (ql << 16) | (uint32_t)(k - lo);
-            en.b = B.b[k];
-            ent[base + pos] = en;
+        for (int64_t k0 = lo + lane; k0 < hi; k0 += 32 * kU) {
+            float v[kU];
+            double b[kU];
+            uint32_t pos[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int64_t k = k0 + 32 * u;
+                if (k < hi) {
+                    v[u] = index_value<NL>(B, s, k);
+                    b[u] = B.b[k];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+                if (k0 + 32 * u < hi)
+                    pos[u] = atomicAdd(&c[(unsigned)bucket_of(v[u], g.inv_w) & mask], 1u);
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int64_t k = k0 + 32 * u;
+                if (k < hi) {
+                    Entry en;
+                    en.mz = v[u];
+                    en.id = (ql << 16) | (uint32_t)(k - lo);
+                    en.b = b[u];
+                    ent[base + pos[u]] = en;
+                }
+            }
         }
+    }
+}
+
+// Sweeping-side order (largest length class first); a block's spectra are
+// ranked per class in shared memory, so that the 17 cursors get one atomic a
+// block and class.
+constexpr int kOrderThreads = 256;
+__global__ void __launch_bounds__(kOrderThreads)
+order_scatter_kernel(SpecSet S, const uint32_t* cls_count, uint32_t* cls_cursor, int32_t* order,
+                     const uint32_t* bad) {
+    if (*bad) return;
+    __shared__ uint32_t s_cnt[kOrderClasses], s_base[kOrderClasses];
+    const int tid = threadIdx.x;
+    for (int64_t s0 = (int64_t)blockIdx.x * kOrderThreads; s0 < S.n;
+         s0 += (int64_t)gridDim.x * kOrderThreads) {
+        if (tid < kOrderClasses) s_cnt[tid] = 0u;
+        __syncthreads();
+        const int64_t s = s0 + tid;
+        int c = 0;
+        uint32_t rank = 0;
+        if (s < S.n) {
+            c = length_class(S.off[s + 1] - S.off[s]);
+            rank = atomicAdd(&s_cnt[c], 1u);
+        }
+        __syncthreads();
+        if (tid < kOrderClasses && s_cnt[tid]) {
+            uint32_t base = 0;
+            for (int k = kOrderClasses - 1; k > tid; --k) base += cls_count[k];
+            s_base[tid] = base + atomicAdd(&cls_cursor[tid], s_cnt[tid]);
+        }
+        __syncthreads();
+        if (s < S.n) order[s_base[c] + rank] = (int32_t)s;
+        __syncthreads();
     }
 }
 
@@ -309,12 +448,6 @@ struct TraceOut {
     unsigned int tag;
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 struct SpillList {
     int2* pairs;  // (reference, query)
     unsigned int* count;
@@ -330,7 +463,7 @@ __device__ __forceinline__ void spill_push(const SpillList& sl, int r, int q, ui
 }
 
 // ---------------------------------------------------------------------------
-// 5. join kernel
+// 4. join kernel
 // ---------------------------------------------------------------------------
 struct JoinParams {
     SpecSet A;  // sweeping side (one spectrum per work item)
@@ -1153,7 +1286,7 @@ join_kernel(JoinParams P) {
 }
 
 // ---------------------------------------------------------------------------
-// 6. pair kernel: one CTA per pair
+// 5. pair kernel: one CTA per pair
 // ---------------------------------------------------------------------------
 struct PairParams {
     SpecSet R;
@@ -1706,11 +1839,6 @@ __global__ void pair_kernel(PairParams P) {
 // so their named barrier is never left half-joined.
 constexpr unsigned long long kPipeWaitNs = 2000000000ull;
 
-__device__ __forceinline__ unsigned long long pipe_clock() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ void pipe_bar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(bar)),
@@ -1726,7 +1854,7 @@ __device__ __forceinline__ void pipe_bar_arrive(uint64_t* bar) {
 __device__ __forceinline__ bool pipe_bar_wait(uint64_t* bar, uint32_t parity,
                                               volatile int* stop) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    const unsigned long long t0 = pipe_clock();
+    const unsigned long long t0 = global_ns();
     for (;;) {
         uint32_t ok;
         asm volatile(
@@ -1738,7 +1866,7 @@ __device__ __forceinline__ bool pipe_bar_wait(uint64_t* bar, uint32_t parity,
             : "memory");
         if (ok) return true;
         if (*stop) return false;
-        if (pipe_clock() - t0 > kPipeWaitNs) return false;
+        if (global_ns() - t0 > kPipeWaitNs) return false;
     }
 }
 
@@ -1966,6 +2094,13 @@ int set_func_smem(T* f, size_t bytes) {
     return raise_func_smem(reinterpret_cast<const void*>(f), bytes);
 }
 
+// Blocks for n spectra at `per` spectra a block, at most 32 a multiprocessor.
+int blocks_for(int64_t n, int per, int sms) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>((n + per - 1) / per, (int64_t)sms * 32));
+}
+constexpr int kPrepPerBlock = kPrepSpectra * (kPrepThreads / 32);
+constexpr int kScatterThreads = 256;  // index scatter: a warp per spectrum
+
 // Launch the join.  Persistent (waves == 0): one resident CTA per slot, each
 // warp pulling work until none is left; CTA b owns global-pool slices
 // 8b..8b+7, so the grid may not exceed the resident CTAs.  Bounded
@@ -2048,14 +2183,11 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     need += bump_size(nR * sizeof(double)) + bump_size(nQ * sizeof(double));
     if (p.mode == 1) {
         need += bump_size(nR * sizeof(int32_t));
-        need += bump_size((size_t)p.n_tiles * (p.nb + 1) * sizeof(uint32_t));
-        need += bump_size((size_t)p.n_tiles * p.nb * sizeof(uint32_t));
-        need += bump_size((size_t)std::max<int64_t>(1, args.qry.n_peaks) * sizeof(Entry));
-        if (args.modified) {  // the neutral-loss index
-            need += bump_size((size_t)p.n_tiles * (p.nb + 1) * sizeof(uint32_t));
-            need += bump_size((size_t)p.n_tiles * p.nb * sizeof(uint32_t));
-            need += bump_size((size_t)std::max<int64_t>(1, args.qry.n_peaks) * sizeof(Entry));
-        }
+        const size_t idx = args.modified ? 2 : 1;  // m/z index, neutral-loss index
+        need += bump_size(idx * (size_t)p.n_tiles * p.nb * sizeof(uint32_t));
+        need += bump_size((size_t)p.n_tiles * scan_chunks(p.nb) * sizeof(uint32_t));
+        need += idx * bump_size((size_t)p.n_tiles * (p.nb + 1) * sizeof(uint32_t));
+        need += idx * bump_size((size_t)std::max<int64_t>(1, args.qry.n_peaks) * sizeof(Entry));
         need += bump_size((size_t)p.spill_cap * sizeof(int2));
         need += bump_size(gpool_bytes);
     }
@@ -2084,24 +2216,29 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     unsigned int* spill_count = reinterpret_cast<unsigned int*>(small + 20);
     unsigned long long* work_join = reinterpret_cast<unsigned long long*>(small + 21);
     unsigned long long* work_pair = reinterpret_cast<unsigned long long*>(small + 22);
+    // the bucket counts lie behind the counters: one memset clears both
+    const size_t idx = p.mode != 1 ? 0 : (args.modified ? 2 : 1);
+    const size_t n_cnt = (size_t)p.n_tiles * p.nb;
+    const int n_chunks = p.n_tiles * scan_chunks(p.nb);
+    uint32_t* cur = idx ? bp.take<uint32_t>(idx * n_cnt) : nullptr;
+    const size_t zeroed = bp.used - (size_t)((char*)small - (char*)ctx->scratch.ptr);
+    uint32_t* cur2 = idx == 2 ? cur + n_cnt : nullptr;
+    uint32_t* sums = idx ? bp.take<uint32_t>(n_chunks) : nullptr;
     double* snR = bp.take<double>(nR);
     double* snQ = bp.take<double>(nQ);
-    CMS_CUDA_TRY(cudaMemsetAsync(small, 0, 64 * sizeof(uint64_t), s));
+    CMS_CUDA_TRY(cudaMemsetAsync(small, 0, zeroed, s));
 
-    const int threads = 256;
-    auto grid_for = [&](int64_t n, int per_block) {
-        int64_t g = (n + per_block - 1) / per_block;
-        return (int)std::max<int64_t>(1, std::min<int64_t>(g, (int64_t)ctx->sm_count * 32));
-    };
+    const IndexGeom g{p.tile, p.n_tiles, p.nb, 1.0 / p.width};
+    const int sms = ctx->sm_count;
     {
-        StageScope sc(ctx, 0, 4, s);
+        StageScope sc(ctx, 0, 2, s);
         const int max_peaks = args.modified ? kModifiedMaxPeaks : CMS_MAX_PEAKS;
-        validate_kernel<<<grid_for(nR, threads), threads, 0, s>>>(args.ref, bad, ctx->err_word,
-                                                                 max_peaks);
-        validate_kernel<<<grid_for(nQ, threads), threads, 0, s>>>(args.qry, bad, ctx->err_word,
-                                                                 max_peaks);
-        norms_kernel<<<grid_for(nR, threads), threads, 0, s>>>(args.ref, snR, bad);
-        norms_kernel<<<grid_for(nQ, threads), threads, 0, s>>>(args.qry, snQ, bad);
+        const PrepSide pr{args.ref, snR, idx ? cls_count : nullptr, nullptr, nullptr};
+        const PrepSide pq{args.qry, snQ, nullptr, cur, cur2};
+        prep_kernel<<<blocks_for(nR, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
+            pr, g, bad, ctx->err_word, max_peaks);
+        prep_kernel<<<blocks_for(nQ, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
+            pq, g, bad, ctx->err_word, max_peaks);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
@@ -2173,42 +2310,35 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     // ---- mode 1: order, index, join, spill ----
     int32_t* order = bp.take<int32_t>(nR);
     uint32_t* tab = bp.take<uint32_t>((size_t)p.n_tiles * (p.nb + 1));
-    uint32_t* cur = bp.take<uint32_t>((size_t)p.n_tiles * p.nb);
     Entry* ent = bp.take<Entry>((size_t)std::max<int64_t>(1, args.qry.n_peaks));
     uint32_t* tab2 = nullptr;
-    uint32_t* cur2 = nullptr;
     Entry* ent2 = nullptr;
     if (args.modified) {
         tab2 = bp.take<uint32_t>((size_t)p.n_tiles * (p.nb + 1));
-        cur2 = bp.take<uint32_t>((size_t)p.n_tiles * p.nb);
         ent2 = bp.take<Entry>((size_t)std::max<int64_t>(1, args.qry.n_peaks));
     }
     int2* spill = bp.take<int2>(p.spill_cap);
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
 
     {
-        StageScope sc(ctx, 1, 2, s);
-        order_count_kernel<<<grid_for(nR, threads), threads, 0, s>>>(args.ref, cls_count, bad);
-        order_scatter_kernel<<<grid_for(nR, threads), threads, 0, s>>>(args.ref, cls_count,
-                                                                       cls_cursor, order, bad);
+        StageScope sc(ctx, 1, 1, s);
+        order_scatter_kernel<<<blocks_for(nR, kOrderThreads, sms), kOrderThreads, 0, s>>>(
+            args.ref, cls_count, cls_cursor, order, bad);
     }
-    IndexGeom g{p.tile, p.n_tiles, p.nb, 1.0 / p.width};
+    const int scatter_blocks = blocks_for(nQ, kScatterThreads / 32, sms);
     {
         StageScope sc(ctx, 2, 3, s);
-        CMS_CUDA_TRY(cudaMemsetAsync(cur, 0, (size_t)p.n_tiles * p.nb * sizeof(uint32_t), s));
-        index_count_kernel<false><<<grid_for(nQ * 32, threads), threads, 0, s>>>(args.qry, g, cur, bad);
-        index_scan_kernel<<<p.n_tiles, 1024, 0, s>>>(g, cur, tab, bad);
-        index_scatter_kernel<false><<<grid_for(nQ * 32, threads), threads, 0, s>>>(args.qry, g, cur,
-                                                                            ent, bad);
+        index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur, sums, bad);
+        index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur, tab, sums, bad);
+        index_scatter_kernel<false><<<scatter_blocks, kScatterThreads, 0, s>>>(args.qry, g, cur, ent,
+                                                                               bad);
     }
     if (args.modified) {  // neutral-loss index: m/z - precursor, same geometry
         StageScope sc(ctx, 2, 3, s);
-        CMS_CUDA_TRY(cudaMemsetAsync(cur2, 0, (size_t)p.n_tiles * p.nb * sizeof(uint32_t), s));
-        index_count_kernel<true><<<grid_for(nQ * 32, threads), threads, 0, s>>>(args.qry, g, cur2,
-                                                                                bad);
-        index_scan_kernel<<<p.n_tiles, 1024, 0, s>>>(g, cur2, tab2, bad);
-        index_scatter_kernel<true><<<grid_for(nQ * 32, threads), threads, 0, s>>>(args.qry, g, cur2,
-                                                                                  ent2, bad);
+        index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur2, sums, bad);
+        index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur2, tab2, sums, bad);
+        index_scatter_kernel<true><<<scatter_blocks, kScatterThreads, 0, s>>>(args.qry, g, cur2,
+                                                                              ent2, bad);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
@@ -2668,15 +2798,11 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     int dev = 0, sms = 0;
     CMS_CUDA_TRY(cudaGetDevice(&dev));
     CMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int threads = 256;
-    auto grid_for = [&](int64_t n) {
-        return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads,
-                                                           (int64_t)sms * 32));
-    };
-    validate_kernel<<<grid_for(n_ref), threads, 0, s>>>(args.ref, bad, err);
-    validate_kernel<<<grid_for(n_q), threads, 0, s>>>(args.qry, bad, err);
-    norms_kernel<<<grid_for(n_ref), threads, 0, s>>>(args.ref, snR, bad);
-    norms_kernel<<<grid_for(n_q), threads, 0, s>>>(args.qry, snQ, bad);
+    const IndexGeom none{1, 1, 1, 1.0};
+    prep_kernel<<<blocks_for(n_ref, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
+        PrepSide{args.ref, snR, nullptr, nullptr, nullptr}, none, bad, err, CMS_MAX_PEAKS);
+    prep_kernel<<<blocks_for(n_q, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
+        PrepSide{args.qry, snQ, nullptr, nullptr, nullptr}, none, bad, err, CMS_MAX_PEAKS);
     CMS_CUDA_TRY(cudaGetLastError());
 
     PairParams pp{};
@@ -2781,12 +2907,13 @@ extern "C" int cms_library_create(cms_ctx* ctx, const float* mz, const double* a
     nb = std::min(nb, 1 << 22);
     L->g = IndexGeom{tile, (int)((n + tile - 1) / tile), nb, 1.0 / w};
     const size_t n_tab = (size_t)L->g.n_tiles * (nb + 1), n_cur = (size_t)L->g.n_tiles * nb;
-    uint32_t* cur = nullptr;
+    const int n_chunks = L->g.n_tiles * scan_chunks(nb);
+    uint32_t* cur = nullptr;  // bucket counts, then the chunk sums
     cudaError_t e = cudaMalloc(&L->bad, 64);
     if (e == cudaSuccess) e = cudaMalloc(&L->sn, sizeof(double) * n);
     if (e == cudaSuccess) e = cudaMalloc(&L->tab, sizeof(uint32_t) * n_tab);
     if (e == cudaSuccess) e = cudaMalloc(&L->ent, sizeof(Entry) * std::max<int64_t>(1, n_peaks));
-    if (e == cudaSuccess) e = cudaMalloc(&cur, sizeof(uint32_t) * n_cur);
+    if (e == cudaSuccess) e = cudaMalloc(&cur, sizeof(uint32_t) * (n_cur + n_chunks));
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         cudaFree(cur);
@@ -2794,20 +2921,17 @@ extern "C" int cms_library_create(cms_ctx* ctx, const float* mz, const double* a
         set_error("cms_library_create: device allocation failed (%s)", cudaGetErrorString(e));
         return CMS_ERR_NOMEM;
     }
-    const int threads = 256;
-    auto grid_for = [&](int64_t cnt) {
-        return (int)std::max<int64_t>(1, std::min<int64_t>((cnt + threads - 1) / threads,
-                                                           (int64_t)ctx->sm_count * 32));
-    };
     e = cudaMemsetAsync(L->bad, 0, 64, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(cur, 0, sizeof(uint32_t) * n_cur, s);
     if (e == cudaSuccess) {
-        validate_kernel<<<grid_for(n), threads, 0, s>>>(L->spec, L->bad, ctx->err_word);
-        norms_kernel<<<grid_for(n), threads, 0, s>>>(L->spec, L->sn, L->bad);
-        index_count_kernel<false><<<grid_for(n * 32), threads, 0, s>>>(L->spec, L->g, cur, L->bad);
-        index_scan_kernel<<<L->g.n_tiles, 1024, 0, s>>>(L->g, cur, L->tab, L->bad);
-        index_scatter_kernel<false><<<grid_for(n * 32), threads, 0, s>>>(L->spec, L->g, cur, L->ent,
-                                                                  L->bad);
+        const int sms = ctx->sm_count;
+        prep_kernel<<<blocks_for(n, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
+            PrepSide{L->spec, L->sn, nullptr, cur, nullptr}, L->g, L->bad, ctx->err_word,
+            CMS_MAX_PEAKS);
+        index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, cur + n_cur, L->bad);
+        index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, L->tab, cur + n_cur, L->bad);
+        index_scatter_kernel<false><<<blocks_for(n, kScatterThreads / 32, sms), kScatterThreads, 0,
+                                      s>>>(L->spec, L->g, cur, L->ent, L->bad);
         e = cudaGetLastError();
     }
     uint32_t hbad = 0;
@@ -2894,29 +3018,23 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     unsigned int* spill_count = reinterpret_cast<unsigned int*>(small + 20);
     unsigned long long* work_join = reinterpret_cast<unsigned long long*>(small + 21);
     unsigned long long* work_pair = reinterpret_cast<unsigned long long*>(small + 22);
+    uint32_t* slots = bp.take<uint32_t>(kSlotWords);  // cleared with the counters before it
+    CMS_CUDA_TRY(cudaMemsetAsync(small, 0, bp.used, s));
     double* snQ = bp.take<double>(n_q);
     int32_t* order = bp.take<int32_t>(n_q);
     int2* spill = bp.take<int2>(spill_cap);
-    uint32_t* slots = bp.take<uint32_t>(kSlotWords);
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
-    CMS_CUDA_TRY(cudaMemsetAsync(small, 0, 64 * sizeof(uint64_t), s));
-    CMS_CUDA_TRY(cudaMemsetAsync(slots, 0, kSlotWords * sizeof(uint32_t), s));
 
-    const int threads = 256;
-    auto grid_for = [&](int64_t cnt) {
-        return (int)std::max<int64_t>(1, std::min<int64_t>((cnt + threads - 1) / threads,
-                                                           (int64_t)ctx->sm_count * 32));
-    };
     {
-        StageScope sc(ctx, 0, 2, s);
-        validate_kernel<<<grid_for(n_q), threads, 0, s>>>(Q, bad, ctx->err_word);
-        norms_kernel<<<grid_for(n_q), threads, 0, s>>>(Q, snQ, bad);
+        StageScope sc(ctx, 0, 1, s);
+        prep_kernel<<<blocks_for(n_q, kPrepPerBlock, ctx->sm_count), kPrepThreads, 0, s>>>(
+            PrepSide{Q, snQ, cls_count, nullptr, nullptr}, lib->g, bad, ctx->err_word,
+            CMS_MAX_PEAKS);
     }
     {
-        StageScope sc(ctx, 1, 2, s);
-        order_count_kernel<<<grid_for(n_q), threads, 0, s>>>(Q, cls_count, bad);
-        order_scatter_kernel<<<grid_for(n_q), threads, 0, s>>>(Q, cls_count, cls_cursor, order,
-                                                               bad);
+        StageScope sc(ctx, 1, 1, s);
+        order_scatter_kernel<<<blocks_for(n_q, kOrderThreads, ctx->sm_count), kOrderThreads, 0, s>>>(
+            Q, cls_count, cls_cursor, order, bad);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
