@@ -27,10 +27,10 @@
 //                        pointer advanced by the index instead of one step at
 //                        a time), test them with exact float32 window bounds
 //                        and push candidates into a per-warp pool (shared
-//                        memory, extended in global memory).  The pool is
-//                        counting-sorted by query; each query's run is then
-//                        resolved greedily: 1-3 candidates in closed form by
-//                        one lane, 4-8 by an 8-lane segment, 9-32 by the warp.
+//                        memory, extended in global memory).  Each query's
+//                        run is then resolved greedily: 1-4 candidates in
+//                        closed form by one lane, 5-8 by an 8-lane segment,
+//                        9-32 by the warp.
 //                        The sweep is load-balanced: a chunk's window entries
 //                        are expanded 32 at a time over the warp, and each
 //                        query's candidates are chained through a per-warp
@@ -79,7 +79,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // ---------------------------------------------------------------------------
 // tile index over the query side
 // ---------------------------------------------------------------------------
-// tile-stream entry: m/z, (query within tile << 16 | peak), intensity weight b
+// tile-stream entry: m/z (also in the neutral-loss index), (query within tile
+// << 16 | peak), intensity weight b
 struct __align__(16) Entry {
     float mz;
     uint32_t id;
@@ -101,16 +102,121 @@ __device__ __forceinline__ long long bucket_of(float x, double inv_w) {
     return __double2ll_rd(__dmul_rn((double)x, inv_w));
 }
 
-// The value an index sorts a peak by: its m/z, or for the neutral-loss index
-// of modified cosine (NL) its m/z minus its spectrum's precursor m/z, computed
-// in float64 and rounded to float32 (the join widens its windows by a margin
-// that covers this rounding and confirms each candidate exactly).
+// The value the neutral-loss index of modified cosine buckets a peak by: its
+// m/z minus its spectrum's precursor m/z, computed in float64 and rounded to
+// float32 (the windows are widened by a margin that covers this rounding, and
+// the join confirms each candidate exactly).
 __device__ __forceinline__ float loss_value(float mz, double prec) {
     return __double2float_rn(__dsub_rn((double)mz, prec));
 }
-template <bool NL>
-__device__ __forceinline__ float index_value(const SpecSet& B, int64_t s, int64_t k) {
-    return NL ? loss_value(B.mz[k], B.prec[s]) : B.mz[k];
+// Neutral-loss window of modified cosine's shifted pass: entries whose
+// m/z - precursor lies within tol of the sweeping peak's, widened by twice
+// the float32 spacing there (the indexed values are rounded to float32) and a
+// float64 rounding allowance, rounded outwards; every entry of its buckets is
+// then tested exactly against the shifted window.
+__device__ __forceinline__ bool nl_window(float mz, double prec, double tol, float& L, float& H) {
+    const double zr = __dsub_rn((double)mz, prec);
+    const float mag = __double2float_ru(fabs(zr) + tol + 1.0);
+    const double m = 2.0 * (double)(nextafterf(mag, INFINITY) - mag) +
+                     1e-9 * (fabs((double)mz) + fabs(prec) + 1.0);
+    L = __double2float_rd(__dsub_rn(__dsub_rn(zr, tol), m));
+    H = __double2float_ru(__dadd_rn(__dadd_rn(zr, tol), m));
+    return isfinite(L) && isfinite(H);
+}
+
+// Exact float32 window of one sweeping peak.
+//
+// The float64 test of the reference (query peak y matches reference peak x iff
+// !(y+shift > x+tol) && !(y+shift < x-tol)) is, for a fixed sweeping peak, a
+// conjunction of a predicate non-decreasing in the indexed peak's m/z and one
+// non-increasing in it.  So the float32 values it accepts form one interval
+// [L, H] of float32 numbers.  It is found once per sweeping peak by rounding
+// an estimate and stepping with nextafterf until the float64 predicates flip;
+// each entry is then tested with two float32 compares, with exactly the same
+// outcome as the float64 test.  The estimate is within an ulp or two; the
+// step loops are capped, and a peak that does not converge (non-finite input)
+// gets an empty window and an error flag.
+template <bool A_IS_REF, bool NOSHIFT>
+struct Window {
+    // A_IS_REF: x = sweeping reference peak; lo/hi = x -+ tol
+    // else:     c = sweeping query peak + shift
+    __device__ __forceinline__ static bool not_below(float y, double lo, double c, double tol,
+                                                     double shift) {
+        if (A_IS_REF) return !(__dadd_rn((double)y, shift) < lo);
+        return !(c > __dadd_rn((double)y, tol));
+    }
+    __device__ __forceinline__ static bool not_above(float y, double hi, double c, double tol,
+                                                     double shift) {
+        if (A_IS_REF) return !(__dadd_rn((double)y, shift) > hi);
+        return !(c < __dsub_rn((double)y, tol));
+    }
+    __device__ static bool bounds(float mzA, double tol, double shift, float& L, float& H) {
+        const double x = (double)mzA;
+        if (A_IS_REF && NOSHIFT) {
+            // y (float32, exact in float64) is accepted iff lo <= y <= hi: the
+            // interval ends are lo rounded up and hi rounded down to float32
+            L = __double2float_ru(__dsub_rn(x, tol));
+            H = __double2float_rd(__dadd_rn(x, tol));
+            return isfinite(L) && isfinite(H);
+        }
+        double lo = 0.0, hi = 0.0, c = 0.0, el, eh;
+        if (A_IS_REF) {
+            lo = __dsub_rn(x, tol);
+            hi = __dadd_rn(x, tol);
+            el = __dsub_rn(lo, shift);
+            eh = __dsub_rn(hi, shift);
+        } else {
+            c = __dadd_rn(x, shift);
+            el = __dsub_rn(c, tol);
+            eh = __dadd_rn(c, tol);
+        }
+        float l = __double2float_rd(el), h = __double2float_ru(eh);
+        int k = 0;
+        for (; k < 16 && !not_below(l, lo, c, tol, shift); ++k) l = nextafterf(l, INFINITY);
+        for (; k < 32 && not_below(nextafterf(l, -INFINITY), lo, c, tol, shift); ++k)
+            l = nextafterf(l, -INFINITY);
+        for (; k < 48 && !not_above(h, hi, c, tol, shift); ++k) h = nextafterf(h, -INFINITY);
+        for (; k < 64 && not_above(nextafterf(h, INFINITY), hi, c, tol, shift); ++k)
+            h = nextafterf(h, INFINITY);
+        const bool ok = k < 64 && isfinite(l) && isfinite(h) && not_below(l, lo, c, tol, shift) &&
+                        not_above(h, hi, c, tol, shift);
+        L = l;
+        H = h;
+        return ok;
+    }
+};
+
+// What the join needs to know of a sweeping peak, computed once per call: its
+// window [lo, hi] in the indexed side's float32 m/z and the window's first and
+// last bucket (first > last: the range wraps around the hashed table;
+// kNoBucket: no entry can match).
+struct __align__(16) Probe {
+    float lo, hi;
+    uint32_t bl, bh;
+};
+constexpr uint32_t kNoBucket = 0xffffffffu;
+
+__device__ __forceinline__ uint2 bucket_range(float L, float H, const IndexGeom& g) {
+    if (!(L <= H)) return make_uint2(kNoBucket, 0u);
+    const long long blo = bucket_of(L, g.inv_w), bhi = bucket_of(H, g.inv_w);
+    if (bhi - blo + 1 >= g.nb) return make_uint2(0u, (unsigned)g.nb - 1u);
+    const unsigned mask = (unsigned)(g.nb - 1);
+    return make_uint2((unsigned)blo & mask, (unsigned)bhi & mask);
+}
+
+// A sweeping spectrum in the order the join takes them.
+struct __align__(16) SweepItem {
+    int64_t a0;   // its first peak
+    double sn;    // its norm
+    double rn;    // 1 / norm (recip_norm)
+    int32_t a;    // its index
+    int32_t na;   // its peaks
+};
+
+// 1 / norm for the join's division-free score, NaN (which sends the score to
+// the division) for norms whose products with it could leave the normal range
+__device__ __forceinline__ double recip_norm(double sn) {
+    return sn >= 1e-100 && sn <= 1e100 ? __drcp_rn(sn) : __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // ---------------------------------------------------------------------------
@@ -124,10 +230,42 @@ __device__ __forceinline__ int length_class(int64_t len) {
 struct PrepSide {
     SpecSet S;
     double* sn;           // sqrt(sum_k (a_k * b_k)^2), summed in peak order
+    double* rn;           // recip_norm(sn) (null: not wanted)
     uint32_t* cls_count;  // spectra per length class (null: not wanted)
     uint32_t* cnt;        // peaks per (tile, bucket) of the m/z index (null: not wanted)
     uint32_t* cnt2;       // the same of the neutral-loss index (null: not wanted)
+    Probe* probe;         // per peak, for the sweeping side (null: not wanted)
+    uint2* probe2;        // per peak, its shifted window's buckets (null: not wanted)
+    double tol, shift;    // of the windows
+    int is_ref;           // the sweeping side is the reference side
 };
+
+// The windows and buckets of one sweeping peak.
+__device__ void make_probe(const PrepSide& P, const IndexGeom& g, int64_t s, int64_t k,
+                           uint32_t* err) {
+    const float mz = P.S.mz[k];
+    Probe p{1.0f, 0.0f, kNoBucket, 0u};
+    float L, H;
+    const bool ok = !P.is_ref        ? Window<false, false>::bounds(mz, P.tol, P.shift, L, H)
+                    : P.shift == 0.0 ? Window<true, true>::bounds(mz, P.tol, P.shift, L, H)
+                                     : Window<true, false>::bounds(mz, P.tol, P.shift, L, H);
+    if (ok) {
+        const uint2 b = bucket_range(L, H, g);
+        p = Probe{L, H, b.x, b.y};
+    } else {
+        atomicOr(err, kErrBadOffsets);
+    }
+    *reinterpret_cast<uint4*>(&P.probe[k]) =
+        make_uint4(__float_as_uint(p.lo), __float_as_uint(p.hi), p.bl, p.bh);
+    if (P.probe2) {
+        uint2 b = make_uint2(kNoBucket, 0u);
+        if (nl_window(mz, P.S.prec[s], P.tol, L, H))
+            b = bucket_range(L, H, g);
+        else
+            atomicOr(err, kErrBadOffsets);
+        P.probe2[k] = b;
+    }
+}
 
 // cnt / cnt2 have geometry g.  Offsets out of order or range and spectra above
 // max_peaks raise the error word and *bad, which stops every later kernel of
@@ -219,7 +357,18 @@ prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks
                 for (int k = 0; k < 32; ++k) acc = __dadd_rn(acc, tile[lane][k]);
             }
         }
-        if (lane < kPrepSpectra && s0 + lane < n) P.sn[s0 + lane] = sqrt(acc);
+        if (lane < kPrepSpectra && s0 + lane < n) {
+            const double sn = sqrt(acc);
+            P.sn[s0 + lane] = sn;
+            if (P.rn) P.rn[s0 + lane] = recip_norm(sn);
+        }
+        if (P.probe)
+#pragma unroll 1
+            for (int j = 0; j < kPrepSpectra; ++j) {
+                const int64_t lj = __shfl_sync(full, lo, j);
+                const int nj = __shfl_sync(full, len, j);
+                for (int i = lane; i < nj; i += 32) make_probe(P, g, s0 + j, lj + i, err);
+            }
         __syncwarp();
     }
     __syncthreads();
@@ -326,7 +475,7 @@ index_scan_kernel(IndexGeom g, uint32_t* cnt_cur, uint32_t* tab, const uint32_t*
 // (4.7 M peaks: 110 us; one chunk at a time 135 us).
 template <bool NL>
 __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entry* ent,
-                                     const uint32_t* bad) {
+                                     double* ent_a, const uint32_t* bad) {
     if (*bad) return;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -340,15 +489,17 @@ __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entr
         const int64_t lo = B.off[s], hi = B.off[s + 1];
         uint32_t* c = cur + t * (int64_t)g.nb;
         for (int64_t k0 = lo + lane; k0 < hi; k0 += 32 * kU) {
-            float v[kU];
-            double b[kU];
+            float v[kU], mz[kU];
+            double b[kU], a[kU];
             uint32_t pos[kU];
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const int64_t k = k0 + 32 * u;
                 if (k < hi) {
-                    v[u] = index_value<NL>(B, s, k);
+                    mz[u] = B.mz[k];
+                    v[u] = NL ? loss_value(mz[u], B.prec[s]) : mz[u];
                     b[u] = B.b[k];
+                    if (ent_a) a[u] = B.a[k];
                 }
             }
 #pragma unroll
@@ -360,10 +511,11 @@ __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entr
                 const int64_t k = k0 + 32 * u;
                 if (k < hi) {
                     Entry en;
-                    en.mz = v[u];
+                    en.mz = mz[u];
                     en.id = (ql << 16) | (uint32_t)(k - lo);
                     en.b = b[u];
                     ent[base + pos[u]] = en;
+                    if (ent_a) ent_a[base + pos[u]] = a[u];
                 }
             }
         }
@@ -375,8 +527,8 @@ __global__ void index_scatter_kernel(SpecSet B, IndexGeom g, uint32_t* cur, Entr
 // block and class.
 constexpr int kOrderThreads = 256;
 __global__ void __launch_bounds__(kOrderThreads)
-order_scatter_kernel(SpecSet S, const uint32_t* cls_count, uint32_t* cls_cursor, int32_t* order,
-                     const uint32_t* bad) {
+order_scatter_kernel(SpecSet S, const double* sn, const uint32_t* cls_count, uint32_t* cls_cursor,
+                     SweepItem* items, const uint32_t* bad) {
     if (*bad) return;
     __shared__ uint32_t s_cnt[kOrderClasses], s_base[kOrderClasses];
     const int tid = threadIdx.x;
@@ -387,8 +539,14 @@ order_scatter_kernel(SpecSet S, const uint32_t* cls_count, uint32_t* cls_cursor,
         const int64_t s = s0 + tid;
         int c = 0;
         uint32_t rank = 0;
+        SweepItem it{};
         if (s < S.n) {
-            c = length_class(S.off[s + 1] - S.off[s]);
+            it.a0 = S.off[s];
+            it.na = (int32_t)(S.off[s + 1] - it.a0);
+            it.a = (int32_t)s;
+            it.sn = sn[s];
+            it.rn = recip_norm(it.sn);
+            c = length_class(it.na);
             rank = atomicAdd(&s_cnt[c], 1u);
         }
         __syncthreads();
@@ -398,7 +556,7 @@ order_scatter_kernel(SpecSet S, const uint32_t* cls_count, uint32_t* cls_cursor,
             s_base[tid] = base + atomicAdd(&cls_cursor[tid], s_cnt[tid]);
         }
         __syncthreads();
-        if (s < S.n) order[s_base[c] + rank] = (int32_t)s;
+        if (s < S.n) items[s_base[c] + rank] = it;
         __syncthreads();
     }
 }
@@ -468,16 +626,19 @@ __device__ __forceinline__ void spill_push(const SpillList& sl, int r, int q, ui
 struct JoinParams {
     SpecSet A;  // sweeping side (one spectrum per work item)
     SpecSet B;  // indexed side (tiles)
-    const double* snA;
+    const SweepItem* items;  // sweeping spectra, largest length class first
+    const Probe* probe;      // per sweeping peak: window and buckets
+    const uint2* probe2;     // modified cosine: buckets of the shifted window
     const double* snB;
-    const int32_t* a_order;
+    const double* rnB;
     const uint32_t* tab;
     const Entry* ent;
+    const double* ent_a;   // m/z weight a of each tile-stream entry (null: 1.0)
     const uint32_t* tab2;  // modified cosine: neutral-loss index (m/z - precursor)
     const Entry* ent2;
+    const double* ent2_a;
     IndexGeom g;
     double tol;
-    double shift;
     int match_limit;
     float init_width_scale;  // first sub-range width = scale / n_A_peaks (0: whole tile)
     // first sub-range width per length class of the sweeping spectrum (the
@@ -485,7 +646,7 @@ struct JoinParams {
     int width_by_class[kOrderClasses];
     int warp_smem_bytes;     // per-warp slice of dynamic shared memory
     int pool_max;            // candidates a sweep may hold: kPoolMax, or kPool without gpool
-    int max_fetch;           // fetches of kFetch items per warp before it exits (0: no limit)
+    int max_fetch;           // work items per warp before it exits (0: no limit)
     unsigned char* gpool;    // global pool extension, kGPool * 16 bytes per warp (or null)
     // bounded launches: a CTA claims one of n_slots global-pool slices (a bit
     // of `slots`) for its lifetime instead of using slice blockIdx.x (null:
@@ -496,17 +657,13 @@ struct JoinParams {
     unsigned long long* work;
     SpillList spill;
     DenseOut dense;
+    int vec_rows;            // dense arrays 16 / 16 / 4-byte aligned: vector zeros
     SparseOut sparse;
     uint32_t* err;
     const uint32_t* bad;
     int sym;  // only pairs (reference i, query j) with i <= j
 };
 
-constexpr int kFetch = 2;                  // work items taken per atomic (2: 0.8% faster than 4)
-// rounds of 32 tile-stream entries a warp loads before testing the first (1
-// measured fastest at 100k x 100k: 42.8 ms against 43.3 for 2 and 46.6 for 3,
-// each extra round costing registers and spills)
-constexpr int kRounds = 1;
 constexpr int kSearchWaves = 4;            // waves of short-lived CTAs per library search
 constexpr int kSlotWords = 64;             // slot bitmap words of a bounded join launch
 constexpr int kPoolMax = 4096;             // candidates per sweep: smem pool + global extension
@@ -514,10 +671,16 @@ constexpr int kGPool = kPoolMax - kPool;   // global extension entries per warp
 static_assert(kPoolMax <= 4096, "pool slots are packed into 12 bits");
 static_assert(kMaxTile <= 4096, "query indices within a range are packed into 12 bits");
 
-// Candidate metadata word: the query's index within the swept range (bits
-// 0-11) and the slot of the previous candidate of the same query (bits 12-23,
-// present when kHasNext is set).  A query's candidates form a chain that
-// starts at the slot its head names (the candidate pushed last).
+// One candidate: key, generation word and a metadata word, which holds the
+// query's index within the swept range (bits 0-11) and the slot of the
+// previous candidate of the same query (bits 12-23, present when kHasNext is
+// set).  A query's candidates form a chain that starts at the slot its head
+// names (the candidate pushed last).
+struct __align__(16) PoolEntry {
+    double key;
+    uint32_t gen;
+    uint32_t meta;
+};
 constexpr uint32_t kHasNext = 1u << 24;
 __device__ __forceinline__ int meta_query(uint32_t m) { return (int)(m & 0xFFFu); }
 __device__ __forceinline__ int meta_next(uint32_t m) { return (int)((m >> 12) & 0xFFFu); }
@@ -525,51 +688,42 @@ __device__ __forceinline__ int meta_next(uint32_t m) { return (int)((m >> 12) & 
 // A warp's candidate pool: the first kPool entries live in shared memory, the
 // rest in a per-warp slice of global scratch (L2-resident), so that a large
 // reference spectrum is swept once even when it has thousands of candidates
-// in a tile.  Slots are indices into the concatenation.
+// in a tile.  Slots are indices into the concatenation; an access is one
+// 16-byte generic load or store (gbase points kPool entries before the slice).
 struct Pool {
-    double* skey;
-    uint32_t* sgen;
-    uint32_t* smeta;
-    double* gkey;
-    uint32_t* ggen;
-    uint32_t* gmeta;
-    __device__ __forceinline__ double key(int i) const { return i < kPool ? skey[i] : gkey[i - kPool]; }
-    __device__ __forceinline__ uint32_t gen(int i) const { return i < kPool ? sgen[i] : ggen[i - kPool]; }
-    __device__ __forceinline__ uint32_t meta(int i) const {
-        return i < kPool ? smeta[i] : gmeta[i - kPool];
+    PoolEntry* sbase;
+    PoolEntry* gbase;
+    __device__ __forceinline__ PoolEntry* at(int i) const { return (i < kPool ? sbase : gbase) + i; }
+    __device__ __forceinline__ PoolEntry get(int i) const {
+        const uint4 v = *reinterpret_cast<const uint4*>(at(i));
+        return PoolEntry{__hiloint2double((int)v.y, (int)v.x), v.z, v.w};
     }
+    __device__ __forceinline__ uint32_t meta(int i) const { return at(i)->meta; }
     __device__ __forceinline__ void put(int i, double k, uint32_t g, uint32_t m) const {
-        if (i < kPool) {
-            skey[i] = k;
-            sgen[i] = g;
-            smeta[i] = m;
-        } else {
-            gkey[i - kPool] = k;
-            ggen[i - kPool] = g;
-            gmeta[i - kPool] = m;
-        }
+        *reinterpret_cast<uint4*>(at(i)) =
+            make_uint4((unsigned)__double2loint(k), (unsigned)__double2hiint(k), g, m);
     }
 };
 
 // Per-warp shared-memory slice (offsets in bytes; the head table's length
 // depends on the tile size, so the slice size is computed at launch).
-//   key   double [kPool]     candidate key
-//   gen   uint32 [kPool]     (p_ref << 16) | p_query
-//   meta  uint32 [kPool]     query in range | previous candidate of the query
-//   head  uint32 [tile/2]    two 16-bit heads per word, one per query of the
-//                            range: (epoch << 12) | slot of its last candidate;
-//                            a head of another epoch means "no candidate yet"
+//   pool  PoolEntry [kPool]
+//   head  uint16 [tile]      one per query of the range: (epoch << 12) | slot of
+//                            its last candidate; a head of another epoch means
+//                            "no candidate yet"
+//   rec   uint4 [32]         sweep: the chunk's peaks with window entries, in order:
+//                            stream offset, window, lane.  Resolution: uint16 queue
+//                            of chain heads with two or more candidates
 //   wa    double [32]        per-lane sweeping-peak weight of the current chunk
-//   lh    float2 [32]        per-lane float32 window [L, H] of the current chunk
-//   runs  uint32 [kLongRuns] runs of 4..32 candidates queued for the warp:
+//   runs  uint32 [kLongRuns] runs of 5..32 candidates queued for the warp:
 //                            slot of the chain head | length << 12; runs of at
 //                            most kMidRun from the front, longer ones from the back
-//   x     float  [32]        per-lane sweeping-peak m/z (modified cosine's exact test)
 //   t0    uint64             %globaltimer at the current item's start (trace only)
 constexpr int kLongRuns = 64;
-__host__ __device__ constexpr int head_words(int tile) { return (((tile + 1) / 2) + 3) & ~3; }
+constexpr int kQueue = 256;
+__host__ __device__ constexpr int head_bytes(int tile) { return (2 * tile + 15) & ~15; }
 __host__ __device__ constexpr int warp_slice_bytes(int tile) {
-    return 16 * kPool + 4 * head_words(tile) + 8 * 32 + 8 * 32 + 4 * kLongRuns + 4 * 32 + 16;
+    return 16 * kPool + head_bytes(tile) + 16 * 32 + 8 * 32 + 4 * kLongRuns + 16;
 }
 
 // Reference peak of a candidate's generation word.  Modified cosine marks
@@ -581,98 +735,44 @@ __device__ __forceinline__ uint32_t gen_p1(uint32_t g) {
     return MODIFIED ? ((g >> 16) & 0x7FFFu) : (g >> 16);
 }
 
-// Neutral-loss window of modified cosine's shifted pass: entries whose
-// m/z - precursor lies within tol of the sweeping peak's, widened by twice
-// the float32 spacing there (the stored values are rounded to float32) and a
-// float64 rounding allowance, rounded outwards; every entry inside is then
-// confirmed with the exact test of the shifted window.
-__device__ __forceinline__ bool nl_window(float mz, double prec, double tol, float& L, float& H) {
-    const double zr = __dsub_rn((double)mz, prec);
-    const float mag = __double2float_ru(fabs(zr) + tol + 1.0);
-    const double m = 2.0 * (double)(nextafterf(mag, INFINITY) - mag) +
-                     1e-9 * (fabs((double)mz) + fabs(prec) + 1.0);
-    L = __double2float_rd(__dsub_rn(__dsub_rn(zr, tol), m));
-    H = __double2float_ru(__dadd_rn(__dadd_rn(zr, tol), m));
-    return isfinite(L) && isfinite(H);
+// float32 of score / (nr * nq) with both operations rounded in float64, as the
+// reference order has it, mostly without the division: rr and rq are the
+// norms' reciprocals (NaN when a norm is out of [1e-100, 1e100]), so
+// (score * rr) * rq is within 3 * 2^-52 of the quotient, and when the float32
+// values of both ends of a band of 2^-49 around it agree, the quotient rounds
+// to that value too.  Otherwise (about one in 10^7, zero norms and scores
+// below 1e-30) the quotient itself.
+__device__ __forceinline__ float cosine_of(double score, double rr, double rq, double nr,
+                                           const double* nq) {
+    const double x = __dmul_rn(__dmul_rn(score, rr), rq);
+    const float lo = (float)__dmul_rn(x, 1.0 - 0x1p-49), hi = (float)__dmul_rn(x, 1.0 + 0x1p-49);
+    if (lo == hi && lo > 1e-30f) return lo;
+    return (float)__ddiv_rn(score, __dmul_rn(nr, *nq));
 }
 
-// Exact float32 window of one sweeping peak.
-//
-// The float64 test of the reference (query peak y matches reference peak x iff
-// !(y+shift > x+tol) && !(y+shift < x-tol)) is, for a fixed sweeping peak, a
-// conjunction of a predicate non-decreasing in the indexed peak's m/z and one
-// non-increasing in it.  So the float32 values it accepts form one interval
-// [L, H] of float32 numbers.  It is found once per sweeping peak by rounding
-// an estimate and stepping with nextafterf until the float64 predicates flip;
-// each entry is then tested with two float32 compares, with exactly the same
-// outcome as the float64 test.  The estimate is within an ulp or two; the
-// step loops are capped, and a peak that does not converge (non-finite input)
-// gets an empty window and an error flag.
-template <bool A_IS_REF, bool NOSHIFT>
-struct Window {
-    // A_IS_REF: x = sweeping reference peak; lo/hi = x -+ tol
-    // else:     c = sweeping query peak + shift
-    __device__ __forceinline__ static bool not_below(float y, double lo, double c, double tol,
-                                                     double shift) {
-        if (A_IS_REF) return !(__dadd_rn((double)y, shift) < lo);
-        return !(c > __dadd_rn((double)y, tol));
-    }
-    __device__ __forceinline__ static bool not_above(float y, double hi, double c, double tol,
-                                                     double shift) {
-        if (A_IS_REF) return !(__dadd_rn((double)y, shift) > hi);
-        return !(c < __dsub_rn((double)y, tol));
-    }
-    __device__ static bool bounds(float mzA, double tol, double shift, float& L, float& H) {
-        const double x = (double)mzA;
-        if (A_IS_REF && NOSHIFT) {
-            // y (float32, exact in float64) is accepted iff lo <= y <= hi: the
-            // interval ends are lo rounded up and hi rounded down to float32
-            L = __double2float_ru(__dsub_rn(x, tol));
-            H = __double2float_rd(__dadd_rn(x, tol));
-            return isfinite(L) && isfinite(H);
-        }
-        double lo = 0.0, hi = 0.0, c = 0.0, el, eh;
-        if (A_IS_REF) {
-            lo = __dsub_rn(x, tol);
-            hi = __dadd_rn(x, tol);
-            el = __dsub_rn(lo, shift);
-            eh = __dsub_rn(hi, shift);
-        } else {
-            c = __dadd_rn(x, shift);
-            el = __dsub_rn(c, tol);
-            eh = __dadd_rn(c, tol);
-        }
-        float l = __double2float_rd(el), h = __double2float_ru(eh);
-        int k = 0;
-        for (; k < 16 && !not_below(l, lo, c, tol, shift); ++k) l = nextafterf(l, INFINITY);
-        for (; k < 32 && not_below(nextafterf(l, -INFINITY), lo, c, tol, shift); ++k)
-            l = nextafterf(l, -INFINITY);
-        for (; k < 48 && !not_above(h, hi, c, tol, shift); ++k) h = nextafterf(h, -INFINITY);
-        for (; k < 64 && not_above(nextafterf(h, INFINITY), hi, c, tol, shift); ++k)
-            h = nextafterf(h, INFINITY);
-        const bool ok = k < 64 && isfinite(l) && isfinite(h) && not_below(l, lo, c, tol, shift) &&
-                        not_above(h, hi, c, tol, shift);
-        L = l;
-        H = h;
-        return ok;
-    }
-};
-
-// Three CTAs (24 warps) per SM: up to 85 registers a thread.
-template <bool A_IS_REF, bool SPARSE, bool NOSHIFT, bool MODIFIED>
+// Bound by instruction issue and latency together (about 13 cycles between a
+// warp's instructions at six warps a scheduler), not by memory: 50000 x 50000
+// lognormal spectra, dense, move 11.4 B a pair at a quarter of the copy rate.
+// So what counts is the length of an item's instruction chain: windows and
+// buckets come ready-made per sweeping peak, item descriptors in order, a
+// pool entry is one 16-byte access, and owners of one candidate do not wait
+// for the code of longer runs (50000 x 50000: 11.45 ms with all of that done
+// per item, 9.9 ms now).
+// Three CTAs (24 warps) per SM: up to 80 registers a thread.
+template <bool A_IS_REF, bool SPARSE, bool MODIFIED>
 __global__ void __launch_bounds__(kJoinThreads, 3)
 join_kernel(JoinParams P) {
     if (*P.bad) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int hw = head_words(P.g.tile);
+    const int hb = head_bytes(P.g.tile);
     unsigned char* slice = smem_raw + (size_t)(threadIdx.x >> 5) * P.warp_smem_bytes;
     uint32_t* head = reinterpret_cast<uint32_t*>(slice + 16 * kPool);
-    double* s_wa = reinterpret_cast<double*>(slice + 16 * kPool + 4 * hw);
-    float2* s_lh = reinterpret_cast<float2*>(slice + 16 * kPool + 4 * hw + 8 * 32);
-    uint32_t* long_runs = reinterpret_cast<uint32_t*>(slice + 16 * kPool + 4 * hw + 16 * 32);
-    float* s_x = reinterpret_cast<float*>(slice + 16 * kPool + 4 * hw + 16 * 32 + 4 * kLongRuns);
-    unsigned long long* s_t0 = reinterpret_cast<unsigned long long*>(
-        slice + 16 * kPool + 4 * hw + 16 * 32 + 4 * kLongRuns + 4 * 32);
+    uint4* s_rec = reinterpret_cast<uint4*>(slice + 16 * kPool + hb);
+    uint16_t* queue = reinterpret_cast<uint16_t*>(s_rec);
+    double* s_wa = reinterpret_cast<double*>(slice + 16 * kPool + hb + 16 * 32);
+    uint32_t* long_runs = reinterpret_cast<uint32_t*>(slice + 16 * kPool + hb + 24 * 32);
+    unsigned long long* s_t0 = reinterpret_cast<unsigned long long*>(slice + 16 * kPool + hb +
+                                                                     24 * 32 + 4 * kLongRuns);
     // Global-pool slice of this CTA: blockIdx.x, or under bounded launches a
     // slice claimed from the slot bitmap (at most n_slots CTAs are resident at
     // once, so one is free; if a release has not landed yet the CTA runs with
@@ -707,71 +807,74 @@ join_kernel(JoinParams P) {
     }
     const int pool_max = (P.gpool && pslot >= 0) ? P.pool_max : kPool;
     Pool pool;
-    {
-        const size_t gw = (size_t)(pslot >= 0 ? pslot : 0) * kJoinWarps + (threadIdx.x >> 5);
-        unsigned char* g = (P.gpool && pslot >= 0) ? P.gpool + gw * (size_t)kGPool * 16 : nullptr;
-        pool.skey = reinterpret_cast<double*>(slice);
-        pool.sgen = reinterpret_cast<uint32_t*>(slice + 8 * kPool);
-        pool.smeta = reinterpret_cast<uint32_t*>(slice + 12 * kPool);
-        pool.gkey = reinterpret_cast<double*>(g);
-        pool.ggen = reinterpret_cast<uint32_t*>(g ? g + 8 * kGPool : nullptr);
-        pool.gmeta = reinterpret_cast<uint32_t*>(g ? g + 12 * kGPool : nullptr);
-    }
+    pool.sbase = reinterpret_cast<PoolEntry*>(slice);
+    pool.gbase = pool.sbase;
+    if (P.gpool && pslot >= 0)
+        pool.gbase = reinterpret_cast<PoolEntry*>(P.gpool) +
+                     ((size_t)pslot * kJoinWarps + (threadIdx.x >> 5)) * (size_t)kGPool - kPool;
 
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     const unsigned below = (1u << lane) - 1u;
+    const unsigned upto = below | (1u << lane);
     const int64_t nA = P.A.n;
     const int64_t n_items = nA * (int64_t)P.g.n_tiles;
-    const unsigned nbmask = (unsigned)(P.g.nb - 1);
-    const Entry* __restrict__ ent = P.ent;
-    const uint32_t* __restrict__ tab = P.tab;
     // epoch of the head table (1..15): every swept range takes the next one,
     // so heads left by earlier ranges read as empty without clearing the
     // table; it is cleared once per 15 ranges (and before the first)
     unsigned epoch = 15;
 
+    // the next item's index is fetched while the current one is processed
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(P.work, 1ull);
     for (int fetches = 0; P.max_fetch == 0 || fetches < P.max_fetch; ++fetches) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(P.work, (unsigned long long)kFetch);
-        base = __shfl_sync(full, base, 0);
-        if ((int64_t)base >= n_items) break;
-        // item = t * nA + ai: one division per fetch, then step ai
-        int64_t tt = (int64_t)base / nA, ai = (int64_t)base - tt * nA;
-        for (int f = 0; f < kFetch && (int64_t)(base + f) < n_items; ++f, ++ai) {
-        while (ai >= nA) {
-            ai -= nA;
-            ++tt;
+        const unsigned long long item = __shfl_sync(full, next, 0);
+        if ((int64_t)item >= n_items) break;
+        if (lane == 0 && (P.max_fetch == 0 || fetches + 1 < P.max_fetch))
+            next = atomicAdd(P.work, 1ull);
+        int t;
+        SweepItem A;
+        {
+            int64_t ai;
+            if (n_items <= 0xffffffffll) {
+                t = (int)((unsigned)item / (unsigned)nA);
+                ai = (unsigned)item - (unsigned)t * (unsigned)nA;
+            } else {
+                t = (int)((int64_t)item / nA);
+                ai = (int64_t)item - (int64_t)t * nA;
+            }
+            A = P.items[ai];
         }
         if (P.trace.rec && lane == 0) *s_t0 = global_ns();
-        const int t = (int)tt;
-        const int a = P.a_order[ai];
-        const int64_t a0 = P.A.off[a];
-        const int na = (int)(P.A.off[a + 1] - a0);
+        const int a = A.a, na = A.na;
         const int b_begin = t * P.g.tile;
         const int tn = (int)min((int64_t)P.g.tile, P.B.n - b_begin);
         const int64_t tbase = P.B.off[b_begin];
-        const uint32_t* T = tab + (int64_t)t * (P.g.nb + 1);
+        const uint32_t* T = P.tab + (int64_t)t * (P.g.nb + 1);
         const uint32_t* T2 = MODIFIED ? P.tab2 + (int64_t)t * (P.g.nb + 1) : nullptr;
-        const double snA = P.snA[a];
-        // a resolved run's result, stored straight into the dense output
-        auto put_dense = [&](int bq, float sc, int mt) {
-            const int64_t o = (int64_t)(A_IS_REF ? a : bq) * P.dense.ld + (A_IS_REF ? bq : a);
-            __stcs(&P.dense.score[o], sc);
-            __stcs(&P.dense.matches[o], mt);
-        };
-        auto store_result_n = [&](int bq, double score, int mt, double snB) {
-            const float sc =
-                (float)__ddiv_rn(score, A_IS_REF ? __dmul_rn(snA, snB) : __dmul_rn(snB, snA));
+        // dense position of (this spectrum, query b_begin); the join's dense
+        // output always has the sweeping spectrum as its row
+        const int64_t row = SPARSE ? 0 : (int64_t)a * P.dense.ld + b_begin;
+        // a resolved run's score and count, for query q of the tile
+        auto store_result = [&](int q, double score, int mt, double rnB) {
+            const double* nb = P.snB + b_begin + q;
+            const float sc = cosine_of(score, A.rn, rnB, A.sn, nb);
             if (SPARSE) {
                 if (sc >= P.sparse.threshold)
-                    emit_hit(P.sparse, A_IS_REF ? a : bq, A_IS_REF ? bq : a, sc, mt, 0);
+                    emit_hit(P.sparse, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a, sc,
+                             mt, 0);
             } else {
-                put_dense(bq, sc, mt);
+                __stcs(P.dense.score + row + q, sc);
+                __stcs(P.dense.matches + row + q, mt);
             }
         };
-        auto store_result = [&](int bq, double score, int mt) {
-            store_result_n(bq, score, mt, P.snB[bq]);
+        // a run for the pair kernel (its dense cells marked until then)
+        auto spill_run = [&](int q) {
+            spill_push(P.spill, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a, P.err);
+            if (!SPARSE) {
+                __stcs(P.dense.score + row + q, __int_as_float(0x7fc00000));
+                __stcs(P.dense.matches + row + q, -1);
+            }
         };
 
         int width = tn;
@@ -794,171 +897,149 @@ join_kernel(JoinParams P) {
             const int rw = range_hi - range_lo;
             epoch = epoch == 15 ? 1u : epoch + 1u;
             if (epoch == 1u)
-                for (int w = 4 * lane; w < hw; w += 128)
-                    *reinterpret_cast<uint4*>(head + w) = make_uint4(0u, 0u, 0u, 0u);
+                for (int w = lane; w < hb / 16; w += 32)
+                    reinterpret_cast<uint4*>(head)[w] = make_uint4(0u, 0u, 0u, 0u);
             __syncwarp();
             // ---- sweep: candidates of (a, queries [range_lo, range_hi)) ----
             // Each lane takes one sweeping peak of a 32-peak chunk and finds
             // the tile-stream entries of its window's buckets (one run, or two
-            // when the hashed bucket range wraps).  The chunk's entries are
-            // then processed 32 at a time, flat entry k by lane k % 32, which
-            // finds the peak that owns it by a binary search over the warp's
-            // inclusive entry counts: every lane tests an entry in every
-            // round, however unevenly the entries fall among the peaks.
+            // when the hashed bucket range wraps: then the chunk takes a second
+            // turn for the wrapped parts).  The chunk's entries are processed
+            // 32 at a time, flat entry k by lane k % 32, so that every lane
+            // tests an entry in every round, however unevenly the entries fall
+            // among the peaks.  The peaks that have entries leave a record each,
+            // in order; a round's first entries of peaks are or-ed into a mask
+            // over its 32 positions, so the owner of an entry is the count of
+            // mask bits up to its position (one reduction, one population count
+            // and one shared-memory read; a binary search by shuffles over the
+            // entry counts took five dependent shuffles).
             // Latency is hidden by running ahead: a step's bucket-table loads
             // are issued one step early (steps are chunks, or chunk x pass
-            // for modified cosine), the peaks a probe needs one chunk early,
-            // and the entries of kRounds rounds are loaded before the first is
-            // tested.
+            // for modified cosine), the probes they need one chunk early.
             int n = 0;  // candidates found (warp-uniform)
             constexpr int kPasses = MODIFIED ? 2 : 1;
             const int n_steps = ((na + 31) >> 5) * kPasses;
-            float mz_c = 0.f, mz_n = 0.f;  // chunks c, c+1
+            const Probe none{1.0f, 0.0f, kNoBucket, 0u};
+            Probe pr = none, pn = none;  // probes of this step's and the next chunk
             double w_c = 0.0, w_n = 0.0;
-            auto load_peak = [&](int pp, float& mz, double& w) {
+            auto load_peak = [&](int pp, Probe& x, double& w) {
+                x = none;
                 if (pp < na) {
-                    mz = P.A.mz[a0 + pp];
-                    w = __dmul_rn(peak_a(P.A.a, a0 + pp), P.A.b[a0 + pp]);
+                    const int4 v = __ldg(reinterpret_cast<const int4*>(P.probe + A.a0 + pp));
+                    x = Probe{__int_as_float(v.x), __int_as_float(v.y), (uint32_t)v.z, (uint32_t)v.w};
+                    w = A_IS_REF ? __dmul_rn(peak_a(P.A.a, A.a0 + pp), P.A.b[A.a0 + pp])
+                                 : P.A.b[A.a0 + pp];
                 }
             };
-            load_peak(lane, mz_c, w_c);
-            load_peak(32 + lane, mz_n, w_n);
-            // one step's window and raw bucket-table values (consumed a step later)
-            float pL = 1.0f, pH = 0.0f;
-            uint32_t pt0 = 0, pt1 = 0, pt2 = 0, pt3 = 0;
-            auto probe = [&](bool valid, float mz, bool shifted) {
-                pL = 1.0f;
-                pH = 0.0f;
-                pt0 = pt1 = pt2 = pt3 = 0u;
-                if (!valid) return;
-                const bool ok = (MODIFIED && shifted)
-                                    ? nl_window(mz, P.A.prec[a], P.tol, pL, pH)
-                                    : Window<A_IS_REF, NOSHIFT>::bounds(mz, P.tol, P.shift, pL, pH);
-                if (!ok) {
-                    atomicOr(P.err, kErrBadOffsets);
-                    pL = 1.0f;
-                    pH = 0.0f;
-                    return;
-                }
-                if (!(pL <= pH)) return;
-                const uint32_t* TT = (MODIFIED && shifted) ? T2 : T;
-                const long long blo = bucket_of(pL, P.g.inv_w);
-                const long long bhi = bucket_of(pH, P.g.inv_w);
-                if (bhi - blo + 1 >= P.g.nb) {
-                    pt0 = __ldg(&TT[0]);
-                    pt1 = __ldg(&TT[P.g.nb]);
+            // raw bucket-table values: entries [t0, t1), and [0, t2) when wrapped
+            auto table = [&](const uint32_t* TT, uint32_t bl, uint32_t bh, uint32_t& t0,
+                             uint32_t& t1, uint32_t& t2) {
+                t0 = t1 = t2 = 0u;
+                if (bl == kNoBucket) return;
+                t0 = __ldg(&TT[bl]);
+                if (bl <= bh) {
+                    t1 = __ldg(&TT[bh + 1]);
                 } else {
-                    const unsigned bl = (unsigned)blo & nbmask, bh = (unsigned)bhi & nbmask;
-                    pt0 = __ldg(&TT[bl]);
-                    if (bl <= bh) {
-                        pt1 = __ldg(&TT[bh + 1]);
-                    } else {  // wrapped: [bl, nb) then [0, bh]
-                        pt1 = __ldg(&TT[P.g.nb]);
-                        pt2 = __ldg(&TT[0]);
-                        pt3 = __ldg(&TT[bh + 1]);
-                    }
+                    t1 = __ldg(&TT[P.g.nb]);
+                    t2 = __ldg(&TT[bh + 1]);
                 }
             };
-            probe(lane < na, mz_c, false);
+            load_peak(lane, pr, w_c);
+            load_peak(32 + lane, pn, w_n);
+            uint32_t t0, t1, t2;
+            table(T, pr.bl, pr.bh, t0, t1, t2);
             for (int st = 0; st < n_steps; ++st) {
                 const int pass = MODIFIED ? (st & 1) : 0;
                 const int pc = (MODIFIED ? (st >> 1) : st) * 32;
-                const int p = pc + lane;
-                // this step's probe
-                const float L = pL, H = pH;
-                const uint32_t r0b = pt0, c0 = pt1 - pt0, r1b = pt2, c1 = pt3 - pt2;
-                if (pass == 0) {
-                    s_wa[lane] = w_c;
-                    if (MODIFIED) s_x[lane] = mz_c;
+                const uint32_t r0 = t0, c0 = t1 - t0, c1 = t2;
+                // window of the record; the shifted pass tests with the peak's m/z
+                float x0 = pr.lo, x1 = pr.hi;
+                if (MODIFIED && pass) x0 = pc + lane < na ? __ldg(&P.A.mz[A.a0 + pc + lane]) : 0.f;
+                if (pass == 0) s_wa[lane] = w_c;
+                // the next step's table values, in flight during this step's rounds
+                if (MODIFIED && pass == 0) {
+                    uint2 b2 = make_uint2(kNoBucket, 0u);
+                    if (pc + lane < na) b2 = __ldg(&P.probe2[A.a0 + pc + lane]);
+                    table(T2, b2.x, b2.y, t0, t1, t2);
+                } else {
+                    pr = pn;
+                    w_c = w_n;
+                    table(T, pr.bl, pr.bh, t0, t1, t2);
+                    load_peak(pc + 64 + lane, pn, w_n);
                 }
-                // the next step's probe, in flight during this step's rounds
-                if (st + 1 < n_steps) {
-                    if (MODIFIED && pass == 0)
-                        probe(p < na, mz_c, true);
-                    else
-                        probe(p + 32 < na, mz_n, false);
-                }
-                const Entry* EE = (MODIFIED && pass) ? P.ent2 : ent;
-                s_lh[lane] = make_float2(L, H);
-                const uint32_t c = c0 + c1;
-                uint32_t incl = c;
+                const Entry* EE = ((MODIFIED && pass) ? P.ent2 : P.ent) + tbase;
+                const double* EA = (MODIFIED && pass) ? P.ent2_a : P.ent_a;
+                const int turns = __any_sync(full, c1 != 0u) ? 2 : 1;
+                for (int turn = 0; turn < turns; ++turn) {
+                    const uint32_t c = turn ? c1 : c0;
+                    uint32_t incl = c;
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const uint32_t v = __shfl_up_sync(full, incl, d);
-                    if (lane >= d) incl += v;
-                }
-                const uint32_t excl = incl - c;
-                const uint32_t E = __shfl_sync(full, incl, 31);
-                const bool wrapped = __any_sync(full, c1 != 0u);
-                const uint32_t off0 = r0b - excl;  // entry k of lane l: r0b + (k - excl)
-                __syncwarp();
-                // position of flat entry k, and the lane (peak) that owns it
-                auto locate = [&](uint32_t k, int& o) -> uint32_t {
-                    o = 0;
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1) {
-                        const uint32_t v = __shfl_sync(full, incl, o + step - 1);
-                        if (v <= k) o += step;
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t v = __shfl_up_sync(full, incl, d);
+                        if (lane >= d) incl += v;
                     }
-                    if (!wrapped) return __shfl_sync(full, off0, o & 31) + k;
-                    const uint32_t oex = __shfl_sync(full, excl, o & 31);
-                    const uint32_t oc0 = __shfl_sync(full, c0, o & 31);
-                    const uint32_t or0 = __shfl_sync(full, r0b, o & 31);
-                    const uint32_t or1 = __shfl_sync(full, r1b, o & 31);
-                    const uint32_t e = k - oex;
-                    return e < oc0 ? or0 + e : or1 + (e - oc0);
-                };
-                for (uint32_t kb = 0; kb < E; kb += 32 * kRounds) {
-                    // kRounds rounds' entries in flight before the first is tested
-                    int ow[kRounds];
-                    Entry enb[kRounds];
-#pragma unroll
-                    for (int u = 0; u < kRounds; ++u) {
-                        const uint32_t k = kb + 32u * u + (uint32_t)lane;
-                        const uint32_t pos = locate(k, ow[u]);
-                        enb[u].id = 0;
-                        if (k < E) enb[u] = EE[tbase + pos];
-                    }
-#pragma unroll
-                    for (int u = 0; u < kRounds; ++u) {
-                        if (kb + 32u * u >= E) break;
-                        const uint32_t k = kb + 32u * u + (uint32_t)lane;
-                        const int o = ow[u];
-                        const Entry en = enb[u];
+                    const uint32_t excl = incl - c;
+                    const uint32_t E = __shfl_sync(full, incl, 31);
+                    const unsigned some = __ballot_sync(full, c != 0u);
+                    if (c != 0u)
+                        s_rec[__popc(some & below)] =
+                            make_uint4((turn ? 0u : r0) - excl, __float_as_uint(x0),
+                                       __float_as_uint(x1), (unsigned)lane);
+                    __syncwarp();
+                    int started = -1;  // records whose first entry lies before the round, minus 1
+                    for (uint32_t kb = 0; kb < E; kb += 32) {
+                        const uint32_t d = excl - kb;
+                        const unsigned first =
+                            __reduce_or_sync(full, (c != 0u && d < 32u) ? 1u << d : 0u);
+                        const int ri = started + __popc(first & upto);
+                        started += __popc(first);
+                        const uint32_t k = kb + (uint32_t)lane;
                         bool cand = false;
+                        int o = 0, bq = 0, pB = 0;
+                        uint32_t pos = 0;
+                        double eb = 0.0;
                         if (k < E) {
-                            const float2 lh = s_lh[o];
-                            const int bq = (int)(en.id >> 16);
-                            cand = en.mz >= lh.x && en.mz <= lh.y && bq >= range_lo && bq < range_hi;
-                            if (MODIFIED && pass && cand) {
+                            const uint4 rec = s_rec[ri];
+                            pos = rec.x + k;
+                            const int4 v = __ldg(reinterpret_cast<const int4*>(EE + pos));
+                            const float mz = __int_as_float(v.x);
+                            o = (int)rec.w;
+                            bq = (int)((unsigned)v.y >> 16);
+                            pB = v.y & 0xFFFF;
+                            eb = __hiloint2double(v.w, v.z);
+                            cand = bq >= range_lo && bq < range_hi;
+                            if (MODIFIED && pass) {
                                 // the shifted window exactly as matchms tests it:
                                 // mz2 = mz_q + (prec_ref - prec_q) against mz_ref -+ tol
-                                const int qb = b_begin + bq;
-                                const float y = P.B.mz[P.B.off[qb] + (en.id & 0xFFFFu)];
-                                const double mz2 =
-                                    __dadd_rn((double)y, __dsub_rn(P.A.prec[a], P.B.prec[qb]));
-                                const double x = (double)s_x[o];
-                                cand = !(mz2 > __dadd_rn(x, P.tol)) && !(mz2 < __dsub_rn(x, P.tol));
+                                if (cand) {
+                                    const double mz2 = __dadd_rn(
+                                        (double)mz, __dsub_rn(P.A.prec[a], P.B.prec[b_begin + bq]));
+                                    const double x = (double)__uint_as_float(rec.y);
+                                    cand = !(mz2 > __dadd_rn(x, P.tol)) && !(mz2 < __dsub_rn(x, P.tol));
+                                }
+                            } else {
+                                cand = cand && mz >= __uint_as_float(rec.y) &&
+                                       mz <= __uint_as_float(rec.z);
                             }
                         }
                         const unsigned bal = __ballot_sync(full, cand);
                         const int slot = n + __popc(bal & below);
                         n += __popc(bal);
                         if (cand && slot < pool_max) {
-                            const int bq = (int)(en.id >> 16);
-                            const int pB = (int)(en.id & 0xFFFFu);
                             const int pa = pc + o;
-                            const double aB = P.B.a ? P.B.a[P.B.off[b_begin + bq] + pB] : 1.0;
                             double key;
                             uint32_t gen;
                             if (A_IS_REF) {
-                                key = __dmul_rn(__dmul_rn(s_wa[o], aB), en.b);
+                                key = s_wa[o];
+                                if (EA) key = __dmul_rn(key, EA[tbase + pos]);
+                                key = __dmul_rn(key, eb);
                                 gen = ((uint32_t)pa << 16) | (uint32_t)pB;
                                 if (MODIFIED) gen |= (uint32_t)pass << 31;
                             } else {
-                                const double wB = __dmul_rn(aB, en.b);
-                                key = __dmul_rn(__dmul_rn(wB, peak_a(P.A.a, a0 + pa)),
-                                                P.A.b[a0 + pa]);
+                                key = eb;
+                                if (EA) key = __dmul_rn(EA[tbase + pos], eb);
+                                if (P.A.a) key = __dmul_rn(key, P.A.a[A.a0 + pa]);
+                                key = __dmul_rn(key, s_wa[o]);
                                 gen = ((uint32_t)pB << 16) | (uint32_t)pa;
                             }
                             // push onto the query's chain: swap the new slot into
@@ -979,16 +1060,12 @@ join_kernel(JoinParams P) {
                             if ((ph >> 12) == epoch) m |= ((ph & 0xFFFu) << 12) | kHasNext;
                             pool.put(slot, key, gen, m);
                         }
+                        if (n > pool_max) break;
                     }
+                    __syncwarp();  // s_rec / s_wa are rewritten by the next turn or step
                     if (n > pool_max) break;
                 }
-                __syncwarp();  // s_lh / s_wa / s_x are rewritten by the next step
                 if (n > pool_max) break;
-                if (pass == kPasses - 1) {  // next chunk: rotate the prefetched peaks
-                    mz_c = mz_n;
-                    w_c = w_n;
-                    load_peak(pc + 64 + lane, mz_n, w_n);
-                }
             }
             __syncwarp();
             if (n > pool_max) {
@@ -1000,15 +1077,8 @@ join_kernel(JoinParams P) {
                 }
                 // a single pair has more candidates than the pool: pair kernel
                 if (lane == 0) {
-                    const int bq = b_begin + range_lo;
-                    const int rr = A_IS_REF ? a : bq, qq = A_IS_REF ? bq : a;
-                    spill_push(P.spill, rr, qq, P.err);
-                    if (!SPARSE) {
-                        const int64_t o = (int64_t)rr * P.dense.ld + qq;
-                        P.dense.score[o] = __int_as_float(0x7fc00000);
-                        P.dense.matches[o] = -1;
-                        P.dense.overflow[o] = 0;
-                    }
+                    spill_run(range_lo);
+                    if (!SPARSE) P.dense.overflow[row + range_lo] = 0;
                 }
                 __syncwarp();
                 range_lo = range_hi;
@@ -1023,38 +1093,47 @@ join_kernel(JoinParams P) {
             // before the runs are resolved, so that the lines are still in L2
             // when the results land in them (zeroing before the sweep let L2
             // evict ~1/3 of them first: +40% DRAM traffic).  Four queries per
-            // lane, 16-byte streaming stores when aligned.
+            // lane and 16-byte streaming stores from the first aligned query on,
+            // whatever the row's own alignment.
             if (!SPARSE) {
-                const int64_t row = (int64_t)a * P.dense.ld + b_begin + range_lo;
-                int qv = 0;
-                if ((row & 3) == 0 && (P.dense.ld & 3) == 0) {
-                    for (; qv + 128 <= rw; qv += 128) {
-                        const int64_t o = row + qv + 4 * lane;
+                const int64_t r = row + range_lo;
+                auto zero1 = [&](int64_t o) {
+                    __stcs(P.dense.score + o, 0.f);
+                    __stcs(P.dense.matches + o, 0);
+                    __stcs(P.dense.overflow + o, (unsigned char)0);
+                };
+                if (P.vec_rows) {
+                    const int pre = min(rw, (int)(-r & 3));
+                    const int nv = (rw - pre) >> 2;
+                    if (lane < pre) zero1(r + lane);
+                    for (int v = lane; v < nv; v += 32) {
+                        const int64_t o = r + pre + 4 * v;
                         __stcs(reinterpret_cast<float4*>(P.dense.score + o),
                                make_float4(0.f, 0.f, 0.f, 0.f));
                         __stcs(reinterpret_cast<int4*>(P.dense.matches + o), make_int4(0, 0, 0, 0));
                         __stcs(reinterpret_cast<uchar4*>(P.dense.overflow + o),
                                make_uchar4(0, 0, 0, 0));
                     }
-                }
-                for (int qr = qv + lane; qr < rw; qr += 32) {
-                    __stcs(&P.dense.score[row + qr], 0.f);
-                    __stcs(&P.dense.matches[row + qr], 0);
-                    __stcs(&P.dense.overflow[row + qr], (unsigned char)0);
+                    if (lane < ((rw - pre) & 3)) zero1(r + pre + 4 * nv + lane);
+                } else {
+                    for (int qr = lane; qr < rw; qr += 32) zero1(r + qr);
                 }
             }
             __syncwarp();
 
             // ---- resolve each query's run ----
             // Slot s owns its query's run when the query's head names it (it
-            // was pushed last); the owner walks the chain.  Runs of 1 to 3
-            // candidates are resolved by their lane in closed form; runs of
-            // 4..32 are queued and resolved by the warp; longer runs (or runs
-            // reaching match_limit) go to the pair kernel.
-            int n_mid = 0, n_big = 0;
+            // was pushed last).  Runs of one candidate, most of them, are
+            // stored at once; the owners of longer runs are queued and taken 32
+            // at a time, a lane walking its run's chain: 2 to 4 candidates are
+            // resolved there in closed form (the queue keeps the lanes of that
+            // code busy: an owner loop that did both ran it for a few lanes in
+            // every step), 5..32 go to a second queue resolved by the warp, and
+            // longer runs (or runs reaching match_limit) to the pair kernel.
+            int n_mid = 0, n_big = 0, n_queue = 0;
             auto flush_long = [&]() {
                 __syncwarp();
-                // runs of 4..8 candidates, four at a time: each 8-lane segment
+                // runs of 5..8 candidates, four at a time: each 8-lane segment
                 // sorts one run's (key, gen) descending in registers (bitonic),
                 // then resolves it greedily by segment-wise ballot
                 const int seg = lane >> 3, tq = lane & 7;
@@ -1065,12 +1144,16 @@ join_kernel(JoinParams P) {
                     const int L = valid ? (int)(e >> 12) : 0;
                     double k = -INFINITY;
                     uint32_t g = 0;
+                    int q = 0;
                     if (tq < L) {
                         int sl = s0;
                         for (int h = 0; h < tq; ++h) sl = meta_next(pool.meta(sl));
-                        k = pool.key(sl);
-                        g = pool.gen(sl);
+                        const PoolEntry x = pool.get(sl);
+                        k = x.key;
+                        g = x.gen;
+                        q = range_lo + meta_query(x.meta);
                     }
+                    const double rnB = (valid && tq == 0) ? P.rnB[b_begin + q] : 0.0;
 #pragma unroll
                     for (int kk = 2; kk <= kMidRun; kk <<= 1) {
 #pragma unroll
@@ -1105,8 +1188,7 @@ join_kernel(JoinParams P) {
                         }
                         bal = __ballot_sync(full, alive);
                     }
-                    if (valid && tq == 0)
-                        store_result(b_begin + range_lo + meta_query(pool.meta(s0)), score, mt);
+                    if (valid && tq == 0) store_result(q, score, mt, rnB);
                 }
                 // runs of 9..32 candidates, one at a time on the whole warp
                 for (int r = 0; r < n_big; ++r) {
@@ -1115,11 +1197,14 @@ join_kernel(JoinParams P) {
                     const int L = (int)(e >> 12);
                     double k = -INFINITY;
                     uint32_t g = 0;
+                    int q = 0;
                     if (lane < L) {
                         int sl = s0;
                         for (int h = 0; h < lane; ++h) sl = meta_next(pool.meta(sl));
-                        k = pool.key(sl);
-                        g = pool.gen(sl);
+                        const PoolEntry x = pool.get(sl);
+                        k = x.key;
+                        g = x.gen;
+                        q = range_lo + meta_query(x.meta);
                     }
 #pragma unroll
                     for (int kk = 2; kk <= 32; kk <<= 1) {
@@ -1153,111 +1238,138 @@ join_kernel(JoinParams P) {
                             alive = false;
                         bal = __ballot_sync(full, alive);
                     }
-                    if (lane == 0)
-                        store_result(b_begin + range_lo + meta_query(pool.meta(s0)), score, mt);
+                    if (lane == 0) store_result(q, score, mt, P.rnB[b_begin + q]);
                 }
                 __syncwarp();
                 n_mid = 0;
                 n_big = 0;
             };
-            for (int c = 0; c < n; c += 32) {
-                const int s = c + lane;
-                bool own = false;
-                int L = 0, qr = 0;
-                double snB_own = 0.0;
-                double k0 = 0.0, k1 = 0.0, k2 = 0.0;
-                uint32_t g0 = 0, g1 = 0, g2 = 0;
-                if (s < n) {
-                    const uint32_t m0 = pool.meta(s);
-                    qr = meta_query(m0);
-                    const unsigned h = (head[qr >> 1] >> ((qr & 1) * 16)) & 0xFFFu;
-                    own = h == (unsigned)s;
-                    if (own) {
-                        // the query norm's load starts before the chain walk
-                        snB_own = P.snB[b_begin + range_lo + qr];
-                        k0 = pool.key(s);
-                        g0 = pool.gen(s);
-                        L = 1;
-                        if (m0 & kHasNext) {
-                            const int s1 = meta_next(m0);
-                            const uint32_t m1 = pool.meta(s1);
-                            k1 = pool.key(s1);
-                            g1 = pool.gen(s1);
-                            L = 2;
-                            if (m1 & kHasNext) {
-                                const int s2 = meta_next(m1);
-                                uint32_t m2 = pool.meta(s2);
-                                k2 = pool.key(s2);
-                                g2 = pool.gen(s2);
-                                L = 3;
+            auto flush_queue = [&]() {
+                __syncwarp();
+                for (int c = 0; c < n_queue; c += 32) {
+                    int L = 0, q = 0, s = 0;
+                    double rnB = 0.0;
+                    double k0 = 0.0, k1 = 0.0, k2 = -INFINITY, k3 = -INFINITY;
+                    uint32_t g0 = 0, g1 = 0, g2 = 0, g3 = 0;
+                    if (c + lane < n_queue) {
+                        s = queue[c + lane];
+                        PoolEntry x = pool.get(s);
+                        q = range_lo + meta_query(x.meta);
+                        rnB = P.rnB[b_begin + q];
+                        k0 = x.key;
+                        g0 = x.gen;
+                        x = pool.get(meta_next(x.meta));
+                        k1 = x.key;
+                        g1 = x.gen;
+                        L = 2;
+                        if (x.meta & kHasNext) {
+                            x = pool.get(meta_next(x.meta));
+                            k2 = x.key;
+                            g2 = x.gen;
+                            L = 3;
+                            if (x.meta & kHasNext) {
+                                x = pool.get(meta_next(x.meta));
+                                k3 = x.key;
+                                g3 = x.gen;
+                                L = 4;
                                 // longer runs: count the rest (up to kLongRun + 1)
-                                while ((m2 & kHasNext) && L <= kLongRun) {
-                                    m2 = pool.meta(meta_next(m2));
+                                uint32_t m = x.meta;
+                                while ((m & kHasNext) && L <= kLongRun) {
+                                    m = pool.meta(meta_next(m));
                                     ++L;
                                 }
                             }
                         }
                     }
-                }
-                const bool is_long = own && L > 3 && L <= kLongRun && L < P.match_limit;
-                const bool is_mid = is_long && L <= kMidRun;
-                const unsigned mb = __ballot_sync(full, is_mid);
-                const unsigned bb = __ballot_sync(full, is_long && !is_mid);
-                if (n_mid + n_big + __popc(mb) + __popc(bb) > kLongRuns) flush_long();
-                const unsigned run = (unsigned)s | ((unsigned)L << 12);
-                if (is_mid)
-                    long_runs[n_mid + __popc(mb & below)] = run;
-                else if (is_long)
-                    long_runs[kLongRuns - 1 - (n_big + __popc(bb & below))] = run;
-                n_mid += __popc(mb);
-                n_big += __popc(bb);
-                if (own && !is_long) {
-                    const int bq = b_begin + range_lo + qr;
-                    if (L >= P.match_limit || L > kLongRun) {
-                        spill_push(P.spill, A_IS_REF ? a : bq, A_IS_REF ? bq : a, P.err);
-                        if (!SPARSE) put_dense(bq, __int_as_float(0x7fc00000), -1);
-                    } else {
-                        // one to three candidates: sorting network, then greedy
+                    const bool to_pair = L >= P.match_limit || L > kLongRun;
+                    const bool is_long = L > 4 && !to_pair;
+                    const bool is_mid = is_long && L <= kMidRun;
+                    const unsigned mb = __ballot_sync(full, is_mid);
+                    const unsigned bb = __ballot_sync(full, is_long && !is_mid);
+                    if (n_mid + n_big + __popc(mb) + __popc(bb) > kLongRuns) flush_long();
+                    const unsigned run = (unsigned)s | ((unsigned)L << 12);
+                    if (is_mid)
+                        long_runs[n_mid + __popc(mb & below)] = run;
+                    else if (is_long)
+                        long_runs[kLongRuns - 1 - (n_big + __popc(bb & below))] = run;
+                    n_mid += __popc(mb);
+                    n_big += __popc(bb);
+                    if (to_pair) spill_run(q);
+                    if (L != 0 && !is_long && !to_pair) {
+                        // two to four candidates: sorting network (absent ones hold
+                        // -infinity and stay last), then greedy
+                        auto order = [](double& ka, uint32_t& ga, double& kb, uint32_t& gb) {
+                            if (before(kb, gb, ka, ga)) {
+                                const double tk = ka;
+                                ka = kb;
+                                kb = tk;
+                                const uint32_t tg = ga;
+                                ga = gb;
+                                gb = tg;
+                            }
+                        };
+                        auto clash = [](uint32_t ga, uint32_t gb) {
+                            return gen_p1<MODIFIED>(ga) == gen_p1<MODIFIED>(gb) ||
+                                   (ga & 0xFFFFu) == (gb & 0xFFFFu);
+                        };
+                        order(k0, g0, k1, g1);
+                        if (L > 2) {
+                            order(k2, g2, k3, g3);
+                            order(k0, g0, k2, g2);
+                            order(k1, g1, k3, g3);
+                            order(k1, g1, k2, g2);
+                        }
                         double score = k0;
                         int mt = 1;
-                        if (L >= 2) {
-                            auto order = [](double& ka, uint32_t& ga, double& kb, uint32_t& gb) {
-                                if (before(kb, gb, ka, ga)) {
-                                    const double tk = ka;
-                                    ka = kb;
-                                    kb = tk;
-                                    const uint32_t tg = ga;
-                                    ga = gb;
-                                    gb = tg;
-                                }
-                            };
-                            auto clash = [](uint32_t ga, uint32_t gb) {
-                                return gen_p1<MODIFIED>(ga) == gen_p1<MODIFIED>(gb) ||
-                                       (ga & 0xFFFFu) == (gb & 0xFFFFu);
-                            };
-                            order(k0, g0, k1, g1);
-                            if (L == 3) {
-                                order(k1, g1, k2, g2);
-                                order(k0, g0, k1, g1);
-                            }
-                            score = k0;
-                            const bool take1 = !clash(g0, g1);
-                            if (take1) {
-                                score = __dadd_rn(score, k1);
-                                mt = 2;
-                            }
-                            if (L == 3 && !clash(g0, g2) && !(take1 && clash(g1, g2))) {
+                        const bool take1 = !clash(g0, g1);
+                        if (take1) {
+                            score = __dadd_rn(score, k1);
+                            mt = 2;
+                        }
+                        if (L > 2) {
+                            const bool take2 = !clash(g0, g2) && !(take1 && clash(g1, g2));
+                            if (take2) {
                                 score = __dadd_rn(score, k2);
                                 ++mt;
                             }
+                            if (L > 3 && !clash(g0, g3) && !(take1 && clash(g1, g3)) &&
+                                !(take2 && clash(g2, g3))) {
+                                score = __dadd_rn(score, k3);
+                                ++mt;
+                            }
                         }
-                        store_result_n(bq, score, mt, snB_own);
+                        store_result(q, score, mt, rnB);
+                    }
+                    __syncwarp();
+                }
+                __syncwarp();
+                n_queue = 0;
+            };
+            for (int c = 0; c < n; c += 32) {
+                const int s = c + lane;
+                bool more = false;
+                if (s < n) {
+                    const PoolEntry x = pool.get(s);
+                    const int qr = meta_query(x.meta);
+                    const unsigned h = (head[qr >> 1] >> ((qr & 1) * 16)) & 0xFFFu;
+                    if (h == (unsigned)s) {
+                        more = (x.meta & kHasNext) != 0u;
+                        if (!more) {
+                            const int q = range_lo + qr;
+                            if (P.match_limit > 1)
+                                store_result(q, x.key, 1, P.rnB[b_begin + q]);
+                            else
+                                spill_run(q);
+                        }
                     }
                 }
+                const unsigned mb = __ballot_sync(full, more);
+                if (n_queue + __popc(mb) > kQueue) flush_queue();
+                if (more) queue[n_queue + __popc(mb & below)] = (uint16_t)s;
+                n_queue += __popc(mb);
             }
-            __syncwarp();
+            flush_queue();
             flush_long();
-            __syncwarp();
             range_lo = range_hi;
             if (n < pool_max / 4) width = min(tn, width * 2);
         }
@@ -1269,11 +1381,10 @@ join_kernel(JoinParams P) {
                 asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
                 unsigned long long* r = P.trace.rec + 4 * k;
                 r[0] = (unsigned long long)P.trace.tag | ((unsigned long long)smid << 32);
-                r[1] = base + (unsigned long long)f;
+                r[1] = item;
                 r[2] = *s_t0;
                 r[3] = global_ns();
             }
-        }
         }
     }
     if (P.slots) {  // give the global-pool slice back
@@ -2105,14 +2216,14 @@ constexpr int kScatterThreads = 256;  // index scatter: a warp per spectrum
 // warp pulling work until none is left; CTA b owns global-pool slices
 // 8b..8b+7, so the grid may not exceed the resident CTAs.  Bounded
 // (waves > 0): `waves` times the resident CTAs, each warp exiting after an
-// equal share of fetches, so that the SMs free up CTA by CTA and concurrent
+// equal share of items, so that the SMs free up CTA by CTA and concurrent
 // launches on other streams are scheduled in between while every wave stays
 // full; each CTA claims a global-pool slice from jp.slots (zeroed by the
 // caller) for its lifetime.
-template <bool A_IS_REF, bool SPARSE, bool NOSHIFT, bool MODIFIED>
+template <bool A_IS_REF, bool SPARSE, bool MODIFIED>
 int launch_join(cms_ctx* ctx, JoinParams jp, size_t smem, size_t gpool_warps, int64_t n_items,
                 cudaStream_t s, int waves = 0) {
-    auto* kern = join_kernel<A_IS_REF, SPARSE, NOSHIFT, MODIFIED>;
+    auto* kern = join_kernel<A_IS_REF, SPARSE, MODIFIED>;
     if (const int rc = set_func_smem(kern, smem)) return rc;
     jp.trace = TraceOut{ctx->trace_rec, ctx->trace_count, ctx->trace_cap, ctx->trace_tag};
     int per_sm = 1;
@@ -2120,10 +2231,9 @@ int launch_join(cms_ctx* ctx, JoinParams jp, size_t smem, size_t gpool_warps, in
     const int64_t resident = (int64_t)ctx->sm_count * std::max(1, per_sm);
     int64_t grid;
     if (waves > 0) {
-        const int64_t fetches = std::max<int64_t>(1, (n_items + kFetch - 1) / kFetch);
-        grid = std::min<int64_t>(resident * waves, (fetches + kJoinWarps - 1) / kJoinWarps);
+        grid = std::min<int64_t>(resident * waves, (n_items + kJoinWarps - 1) / kJoinWarps);
         grid = std::max<int64_t>(1, grid);
-        const int64_t per_warp = (fetches + grid * kJoinWarps - 1) / (grid * kJoinWarps);
+        const int64_t per_warp = (n_items + grid * kJoinWarps - 1) / (grid * kJoinWarps);
         if (per_warp > INT32_MAX) {
             set_error("cms_cosine_greedy: too many work items for one launch");
             return CMS_ERR_UNSUPPORTED;
@@ -2182,12 +2292,17 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     need += bump_size(64 * sizeof(uint64_t));            // flags, counters
     need += bump_size(nR * sizeof(double)) + bump_size(nQ * sizeof(double));
     if (p.mode == 1) {
-        need += bump_size(nR * sizeof(int32_t));
+        need += bump_size(nR * sizeof(SweepItem)) + bump_size(nQ * sizeof(double));
+        need += bump_size((size_t)std::max<int64_t>(1, args.ref.n_peaks) * sizeof(Probe));
+        if (args.modified)
+            need += bump_size((size_t)std::max<int64_t>(1, args.ref.n_peaks) * sizeof(uint2));
         const size_t idx = args.modified ? 2 : 1;  // m/z index, neutral-loss index
         need += bump_size(idx * (size_t)p.n_tiles * p.nb * sizeof(uint32_t));
         need += bump_size((size_t)p.n_tiles * scan_chunks(p.nb) * sizeof(uint32_t));
         need += idx * bump_size((size_t)p.n_tiles * (p.nb + 1) * sizeof(uint32_t));
         need += idx * bump_size((size_t)std::max<int64_t>(1, args.qry.n_peaks) * sizeof(Entry));
+        if (args.qry.a)
+            need += idx * bump_size((size_t)std::max<int64_t>(1, args.qry.n_peaks) * sizeof(double));
         need += bump_size((size_t)p.spill_cap * sizeof(int2));
         need += bump_size(gpool_bytes);
     }
@@ -2224,6 +2339,10 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     const size_t zeroed = bp.used - (size_t)((char*)small - (char*)ctx->scratch.ptr);
     uint32_t* cur2 = idx == 2 ? cur + n_cnt : nullptr;
     uint32_t* sums = idx ? bp.take<uint32_t>(n_chunks) : nullptr;
+    double* rnQ = idx ? bp.take<double>(nQ) : nullptr;
+    const size_t ref_peaks = (size_t)std::max<int64_t>(1, args.ref.n_peaks);
+    Probe* probe = idx ? bp.take<Probe>(ref_peaks) : nullptr;
+    uint2* probe2 = idx == 2 ? bp.take<uint2>(ref_peaks) : nullptr;
     double* snR = bp.take<double>(nR);
     double* snQ = bp.take<double>(nQ);
     CMS_CUDA_TRY(cudaMemsetAsync(small, 0, zeroed, s));
@@ -2233,8 +2352,10 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     {
         StageScope sc(ctx, 0, 2, s);
         const int max_peaks = args.modified ? kModifiedMaxPeaks : CMS_MAX_PEAKS;
-        const PrepSide pr{args.ref, snR, idx ? cls_count : nullptr, nullptr, nullptr};
-        const PrepSide pq{args.qry, snQ, nullptr, cur, cur2};
+        const PrepSide pr{args.ref, snR,   nullptr, idx ? cls_count : nullptr, nullptr, nullptr,
+                          probe,    probe2, args.tol, args.shift, 1};
+        const PrepSide pq{args.qry, snQ,     rnQ, nullptr, cur, cur2,
+                          nullptr,  nullptr, 0.0, 0.0, 0};
         prep_kernel<<<blocks_for(nR, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
             pr, g, bad, ctx->err_word, max_peaks);
         prep_kernel<<<blocks_for(nQ, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
@@ -2308,14 +2429,18 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     }
 
     // ---- mode 1: order, index, join, spill ----
-    int32_t* order = bp.take<int32_t>(nR);
+    SweepItem* items = bp.take<SweepItem>(nR);
+    const size_t q_peaks = (size_t)std::max<int64_t>(1, args.qry.n_peaks);
     uint32_t* tab = bp.take<uint32_t>((size_t)p.n_tiles * (p.nb + 1));
-    Entry* ent = bp.take<Entry>((size_t)std::max<int64_t>(1, args.qry.n_peaks));
+    Entry* ent = bp.take<Entry>(q_peaks);
+    double* ent_a = args.qry.a ? bp.take<double>(q_peaks) : nullptr;
     uint32_t* tab2 = nullptr;
     Entry* ent2 = nullptr;
+    double* ent2_a = nullptr;
     if (args.modified) {
         tab2 = bp.take<uint32_t>((size_t)p.n_tiles * (p.nb + 1));
-        ent2 = bp.take<Entry>((size_t)std::max<int64_t>(1, args.qry.n_peaks));
+        ent2 = bp.take<Entry>(q_peaks);
+        if (args.qry.a) ent2_a = bp.take<double>(q_peaks);
     }
     int2* spill = bp.take<int2>(p.spill_cap);
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
@@ -2323,7 +2448,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     {
         StageScope sc(ctx, 1, 1, s);
         order_scatter_kernel<<<blocks_for(nR, kOrderThreads, sms), kOrderThreads, 0, s>>>(
-            args.ref, cls_count, cls_cursor, order, bad);
+            args.ref, snR, cls_count, cls_cursor, items, bad);
     }
     const int scatter_blocks = blocks_for(nQ, kScatterThreads / 32, sms);
     {
@@ -2331,30 +2456,33 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur, sums, bad);
         index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur, tab, sums, bad);
         index_scatter_kernel<false><<<scatter_blocks, kScatterThreads, 0, s>>>(args.qry, g, cur, ent,
-                                                                               bad);
+                                                                               ent_a, bad);
     }
     if (args.modified) {  // neutral-loss index: m/z - precursor, same geometry
         StageScope sc(ctx, 2, 3, s);
         index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur2, sums, bad);
         index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(g, cur2, tab2, sums, bad);
-        index_scatter_kernel<true><<<scatter_blocks, kScatterThreads, 0, s>>>(args.qry, g, cur2,
-                                                                              ent2, bad);
+        index_scatter_kernel<true><<<scatter_blocks, kScatterThreads, 0, s>>>(
+            args.qry, g, cur2, ent2, ent2_a, bad);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
     JoinParams jp{};
     jp.A = args.ref;
     jp.B = args.qry;
-    jp.snA = snR;
+    jp.items = items;
+    jp.probe = probe;
+    jp.probe2 = probe2;
     jp.snB = snQ;
-    jp.a_order = order;
+    jp.rnB = rnQ;
     jp.tab = tab;
     jp.ent = ent;
+    jp.ent_a = ent_a;
     jp.tab2 = tab2;
     jp.ent2 = ent2;
+    jp.ent2_a = ent2_a;
     jp.g = g;
     jp.tol = args.tol;
-    jp.shift = args.shift;
     jp.match_limit = args.match_limit;
     jp.init_width_scale = 0.f;
     for (int c = 0; c < kOrderClasses; ++c) jp.width_by_class[c] = p.width_by_class[c];
@@ -2371,6 +2499,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     jp.work = work_join;
     jp.spill = SpillList{spill, spill_count, p.spill_cap};
     jp.dense = pp.dense;
+    jp.vec_rows = (((uintptr_t)pp.dense.score | (uintptr_t)pp.dense.matches) & 15) == 0 &&
+                  ((uintptr_t)pp.dense.overflow & 3) == 0;
     jp.sparse = pp.sparse;
     jp.err = ctx->err_word;
     jp.bad = bad;
@@ -2378,22 +2508,13 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     const size_t join_smem = (size_t)warp_slice_bytes(p.tile) * kJoinWarps;
     {
         StageScope sc(ctx, 3, 1, s);
-        const bool noshift = args.shift == 0.0;
-        const int64_t items = nR * (int64_t)p.n_tiles;
-        if (args.modified)  // shift 0 at the first pass; the second takes it per pair
-            rc = sparse ? launch_join<true, true, true, true>(ctx, jp, join_smem, gpool_warps, items, s)
-                        : launch_join<true, false, true, true>(ctx, jp, join_smem, gpool_warps, items,
-                                                                s);
+        const int64_t n = nR * (int64_t)p.n_tiles;
+        if (args.modified)
+            rc = sparse ? launch_join<true, true, true>(ctx, jp, join_smem, gpool_warps, n, s)
+                        : launch_join<true, false, true>(ctx, jp, join_smem, gpool_warps, n, s);
         else
-        rc = sparse
-                 ? (noshift ? launch_join<true, true, true, false>(ctx, jp, join_smem, gpool_warps,
-                                                                   items, s)
-                            : launch_join<true, true, false, false>(ctx, jp, join_smem, gpool_warps,
-                                                                    items, s))
-                 : (noshift ? launch_join<true, false, true, false>(ctx, jp, join_smem, gpool_warps,
-                                                                    items, s)
-                            : launch_join<true, false, false, false>(ctx, jp, join_smem, gpool_warps,
-                                                                     items, s));
+            rc = sparse ? launch_join<true, true, false>(ctx, jp, join_smem, gpool_warps, n, s)
+                        : launch_join<true, false, false>(ctx, jp, join_smem, gpool_warps, n, s);
         if (rc) return rc;
     }
     CMS_CUDA_TRY(cudaGetLastError());
@@ -2800,9 +2921,9 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     CMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const IndexGeom none{1, 1, 1, 1.0};
     prep_kernel<<<blocks_for(n_ref, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-        PrepSide{args.ref, snR, nullptr, nullptr, nullptr}, none, bad, err, CMS_MAX_PEAKS);
+        PrepSide{args.ref, snR}, none, bad, err, CMS_MAX_PEAKS);
     prep_kernel<<<blocks_for(n_q, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-        PrepSide{args.qry, snQ, nullptr, nullptr, nullptr}, none, bad, err, CMS_MAX_PEAKS);
+        PrepSide{args.qry, snQ}, none, bad, err, CMS_MAX_PEAKS);
     CMS_CUDA_TRY(cudaGetLastError());
 
     PairParams pp{};
@@ -2849,8 +2970,10 @@ struct cms_library {
     int match_limit = 1;
     cms::IndexGeom g{};
     double* sn = nullptr;
+    double* rn = nullptr;
     uint32_t* tab = nullptr;
     cms::Entry* ent = nullptr;
+    double* ent_a = nullptr;  // only with m/z weights
     uint32_t* bad = nullptr;
 };
 
@@ -2858,8 +2981,10 @@ namespace {
 void library_free(cms_library* L) {
     if (!L) return;
     cudaFree(L->sn);
+    cudaFree(L->rn);
     cudaFree(L->tab);
     cudaFree(L->ent);
+    cudaFree(L->ent_a);
     cudaFree(L->bad);
     delete L;
 }
@@ -2911,6 +3036,9 @@ extern "C" int cms_library_create(cms_ctx* ctx, const float* mz, const double* a
     uint32_t* cur = nullptr;  // bucket counts, then the chunk sums
     cudaError_t e = cudaMalloc(&L->bad, 64);
     if (e == cudaSuccess) e = cudaMalloc(&L->sn, sizeof(double) * n);
+    if (e == cudaSuccess) e = cudaMalloc(&L->rn, sizeof(double) * n);
+    if (e == cudaSuccess && a)
+        e = cudaMalloc(&L->ent_a, sizeof(double) * std::max<int64_t>(1, n_peaks));
     if (e == cudaSuccess) e = cudaMalloc(&L->tab, sizeof(uint32_t) * n_tab);
     if (e == cudaSuccess) e = cudaMalloc(&L->ent, sizeof(Entry) * std::max<int64_t>(1, n_peaks));
     if (e == cudaSuccess) e = cudaMalloc(&cur, sizeof(uint32_t) * (n_cur + n_chunks));
@@ -2926,12 +3054,12 @@ extern "C" int cms_library_create(cms_ctx* ctx, const float* mz, const double* a
     if (e == cudaSuccess) {
         const int sms = ctx->sm_count;
         prep_kernel<<<blocks_for(n, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-            PrepSide{L->spec, L->sn, nullptr, cur, nullptr}, L->g, L->bad, ctx->err_word,
+            PrepSide{L->spec, L->sn, L->rn, nullptr, cur}, L->g, L->bad, ctx->err_word,
             CMS_MAX_PEAKS);
         index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, cur + n_cur, L->bad);
         index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, L->tab, cur + n_cur, L->bad);
         index_scatter_kernel<false><<<blocks_for(n, kScatterThreads / 32, sms), kScatterThreads, 0,
-                                      s>>>(L->spec, L->g, cur, L->ent, L->bad);
+                                      s>>>(L->spec, L->g, cur, L->ent, L->ent_a, L->bad);
         e = cudaGetLastError();
     }
     uint32_t hbad = 0;
@@ -3006,7 +3134,9 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
         (size_t)std::min(ctx->sm_count * 4, kSlotWords * 32) * kJoinWarps;
     const size_t gpool_bytes = gpool_warps * (size_t)kGPool * 16;
     size_t need = bump_size(64 * sizeof(uint64_t)) + bump_size(n_q * sizeof(double)) +
-                  bump_size(n_q * sizeof(int32_t)) + bump_size((size_t)spill_cap * sizeof(int2)) +
+                  bump_size(n_q * sizeof(SweepItem)) +
+                  bump_size((size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(Probe)) +
+                  bump_size((size_t)spill_cap * sizeof(int2)) +
                   bump_size(kSlotWords * sizeof(uint32_t)) + bump_size(gpool_bytes) + 4096;
     int rc = arena_reserve(ctx, ctx->scratch, need, s);
     if (rc) return rc;
@@ -3021,20 +3151,23 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     uint32_t* slots = bp.take<uint32_t>(kSlotWords);  // cleared with the counters before it
     CMS_CUDA_TRY(cudaMemsetAsync(small, 0, bp.used, s));
     double* snQ = bp.take<double>(n_q);
-    int32_t* order = bp.take<int32_t>(n_q);
+    SweepItem* sweep = bp.take<SweepItem>(n_q);
+    Probe* probe = bp.take<Probe>((size_t)std::max<int64_t>(1, n_q_peaks));
     int2* spill = bp.take<int2>(spill_cap);
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
 
     {
         StageScope sc(ctx, 0, 1, s);
         prep_kernel<<<blocks_for(n_q, kPrepPerBlock, ctx->sm_count), kPrepThreads, 0, s>>>(
-            PrepSide{Q, snQ, cls_count, nullptr, nullptr}, lib->g, bad, ctx->err_word,
+            PrepSide{Q, snQ, nullptr, cls_count, nullptr, nullptr, probe, nullptr, lib->tol,
+                     lib->shift, 0},
+            lib->g, bad, ctx->err_word,
             CMS_MAX_PEAKS);
     }
     {
         StageScope sc(ctx, 1, 1, s);
         order_scatter_kernel<<<blocks_for(n_q, kOrderThreads, ctx->sm_count), kOrderThreads, 0, s>>>(
-            Q, cls_count, cls_cursor, order, bad);
+            Q, snQ, cls_count, cls_cursor, sweep, bad);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
@@ -3043,14 +3176,15 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     JoinParams jp{};  // width_by_class zero: widths from cand_per_pair
     jp.A = Q;
     jp.B = lib->spec;
-    jp.snA = snQ;
+    jp.items = sweep;
+    jp.probe = probe;
     jp.snB = lib->sn;
-    jp.a_order = order;
+    jp.rnB = lib->rn;
     jp.tab = lib->tab;
     jp.ent = lib->ent;
+    jp.ent_a = lib->ent_a;
     jp.g = lib->g;
     jp.tol = lib->tol;
-    jp.shift = lib->shift;
     jp.match_limit = lib->match_limit;
     // A search runs as kSearchWaves waves of short-lived CTAs (an equal share
     // of fetches per warp) so that searches on other streams interleave with
@@ -3073,9 +3207,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     jp.bad = bad;
     {
         StageScope sc(ctx, 3, 1, s);
-        rc = launch_join<false, true, false, false>(ctx, jp,
-                                                    (size_t)jp.warp_smem_bytes * kJoinWarps,
-                                                    gpool_warps, items, s, kSearchWaves);
+        rc = launch_join<false, true, false>(ctx, jp, (size_t)jp.warp_smem_bytes * kJoinWarps,
+                                             gpool_warps, items, s, kSearchWaves);
         if (rc) return rc;
     }
     PairParams pp{};
