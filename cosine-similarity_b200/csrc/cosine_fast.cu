@@ -62,10 +62,16 @@ namespace {
 constexpr int kJoinWarps = 8;
 constexpr int kJoinThreads = kJoinWarps * 32;
 constexpr int kPool = 256;        // candidate pool entries per warp
-constexpr int kLongRun = 32;      // longer runs go to the pair kernel
 constexpr int kMidRun = 8;        // runs up to this length are resolved four per warp step
 constexpr int kMaxTile = 4096;    // max query spectra per tile
 constexpr int kOrderClasses = 17; // log2 length classes (0..16)
+// Length classes (512 peaks and more) whose spectra the join takes first,
+// against every tile: one of them against the last tile, begun when the other
+// warps are nearly done, would be waited for (12345 symmetric: 1.90 ms tile by
+// tile, 1.70 ms with them first; 1000 queries against a library 1.78 and 1.67).
+// Not for modified cosine, whose few large spectra are slower when they all
+// run together (8.8 ms tile by tile, 9.5 with them first).
+constexpr int kLargeClass = 10;
 constexpr int kModifiedMaxPeaks = 32767;  // modified cosine: reference peak index in 15 bits
 
 __device__ __forceinline__ double peak_a(const double* a, int64_t i) { return a ? a[i] : 1.0; }
@@ -207,10 +213,10 @@ __device__ __forceinline__ uint2 bucket_range(float L, float H, const IndexGeom&
 // A sweeping spectrum in the order the join takes them.
 struct __align__(16) SweepItem {
     int64_t a0;   // its first peak
-    double sn;    // its norm
-    double rn;    // 1 / norm (recip_norm)
     int32_t a;    // its index
     int32_t na;   // its peaks
+    double rn;    // 1 / norm (recip_norm)
+    double pad;
 };
 
 // 1 / norm for the join's division-free score, NaN (which sends the score to
@@ -235,6 +241,7 @@ struct PrepSide {
     uint32_t* cnt;        // peaks per (tile, bucket) of the m/z index (null: not wanted)
     uint32_t* cnt2;       // the same of the neutral-loss index (null: not wanted)
     Probe* probe;         // per peak, for the sweeping side (null: not wanted)
+    double* w;            // per peak a * b (null: not wanted)
     uint2* probe2;        // per peak, its shifted window's buckets (null: not wanted)
     double tol, shift;    // of the windows
     int is_ref;           // the sweeping side is the reference side
@@ -326,6 +333,14 @@ prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks
                 z[j] = (in && P.cnt) ? P.S.mz[k] : 0.f;
             }
         };
+        auto weights = [&](int c) {
+            if (!P.w) return;
+#pragma unroll
+            for (int j = 0; j < kPrepSpectra; ++j) {
+                const int64_t k = __shfl_sync(full, lo, j) + c + lane;
+                if (c + lane < __shfl_sync(full, len, j)) P.w[k] = __dmul_rn(w[j], v[j]);
+            }
+        };
         auto count = [&](int c) {
             if (!P.cnt) return;
 #pragma unroll
@@ -349,6 +364,7 @@ prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks
                 tile[j][lane] = __dmul_rn(x, x);
             }
             count(c);
+            weights(c);
             __syncwarp();
             if (c + 32 < longest) load(c + 32);
             // past a spectrum's end the tile holds +0.0, which leaves the sum as it is
@@ -544,8 +560,7 @@ order_scatter_kernel(SpecSet S, const double* sn, const uint32_t* cls_count, uin
             it.a0 = S.off[s];
             it.na = (int32_t)(S.off[s + 1] - it.a0);
             it.a = (int32_t)s;
-            it.sn = sn[s];
-            it.rn = recip_norm(it.sn);
+            it.rn = recip_norm(sn[s]);
             c = length_class(it.na);
             rank = atomicAdd(&s_cnt[c], 1u);
         }
@@ -627,8 +642,11 @@ struct JoinParams {
     SpecSet A;  // sweeping side (one spectrum per work item)
     SpecSet B;  // indexed side (tiles)
     const SweepItem* items;  // sweeping spectra, largest length class first
+    const uint32_t* cls_count;  // their number per length class
     const Probe* probe;      // per sweeping peak: window and buckets
     const uint2* probe2;     // modified cosine: buckets of the shifted window
+    const double* w;         // per sweeping peak: its weight in the key
+    const double* snA;
     const double* snB;
     const double* rnB;
     const uint32_t* tab;
@@ -664,6 +682,12 @@ struct JoinParams {
     int sym;  // only pairs (reference i, query j) with i <= j
 };
 
+// Tile-stream entries a lane has in flight in a round, and pool slots when
+// owners are looked up.  Two entries are 3% faster where chunks have hundreds
+// (50000 x 50000 lognormal) and 5 to 20% slower where they have about 70 (1024 x
+// 1024 uniform, modified cosine); two slots are 1 to 3% faster everywhere.
+constexpr int kIlp = 1;
+constexpr int kIlpR = 2;
 constexpr int kSearchWaves = 4;            // waves of short-lived CTAs per library search
 constexpr int kSlotWords = 64;             // slot bitmap words of a bounded join launch
 constexpr int kPoolMax = 4096;             // candidates per sweep: smem pool + global extension
@@ -715,7 +739,8 @@ struct Pool {
 //                            stream offset, window, lane.  Resolution: uint16 queue
 //                            of chain heads with two or more candidates
 //   wa    double [32]        per-lane sweeping-peak weight of the current chunk
-//   runs  uint32 [kLongRuns] runs of 5..32 candidates queued for the warp:
+//                            Resolution: accepted keys of a long run in order
+//   runs  uint32 [kLongRuns] runs of five or more candidates queued for the warp:
 //                            slot of the chain head | length << 12; runs of at
 //                            most kMidRun from the front, longer ones from the back
 //   t0    uint64             %globaltimer at the current item's start (trace only)
@@ -735,6 +760,11 @@ __device__ __forceinline__ uint32_t gen_p1(uint32_t g) {
     return MODIFIED ? ((g >> 16) & 0x7FFFu) : (g >> 16);
 }
 
+// Kept out of line: the division's code would be in the join several times.
+__device__ __noinline__ float cosine_exact(double score, const double* nr, const double* nq) {
+    return (float)__ddiv_rn(score, __dmul_rn(*nr, *nq));
+}
+
 // float32 of score / (nr * nq) with both operations rounded in float64, as the
 // reference order has it, mostly without the division: rr and rq are the
 // norms' reciprocals (NaN when a norm is out of [1e-100, 1e100]), so
@@ -742,12 +772,12 @@ __device__ __forceinline__ uint32_t gen_p1(uint32_t g) {
 // values of both ends of a band of 2^-49 around it agree, the quotient rounds
 // to that value too.  Otherwise (about one in 10^7, zero norms and scores
 // below 1e-30) the quotient itself.
-__device__ __forceinline__ float cosine_of(double score, double rr, double rq, double nr,
+__device__ __forceinline__ float cosine_of(double score, double rr, double rq, const double* nr,
                                            const double* nq) {
     const double x = __dmul_rn(__dmul_rn(score, rr), rq);
     const float lo = (float)__dmul_rn(x, 1.0 - 0x1p-49), hi = (float)__dmul_rn(x, 1.0 + 0x1p-49);
     if (lo == hi && lo > 1e-30f) return lo;
-    return (float)__ddiv_rn(score, __dmul_rn(nr, *nq));
+    return cosine_exact(score, nr, nq);
 }
 
 // Bound by instruction issue and latency together (about 13 cycles between a
@@ -757,7 +787,9 @@ __device__ __forceinline__ float cosine_of(double score, double rr, double rq, d
 // buckets come ready-made per sweeping peak, item descriptors in order, a
 // pool entry is one 16-byte access, and owners of one candidate do not wait
 // for the code of longer runs (50000 x 50000: 11.45 ms with all of that done
-// per item, 9.9 ms now).
+// per item, 9.6 ms now).  The code is kept short, 45 KB instead of 126 KB:
+// modified cosine 13.2 -> 8.8 ms and 1024 x 1024 328 -> 272 us together with
+// the comparison instead of the sorting of long runs.
 // Three CTAs (24 warps) per SM: up to 80 registers a thread.
 template <bool A_IS_REF, bool SPARSE, bool MODIFIED>
 __global__ void __launch_bounds__(kJoinThreads, 3)
@@ -766,7 +798,7 @@ join_kernel(JoinParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int hb = head_bytes(P.g.tile);
     unsigned char* slice = smem_raw + (size_t)(threadIdx.x >> 5) * P.warp_smem_bytes;
-    uint32_t* head = reinterpret_cast<uint32_t*>(slice + 16 * kPool);
+    uint16_t* head = reinterpret_cast<uint16_t*>(slice + 16 * kPool);
     uint4* s_rec = reinterpret_cast<uint4*>(slice + 16 * kPool + hb);
     uint16_t* queue = reinterpret_cast<uint16_t*>(s_rec);
     double* s_wa = reinterpret_cast<double*>(slice + 16 * kPool + hb + 16 * 32);
@@ -824,6 +856,9 @@ join_kernel(JoinParams P) {
     // table; it is cleared once per 15 ranges (and before the first)
     unsigned epoch = 15;
 
+    int64_t n_large = 0;
+    if (!MODIFIED)
+        for (int c = kLargeClass; c < kOrderClasses; ++c) n_large += P.cls_count[c];
     // the next item's index is fetched while the current one is processed
     unsigned long long next = 0;
     if (lane == 0) next = atomicAdd(P.work, 1ull);
@@ -835,15 +870,24 @@ join_kernel(JoinParams P) {
         int t;
         SweepItem A;
         {
+            // large spectra over all tiles, then the others tile by tile
+            const bool small = (int64_t)item >= n_large * P.g.n_tiles;
+            const int64_t j = small ? (int64_t)item - n_large * P.g.n_tiles : (int64_t)item;
+            const int64_t m = small ? nA - n_large : n_large;
             int64_t ai;
             if (n_items <= 0xffffffffll) {
-                t = (int)((unsigned)item / (unsigned)nA);
-                ai = (unsigned)item - (unsigned)t * (unsigned)nA;
+                t = (int)((unsigned)j / (unsigned)m);
+                ai = (unsigned)j - (unsigned)t * (unsigned)m;
             } else {
-                t = (int)((int64_t)item / nA);
-                ai = (int64_t)item - (int64_t)t * nA;
+                t = (int)(j / m);
+                ai = j - (int64_t)t * m;
             }
-            A = P.items[ai];
+            const int4* it = reinterpret_cast<const int4*>(P.items + ai + (small ? n_large : 0));
+            const int4 x = __ldg(it);
+            A.a0 = ((int64_t)x.y << 32) | (unsigned)x.x;
+            A.a = x.z;
+            A.na = x.w;
+            A.rn = __ldg(reinterpret_cast<const double*>(it + 1));
         }
         if (P.trace.rec && lane == 0) *s_t0 = global_ns();
         const int a = A.a, na = A.na;
@@ -854,26 +898,25 @@ join_kernel(JoinParams P) {
         const uint32_t* T2 = MODIFIED ? P.tab2 + (int64_t)t * (P.g.nb + 1) : nullptr;
         // dense position of (this spectrum, query b_begin); the join's dense
         // output always has the sweeping spectrum as its row
-        const int64_t row = SPARSE ? 0 : (int64_t)a * P.dense.ld + b_begin;
+        auto row = [&]() { return SPARSE ? 0 : (int64_t)a * P.dense.ld + b_begin; };
         // a resolved run's score and count, for query q of the tile
         auto store_result = [&](int q, double score, int mt, double rnB) {
-            const double* nb = P.snB + b_begin + q;
-            const float sc = cosine_of(score, A.rn, rnB, A.sn, nb);
+            const float sc = cosine_of(score, A.rn, rnB, P.snA + a, P.snB + b_begin + q);
             if (SPARSE) {
                 if (sc >= P.sparse.threshold)
                     emit_hit(P.sparse, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a, sc,
                              mt, 0);
             } else {
-                __stcs(P.dense.score + row + q, sc);
-                __stcs(P.dense.matches + row + q, mt);
+                __stcs(P.dense.score + row() + q, sc);
+                __stcs(P.dense.matches + row() + q, mt);
             }
         };
         // a run for the pair kernel (its dense cells marked until then)
         auto spill_run = [&](int q) {
             spill_push(P.spill, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a, P.err);
             if (!SPARSE) {
-                __stcs(P.dense.score + row + q, __int_as_float(0x7fc00000));
-                __stcs(P.dense.matches + row + q, -1);
+                __stcs(P.dense.score + row() + q, __int_as_float(0x7fc00000));
+                __stcs(P.dense.matches + row() + q, -1);
             }
         };
 
@@ -919,33 +962,34 @@ join_kernel(JoinParams P) {
             int n = 0;  // candidates found (warp-uniform)
             constexpr int kPasses = MODIFIED ? 2 : 1;
             const int n_steps = ((na + 31) >> 5) * kPasses;
-            const Probe none{1.0f, 0.0f, kNoBucket, 0u};
-            Probe pr = none, pn = none;  // probes of this step's and the next chunk
+            // this step's probe (pr) and the next chunk's (pn)
+            Probe pr, pn;
+            uint2 pr2 = make_uint2(kNoBucket, 0u), pn2 = pr2;  // shifted pass: buckets, m/z
+            float mz_c = 0.f, mz_n = 0.f;
             double w_c = 0.0, w_n = 0.0;
-            auto load_peak = [&](int pp, Probe& x, double& w) {
-                x = none;
+            auto load_peak = [&](int pp, Probe& x, uint2& x2, float& mz, double& w) {
+                x = Probe{1.0f, 0.0f, kNoBucket, 0u};
+                if (MODIFIED) x2 = make_uint2(kNoBucket, 0u);
                 if (pp < na) {
                     const int4 v = __ldg(reinterpret_cast<const int4*>(P.probe + A.a0 + pp));
                     x = Probe{__int_as_float(v.x), __int_as_float(v.y), (uint32_t)v.z, (uint32_t)v.w};
-                    w = A_IS_REF ? __dmul_rn(peak_a(P.A.a, A.a0 + pp), P.A.b[A.a0 + pp])
-                                 : P.A.b[A.a0 + pp];
+                    w = __ldg(P.w + A.a0 + pp);
+                    if (MODIFIED) {
+                        x2 = __ldg(P.probe2 + A.a0 + pp);
+                        mz = __ldg(P.A.mz + A.a0 + pp);
+                    }
                 }
             };
             // raw bucket-table values: entries [t0, t1), and [0, t2) when wrapped
             auto table = [&](const uint32_t* TT, uint32_t bl, uint32_t bh, uint32_t& t0,
                              uint32_t& t1, uint32_t& t2) {
-                t0 = t1 = t2 = 0u;
-                if (bl == kNoBucket) return;
-                t0 = __ldg(&TT[bl]);
-                if (bl <= bh) {
-                    t1 = __ldg(&TT[bh + 1]);
-                } else {
-                    t1 = __ldg(&TT[P.g.nb]);
-                    t2 = __ldg(&TT[bh + 1]);
-                }
+                const bool some = bl != kNoBucket, wraps = some && bl > bh;
+                t0 = some ? __ldg(TT + bl) : 0u;
+                t1 = some ? __ldg(TT + (wraps ? (uint32_t)P.g.nb : bh + 1u)) : 0u;
+                t2 = wraps ? __ldg(TT + bh + 1u) : 0u;
             };
-            load_peak(lane, pr, w_c);
-            load_peak(32 + lane, pn, w_n);
+            load_peak(lane, pr, pr2, mz_c, w_c);
+            load_peak(32 + lane, pn, pn2, mz_n, w_n);
             uint32_t t0, t1, t2;
             table(T, pr.bl, pr.bh, t0, t1, t2);
             for (int st = 0; st < n_steps; ++st) {
@@ -953,19 +997,20 @@ join_kernel(JoinParams P) {
                 const int pc = (MODIFIED ? (st >> 1) : st) * 32;
                 const uint32_t r0 = t0, c0 = t1 - t0, c1 = t2;
                 // window of the record; the shifted pass tests with the peak's m/z
-                float x0 = pr.lo, x1 = pr.hi;
-                if (MODIFIED && pass) x0 = pc + lane < na ? __ldg(&P.A.mz[A.a0 + pc + lane]) : 0.f;
+                const float x0 = (MODIFIED && pass) ? mz_c : pr.lo, x1 = pr.hi;
                 if (pass == 0) s_wa[lane] = w_c;
                 // the next step's table values, in flight during this step's rounds
                 if (MODIFIED && pass == 0) {
-                    uint2 b2 = make_uint2(kNoBucket, 0u);
-                    if (pc + lane < na) b2 = __ldg(&P.probe2[A.a0 + pc + lane]);
-                    table(T2, b2.x, b2.y, t0, t1, t2);
+                    table(T2, pr2.x, pr2.y, t0, t1, t2);
                 } else {
                     pr = pn;
                     w_c = w_n;
+                    if (MODIFIED) {
+                        pr2 = pn2;
+                        mz_c = mz_n;
+                    }
                     table(T, pr.bl, pr.bh, t0, t1, t2);
-                    load_peak(pc + 64 + lane, pn, w_n);
+                    load_peak(pc + 64 + lane, pn, pn2, mz_n, w_n);
                 }
                 const Entry* EE = ((MODIFIED && pass) ? P.ent2 : P.ent) + tbase;
                 const double* EA = (MODIFIED && pass) ? P.ent2_a : P.ent_a;
@@ -987,78 +1032,123 @@ join_kernel(JoinParams P) {
                                        __float_as_uint(x1), (unsigned)lane);
                     __syncwarp();
                     int started = -1;  // records whose first entry lies before the round, minus 1
-                    for (uint32_t kb = 0; kb < E; kb += 32) {
-                        const uint32_t d = excl - kb;
-                        const unsigned first =
-                            __reduce_or_sync(full, (c != 0u && d < 32u) ? 1u << d : 0u);
-                        const int ri = started + __popc(first & upto);
-                        started += __popc(first);
-                        const uint32_t k = kb + (uint32_t)lane;
-                        bool cand = false;
-                        int o = 0, bq = 0, pB = 0;
-                        uint32_t pos = 0;
-                        double eb = 0.0;
-                        if (k < E) {
-                            const uint4 rec = s_rec[ri];
-                            pos = rec.x + k;
-                            const int4 v = __ldg(reinterpret_cast<const int4*>(EE + pos));
-                            const float mz = __int_as_float(v.x);
-                            o = (int)rec.w;
-                            bq = (int)((unsigned)v.y >> 16);
-                            pB = v.y & 0xFFFF;
-                            eb = __hiloint2double(v.w, v.z);
-                            cand = bq >= range_lo && bq < range_hi;
+#pragma unroll 1
+                    for (uint32_t kb = 0; kb < E; kb += 32 * kIlp) {
+                        // kIlp entries a lane, loaded before the first is tested
+                        uint4 rec[kIlp];
+                        int4 v[kIlp];
+                        double ea[kIlp];
+                        bool cand[kIlp];
+                        int slot[kIlp];
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            const uint32_t d = excl - (kb + 32u * u);
+                            const unsigned first =
+                                __reduce_or_sync(full, (c != 0u && d < 32u) ? 1u << d : 0u);
+                            const int ri = started + __popc(first & upto);
+                            started += __popc(first);
+                            const uint32_t k = kb + 32u * u + (uint32_t)lane;
+                            cand[u] = k < E;
+                            rec[u] = make_uint4(0u, 0u, 0u, 0u);
+                            v[u] = make_int4(0, 0, 0, 0);
+                            ea[u] = 1.0;
+                            if (k < E) {
+                                rec[u] = s_rec[ri];
+                                v[u] = __ldg(reinterpret_cast<const int4*>(EE + (rec[u].x + k)));
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            const int bq = (int)((unsigned)v[u].y >> 16);
+                            const float mz = __int_as_float(v[u].x);
+                            cand[u] = cand[u] && bq >= range_lo && bq < range_hi;
                             if (MODIFIED && pass) {
                                 // the shifted window exactly as matchms tests it:
                                 // mz2 = mz_q + (prec_ref - prec_q) against mz_ref -+ tol
-                                if (cand) {
+                                if (cand[u]) {
                                     const double mz2 = __dadd_rn(
                                         (double)mz, __dsub_rn(P.A.prec[a], P.B.prec[b_begin + bq]));
-                                    const double x = (double)__uint_as_float(rec.y);
-                                    cand = !(mz2 > __dadd_rn(x, P.tol)) && !(mz2 < __dsub_rn(x, P.tol));
+                                    const double x = (double)__uint_as_float(rec[u].y);
+                                    cand[u] = !(mz2 > __dadd_rn(x, P.tol)) &&
+                                              !(mz2 < __dsub_rn(x, P.tol));
                                 }
                             } else {
-                                cand = cand && mz >= __uint_as_float(rec.y) &&
-                                       mz <= __uint_as_float(rec.z);
+                                cand[u] = cand[u] && mz >= __uint_as_float(rec[u].y) &&
+                                          mz <= __uint_as_float(rec[u].z);
+                            }
+                            if (EA && cand[u])
+                                ea[u] = __ldg(EA + tbase + (rec[u].x + kb + 32u * u + lane));
+                        }
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            const unsigned bal = __ballot_sync(full, cand[u]);
+                            slot[u] = n + __popc(bal & below);
+                            n += __popc(bal);
+                            cand[u] = cand[u] && slot[u] < pool_max;
+                        }
+                        // push onto the queries' chains: the slot is written into its
+                        // query's 16-bit head and read back; where several lanes (or
+                        // entries) wrote the same head, those that do not find their
+                        // slot go again, behind the one that got in.  The head read
+                        // first, if of this epoch, is the chain's next element.
+                        unsigned ph[kIlp];
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            ph[u] = 0u;
+                            if (cand[u]) ph[u] = head[((unsigned)v[u].y >> 16) - range_lo];
+                        }
+                        __syncwarp();
+                        bool lost[kIlp];
+                        auto claim = [&](int u) {
+                            return (uint16_t)((epoch << 12) | (unsigned)slot[u]);
+                        };
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u)
+                            if (cand[u]) head[((unsigned)v[u].y >> 16) - range_lo] = claim(u);
+                        __syncwarp();
+                        bool any = false;
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            lost[u] = cand[u] && head[((unsigned)v[u].y >> 16) - range_lo] != claim(u);
+                            any = any || lost[u];
+                        }
+                        while (__any_sync(full, any)) {
+#pragma unroll
+                            for (int u = 0; u < kIlp; ++u)
+                                if (lost[u]) ph[u] = head[((unsigned)v[u].y >> 16) - range_lo];
+                            __syncwarp();
+#pragma unroll
+                            for (int u = 0; u < kIlp; ++u)
+                                if (lost[u]) head[((unsigned)v[u].y >> 16) - range_lo] = claim(u);
+                            __syncwarp();
+                            any = false;
+#pragma unroll
+                            for (int u = 0; u < kIlp; ++u) {
+                                lost[u] =
+                                    lost[u] && head[((unsigned)v[u].y >> 16) - range_lo] != claim(u);
+                                any = any || lost[u];
                             }
                         }
-                        const unsigned bal = __ballot_sync(full, cand);
-                        const int slot = n + __popc(bal & below);
-                        n += __popc(bal);
-                        if (cand && slot < pool_max) {
-                            const int pa = pc + o;
+#pragma unroll
+                        for (int u = 0; u < kIlp; ++u) {
+                            if (!cand[u]) continue;
+                            const int pB = v[u].y & 0xFFFF, pa = pc + (int)rec[u].w;
+                            const double eb = __hiloint2double(v[u].w, v[u].z), wa = s_wa[rec[u].w];
                             double key;
                             uint32_t gen;
                             if (A_IS_REF) {
-                                key = s_wa[o];
-                                if (EA) key = __dmul_rn(key, EA[tbase + pos]);
-                                key = __dmul_rn(key, eb);
+                                key = EA ? __dmul_rn(__dmul_rn(wa, ea[u]), eb) : __dmul_rn(wa, eb);
                                 gen = ((uint32_t)pa << 16) | (uint32_t)pB;
                                 if (MODIFIED) gen |= (uint32_t)pass << 31;
                             } else {
-                                key = eb;
-                                if (EA) key = __dmul_rn(EA[tbase + pos], eb);
+                                key = EA ? __dmul_rn(ea[u], eb) : eb;
                                 if (P.A.a) key = __dmul_rn(key, P.A.a[A.a0 + pa]);
-                                key = __dmul_rn(key, s_wa[o]);
+                                key = __dmul_rn(key, wa);
                                 gen = ((uint32_t)pB << 16) | (uint32_t)pa;
                             }
-                            // push onto the query's chain: swap the new slot into
-                            // its 16-bit head; the old head, if of this epoch, is
-                            // the chain's next element
-                            const int qr = bq - range_lo;
-                            uint32_t* hp = head + (qr >> 1);
-                            const unsigned sh = (unsigned)(qr & 1) * 16u;
-                            const unsigned nh = (epoch << 12) | (unsigned)slot;
-                            unsigned cur = *reinterpret_cast<volatile uint32_t*>(hp), assumed, ph;
-                            do {
-                                assumed = cur;
-                                ph = (assumed >> sh) & 0xFFFFu;
-                                cur = atomicCAS(hp, assumed,
-                                                (assumed & ~(0xFFFFu << sh)) | (nh << sh));
-                            } while (cur != assumed);
-                            uint32_t m = (uint32_t)qr;
-                            if ((ph >> 12) == epoch) m |= ((ph & 0xFFFu) << 12) | kHasNext;
-                            pool.put(slot, key, gen, m);
+                            uint32_t m = ((unsigned)v[u].y >> 16) - range_lo;
+                            if ((ph[u] >> 12) == epoch) m |= ((ph[u] & 0xFFFu) << 12) | kHasNext;
+                            pool.put(slot[u], key, gen, m);
                         }
                         if (n > pool_max) break;
                     }
@@ -1078,7 +1168,7 @@ join_kernel(JoinParams P) {
                 // a single pair has more candidates than the pool: pair kernel
                 if (lane == 0) {
                     spill_run(range_lo);
-                    if (!SPARSE) P.dense.overflow[row + range_lo] = 0;
+                    if (!SPARSE) P.dense.overflow[row() + range_lo] = 0;
                 }
                 __syncwarp();
                 range_lo = range_hi;
@@ -1096,7 +1186,7 @@ join_kernel(JoinParams P) {
             // lane and 16-byte streaming stores from the first aligned query on,
             // whatever the row's own alignment.
             if (!SPARSE) {
-                const int64_t r = row + range_lo;
+                const int64_t r = row() + range_lo;
                 auto zero1 = [&](int64_t o) {
                     __stcs(P.dense.score + o, 0.f);
                     __stcs(P.dense.matches + o, 0);
@@ -1131,245 +1221,245 @@ join_kernel(JoinParams P) {
             // every step), 5..32 go to a second queue resolved by the warp, and
             // longer runs (or runs reaching match_limit) to the pair kernel.
             int n_mid = 0, n_big = 0, n_queue = 0;
-            auto flush_long = [&]() {
-                __syncwarp();
-                // runs of 5..8 candidates, four at a time: each 8-lane segment
-                // sorts one run's (key, gen) descending in registers (bitonic),
-                // then resolves it greedily by segment-wise ballot
-                const int seg = lane >> 3, tq = lane & 7;
-                for (int r = 0; r < n_mid; r += 4) {
-                    const bool valid = r + seg < n_mid;
-                    const unsigned e = valid ? long_runs[r + seg] : 0u;
-                    const int s0 = (int)(e & 0xFFFu);
-                    const int L = valid ? (int)(e >> 12) : 0;
-                    double k = -INFINITY;
-                    uint32_t g = 0;
-                    int q = 0;
-                    if (tq < L) {
-                        int sl = s0;
-                        for (int h = 0; h < tq; ++h) sl = meta_next(pool.meta(sl));
-                        const PoolEntry x = pool.get(sl);
-                        k = x.key;
-                        g = x.gen;
-                        q = range_lo + meta_query(x.meta);
-                    }
-                    const double rnB = (valid && tq == 0) ? P.rnB[b_begin + q] : 0.0;
+            // Every queue is worked off at one place in the code, when it may not
+            // take another step's slots or nothing is left to come: copies of it
+            // wherever it is needed made three quarters of the kernel's code.
+#pragma unroll 1
+            for (int c = 0;; c += 32 * kIlpR) {
+                const bool last = c >= n;
+                if (!last) {
+                    // kIlpR slots a lane, their loads in flight together
+                    PoolEntry x[kIlpR];
+                    double rnB[kIlpR];
+                    bool own[kIlpR], more[kIlpR];
 #pragma unroll
-                    for (int kk = 2; kk <= kMidRun; kk <<= 1) {
+                    for (int u = 0; u < kIlpR; ++u) {
+                        const int sl = c + 32 * u + lane;
+                        own[u] = sl < n;
+                        x[u] = PoolEntry{0.0, 0u, 0u};
+                        if (own[u]) x[u] = pool.get(sl);
+                    }
 #pragma unroll
-                        for (int j = kk >> 1; j > 0; j >>= 1) {
-                            const double ok = __shfl_xor_sync(full, k, j);
-                            const uint32_t og = __shfl_xor_sync(full, g, j);
-                            const bool lower = (tq & j) == 0;
-                            const bool desc = (tq & kk) == 0;
-                            const bool mine_first = before(k, g, ok, og);
-                            const bool keep = (lower == desc) ? mine_first : !mine_first;
-                            if (!keep) {
-                                k = ok;
-                                g = og;
-                            }
-                        }
+                    for (int u = 0; u < kIlpR; ++u) {
+                        const int qr = meta_query(x[u].meta);
+                        own[u] = own[u] && (head[qr] & 0xFFFu) == (unsigned)(c + 32 * u + lane);
+                        more[u] = own[u] && ((x[u].meta & kHasNext) || P.match_limit <= 1);
+                        rnB[u] = 0.0;
+                        if (own[u] && !more[u]) rnB[u] = __ldg(P.rnB + b_begin + range_lo + qr);
                     }
-                    bool alive = tq < L;
-                    unsigned bal = __ballot_sync(full, alive);
-                    double score = 0.0;
-                    int mt = 0;
-                    while (bal) {
-                        const unsigned mine = (bal >> (seg * 8)) & 0xFFu;
-                        const int leader = mine ? seg * 8 + __ffs(mine) - 1 : lane;
-                        const uint32_t lg = __shfl_sync(full, g, leader);
-                        const double lk = __shfl_sync(full, k, leader);
-                        if (mine) {
-                            score = __dadd_rn(score, lk);
-                            ++mt;
-                            if (lane == leader || gen_p1<MODIFIED>(g) == gen_p1<MODIFIED>(lg) ||
-                                ((g & 0xFFFFu) == (lg & 0xFFFFu)))
-                                alive = false;
-                        }
-                        bal = __ballot_sync(full, alive);
+#pragma unroll
+                    for (int u = 0; u < kIlpR; ++u) {
+                        if (own[u] && !more[u])
+                            store_result(range_lo + meta_query(x[u].meta), x[u].key, 1, rnB[u]);
+                        const unsigned mb = __ballot_sync(full, more[u]);
+                        if (more[u])
+                            queue[n_queue + __popc(mb & below)] = (uint16_t)(c + 32 * u + lane);
+                        n_queue += __popc(mb);
                     }
-                    if (valid && tq == 0) store_result(q, score, mt, rnB);
                 }
-                // runs of 9..32 candidates, one at a time on the whole warp
-                for (int r = 0; r < n_big; ++r) {
-                    const unsigned e = long_runs[kLongRuns - 1 - r];
-                    const int s0 = (int)(e & 0xFFFu);
-                    const int L = (int)(e >> 12);
-                    double k = -INFINITY;
-                    uint32_t g = 0;
-                    int q = 0;
-                    if (lane < L) {
-                        int sl = s0;
-                        for (int h = 0; h < lane; ++h) sl = meta_next(pool.meta(sl));
-                        const PoolEntry x = pool.get(sl);
-                        k = x.key;
-                        g = x.gen;
-                        q = range_lo + meta_query(x.meta);
-                    }
-#pragma unroll
-                    for (int kk = 2; kk <= 32; kk <<= 1) {
-#pragma unroll
-                        for (int j = kk >> 1; j > 0; j >>= 1) {
-                            const double ok = __shfl_xor_sync(full, k, j);
-                            const uint32_t og = __shfl_xor_sync(full, g, j);
-                            const bool lower = (lane & j) == 0;
-                            const bool desc = (lane & kk) == 0;
-                            // the lower lane of a descending pair keeps the larger
-                            const bool mine_first = before(k, g, ok, og);
-                            const bool keep = (lower == desc) ? mine_first : !mine_first;
-                            if (!keep) {
-                                k = ok;
-                                g = og;
-                            }
-                        }
-                    }
-                    bool alive = lane < L;
-                    unsigned bal = __ballot_sync(full, alive);
-                    double score = 0.0;
-                    int mt = 0;
-                    while (bal) {
-                        const int leader = __ffs(bal) - 1;
-                        const uint32_t lg = __shfl_sync(full, g, leader);
-                        const double lk = __shfl_sync(full, k, leader);
-                        score = __dadd_rn(score, lk);
-                        ++mt;
-                        if (lane == leader || gen_p1<MODIFIED>(g) == gen_p1<MODIFIED>(lg) ||
-                            ((g & 0xFFFFu) == (lg & 0xFFFFu)))
-                            alive = false;
-                        bal = __ballot_sync(full, alive);
-                    }
-                    if (lane == 0) store_result(q, score, mt, P.rnB[b_begin + q]);
-                }
+                if (!last && n_queue <= kQueue - 32 * kIlpR) continue;
                 __syncwarp();
-                n_mid = 0;
-                n_big = 0;
-            };
-            auto flush_queue = [&]() {
-                __syncwarp();
-                for (int c = 0; c < n_queue; c += 32) {
-                    int L = 0, q = 0, s = 0;
-                    double rnB = 0.0;
-                    double k0 = 0.0, k1 = 0.0, k2 = -INFINITY, k3 = -INFINITY;
-                    uint32_t g0 = 0, g1 = 0, g2 = 0, g3 = 0;
-                    if (c + lane < n_queue) {
-                        s = queue[c + lane];
-                        PoolEntry x = pool.get(s);
-                        q = range_lo + meta_query(x.meta);
-                        rnB = P.rnB[b_begin + q];
-                        k0 = x.key;
-                        g0 = x.gen;
-                        x = pool.get(meta_next(x.meta));
-                        k1 = x.key;
-                        g1 = x.gen;
-                        L = 2;
-                        if (x.meta & kHasNext) {
-                            x = pool.get(meta_next(x.meta));
-                            k2 = x.key;
-                            g2 = x.gen;
-                            L = 3;
+#pragma unroll 1
+                for (int qc = 0;; qc += 32) {
+                    const bool qlast = qc >= n_queue;
+                    if (!qlast) {
+                        int L = 0, q = 0, s = 0;
+                        double rnB = 0.0;
+                        double k0 = 0.0, k1 = 0.0, k2 = -INFINITY, k3 = -INFINITY;
+                        uint32_t g0 = 0, g1 = 0, g2 = 0, g3 = 0;
+                        if (qc + lane < n_queue) {
+                            s = queue[qc + lane];
+                            PoolEntry x = pool.get(s);
+                            q = range_lo + meta_query(x.meta);
+                            rnB = __ldg(P.rnB + b_begin + q);
+                            k0 = x.key;
+                            g0 = x.gen;
+                            L = 1;
                             if (x.meta & kHasNext) {
                                 x = pool.get(meta_next(x.meta));
-                                k3 = x.key;
-                                g3 = x.gen;
-                                L = 4;
-                                // longer runs: count the rest (up to kLongRun + 1)
-                                uint32_t m = x.meta;
-                                while ((m & kHasNext) && L <= kLongRun) {
-                                    m = pool.meta(meta_next(m));
-                                    ++L;
+                                k1 = x.key;
+                                g1 = x.gen;
+                                L = 2;
+                                if (x.meta & kHasNext) {
+                                    x = pool.get(meta_next(x.meta));
+                                    k2 = x.key;
+                                    g2 = x.gen;
+                                    L = 3;
+                                    if (x.meta & kHasNext) {
+                                        x = pool.get(meta_next(x.meta));
+                                        k3 = x.key;
+                                        g3 = x.gen;
+                                        L = 4;
+                                        // longer runs: count on to kMidRun + 1
+                                        uint32_t m = x.meta;
+#pragma unroll 1
+                                        while ((m & kHasNext) && L <= kMidRun) {
+                                            m = pool.meta(meta_next(m));
+                                            ++L;
+                                        }
+                                    }
                                 }
                             }
                         }
+                        __syncwarp();
+                        const bool to_pair = L >= P.match_limit;
+                        const bool is_long = L > 4 && !to_pair;
+                        const bool is_mid = is_long && L <= kMidRun;
+                        const unsigned mb = __ballot_sync(full, is_mid);
+                        const unsigned bb = __ballot_sync(full, is_long && !is_mid);
+                        const unsigned run = (unsigned)s | ((unsigned)L << 12);
+                        if (is_mid)
+                            long_runs[n_mid + __popc(mb & below)] = run;
+                        else if (is_long)
+                            long_runs[kLongRuns - 1 - (n_big + __popc(bb & below))] = run;
+                        n_mid += __popc(mb);
+                        n_big += __popc(bb);
+                        if (to_pair) spill_run(q);
+                        if (L != 0 && !is_long && !to_pair) {
+                            // two to four candidates: sorting network (absent ones hold
+                            // -infinity and stay last), then greedy
+                            auto order = [](double& ka, uint32_t& ga, double& kb, uint32_t& gb) {
+                                if (before(kb, gb, ka, ga)) {
+                                    const double tk = ka;
+                                    ka = kb;
+                                    kb = tk;
+                                    const uint32_t tg = ga;
+                                    ga = gb;
+                                    gb = tg;
+                                }
+                            };
+                            auto clash = [](uint32_t ga, uint32_t gb) {
+                                return gen_p1<MODIFIED>(ga) == gen_p1<MODIFIED>(gb) || ((ga ^ gb) & 0xFFFFu) == 0u;
+                            };
+                            order(k0, g0, k1, g1);
+                            if (L > 2) {
+                                order(k2, g2, k3, g3);
+                                order(k0, g0, k2, g2);
+                                order(k1, g1, k3, g3);
+                                order(k1, g1, k2, g2);
+                            }
+                            double score = k0;
+                            int mt = 1;
+                            const bool take1 = !clash(g0, g1);
+                            if (take1) {
+                                score = __dadd_rn(score, k1);
+                                mt = 2;
+                            }
+                            if (L > 2) {
+                                const bool take2 = !clash(g0, g2) && !(take1 && clash(g1, g2));
+                                if (take2) {
+                                    score = __dadd_rn(score, k2);
+                                    ++mt;
+                                }
+                                if (L > 3 && !clash(g0, g3) && !(take1 && clash(g1, g3)) && !(take2 && clash(g2, g3))) {
+                                    score = __dadd_rn(score, k3);
+                                    ++mt;
+                                }
+                            }
+                            store_result(q, score, mt, rnB);
+                        }
                     }
-                    const bool to_pair = L >= P.match_limit || L > kLongRun;
-                    const bool is_long = L > 4 && !to_pair;
-                    const bool is_mid = is_long && L <= kMidRun;
-                    const unsigned mb = __ballot_sync(full, is_mid);
-                    const unsigned bb = __ballot_sync(full, is_long && !is_mid);
-                    if (n_mid + n_big + __popc(mb) + __popc(bb) > kLongRuns) flush_long();
-                    const unsigned run = (unsigned)s | ((unsigned)L << 12);
-                    if (is_mid)
-                        long_runs[n_mid + __popc(mb & below)] = run;
-                    else if (is_long)
-                        long_runs[kLongRuns - 1 - (n_big + __popc(bb & below))] = run;
-                    n_mid += __popc(mb);
-                    n_big += __popc(bb);
-                    if (to_pair) spill_run(q);
-                    if (L != 0 && !is_long && !to_pair) {
-                        // two to four candidates: sorting network (absent ones hold
-                        // -infinity and stay last), then greedy
-                        auto order = [](double& ka, uint32_t& ga, double& kb, uint32_t& gb) {
-                            if (before(kb, gb, ka, ga)) {
-                                const double tk = ka;
-                                ka = kb;
-                                kb = tk;
-                                const uint32_t tg = ga;
-                                ga = gb;
-                                gb = tg;
+                    if (n_mid + n_big > kLongRuns - 32 || (qlast && last)) {
+                        __syncwarp();
+                        // runs of 5..8 candidates, four at a time on 8-lane segments, then the longer
+                        // ones, one at a time on the whole warp; more than 32 candidates, or match_limit,
+                        // go to the pair kernel
+                        const int mids = (n_mid + 3) >> 2;
+#pragma unroll 1
+                        for (int r = 0; r < mids + n_big; ++r) {
+                            const bool mid = r < mids;
+                            double k = -INFINITY, rnB = 0.0;
+                            uint32_t g = 0;
+                            int q = 0, L = 0, at = -1;  // this lane's candidate
+                            if (mid) {
+                                const int i = 4 * r + (lane >> 3);
+                                const unsigned e = i < n_mid ? long_runs[i] : 0u;
+                                L = (int)(e >> 12);
+                                if ((lane & 7) < L) {
+                                    at = (int)(e & 0xFFFu);
+#pragma unroll 1
+                                    for (int h = 0; h < (lane & 7); ++h) at = meta_next(pool.meta(at));
+                                }
+                            } else {
+                                // lane i walks i steps; L is known when the walk ends
+                                at = (int)(long_runs[kLongRuns - 1 - (r - mids)] & 0xFFFu);
+                                uint32_t m = pool.meta(at);
+                                q = range_lo + meta_query(m);
+#pragma unroll 1
+                                for (int h = 0; h < lane && at >= 0; ++h) {
+                                    at = (m & kHasNext) ? meta_next(m) : -1;
+                                    if (at >= 0) m = pool.meta(at);
+                                }
+                                __syncwarp();
+                                L = __popc(__ballot_sync(full, at >= 0));
+                                if (__any_sync(full, lane == 31 && at >= 0 && (m & kHasNext)) ||
+                                    L >= P.match_limit) {
+                                    if (lane == 0) spill_run(q);
+                                    __syncwarp();
+                                    continue;
+                                }
                             }
-                        };
-                        auto clash = [](uint32_t ga, uint32_t gb) {
-                            return gen_p1<MODIFIED>(ga) == gen_p1<MODIFIED>(gb) ||
-                                   (ga & 0xFFFFu) == (gb & 0xFFFFu);
-                        };
-                        order(k0, g0, k1, g1);
-                        if (L > 2) {
-                            order(k2, g2, k3, g3);
-                            order(k0, g0, k2, g2);
-                            order(k1, g1, k3, g3);
-                            order(k1, g1, k2, g2);
-                        }
-                        double score = k0;
-                        int mt = 1;
-                        const bool take1 = !clash(g0, g1);
-                        if (take1) {
-                            score = __dadd_rn(score, k1);
-                            mt = 2;
-                        }
-                        if (L > 2) {
-                            const bool take2 = !clash(g0, g2) && !(take1 && clash(g1, g2));
-                            if (take2) {
-                                score = __dadd_rn(score, k2);
-                                ++mt;
+                            if (at >= 0) {
+                                const PoolEntry x = pool.get(at);
+                                k = x.key;
+                                g = x.gen;
+                                q = range_lo + meta_query(x.meta);
+                                rnB = __ldg(P.rnB + b_begin + q);
                             }
-                            if (L > 3 && !clash(g0, g3) && !(take1 && clash(g1, g3)) &&
-                                !(take2 && clash(g2, g3))) {
-                                score = __dadd_rn(score, k3);
-                                ++mt;
+                            __syncwarp();
+                            // Every lane compares its candidate with each of its run's, which yields
+                            // the mask of those that precede it in greedy order, and of those among
+                            // them that clash with it; lanes then decide as soon as every preceding
+                            // clashing lane has (the first always can), usually in two or three
+                            // rounds, and accepted keys are added in greedy order through s_wa.
+                            const int seg = mid ? 8 : 32, tq = lane & (seg - 1), sb = lane - tq;
+                            unsigned prec = 0u, clash = 0u;
+                            const int most = mid ? kMidRun : L;
+#pragma unroll 1
+                            for (int j = 0; j < most; j += 4) {
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    const int from = (sb + j + u) & 31;
+                                    const double ok = __shfl_sync(full, k, from);
+                                    const uint32_t og = __shfl_sync(full, g, from);
+                                    const bool p = j + u < L && before(ok, og, k, g);
+                                    const bool x = gen_p1<MODIFIED>(g) == gen_p1<MODIFIED>(og) ||
+                                                   ((g ^ og) & 0xFFFFu) == 0u;
+                                    prec |= p ? 1u << from : 0u;
+                                    clash |= p && x ? 1u << from : 0u;
+                                }
                             }
+                            unsigned dec = __ballot_sync(full, tq >= L), acc = 0u;
+#pragma unroll 1
+                            while (dec != full) {
+                                bool my_dec = (dec >> lane) & 1u, my_acc = (acc >> lane) & 1u;
+                                if (!my_dec && (clash & ~dec) == 0u) {
+                                    my_dec = true;
+                                    my_acc = (clash & acc) == 0u;
+                                }
+                                dec = __ballot_sync(full, my_dec);
+                                acc = __ballot_sync(full, my_acc);
+                            }
+                            if ((acc >> lane) & 1u) s_wa[sb + __popc(prec & acc)] = k;
+                            __syncwarp();
+                            if (L && tq == 0) {
+                                const int mt = __popc(mid ? (acc >> sb) & 0xFFu : acc);
+                                double score = 0.0;
+#pragma unroll 1
+                                for (int i = 0; i < mt; ++i) score = __dadd_rn(score, s_wa[sb + i]);
+                                store_result(q, score, mt, rnB);
+                            }
+                            __syncwarp();
                         }
-                        store_result(q, score, mt, rnB);
+                        n_mid = 0;
+                        n_big = 0;
                     }
-                    __syncwarp();
+                    if (qlast) break;
                 }
-                __syncwarp();
                 n_queue = 0;
-            };
-            for (int c = 0; c < n; c += 32) {
-                const int s = c + lane;
-                bool more = false;
-                if (s < n) {
-                    const PoolEntry x = pool.get(s);
-                    const int qr = meta_query(x.meta);
-                    const unsigned h = (head[qr >> 1] >> ((qr & 1) * 16)) & 0xFFFu;
-                    if (h == (unsigned)s) {
-                        more = (x.meta & kHasNext) != 0u;
-                        if (!more) {
-                            const int q = range_lo + qr;
-                            if (P.match_limit > 1)
-                                store_result(q, x.key, 1, P.rnB[b_begin + q]);
-                            else
-                                spill_run(q);
-                        }
-                    }
-                }
-                const unsigned mb = __ballot_sync(full, more);
-                if (n_queue + __popc(mb) > kQueue) flush_queue();
-                if (more) queue[n_queue + __popc(mb & below)] = (uint16_t)s;
-                n_queue += __popc(mb);
+                __syncwarp();
+                if (last) break;
             }
-            flush_queue();
-            flush_long();
             range_lo = range_hi;
             if (n < pool_max / 4) width = min(tn, width * 2);
         }
@@ -2296,6 +2386,8 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         need += bump_size((size_t)std::max<int64_t>(1, args.ref.n_peaks) * sizeof(Probe));
         if (args.modified)
             need += bump_size((size_t)std::max<int64_t>(1, args.ref.n_peaks) * sizeof(uint2));
+        if (args.ref.a)
+            need += bump_size((size_t)std::max<int64_t>(1, args.ref.n_peaks) * sizeof(double));
         const size_t idx = args.modified ? 2 : 1;  // m/z index, neutral-loss index
         need += bump_size(idx * (size_t)p.n_tiles * p.nb * sizeof(uint32_t));
         need += bump_size((size_t)p.n_tiles * scan_chunks(p.nb) * sizeof(uint32_t));
@@ -2342,6 +2434,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     double* rnQ = idx ? bp.take<double>(nQ) : nullptr;
     const size_t ref_peaks = (size_t)std::max<int64_t>(1, args.ref.n_peaks);
     Probe* probe = idx ? bp.take<Probe>(ref_peaks) : nullptr;
+    double* wR = idx && args.ref.a ? bp.take<double>(ref_peaks) : nullptr;
     uint2* probe2 = idx == 2 ? bp.take<uint2>(ref_peaks) : nullptr;
     double* snR = bp.take<double>(nR);
     double* snQ = bp.take<double>(nQ);
@@ -2353,9 +2446,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         StageScope sc(ctx, 0, 2, s);
         const int max_peaks = args.modified ? kModifiedMaxPeaks : CMS_MAX_PEAKS;
         const PrepSide pr{args.ref, snR,   nullptr, idx ? cls_count : nullptr, nullptr, nullptr,
-                          probe,    probe2, args.tol, args.shift, 1};
-        const PrepSide pq{args.qry, snQ,     rnQ, nullptr, cur, cur2,
-                          nullptr,  nullptr, 0.0, 0.0, 0};
+                          probe,    wR,    probe2, args.tol, args.shift, 1};
+        const PrepSide pq{args.qry, snQ, rnQ, nullptr, cur, cur2};
         prep_kernel<<<blocks_for(nR, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
             pr, g, bad, ctx->err_word, max_peaks);
         prep_kernel<<<blocks_for(nQ, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
@@ -2473,8 +2565,11 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     jp.items = items;
     jp.probe = probe;
     jp.probe2 = probe2;
+    jp.w = wR ? wR : args.ref.b;
+    jp.snA = snR;
     jp.snB = snQ;
     jp.rnB = rnQ;
+    jp.cls_count = cls_count;
     jp.tab = tab;
     jp.ent = ent;
     jp.ent_a = ent_a;
@@ -3159,8 +3254,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     {
         StageScope sc(ctx, 0, 1, s);
         prep_kernel<<<blocks_for(n_q, kPrepPerBlock, ctx->sm_count), kPrepThreads, 0, s>>>(
-            PrepSide{Q, snQ, nullptr, cls_count, nullptr, nullptr, probe, nullptr, lib->tol,
-                     lib->shift, 0},
+            PrepSide{Q, snQ, nullptr, cls_count, nullptr, nullptr, probe, nullptr, nullptr,
+                     lib->tol, lib->shift, 0},
             lib->g, bad, ctx->err_word,
             CMS_MAX_PEAKS);
     }
@@ -3178,8 +3273,11 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     jp.B = lib->spec;
     jp.items = sweep;
     jp.probe = probe;
+    jp.w = Q.b;
+    jp.snA = snQ;
     jp.snB = lib->sn;
     jp.rnB = lib->rn;
+    jp.cls_count = cls_count;
     jp.tab = lib->tab;
     jp.ent = lib->ent;
     jp.ent_a = lib->ent_a;
