@@ -9,10 +9,10 @@
 //                          or |r - q| / ((r + q) / 2) * 1e6 <= tolerance
 //                          (ppm), in IEEE float64 in that order of
 //                          operations.  Output: one byte (0/1) per pair.
-//                          Pure output bandwidth: a CTA takes a tile of 64
-//                          rows x 4096 columns, each thread 16 columns whose
-//                          query values stay in registers over the 64 rows,
-//                          one 16-byte store per row when the row is aligned.
+//                          Bound by the output's write: float32 bounds per row
+//                          decide all but the pairs within rounding of the
+//                          tolerance, and rows of any alignment are written in
+//                          16-byte stores.
 //   intersect_mz_kernel    IntersectMz: |set(mz_r) & set(mz_q)| / |set(mz_r)
 //                          | set(mz_q)| * scaling on the exact float64 m/z
 //                          values (0 when both are empty), through a hashed
@@ -23,6 +23,7 @@
 //                          scaling * inter / union in float64 for the whole
 //                          tile row.
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "cms_internal.cuh"
@@ -32,8 +33,7 @@ namespace {
 
 constexpr int kMassThreads = 256;
 constexpr int kMassCols = 16;                              // columns per thread
-constexpr int kMassTileCols = kMassThreads * kMassCols;    // 4096
-constexpr int kMassTileRows = 64;
+constexpr int kMassWarpCols = 32 * kMassCols;              // 512
 constexpr int kIxThreads = 256;
 
 __device__ __forceinline__ bool mass_ok(double r, double q, double tol, int ppm) {
@@ -44,36 +44,226 @@ __device__ __forceinline__ bool mass_ok(double r, double q, double tol, int ppm)
     return __dmul_rn(__ddiv_rn(d, mean), 1e6) <= tol;
 }
 
-__global__ void __launch_bounds__(kMassThreads) mass_match_kernel(const double* __restrict__ ref,
-                                                                  int64_t n_ref,
-                                                                  const double* __restrict__ q,
-                                                                  int64_t n_q, double tol, int ppm,
-                                                                  uint8_t* __restrict__ out,
-                                                                  int64_t ld, int vec) {
-    const int64_t col_tiles = (n_q + kMassTileCols - 1) / kMassTileCols;
-    const int64_t tiles = col_tiles * ((n_ref + kMassTileRows - 1) / kMassTileRows);
-    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int64_t rt = t / col_tiles, ct = t - rt * col_tiles;
-        const int64_t j0 = ct * kMassTileCols + (int64_t)threadIdx.x * kMassCols;
-        const int64_t i0 = rt * kMassTileRows, i1 = min(n_ref, i0 + kMassTileRows);
-        if (j0 >= n_q) continue;
-        const int nc = (int)min((int64_t)kMassCols, n_q - j0);
-        double qv[kMassCols];
+// The float32 bounds of one row's matches in ppm.  In exact arithmetic the
+// matching q > 0 of a row r > 0 form an interval; rounding blurs its ends by far
+// less than the margin below, so with x = float32(q), rounded to nearest,
+//   x < out_lo or x > out_hi:  no match;   x > in_lo and x < in_hi:  a match
+// (rounding is monotone, and a float32 strictly above in_lo comes from a q
+// above in_lo); what lies between is tested as the definition says.  Rows the
+// argument does not hold for (r not positive or extreme; a tolerance above 5e5,
+// where the ratio's bound of 2e6 gets near) take every column that way, and so
+// do negative q, whose mean may be negative.  mid and half describe [out_lo,
+// out_hi] once more, rounded outwards far enough that float32(|x - mid|) <= half
+// for every x inside.
+struct MassRow {
+    float mid, half, out_lo, out_hi;
+    float in_lo, in_hi, pad0, pad1;
+};
+__device__ __forceinline__ MassRow mass_row(double r, double tol) {
+    MassRow w{0.0f, INFINITY, -INFINITY, INFINITY, INFINITY, -INFINITY, 0.0f, 0.0f};
+    if (!(tol >= 0.0 && tol <= 5e5 && r >= 1e-150 && r <= 1e150)) return w;
+    const double h = tol * 0.5e-6, m = r * 4e-15;
+    const double lo = r * (1.0 - h) / (1.0 + h), hi = r * (1.0 + h) / (1.0 - h);
+    w.out_lo = __double2float_rd(lo - m);
+    w.out_hi = __double2float_ru(hi + m);
+    w.in_lo = __double2float_ru(lo + m);
+    w.in_hi = __double2float_rd(hi - m);
+    if (w.out_hi < 1e30f) {
+        w.mid = __double2float_rn(0.5 * ((double)w.out_lo + (double)w.out_hi));
+        const double up = (double)w.out_hi - (double)w.mid, down = (double)w.mid - (double)w.out_lo;
+        w.half = __double2float_ru(fmax(up, down) * (1.0 + 0x1p-20) + 1e-30);
+    }
+    return w;
+}
+
+// One pair, from the row's bounds or, between them, as defined.
+__device__ __forceinline__ bool ppm_ok(const double* r, const double* q, const MassRow& w, double tol) {
+    const double v = *q;
+    const float f = __double2float_rn(v);
+    if (f > w.in_lo && f < w.in_hi && !(v < 0.0)) return true;
+    if (!(f >= w.out_lo && f <= w.out_hi) && !(v < 0.0)) return false;
+    return mass_ok(*r, v, tol, 1);
+}
+
+// two float32 sums in one instruction
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+// bits 0..3 of m as the bytes of a word
+__device__ __forceinline__ uint32_t nibble_bytes(uint32_t m) {
+    return ((m & 0xFu) * 0x00204081u) & 0x01010101u;
+}
+
+// Writes 32 lanes' 16-bit masks (any: ballot of those that may be nonzero) as 512
+// bytes at row..row + 511, `mine` being this lane's first byte: aligned 16-byte
+// stores whatever the row's alignment, a lane's piece shifted together with its
+// neighbour's, and the 16 bytes left at the two ends of the 512 one by one.
+__device__ __forceinline__ void store_masks(uint8_t* mine, int lane, uint32_t mask, unsigned any) {
+    const unsigned full = 0xffffffffu;
+    const int sh = (int)(-(uintptr_t)mine & 15);  // bytes up to the next boundary
+    uint4 piece = make_uint4(0u, 0u, 0u, 0u);
+    if (any) {
+        const uint32_t next = __shfl_down_sync(full, mask, 1);
+        const uint32_t m = ((mask | (next << 16)) >> sh) & 0xFFFFu;
+        piece = make_uint4(nibble_bytes(m), nibble_bytes(m >> 4), nibble_bytes(m >> 8),
+                           nibble_bytes(m >> 12));
+    }
+    if (sh == 0) {
+        __stcs(reinterpret_cast<uint4*>(mine), piece);
+        return;
+    }
+    if (lane < 31) __stcs(reinterpret_cast<uint4*>(mine + sh), piece);
+    const uint32_t end = __shfl_sync(full, mask, lane < sh ? 0 : 31);
+    uint8_t* row = mine - 16 * lane;
+    if (lane < 16)
+        row[lane < sh ? lane : kMassWarpCols - 16 + lane] = (uint8_t)((end >> lane) & 1u);
+}
+
+// The last columns of a row, 32 bytes at a time.
+__device__ __forceinline__ void store_tail(uint8_t* row, int lane, uint32_t mask, int cols) {
+    for (int k = 0; k < cols; k += 32) {
+        const uint32_t m = __shfl_sync(0xffffffffu, mask, (k + lane) >> 4);
+        if (k + lane < cols) row[k + lane] = (uint8_t)((m >> (lane & 15)) & 1u);
+    }
+}
+
+// A warp takes `rows` rows x 512 columns, 16 consecutive columns a lane.
+//
+// Dalton: the columns' float64 values stay in registers, a subtraction and a
+// compare per pair; bound by the write (40000 x 50000: 406 us, 75% of the copy
+// rate; 49999 columns 566 us, where a store per byte took 5960 us).
+//
+// ppm: a float64 division per pair took 2240 us, seven times the write.  Most
+// rows match none of a warp's columns; the smallest float32 |x - mid| of a
+// lane's columns (one and a half instructions per pair) shows it, and zeros go
+// out.  A few lanes that may have a match are looked at by half a warp each, a
+// column a lane; many at once make their masks themselves.  420 us (49999
+// columns: 487 us, 6030 us with a store per byte).
+template <bool PPM>
+__global__ void __launch_bounds__(kMassThreads, 3)
+mass_match_kernel(const double* __restrict__ ref, int64_t n_ref, const double* __restrict__ q,
+                  int64_t n_q, double tol, uint8_t* __restrict__ out, int64_t ld, int rows) {
+    __shared__ __align__(16) MassRow s_row[kMassThreads / 32][32];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t col_blocks = (n_q + kMassWarpCols - 1) / kMassWarpCols;
+    const int64_t units = col_blocks * ((n_ref + rows - 1) / rows);
+    const int64_t warps = (int64_t)gridDim.x * (kMassThreads / 32);
+    MassRow* const bounds = s_row[threadIdx.x >> 5];
+    for (int64_t t = (int64_t)blockIdx.x * (kMassThreads / 32) + (threadIdx.x >> 5); t < units;
+         t += warps) {
+        const int64_t rb = t / col_blocks, c0 = (t - rb * col_blocks) * kMassWarpCols;
+        const int cols = (int)min((int64_t)kMassWarpCols, n_q - c0);
+        const double* const qc = q + c0;  // this warp's columns
+        const double* rp = ref + rb * rows;
+        int left = (int)min((int64_t)rows, n_ref - rb * rows);
+        uint8_t* mine = out + rb * rows * ld + c0 + kMassCols * lane;
+        if (!PPM) {
+            double v[kMassCols];
 #pragma unroll
-        for (int k = 0; k < kMassCols; ++k) qv[k] = k < nc ? q[j0 + k] : 0.0;
-        for (int64_t i = i0; i < i1; ++i) {
-            const double r = ref[i];
-            uint8_t* o = out + i * ld + j0;
-            if (vec && nc == kMassCols) {
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
+            for (int k = 0; k < kMassCols; ++k)
+                v[k] = kMassCols * lane + k < cols ? qc[kMassCols * lane + k]
+                                                   : __longlong_as_double(0x7ff8000000000000ll);
+            if (cols == kMassWarpCols && ((ld | (int64_t)(uintptr_t)out) & 15) == 0) {
+                // aligned rows: bytes straight into their words
+                for (; left; --left, ++rp, mine += ld) {
+                    const double r = *rp;
+                    uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                    for (int k = 0; k < kMassCols; ++k)
+                        w[k >> 2] |= (uint32_t)mass_ok(r, v[k], tol, 0) << (8 * (k & 3));
+                    __stcs(reinterpret_cast<uint4*>(mine), make_uint4(w[0], w[1], w[2], w[3]));
+                }
+                continue;
+            }
+            for (; left; --left, ++rp, mine += ld) {
+                const double r = *rp;
+                uint32_t mask = 0u;
 #pragma unroll
                 for (int k = 0; k < kMassCols; ++k)
-                    w[k >> 2] |= (uint32_t)mass_ok(r, qv[k], tol, ppm) << (8 * (k & 3));
-                __stcs(reinterpret_cast<uint4*>(o), make_uint4(w[0], w[1], w[2], w[3]));
-            } else {
+                    if (mass_ok(r, v[k], tol, 0)) mask |= 1u << k;
+                if (cols == kMassWarpCols)
+                    store_masks(mine, lane, mask, 1u);
+                else
+                    store_tail(mine - kMassCols * lane, lane, mask, cols);
+            }
+            continue;
+        }
+        float2 x[kMassCols / 2];
+        uint32_t odd = 0u;
 #pragma unroll
-                for (int k = 0; k < kMassCols; ++k)
-                    if (k < nc) o[k] = (uint8_t)mass_ok(r, qv[k], tol, ppm);
+        for (int k = 0; k < kMassCols; ++k) {
+            const double v = kMassCols * lane + k < cols ? qc[kMassCols * lane + k]
+                                                         : __longlong_as_double(0x7ff8000000000000ll);
+            (k & 1 ? x[k / 2].y : x[k / 2].x) = __double2float_rn(v);
+            odd |= (v < 0.0 ? 1u : 0u) << k;
+            if ((k & 3) == 3) asm volatile("" ::: "memory");  // four loads in flight, not sixteen
+        }
+        for (; left > 0; left -= 32, rp += 32) {
+            const int nr = min(32, left);
+            __syncwarp();
+            if (lane < nr) bounds[lane] = mass_row(rp[lane], tol);
+            __syncwarp();
+#pragma unroll 1
+            for (int rr = 0; rr < nr; ++rr, mine += ld) {
+                float a = INFINITY, b = INFINITY;  // a NaN (past the end) never is least
+                {
+                    const float2 w = *reinterpret_cast<const float2*>(&bounds[rr]);
+                    const float2 neg = make_float2(-w.x, -w.x);
+#pragma unroll
+                    for (int k = 0; k < kMassCols / 2; ++k) {
+                        const float2 d = add2(x[k], neg);
+                        a = fminf(a, fabsf(d.x));
+                        b = fminf(b, fabsf(d.y));
+                    }
+                    a = fminf(a, b);
+                    b = w.y;
+                }
+                const unsigned any = __ballot_sync(full, a <= b || odd != 0u);
+                uint32_t mask = 0u;
+                if (any) {
+                    if (__popc(any) <= 4) {
+                        // half a warp for each of the lanes, a column a lane
+                        for (unsigned m = any; m;) {
+                            const int l0 = __ffs(m) - 1;
+                            m &= m - 1u;
+                            const int l1 = m ? __ffs(m) - 1 : -1;
+                            m &= m - 1u;
+                            const int l = lane < 16 ? l0 : l1, j = 16 * l + (lane & 15);
+                            const bool ok = l >= 0 && j < cols && ppm_ok(rp + rr, qc + j, bounds[rr], tol);
+                            const unsigned hit = __ballot_sync(full, ok);
+                            if (lane == l0) mask = hit & 0xFFFFu;
+                            if (lane == l1) mask = hit >> 16;
+                        }
+                    } else {
+                        if ((any >> lane) & 1u) {
+                            uint32_t rest = odd;
+                            const MassRow& w = bounds[rr];
+#pragma unroll
+                            for (int k = 0; k < kMassCols; ++k) {
+                                const float v = k & 1 ? x[k / 2].y : x[k / 2].x;
+                                if (v >= w.out_lo && v <= w.out_hi) rest |= 1u << k;
+                                if (v > w.in_lo && v < w.in_hi) mask |= 1u << k;
+                            }
+                            mask &= ~odd;
+                            for (rest &= ~mask; rest; rest &= rest - 1u) {
+                                const int k = __ffs(rest) - 1;
+                                if (ppm_ok(rp + rr, qc + kMassCols * lane + k, w, tol)) mask |= 1u << k;
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (cols == kMassWarpCols)
+                    store_masks(mine, lane, mask, any);
+                else
+                    store_tail(mine - kMassCols * lane, lane, mask, cols);
             }
         }
     }
@@ -320,14 +510,24 @@ extern "C" int cms_mass_match(const double* ref, int64_t n_ref, const double* q,
         set_error("cms_mass_match: null pointer");
         return CMS_ERR_INVALID;
     }
-    const int vec = (ld % 16 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-    const int64_t tiles = ((n_q + kMassTileCols - 1) / kMassTileCols) *
-                          ((n_ref + kMassTileRows - 1) / kMassTileRows);
+    // Rows a warp takes: 128, so that its columns are loaded once for 64 KB of
+    // output (64: 2% slower, 32: 20%), or fewer where that leaves less than four
+    // units a resident warp.  Ten CTAs per resident one, so that the last wave is
+    // short (one per resident: 572 us instead of 420 for 40000 x 50000 in ppm).
+    const int64_t sms = sm_count_of_current(), col_blocks = (n_q + kMassWarpCols - 1) / kMassWarpCols;
+    int rows = 128;
+    while (rows > 4 && col_blocks * ((n_ref + rows - 1) / rows) < sms * 24 * 4) rows /= 2;
+    const int64_t units = col_blocks * ((n_ref + rows - 1) / rows);
+    const int per_block = kMassThreads / 32;
     const int grid = (int)std::max<int64_t>(
-        1, std::min<int64_t>(tiles, (int64_t)sm_count_of_current() * 8));
-    mass_match_kernel<<<grid, kMassThreads, 0, (cudaStream_t)stream>>>(ref, n_ref, q, n_q,
-                                                                       tolerance, ppm, out, ld,
-                                                                       vec);
+        1, std::min<int64_t>((units + per_block - 1) / per_block, sms * 30));
+    cudaStream_t s = (cudaStream_t)stream;
+    if (ppm)
+        mass_match_kernel<true><<<grid, kMassThreads, 0, s>>>(ref, n_ref, q, n_q, tolerance, out, ld,
+                                                              rows);
+    else
+        mass_match_kernel<false><<<grid, kMassThreads, 0, s>>>(ref, n_ref, q, n_q, tolerance, out,
+                                                               ld, rows);
     CMS_CUDA_TRY(cudaGetLastError());
     return CMS_OK;
 }

@@ -132,3 +132,37 @@ def test_classes(cuda_device):
     sym = CudaIntersectMz().matrix(refs, refs, is_symmetric=True)
     np.testing.assert_array_equal(sym, sym.T)
     np.testing.assert_array_equal(sym, other.intersect_mz(mzs[0], mzs[0]))
+
+
+@pytest.mark.parametrize("n_q", [31, 511, 512, 513, 1040, 2051])
+@pytest.mark.parametrize("ppm,tol", [(False, 0.1), (False, 0.0), (False, 300.0), (False, 1e301),
+                                     (True, 10.0), (True, 0.0), (True, 4e5), (True, 3e6)])
+def test_mass_match_bounds(cuda_device, n_q, ppm, tol):
+    """Row bounds against the definition: values at the tolerance and a few float64
+    steps around it, negative, zero, infinite, NaN and extreme values, at the edges of
+    a warp's 512 columns, rows of every alignment."""
+    import torch
+
+    from cudams import kernels
+
+    rng = np.random.default_rng(n_q)
+    r = rng.uniform(100.0, 1000.0, 67)
+    r[3:12] = [np.nan, np.inf, -np.inf, 0.0, -250.0, 1e-300, 1e200, 1e301, -1e301]
+    q = rng.uniform(50.0, 1200.0, n_q)
+    at = rng.integers(12, 67, n_q)
+    with np.errstate(all="ignore"):
+        edge = r[at] * ((1 + 0.5e-6 * tol) / (1 - 0.5e-6 * tol)) if ppm else r[at] + tol
+    step = rng.integers(-3, 4, n_q)
+    for _ in range(3):
+        edge = np.where(step > 0, np.nextafter(edge, np.inf),
+                        np.where(step < 0, np.nextafter(edge, -np.inf), edge))
+        step -= np.sign(step)
+    q = np.where(rng.random(n_q) < 0.5, edge, q)
+    q[5:16] = [np.nan, np.inf, -np.inf, 0.0, -400.0, -1e-3, 1e-300, 1e200, 1e301, -1e301, r[20]]
+    got = kernels.mass_match_matrix(torch.from_numpy(r).to(_dev()),
+                                    torch.from_numpy(q).to(_dev()), tol, ppm).cpu().numpy()
+    with np.errstate(all="ignore"):  # the oracle's expressions on whole rows (0 / 0 is NaN)
+        d = np.abs(r[:, None] - q[None, :])
+        mean = (r[:, None] + q[None, :]) / 2
+        want = d / mean * 1e6 <= tol if ppm else d <= tol
+    np.testing.assert_array_equal(got.astype(bool), want)
