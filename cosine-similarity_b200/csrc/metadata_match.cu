@@ -17,14 +17,15 @@
 //                          | set(mz_q)| * scaling on the exact float64 m/z
 //                          values (0 when both are empty), through a hashed
 //                          index of the queries' distinct values: per
-//                          (reference, 8192-query tile) the reference's
-//                          distinct values find their (value, query) entries
-//                          and count them per query in shared memory; then
-//                          scaling * inter / union in float64 for the whole
-//                          tile row.
+//                          (reference, query tile) the reference's distinct
+//                          values find their (value, query) entries and count
+//                          them per query in shared memory; the tile's row is
+//                          filled, and scaling * inter / union in float64 is
+//                          stored for the queries that share a value.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <mutex>
 
 #include "cms_internal.cuh"
 
@@ -34,7 +35,10 @@ namespace {
 constexpr int kMassThreads = 256;
 constexpr int kMassCols = 16;                              // columns per thread
 constexpr int kMassWarpCols = 32 * kMassCols;              // 512
-constexpr int kIxThreads = 256;
+// Queries per CTA pass: 54 KB of counters and list, four CTAs of 512 threads a
+// multiprocessor (10007 x 9000 in one pass 308 us, in two of 4504 338 us; 12000 x
+// 12000 in two of 6000 486 us, in one of 12000 503 us).
+constexpr int kIxMaxTile = 9216;
 
 __device__ __forceinline__ bool mass_ok(double r, double q, double tol, int ppm) {
     const double d = fabs(__dsub_rn(r, q));
@@ -283,12 +287,10 @@ __device__ __forceinline__ void spectrum_range(const int64_t* off, int64_t i, in
 // ---- IntersectMz through an index of the queries' distinct m/z values ----
 // Pairs sharing a value are few against R x Q, so instead of merging every
 // pair's peak lists, the queries' distinct (value, query) entries are hashed
-// into buckets (count, scan, scatter), and each (reference, query tile) CTA
-// walks the buckets of its reference's distinct values, counting shared
-// values per query in shared memory, then writes the tile's dense row.
-constexpr int kIxTile = 8192;  // queries per CTA pass (32 KB of counters)
-
-struct IxEntry {
+// into buckets (count, two-launch scan, scatter), and each (reference, query
+// tile) CTA walks the buckets of its reference's distinct values, counting
+// shared values per query in shared memory, then writes the tile's dense row.
+struct __align__(16) IxEntry {
     double v;
     uint32_t q;
     uint32_t pad;
@@ -306,7 +308,9 @@ __device__ __forceinline__ uint32_t ix_bucket(double v, uint32_t mask) {
 
 // one warp per query spectrum: its distinct values (sorted peaks: a value
 // differing from its predecessor) counted per bucket (SCATTER = false) or
-// placed (SCATTER = true); ub[j] = distinct values of query j
+// placed (SCATTER = true); ub[j] = distinct values of query j.  kIxUnroll
+// chunks of 32 peaks have their loads and atomics in flight together.
+constexpr int kIxUnroll = 4;
 template <bool SCATTER>
 __global__ void ix_index_kernel(const double* __restrict__ qmz, const int64_t* __restrict__ qoff,
                                 int64_t n_q, int64_t n_q_peaks, uint32_t mask, uint32_t* cnt_cur,
@@ -317,36 +321,66 @@ __global__ void ix_index_kernel(const double* __restrict__ qmz, const int64_t* _
         int64_t b0, b1;
         spectrum_range(qoff, j, n_q_peaks, b0, b1, (!SCATTER && lane == 0) ? err : nullptr);
         uint32_t distinct = 0;
-        for (int64_t k = b0 + lane; k < b1; k += 32) {
-            const double v = qmz[k];
-            if (k > b0 && qmz[k - 1] == v) continue;
-            ++distinct;
-            const uint32_t h = ix_bucket(v, mask);
+        for (int64_t k0 = b0 + lane; k0 < b1; k0 += 32 * kIxUnroll) {
+            double v[kIxUnroll], before[kIxUnroll];
+            uint32_t pos[kIxUnroll];
+            bool take[kIxUnroll];
+#pragma unroll
+            for (int u = 0; u < kIxUnroll; ++u) {
+                const int64_t k = k0 + 32 * u;
+                v[u] = k < b1 ? qmz[k] : 0.0;
+                before[u] = k < b1 && k > b0 ? qmz[k - 1] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kIxUnroll; ++u) {
+                const int64_t k = k0 + 32 * u;
+                take[u] = k < b1 && !(k > b0 && before[u] == v[u]);
+                if (!take[u]) continue;
+                ++distinct;
+                uint32_t* c = &cnt_cur[ix_bucket(v[u], mask)];
+                if (SCATTER)
+                    pos[u] = atomicAdd(c, 1u);
+                else
+                    atomicAdd(c, 1u);
+            }
             if (SCATTER) {
-                const uint32_t pos = atomicAdd(&cnt_cur[h], 1u);
-                ent[pos] = IxEntry{v, (uint32_t)j, 0u};
-            } else {
-                atomicAdd(&cnt_cur[h], 1u);
+#pragma unroll
+                for (int u = 0; u < kIxUnroll; ++u)
+                    if (take[u])
+                        *reinterpret_cast<uint4*>(&ent[pos[u]]) =
+                            make_uint4((uint32_t)__double2loint(v[u]),
+                                       (uint32_t)__double2hiint(v[u]), (uint32_t)j, 0u);
             }
         }
         if (!SCATTER) {
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) distinct += __shfl_xor_sync(0xffffffffu, distinct, d);
+            distinct = __reduce_add_sync(0xffffffffu, distinct);
             if (lane == 0) ub[j] = distinct;
         }
     }
 }
 
 // Exclusive scan of the bucket counts into tab[0..nb] (cnt_cur becomes the
-// scatter cursor), in three coalesced passes over chunks of kScanChunk
-// buckets: chunk sums, a scan of the sums (one CTA), the chunks' own scans.
-constexpr int kScanThreads = 1024;
-constexpr int kScanPer = 8;
-constexpr int kScanChunk = kScanThreads * kScanPer;  // 8192 buckets
+// scatter cursor): chunk sums, then every chunk's own scan on top of the sums
+// of the chunks before it, both with coalesced accesses.
+constexpr int kScanThreads = 256;
+constexpr int kScanPer = 16;
+constexpr int kScanChunk = kScanThreads * kScanPer;  // 4096 buckets; divides every bucket count
 
-// block-wide exclusive scan of one value per thread; *total gets the sum
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* warp_sums,
-                                                    uint32_t* total) {
+// sum over the block; the same value for every thread
+__device__ __forceinline__ uint32_t block_total(uint32_t x, uint32_t* s_warp) {
+    x = __reduce_add_sync(0xffffffffu, x);
+    __syncthreads();  // s_warp free from an earlier use
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = x;
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) total += s_warp[w];
+    return total;
+}
+
+// exclusive scan over the block of one value per thread
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* s_warp) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t incl = x;
 #pragma unroll
@@ -354,134 +388,155 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* warp_s
         const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += v;
     }
-    __syncthreads();  // warp_sums free from an earlier use
-    if (lane == 31) warp_sums[wid] = incl;
+    __syncthreads();  // s_warp free from an earlier use
+    if (lane == 31) s_warp[wid] = incl;
     __syncthreads();
-    if (wid == 0) {
-        uint32_t v = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0u;
+    uint32_t run = incl - x;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
-            if (lane >= d) v += u;
-        }
-        if (lane < (int)(blockDim.x >> 5)) warp_sums[lane] = v;
-    }
-    __syncthreads();
-    if (total) *total = warp_sums[(blockDim.x >> 5) - 1];
-    return incl - x + (wid > 0 ? warp_sums[wid - 1] : 0u);
+    for (int w = 0; w < THREADS / 32; ++w)
+        if (w < wid) run += s_warp[w];
+    return run;
 }
 
-__global__ void __launch_bounds__(kScanThreads) ix_chunk_sums(const uint32_t* cnt, uint32_t nb,
-                                                              uint32_t* sums) {
-    const uint32_t c0 = blockIdx.x * (uint32_t)kScanChunk;
+__global__ void __launch_bounds__(kScanThreads) ix_chunk_sums(const uint32_t* cnt, uint32_t* sums) {
+    __shared__ uint32_t s_warp[kScanThreads / 32];
+    const uint32_t* c = cnt + (size_t)blockIdx.x * kScanChunk;
     uint32_t x = 0;
 #pragma unroll
-    for (int r = 0; r < kScanPer; ++r) {
-        const uint32_t k = c0 + r * kScanThreads + threadIdx.x;
-        if (k < nb) x += cnt[k];
-    }
-    __shared__ uint32_t ws[32];
-    uint32_t total;
-    block_excl_scan(x, ws, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-// exclusive scan of the chunk sums in place (n_chunks <= kScanChunk), and
-// tab[nb] = the grand total
-__global__ void __launch_bounds__(kScanThreads) ix_scan_sums(uint32_t* sums, int n_chunks,
-                                                             uint32_t* tab, uint32_t nb) {
-    uint32_t v[kScanPer], x = 0;
-#pragma unroll
-    for (int r = 0; r < kScanPer; ++r) {
-        const int k = threadIdx.x * kScanPer + r;
-        v[r] = k < n_chunks ? sums[k] : 0u;
-        x += v[r];
-    }
-    __shared__ uint32_t ws[32];
-    uint32_t total;
-    uint32_t run = block_excl_scan(x, ws, &total);
-#pragma unroll
-    for (int r = 0; r < kScanPer; ++r) {
-        const int k = threadIdx.x * kScanPer + r;
-        if (k < n_chunks) sums[k] = run;
-        run += v[r];
-    }
-    if (threadIdx.x == 0) tab[nb] = total;
+    for (int r = 0; r < kScanPer; ++r) x += c[r * kScanThreads + threadIdx.x];
+    x = block_total(x, s_warp);
+    if (threadIdx.x == 0) sums[blockIdx.x] = x;
 }
 
 __global__ void __launch_bounds__(kScanThreads) ix_chunk_scan(uint32_t* cnt_cur, uint32_t* tab,
-                                                              uint32_t nb,
-                                                              const uint32_t* chunk_base) {
-    const uint32_t k0 = blockIdx.x * (uint32_t)kScanChunk + threadIdx.x * kScanPer;
-    uint32_t v[kScanPer], x = 0;
+                                                              const uint32_t* sums) {
+    __shared__ uint32_t s_val[kScanChunk + kScanThreads];
+    __shared__ uint32_t s_warp[kScanThreads / 32];
+    const int tid = threadIdx.x;
+    uint32_t* c = cnt_cur + (size_t)blockIdx.x * kScanChunk;
+    uint32_t* out = tab + (size_t)blockIdx.x * kScanChunk;
+    // coalesced in, kScanPer consecutive buckets a thread out of shared memory
+    // (a word of padding per kScanPer)
 #pragma unroll
     for (int r = 0; r < kScanPer; ++r) {
-        v[r] = k0 + r < nb ? cnt_cur[k0 + r] : 0u;
-        x += v[r];
+        const int k = r * kScanThreads + tid;
+        s_val[k + k / kScanPer] = c[k];
     }
-    __shared__ uint32_t ws[32];
-    uint32_t run = chunk_base[blockIdx.x] + block_excl_scan(x, ws, nullptr);
+    uint32_t prev = 0;
+    for (int i = tid; i < (int)blockIdx.x; i += kScanThreads) prev += sums[i];
+    prev = block_total(prev, s_warp);
+    uint32_t x = 0;
+#pragma unroll
+    for (int r = 0; r < kScanPer; ++r) x += s_val[tid * (kScanPer + 1) + r];
+    uint32_t run = prev + block_excl_scan<kScanThreads>(x, s_warp);
 #pragma unroll
     for (int r = 0; r < kScanPer; ++r) {
-        if (k0 + r < nb) {
-            tab[k0 + r] = run;
-            cnt_cur[k0 + r] = run;
-        }
-        run += v[r];
+        const uint32_t v = s_val[tid * (kScanPer + 1) + r];
+        s_val[tid * (kScanPer + 1) + r] = run;
+        run += v;
     }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kScanPer; ++r) {
+        const int k = r * kScanThreads + tid;
+        const uint32_t v = s_val[k + k / kScanPer];
+        out[k] = v;
+        c[k] = v;
+    }
+    if (blockIdx.x == gridDim.x - 1 && tid == kScanThreads - 1) out[kScanChunk] = run;
 }
 
-__global__ void __launch_bounds__(kIxThreads) intersect_mz_kernel(
+// One CTA per (reference, tile of `tile` queries).  256 reference values at a
+// time look up their buckets; the buckets' entries, laid end to end, are taken
+// one a thread (owner by binary search over the running counts), so a value
+// that every query has costs no more than its entries.  Counts live in shared
+// memory between references: a query's first hit puts it on a list, the row is
+// filled with the score of no shared value by 16-byte stores, and only the
+// list's queries get a division, their score over the fill, and their counter
+// back to zero.  10007 x 9000, index and all: 308 us (the row write alone: 110
+// us; what is left is the latency of a unit's dependent lookups).  Clearing and
+// scanning 8192 counters per unit, with a float64 division for each query, took
+// 850 us.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) intersect_mz_kernel(
     const double* __restrict__ rmz, const int64_t* __restrict__ roff, int64_t n_ref,
     int64_t n_ref_peaks, int64_t n_q, const uint32_t* __restrict__ tab,
     const IxEntry* __restrict__ ent, const uint32_t* __restrict__ ub, uint32_t mask,
-    double scaling, double* __restrict__ out, int64_t ld, uint32_t* err) {
-    __shared__ uint32_t s_cnt[kIxTile];
-    __shared__ uint32_t s_ua[kIxThreads / 32];
-    const int64_t tiles = (n_q + kIxTile - 1) / kIxTile;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double scaling, double* __restrict__ out, int64_t ld, int tile, uint32_t* err) {
+    extern __shared__ uint32_t s_cnt[];                              // [tile]
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(s_cnt + tile);    // [tile]
+    __shared__ uint32_t s_warp[THREADS / 32];
+    __shared__ uint32_t s_end[THREADS];  // running entry counts of the values
+    __shared__ uint32_t s_first[THREADS];
+    __shared__ double s_v[THREADS];
+    __shared__ unsigned int s_n;
+    const int64_t tiles = (n_q + tile - 1) / tile;
+    const int tid = threadIdx.x;
+    for (int k = tid; k < tile; k += THREADS) s_cnt[k] = 0u;
+    if (tid == 0) s_n = 0u;
+    const double none = __dmul_rn(scaling, 0.0);
     for (int64_t u = blockIdx.x; u < n_ref * tiles; u += gridDim.x) {
-        const int64_t i = u / tiles, j0 = (u - i * tiles) * kIxTile;
-        const int tw = (int)min((int64_t)kIxTile, n_q - j0);
-        __syncthreads();  // the previous unit's readers are done with s_cnt
-        for (int k = threadIdx.x; k < tw; k += blockDim.x) s_cnt[k] = 0u;
-        __syncthreads();
+        const int64_t i = u / tiles, j0 = (u - i * tiles) * tile;
+        const int tw = (int)min((int64_t)tile, n_q - j0);
         int64_t a0, a1;
-        spectrum_range(roff, i, n_ref_peaks, a0, a1,
-                       (threadIdx.x == 0 && j0 == 0) ? err : nullptr);
-        // four threads per distinct reference value, each walking every
-        // fourth entry of its bucket with two loads in flight
-        uint32_t distinct = 0;
-        const int sub = threadIdx.x & 3;
-        for (int64_t k = a0 + (threadIdx.x >> 2); k < a1; k += kIxThreads / 4) {
-            const double v = rmz[k];
-            if (k > a0 && rmz[k - 1] == v) continue;
-            if (sub == 0) ++distinct;
-            const uint32_t h = ix_bucket(v, mask);
-            const uint32_t e1 = tab[h + 1];
-            for (uint32_t e = tab[h] + sub; e < e1; e += 8) {
-                const IxEntry x0 = ent[e];
-                const bool two = e + 4 < e1;
-                IxEntry x1 = x0;
-                if (two) x1 = ent[e + 4];
-                const int64_t c0 = (int64_t)x0.q - j0, c1 = (int64_t)x1.q - j0;
-                if (x0.v == v && c0 >= 0 && c0 < tw) atomicAdd(&s_cnt[c0], 1u);
-                if (two && x1.v == v && c1 >= 0 && c1 < tw) atomicAdd(&s_cnt[c1], 1u);
+        spectrum_range(roff, i, n_ref_peaks, a0, a1, (tid == 0 && j0 == 0) ? err : nullptr);
+        uint32_t ua = 0;  // distinct reference values
+        for (int64_t k0 = a0; k0 < a1; k0 += THREADS) {
+            const int64_t k = k0 + tid;
+            double v = 0.0;
+            bool take = false;
+            if (k < a1) {
+                v = rmz[k];
+                take = !(k > a0 && rmz[k - 1] == v);
             }
+            uint32_t e0 = 0, c = 0;
+            if (take) {
+                const uint32_t h = ix_bucket(v, mask);
+                e0 = tab[h];
+                c = tab[h + 1] - e0;
+            }
+            const uint32_t excl = block_excl_scan<THREADS>(c, s_warp);
+            s_end[tid] = excl + c;
+            s_first[tid] = e0 - excl;
+            s_v[tid] = v;
+            ua += __syncthreads_count(take);
+            const uint32_t total = s_end[THREADS - 1];
+            for (uint32_t e = tid; e < total; e += THREADS) {
+                int o = 0;  // values whose entries end at or before e
+#pragma unroll
+                for (int step = THREADS / 2; step > 0; step >>= 1)
+                    if (s_end[o + step - 1] <= e) o += step;
+                const uint4 x = __ldg(reinterpret_cast<const uint4*>(ent + (s_first[o] + e)));
+                const int64_t q = (int64_t)x.z - j0;
+                if (__hiloint2double((int)x.y, (int)x.x) == s_v[o] && q >= 0 && q < tw &&
+                    atomicAdd(&s_cnt[q], 1u) == 0u)
+                    s_list[atomicAdd(&s_n, 1u)] = (uint16_t)q;
+            }
+            __syncthreads();
         }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) distinct += __shfl_xor_sync(0xffffffffu, distinct, d);
-        if (lane == 0) s_ua[wid] = distinct;
-        __syncthreads();
-        uint32_t ua = 0;
-#pragma unroll
-        for (int w = 0; w < kIxThreads / 32; ++w) ua += s_ua[w];
+        // the row's fill: no shared value (and 0 for two empty spectra)
         double* orow = out + i * ld + j0;
-        for (int k = threadIdx.x; k < tw; k += blockDim.x) {
-            const uint32_t inter = s_cnt[k];
-            const uint32_t uni = ua + ub[j0 + k] - inter;
-            orow[k] = uni == 0u ? 0.0 : __ddiv_rn(__dmul_rn(scaling, (double)inter), (double)uni);
+        if (ua != 0u) {
+            const int pre = min(tw, (int)(((uintptr_t)orow >> 3) & 1));
+            if (tid < pre) orow[tid] = none;
+            const int nv = (tw - pre) >> 1;
+            for (int k = tid; k < nv; k += THREADS)
+                __stcs(reinterpret_cast<double2*>(orow + pre) + k, make_double2(none, none));
+            if (tid < ((tw - pre) & 1)) orow[tw - 1] = none;
+        } else {
+            for (int k = tid; k < tw; k += THREADS) orow[k] = ub[j0 + k] ? none : 0.0;
         }
+        __syncthreads();
+        const unsigned int n = s_n;
+        for (unsigned int k = tid; k < n; k += THREADS) {
+            const int q = s_list[k];
+            const uint32_t inter = s_cnt[q];
+            s_cnt[q] = 0u;
+            orow[q] = __ddiv_rn(__dmul_rn(scaling, (double)inter),
+                                (double)(ua + ub[j0 + q] - inter));
+        }
+        __syncthreads();
+        if (tid == 0) s_n = 0u;
     }
 }
 
@@ -493,6 +548,49 @@ int sm_count_of_current() {
         sms = 148;
     }
     return sms;
+}
+
+// Stream-ordered workspace from a pool of the library's own, one per device,
+// which keeps up to kKeepBytes between calls (the device's default pool gives
+// everything back at each synchronisation: 0.5 ms a call at 10007 x 9000); what
+// is above is returned to the device when a stream is synchronised.  The pool
+// orders reuse between streams and threads itself.
+constexpr uint64_t kKeepBytes = 128ull << 20;
+constexpr int kMaxDevices = 64;
+
+int workspace_alloc(unsigned char** p, size_t bytes, cudaStream_t s) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    int dev = 0;
+    CMS_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) {
+        set_error("device ordinal %d out of range", dev);
+        return CMS_ERR_UNSUPPORTED;
+    }
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.handleTypes = cudaMemHandleTypeNone;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t made;
+            CMS_CUDA_TRY(cudaMemPoolCreate(&made, &props));
+            uint64_t keep = kKeepBytes;
+            const cudaError_t e =
+                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                cudaMemPoolDestroy(made);
+                return cuda_fail(e, "cudaMemPoolSetAttribute");
+            }
+            pools[dev] = made;
+        }
+        pool = pools[dev];
+    }
+    CMS_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, s));
+    return CMS_OK;
 }
 
 }  // namespace
@@ -548,46 +646,52 @@ extern "C" int cms_intersect_mz(const double* ref_mz, const int64_t* ref_off, in
         return CMS_ERR_INVALID;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    // buckets: a power of two >= twice the query peaks (load <= 1/2), 2^26 at most
-    uint32_t nb = 1024;
-    while (nb < (uint64_t)2 * (uint64_t)n_q_peaks && nb < (1u << 26)) nb <<= 1;
+    // buckets: a power of two >= the query peaks, 2^26 at most
+    uint32_t nb = kScanChunk;
+    while (nb < (uint64_t)n_q_peaks && nb < (1u << 26)) nb <<= 1;
     const int sms = sm_count_of_current();
-    uint32_t *cnt = nullptr, *tab = nullptr, *ub = nullptr, *sums = nullptr;
-    IxEntry* ent = nullptr;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&cnt), (size_t)nb * 4, s);
-    if (e == cudaSuccess)
-        e = cudaMallocAsync(reinterpret_cast<void**>(&sums),
-                            (size_t)((nb + kScanChunk - 1) / kScanChunk) * 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&tab), ((size_t)nb + 1) * 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&ub), (size_t)n_q * 4, s);
-    if (e == cudaSuccess)
-        e = cudaMallocAsync(reinterpret_cast<void**>(&ent),
-                            (size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(IxEntry), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, (size_t)nb * 4, s);
-    if (e == cudaSuccess) {
+    const int chunks = (int)(nb / kScanChunk);
+    // one workspace: entries, bucket counts, bucket table, distinct counts, chunk sums
+    const size_t ent_bytes = (size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(IxEntry);
+    const size_t words = (size_t)nb * 2 + 1 + (size_t)n_q + (size_t)chunks;
+    unsigned char* ws = nullptr;
+    if (const int rc = workspace_alloc(&ws, ent_bytes + words * 4, s)) return rc;
+    IxEntry* ent = reinterpret_cast<IxEntry*>(ws);
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(ws + ent_bytes);
+    uint32_t* tab = cnt + nb;
+    uint32_t* ub = tab + nb + 1;
+    uint32_t* sums = ub + n_q;
+    // query tile: the queries split evenly over the fewest tiles of at most
+    // kIxMaxTile (six bytes of shared memory a query)
+    const int64_t tiles = (n_q + kIxMaxTile - 1) / kIxMaxTile;
+    const int tile = (int)(((n_q + tiles - 1) / tiles + 7) & ~int64_t(7));
+    const size_t smem = (size_t)tile * 6;
+    // 512 threads for long rows, 256 where a row is soon filled
+    auto* kern = tile > 2048 ? intersect_mz_kernel<512> : intersect_mz_kernel<256>;
+    const int threads = tile > 2048 ? 512 : 256;
+    int rc = raise_func_smem(reinterpret_cast<const void*>(kern), smem);
+    cudaError_t e = cudaSuccess;
+    if (!rc) e = cudaMemsetAsync(cnt, 0, (size_t)nb * 4, s);
+    if (!rc && e == cudaSuccess) {
         const int igrid = (int)std::max<int64_t>(
             1, std::min<int64_t>((n_q * 32 + 255) / 256, (int64_t)sms * 16));
         ix_index_kernel<false><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt,
                                                      nullptr, ub, device_error);
-        const int n_chunks = (int)((nb + kScanChunk - 1) / kScanChunk);
-        ix_chunk_sums<<<n_chunks, kScanThreads, 0, s>>>(cnt, nb, sums);
-        ix_scan_sums<<<1, kScanThreads, 0, s>>>(sums, n_chunks, tab, nb);
-        ix_chunk_scan<<<n_chunks, kScanThreads, 0, s>>>(cnt, tab, nb, sums);
+        ix_chunk_sums<<<chunks, kScanThreads, 0, s>>>(cnt, sums);
+        ix_chunk_scan<<<chunks, kScanThreads, 0, s>>>(cnt, tab, sums);
         ix_index_kernel<true><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt, ent,
                                                     nullptr, nullptr);
-        const int64_t units = n_ref * ((n_q + kIxTile - 1) / kIxTile);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)sms * 8));
-        intersect_mz_kernel<<<grid, kIxThreads, 0, s>>>(ref_mz, ref_off, n_ref, n_ref_peaks, n_q,
-                                                        tab, ent, ub, nb - 1, scaling, out, ld,
-                                                        device_error);
+        const int64_t units = n_ref * ((n_q + tile - 1) / tile);
+        int per_sm = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+        per_sm = std::max(1, per_sm);
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)sms * per_sm));
+        kern<<<grid, threads, smem, s>>>(ref_mz, ref_off, n_ref, n_ref_peaks, n_q, tab, ent, ub,
+                                         nb - 1, scaling, out, ld, tile, device_error);
         e = cudaGetLastError();
     }
-    // stream-ordered frees: after the kernels above
-    if (ent) cudaFreeAsync(ent, s);
-    if (ub) cudaFreeAsync(ub, s);
-    if (tab) cudaFreeAsync(tab, s);
-    if (cnt) cudaFreeAsync(cnt, s);
-    if (sums) cudaFreeAsync(sums, s);
+    cudaFreeAsync(ws, s);  // stream-ordered: after the kernels above
+    if (rc) return rc;
     CMS_CUDA_TRY(e);
     return CMS_OK;
 }

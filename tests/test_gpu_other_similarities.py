@@ -166,3 +166,24 @@ def test_mass_match_bounds(cuda_device, n_q, ppm, tol):
         mean = (r[:, None] + q[None, :]) / 2
         want = d / mean * 1e6 <= tol if ppm else d <= tol
     np.testing.assert_array_equal(got.astype(bool), want)
+
+
+@pytest.mark.parametrize("scaling", [1.0, -2.5])
+@pytest.mark.parametrize("n_q", [1, 2047, 2049, 9216, 9217])
+def test_intersect_mz_tiles(cuda_device, n_q, scaling):
+    """Query tile edges, a value that every query has, references of more values than
+    a CTA has threads, empty spectra on both sides, rows of both alignments."""
+    from cudams import kernels
+
+    rng = np.random.default_rng(n_q)
+    pool = np.concatenate([[100.25], rng.uniform(101.0, 500.0, 3000)])
+    b = [np.sort(np.concatenate([[100.25], rng.choice(pool, size=int(rng.integers(0, 6)))]))
+         for _ in range(n_q)]
+    if n_q > 3:
+        b[n_q - 2] = np.zeros(0)
+    a = [np.sort(rng.choice(pool, size=k, replace=False)) for k in (1, 40, 511, 513, 1100)]
+    a += [np.zeros(0), np.array([100.25]), np.array([100.25, 100.25, 900.0])]
+    got = kernels.intersect_mz_matrix(*_csr(a), *_csr(b), scaling,
+                                      check_errors=True).cpu().numpy()
+    want = other.intersect_mz(a, b, scaling)
+    np.testing.assert_array_equal(got.view(np.uint64), want.view(np.uint64))
