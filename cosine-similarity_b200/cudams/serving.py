@@ -159,7 +159,7 @@ class SpectrumLibrary:
                 cap = n
             host = [b[:n].cpu().numpy() for b in bufs]
         r, qq, sc, mt, ov = host
-        o = np.lexsort((r, qq))
+        o = np.argsort((qq.astype(np.int64) << 32) | r)  # by query, then library spectrum
         return SearchResult(r[o], qq[o], sc[o], mt[o], ov[o], q.n, self.n,
                             latency_s=time.perf_counter() - t0)
 

@@ -135,8 +135,10 @@ class CudaCosineGreedy(BaseSimilarity):
 
         budget = self.max_device_bytes
         if budget is None:
-            free, _ = torch.cuda.mem_get_info(dev)
-            budget = max(1 << 28, free // 4)
+            budget = 1 << 28  # at least this much whatever is free
+            if n_ref * n_q * _BYTES_PER_PAIR > budget:
+                free, _ = torch.cuda.mem_get_info(dev)
+                budget = max(budget, free // 4)
         rows = max(1, int(budget // max(1, n_q * _BYTES_PER_PAIR)))
         return max(min(n_ref, rows), min(n_ref, int(self.batch_size or 1)))
 
