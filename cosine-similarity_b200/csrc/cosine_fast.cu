@@ -45,7 +45,8 @@
 //                        match_limit truncation, bitonic sort of (key, gen)
 //                        (in registers when there are eight candidates a
 //                        thread, else in shared memory), warp greedy with
-//                        per-chunk conflict masks and used-peak bitmasks.
+//                        used-peak bitmasks and conflict masks over the live
+//                        candidates.
 //   6. mirror_kernel     (symmetric dense calls, csrc/mirror.cu) lower
 //                        triangle copied from the upper one.
 #include <algorithm>
@@ -1620,49 +1621,113 @@ __device__ void sort8_block(unsigned long long* okey, uint32_t* cgen, int m, int
     sync();
 }
 
+constexpr int kGenPeaks = 2;  // reference peaks a thread takes per chunk
+constexpr int kGenIlp = 4;    // candidates a thread has in flight while their keys are made
+
+// Shared scratch of gen_pair: its chunk's reference peak weights, and (cache > 0)
+// the query's first `cache` m/z values.
+struct GenScratch {
+    double* w;     // [kGenPeaks * threads]
+    float* qmz;    // [cache]
+    int cache;
+};
+__host__ __device__ constexpr size_t gen_scratch_bytes(int threads, int cache) {
+    return (size_t)threads * 8 * kGenPeaks + (size_t)cache * 4;
+}
+__device__ __forceinline__ GenScratch gen_scratch(void* p, int threads, int cache) {
+    GenScratch g;
+    g.w = reinterpret_cast<double*>(p);
+    g.qmz = reinterpret_cast<float*>(g.w + kGenPeaks * threads);
+    g.cache = cache;
+    return g;
+}
+
 // Candidates of pair (ri, qi) in generation order, truncated at match_limit,
 // into okey/cgen, by nt threads (tid 0..nt-1, whole warps) with barrier
 // `sync`; s_scan holds one int per warp.  Returns the number generated
 // before truncation stopped it (>= match_limit means overflow).
+//
+// A thread takes a reference peak and finds its window by binary search, in a
+// shared-memory copy of the query's m/z where it fits (eleven dependent reads:
+// from L2 they were most of the time).  It writes its candidates' generation
+// words; the keys are then made one rank a thread, so that the weight loads are
+// independent and no thread waits for one with more candidates.
 template <bool MODIFIED, typename Sync>
 __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned long long* okey,
-                        uint32_t* cgen, int nt, int tid, int* s_scan, Sync sync) {
+                        uint32_t* cgen, int nt, int tid, int* s_scan, const GenScratch& G,
+                        Sync sync) {
     const int lane = tid & 31, wid = tid >> 5, nwarps = nt >> 5;
     const unsigned full = 0xffffffffu;
     const int64_t r0 = P.R.off[ri], q0 = P.Q.off[qi];
     const int nr = (int)(P.R.off[ri + 1] - r0), nq = (int)(P.Q.off[qi + 1] - q0);
     const float* qmz = P.Q.mz + q0;
+    if (nr == 0 || nq == 0) return 0;
+    if (nq <= G.cache) {
+        for (int i = tid; i < nq; i += nt) G.qmz[i] = qmz[i];
+        qmz = G.qmz;
+        sync();
+    }
     int total = 0;
     bool overflow = false;
     // modified cosine generates twice: at shift 0, then at the pair's
     // precursor difference, continuing the same candidate list
 #pragma unroll 1
-    for (int pass = 0; pass < (MODIFIED ? 2 : 1) && !overflow && nr > 0 && nq > 0; ++pass) {
+    for (int pass = 0; pass < (MODIFIED ? 2 : 1) && !overflow; ++pass) {
         const double shift = (MODIFIED && pass) ? __dsub_rn(P.R.prec[ri], P.Q.prec[qi]) : P.shift;
-        for (int pc = 0; pc < nr && !overflow; pc += nt) {
-            const int p1 = pc + tid;
-            int start = 0, cnt = 0;
-            double lo = 0.0, hi = 0.0, w1 = 0.0;
-            if (p1 < nr) {
-                const double mz1 = (double)P.R.mz[r0 + p1];
-                lo = __dsub_rn(mz1, P.tol);
-                hi = __dadd_rn(mz1, P.tol);
-                // first p2 with mz_q + shift >= lo
-                int L = 0, H = nq;
-                while (L < H) {
-                    const int M = (L + H) >> 1;
-                    if (__dadd_rn((double)qmz[M], shift) < lo)
-                        L = M + 1;
-                    else
-                        H = M;
-                }
-                start = L;
-                int k = L;
-                while (k < nq && !(__dadd_rn((double)qmz[k], shift) > hi)) ++k;
-                cnt = k - L;
+#pragma unroll 1
+        for (int pc = 0; pc < nr && !overflow; pc += kGenPeaks * nt) {
+            // kGenPeaks consecutive peaks a thread: a pair that overflows is usually
+            // done after one chunk of 256
+            int start[kGenPeaks], cnt[kGenPeaks], mine = 0;
+            float mz[kGenPeaks];
+#pragma unroll
+            for (int u = 0; u < kGenPeaks; ++u) {
+                const int p1 = pc + kGenPeaks * tid + u;
+                mz[u] = p1 < nr ? P.R.mz[r0 + p1] : 0.f;
             }
-            // exclusive scan of cnt over the nt threads
-            int incl = cnt;
+#pragma unroll
+            for (int u = 0; u < kGenPeaks; ++u) {
+                const int p1 = pc + kGenPeaks * tid + u;
+                start[u] = cnt[u] = 0;
+                if (p1 < nr) {
+                    const double mz1 = (double)mz[u];
+                    // the window as float32 bounds of the query's m/z (exact, see
+                    // Window): first p2 at or above, then on to the last one inside
+                    float wl, wh;
+                    const bool ok = shift == 0.0
+                                        ? Window<true, true>::bounds(mz[u], P.tol, shift, wl, wh)
+                                        : Window<true, false>::bounds(mz[u], P.tol, shift, wl, wh);
+                    int L = 0, H = nq;
+                    if (ok) {
+                        while (L < H) {
+                            const int M = (L + H) >> 1;
+                            if (qmz[M] < wl)
+                                L = M + 1;
+                            else
+                                H = M;
+                        }
+                        start[u] = L;
+                        while (L < nq && qmz[L] <= wh) ++L;
+                    } else {  // not finite: as the definition tests it
+                        const double lo = __dsub_rn(mz1, P.tol), hi = __dadd_rn(mz1, P.tol);
+                        while (L < H) {
+                            const int M = (L + H) >> 1;
+                            if (__dadd_rn((double)qmz[M], shift) < lo)
+                                L = M + 1;
+                            else
+                                H = M;
+                        }
+                        start[u] = L;
+                        while (L < nq && !(__dadd_rn((double)qmz[L], shift) > hi)) ++L;
+                    }
+                    cnt[u] = L - start[u];
+                    if (cnt[u])
+                        G.w[kGenPeaks * tid + u] = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
+                }
+                mine += cnt[u];
+            }
+            // exclusive scan of the counts over the nt threads
+            int incl = mine;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const int v = __shfl_up_sync(full, incl, d);
@@ -1670,28 +1735,42 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
             }
             if (lane == 31) s_scan[wid] = incl;
             sync();
-            if (wid == 0) {
-                int v = lane < nwarps ? s_scan[lane] : 0;
+            int chunk_total = 0, first = incl - mine;
+            for (int w = 0; w < nwarps; ++w) {
+                const int x = s_scan[w];
+                if (w < wid) first += x;
+                chunk_total += x;
+            }
+            const int take = min(chunk_total, P.match_limit - total);
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int u = __shfl_up_sync(full, v, d);
-                    if (lane >= d) v += u;
-                }
-                if (lane < nwarps) s_scan[lane] = v;
+            for (int u = 0; u < kGenPeaks; ++u) {
+                uint32_t gen = ((uint32_t)pass << 31) |
+                               ((uint32_t)(pc + kGenPeaks * tid + u) << 16) | (uint32_t)start[u];
+                const int last = min(take, first + cnt[u]);
+#pragma unroll 1
+                for (int i = first; i < last; ++i) cgen[total + i] = gen++;
+                first += cnt[u];
             }
             sync();
-            const int excl = incl - cnt + (wid > 0 ? s_scan[wid - 1] : 0);
-            const int chunk_total = s_scan[nwarps - 1];
-            if (cnt > 0) {
-                w1 = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
-                for (int i = 0; i < cnt; ++i) {
-                    const int rank = total + excl + i;
-                    if (rank >= P.match_limit) break;
-                    const int p2 = start + i;
-                    const double key =
-                        __dmul_rn(__dmul_rn(w1, peak_a(P.Q.a, q0 + p2)), P.Q.b[q0 + p2]);
-                    okey[rank] = order_key(key);
-                    cgen[rank] = ((uint32_t)pass << 31) | ((uint32_t)p1 << 16) | (uint32_t)p2;
+#pragma unroll 1
+            for (int i0 = tid; i0 < take; i0 += kGenIlp * nt) {
+                double w[kGenIlp], qa[kGenIlp], qb[kGenIlp];
+#pragma unroll
+                for (int u = 0; u < kGenIlp; ++u) {
+                    const int i = i0 + u * nt;
+                    w[u] = qa[u] = qb[u] = 1.0;
+                    if (i < take) {
+                        const uint32_t g = cgen[total + i];
+                        qb[u] = P.Q.b[q0 + (g & 0xFFFFu)];
+                        if (P.Q.a) qa[u] = P.Q.a[q0 + (g & 0xFFFFu)];
+                        w[u] = G.w[(int)gen_p1<MODIFIED>(g) - pc];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kGenIlp; ++u) {
+                    const int i = i0 + u * nt;
+                    if (i < take)
+                        okey[total + i] = order_key(__dmul_rn(__dmul_rn(w[u], qa[u]), qb[u]));
                 }
             }
             total += chunk_total;
@@ -1847,6 +1926,147 @@ __device__ bool sort8_by_word(unsigned long long* okey, uint32_t* cgen,
     return true;
 }
 
+// Bitonic sort, descending, of 8 * nt 32-bit words (thread t ends with positions
+// 8t..8t+7), exchanging through `scratch` (8 * nt words) for distances of 256 and
+// more.
+template <int J>
+__device__ __forceinline__ void words32_local(uint32_t (&c)[8], int base, int kk) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        if (e & J) continue;
+        const uint32_t hi = max(c[e], c[e | J]), lo = min(c[e], c[e | J]);
+        const bool desc = ((base + e) & kk) == 0;
+        c[e] = desc ? hi : lo;
+        c[e | J] = desc ? lo : hi;
+    }
+}
+template <typename Sync>
+__device__ __forceinline__ void sort8_words32(uint32_t* scratch, uint32_t (&c)[8], int m, int nt,
+                                              int tid, Sync sync) {
+    const int base = 8 * tid;
+    const unsigned full = 0xffffffffu;
+#pragma unroll 1
+    for (int kk = 2; kk <= m; kk <<= 1) {
+#pragma unroll 1
+        for (int j = kk >> 1; j >= 8; j >>= 1) {
+            const bool keep_max = ((base & j) == 0) == ((base & kk) == 0);
+            if (j >= 256) {
+                const int pt = tid ^ (j >> 3);
+                sync();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) scratch[e * nt + tid] = c[e];
+                sync();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const uint32_t o = scratch[e * nt + pt];
+                    c[e] = keep_max ? max(c[e], o) : min(c[e], o);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const uint32_t o = __shfl_xor_sync(full, c[e], j >> 3);
+                    c[e] = keep_max ? max(c[e], o) : min(c[e], o);
+                }
+            }
+        }
+        if (kk >= 8) words32_local<4>(c, base, kk);
+        if (kk >= 4) words32_local<2>(c, base, kk);
+        words32_local<1>(c, base, kk);
+    }
+}
+
+// Sorts the m = 8 * nt candidates of okey/cgen (n real ones) into greedy order
+// through one 32-bit word each: the key's float32 (rounded down) without its low
+// R - 1 bits, plus one, above the R-bit index (m = 2^R), zero for padding.  That
+// is the order up to keys whose kept bits tie (about ten neighbours of 1024); the
+// exact (key, gen) order is then restored by odd-even exchanges of neighbours,
+// which end when a pass exchanges nothing.  False, with okey/cgen untouched, when
+// eight passes are not enough or a key is negative or not finite in float32.
+// Against the 64-bit words of sort8_by_word a compare-exchange is two
+// instructions instead of seven and a shuffle one instead of two.
+constexpr int kFixPasses = 8;
+template <typename Sync>
+__device__ bool sort8_by_float(unsigned long long* okey, uint32_t* cgen, void* scratch, int* s_flags,
+                               int n, int m, int nt, int tid, Sync sync) {
+    const int rb = 31 - __clz(m);
+    if (tid <= kFixPasses) s_flags[tid] = 0;
+    sync();
+    uint32_t c[8];
+    bool bad = false;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int i = e * nt + tid;
+        c[e] = (uint32_t)i;
+        if (i < n) {
+            const unsigned long long k = okey[i];
+            const uint32_t f = __float_as_uint(__double2float_rd(key_from_order(k)));
+            bad = bad || f > 0x7f7fffffu || (k >> 63) == 0ull;
+            c[e] |= ((f >> (rb - 1)) + 1u) << rb;
+        }
+    }
+    if (bad) s_flags[kFixPasses] = 1;
+    sync();
+    if (s_flags[kFixPasses]) return false;
+    sort8_words32(reinterpret_cast<uint32_t*>(scratch), c, m, nt, tid, sync);
+    Cand x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int i = (int)(c[e] & (uint32_t)(m - 1));
+        const bool real = c[e] >= (uint32_t)m;
+        x[e].k = real ? okey[i] : 0ull;
+        x[e].g = real ? cgen[i] : 0u;
+    }
+    // ends of each thread's eight, for the exchange with its neighbours
+    unsigned long long* ek = reinterpret_cast<unsigned long long*>(scratch);  // [2 * nt]
+    uint32_t* eg = reinterpret_cast<uint32_t*>(ek + 2 * nt);                  // [2 * nt]
+    auto order = [&](Cand& a, Cand& b, bool& any) {
+        if (cand_gt(b, a)) {
+            const Cand t = a;
+            a = b;
+            b = t;
+            any = true;
+        }
+    };
+#pragma unroll 1
+    for (int pass = 0; pass < kFixPasses; ++pass) {
+        bool any = false;
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) order(x[e], x[e + 1], any);
+#pragma unroll
+        for (int e = 1; e < 7; e += 2) order(x[e], x[e + 1], any);
+        sync();  // the words' or the last pass's readers are done with scratch
+        ek[2 * tid] = x[0].k;
+        eg[2 * tid] = x[0].g;
+        ek[2 * tid + 1] = x[7].k;
+        eg[2 * tid + 1] = x[7].g;
+        sync();
+        if (tid + 1 < nt) {
+            const Cand next{ek[2 * tid + 2], eg[2 * tid + 2]};
+            if (cand_gt(next, x[7])) {
+                x[7] = next;
+                any = true;
+            }
+        }
+        if (tid > 0) {
+            const Cand prev{ek[2 * tid - 1], eg[2 * tid - 1]};
+            const Cand mine{ek[2 * tid], eg[2 * tid]};
+            if (cand_gt(mine, prev)) x[0] = prev;
+        }
+        if (any) s_flags[pass] = 1;
+        sync();
+        if (!s_flags[pass]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                okey[8 * tid + e] = x[e].k;
+                cgen[8 * tid + e] = x[e].g;
+            }
+            sync();
+            return true;
+        }
+    }
+    return false;
+}
+
 // Pads okey/cgen[n, m) and sorts [0, m) descending by (okey, gen), m the
 // power of two >= n: in registers when m = 8 * nt, else in shared memory.
 template <typename Sync>
@@ -1883,47 +2103,74 @@ __device__ void sort_pair(unsigned long long* okey, uint32_t* cgen, int n, int m
     }
 }
 
-// Greedy by one warp over chunks of 32 sorted candidates (used_r / used_q
-// zeroed for the pair's peaks).  Within a chunk a live candidate is accepted
-// iff no earlier accepted one shares its reference or query peak: conflict
-// masks come from __match_any_sync, and lanes decide in rounds, each lane as
-// soon as every earlier conflicting lane has decided (the lowest undecided
-// lane always can, so this ends; usually after one or two rounds).  Accepted
-// keys are summed in sorted order, as the sequential greedy; every lane ends
-// with the same score and match count.
+constexpr int kFill = 2;                    // chunks of 32 candidates looked at together
+constexpr int kQueued = 32 * (kFill + 1);  // at most 31 waiting, plus one look's candidates
+// Greedy by one warp over the sorted candidates.  used_r / used_q, zeroed for
+// the pair's peaks, hold the peaks taken; or, used_q null, used_r is a bitmap over
+// the candidates (n bits, zeroed) of those accepted, and a candidate is compared
+// with each of them (spectra with more peaks than the bitmaps hold).
+//
+// Most candidates have a taken peak when their turn comes, so the live ones are
+// first queued (their positions, in order; `queue` holds kQueued) and resolved 32 at a
+// time: a candidate is accepted iff no earlier accepted one of the batch shares
+// its reference or query peak.  Conflict masks come from __match_any_sync, and
+// lanes decide in rounds, each lane as soon as every earlier conflicting lane has
+// decided (the lowest undecided lane always can, so this ends; usually after two
+// or three rounds).  Accepted keys are summed in sorted order, as the sequential
+// greedy; every lane ends with the same score and match count.
 template <bool MODIFIED>
-__device__ void greedy_pair(const unsigned long long* okey, const uint32_t* cgen,
-                            uint32_t* used_r, uint32_t* used_q, int n, double& score,
+__device__ void greedy_pair(unsigned long long* okey, const uint32_t* cgen, uint32_t* used_r,
+                            uint32_t* used_q, uint16_t* queue, int n, double& score,
                             int& matches) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    // the next chunk's candidates are loaded while this one is resolved
-    // (they do not depend on the used-peak bits)
-    uint32_t g_nx = lane < n ? cgen[lane] : 0u;
-    unsigned long long k_nx = lane < n ? okey[lane] : 0ull;
-    for (int c = 0; c < n; c += 32) {
-        const int i = c + lane;
-        const uint32_t g = g_nx;
-        const unsigned long long ok = k_nx;
-        if (i + 32 < n) {
-            g_nx = cgen[i + 32];
-            k_nx = okey[i + 32];
+    auto free_peaks = [&](uint32_t g) {
+        const int p1 = (int)gen_p1<MODIFIED>(g), p2 = (int)(g & 0xFFFFu);
+        if (used_q)
+            return (((used_r[p1 >> 5] >> (p1 & 31)) | (used_q[p2 >> 5] >> (p2 & 31))) & 1u) == 0u;
+        for (int w = 0; w < (n + 31) / 32; ++w)
+            for (unsigned m = used_r[w]; m; m &= m - 1u) {
+                const uint32_t o = cgen[32 * w + __ffs(m) - 1];
+                if ((int)gen_p1<MODIFIED>(o) == p1 || (int)(o & 0xFFFFu) == p2) return false;
+            }
+        return true;
+    };
+    int queued = 0, c = 0;
+#pragma unroll 1
+    for (;;) {
+#pragma unroll 1
+        while (queued < 32 && c < n) {
+            bool live[kFill];
+#pragma unroll
+            for (int u = 0; u < kFill; ++u) {
+                const int i = c + 32 * u + lane;
+                live[u] = i < n && free_peaks(cgen[i]);
+            }
+#pragma unroll
+            for (int u = 0; u < kFill; ++u) {
+                const unsigned bal = __ballot_sync(full, live[u]);
+                if (live[u]) queue[queued + __popc(bal & below)] = (uint16_t)(c + 32 * u + lane);
+                queued += __popc(bal);
+            }
+            c += 32 * kFill;
         }
-        bool alive = false;
-        if (i < n) {
-            const int p1 = (int)gen_p1<MODIFIED>(g), p2 = g & 0xFFFF;
-            alive = !((used_r[p1 >> 5] >> (p1 & 31)) & 1u) &&
-                    !((used_q[p2 >> 5] >> (p2 & 31)) & 1u);
-        }
+        __syncwarp();
+        if (queued == 0) break;
+        const int take = min(queued, 32);
+        const int pos = lane < take ? queue[lane] : 0;
+        const uint32_t g = cgen[pos];
+        const double key = key_from_order(okey[pos]);
+        const unsigned p1 = gen_p1<MODIFIED>(g), p2 = g & 0xFFFFu;
+        // those queued before the last batch may have lost a peak to it
+        const bool alive = lane < take && free_peaks(g);
         const unsigned live = __ballot_sync(full, alive);
-        if (live == 0u) continue;
-        // dead lanes get values no peak index takes, so they match only
-        // themselves
-        const unsigned m1 = __match_any_sync(full, alive ? gen_p1<MODIFIED>(g) : 0x10000u + lane);
-        const unsigned m2 = __match_any_sync(full, alive ? (g & 0xFFFFu) : 0x10000u + lane);
+        // dead lanes get values no peak index takes, so they match only themselves
+        const unsigned m1 = __match_any_sync(full, alive ? p1 : 0x10000u + lane);
+        const unsigned m2 = __match_any_sync(full, alive ? p2 : 0x10000u + lane);
         const unsigned earlier = (m1 | m2) & live & below;
         unsigned dec = ~live, acc = 0u;
+#pragma unroll 1
         while (dec != full) {
             bool my_dec = (dec >> lane) & 1u, my_acc = (acc >> lane) & 1u;
             if (!my_dec && (earlier & ~dec) == 0u) {
@@ -1934,18 +2181,35 @@ __device__ void greedy_pair(const unsigned long long* okey, const uint32_t* cgen
             acc = __ballot_sync(full, my_acc);
         }
         if ((acc >> lane) & 1u) {
-            const int p1 = (int)gen_p1<MODIFIED>(g), p2 = g & 0xFFFF;
-            atomicOr(&used_r[p1 >> 5], 1u << (p1 & 31));
-            atomicOr(&used_q[p2 >> 5], 1u << (p2 & 31));
+            if (used_q) {
+                atomicOr(&used_r[p1 >> 5], 1u << (p1 & 31));
+                atomicOr(&used_q[p2 >> 5], 1u << (p2 & 31));
+            } else {
+                atomicOr(&used_r[pos >> 5], 1u << (pos & 31));
+            }
         }
-        const double kk = (i < n) ? key_from_order(ok) : 0.0;
-        for (unsigned a = acc; a; a &= a - 1u) {
-            const double k = __shfl_sync(full, kk, __ffs(a) - 1);
-            score = __dadd_rn(score, k);
-        }
+        // accepted keys, in order, over the keys of resolved candidates (there are
+        // at least as many of those, all before the first one queued)
+        __syncwarp();
+        if ((acc >> lane) & 1u)
+            okey[matches + __popc(acc & below)] = (unsigned long long)__double_as_longlong(key);
         matches += __popc(acc);
+        // the rest of the queue moves up
+        uint16_t rest[kFill];
+#pragma unroll
+        for (int u = 0; u < kFill; ++u)
+            rest[u] = 32 * u + lane < queued - take ? queue[32 * (u + 1) + lane] : (uint16_t)0;
+        __syncwarp();
+        queued -= take;
+#pragma unroll
+        for (int u = 0; u < kFill; ++u)
+            if (32 * u + lane < queued) queue[32 * u + lane] = rest[u];
         __syncwarp();
     }
+    // one serial chain of additions, its operands read ahead
+#pragma unroll 8
+    for (int i = 0; i < matches; ++i)
+        score = __dadd_rn(score, __longlong_as_double((long long)okey[i]));
 }
 
 // The pair's outputs (dense, or a sparse hit above the threshold).
@@ -1990,7 +2254,9 @@ __global__ void pair_kernel(PairParams P) {
     uint32_t* cgen = reinterpret_cast<uint32_t*>(okey + P.cap);
     uint32_t* used_r = cgen + P.cap;          // 2048 words: 65536 peaks
     uint32_t* used_q = used_r + 2048;
+    const GenScratch gen = gen_scratch(used_q + 2048, blockDim.x, 0);
     __shared__ int s_scan[32];
+    __shared__ uint16_t s_queue[kQueued];
     __shared__ unsigned long long s_item;
 
     const int tid = threadIdx.x, wid = tid >> 5;
@@ -2008,7 +2274,8 @@ __global__ void pair_kernel(PairParams P) {
         if (item >= n_items) break;
         int64_t ri, qi;
         if (!pair_of(P, item, ri, qi)) continue;
-        const int total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, blockDim.x, tid, s_scan, sync);
+        const int total =
+            gen_pair<MODIFIED>(P, ri, qi, okey, cgen, blockDim.x, tid, s_scan, gen, sync);
         const int n = min(total, P.match_limit);
         double score = 0.0;
         int matches = 0;
@@ -2020,17 +2287,19 @@ __global__ void pair_kernel(PairParams P) {
             int m = 1;
             while (m < n) m <<= 1;
             sort_pair(okey, cgen, n, m, blockDim.x, tid, sync);
-            if (wid == 0) greedy_pair<MODIFIED>(okey, cgen, used_r, used_q, n, score, matches);
+            if (wid == 0)
+                greedy_pair<MODIFIED>(okey, cgen, used_r, used_q, s_queue, n, score, matches);
         }
         if (tid == 0) write_pair<SPARSE>(P, ri, qi, n, score, matches, total >= P.match_limit);
     }
 }
 
 // ---- pipelined pair kernel ----
-// Warps 0..G-1 (the producers, G = blockDim.x / 32 - 1) generate and sort the
-// candidates of the next pair into one of two buffers while warp G (the
-// consumer) runs the greedy of the previous pair from the other buffer, so the
-// producers never wait at a barrier while one warp resolves.  The hand-off
+// The producer warps generate and sort the candidates of the next pair into one
+// of kPipeBufs buffers while kPipeCons consumer warps, pair by pair in turn, run
+// the greedy of earlier pairs, so the producers never wait at a barrier while a
+// warp resolves.  (With one consumer warp and two buffers the greedy, 57
+// thousand cycles a pair against 35 thousand, held the producers up.)  The hand-off
 // is two mbarriers per buffer: `full` (every producer thread arrives after
 // its writes) and `empty` (the consumer, after reading).  Every wait is
 // bounded by %globaltimer (kPipeWaitNs); on expiry the waiting side sets
@@ -2038,6 +2307,27 @@ __global__ void pair_kernel(PairParams P) {
 // side leaves at its next (bounded) wait.  The producers of a CTA take every
 // decision together (one thread decides, a producer barrier publishes it),
 // so their named barrier is never left half-joined.
+//
+// Dense, overflow-heavy spectra (1000 to 2000 peaks, match_limit 1024), 800 x 907:
+// 24.7 ms (39.4 with one consumer, 64-bit words and a chunk-by-chunk greedy).  A
+// CTA's pair takes its producers 34 thousand cycles, 19 generating and 15 sorting,
+// and its consumers 25; four CTAs a multiprocessor at 80 registers (six at 64 with
+// one consumer and two buffers: the same time).  Bound by dependent integer
+// instructions at 57% issue.
+constexpr int kPipeBufs = 3;
+constexpr int kPipeCons = 2;
+constexpr int kPipeUsed = 256;   // words of each used-peak bitmap: spectra of up to 8192 peaks
+constexpr int kPipeCache = 2048; // query m/z values kept in shared memory while generating
+// shared memory of np producer threads and buffers of cap candidates; the
+// scratch serves gen_pair, then the sorts (a 64-bit word per candidate and one
+// more per eight: 72 bytes a thread)
+constexpr size_t pipe_scratch_bytes(int np) {
+    return std::max<size_t>(gen_scratch_bytes(np, kPipeCache), (size_t)np * 72);
+}
+constexpr size_t pipe_smem_bytes(int cap, int np) {
+    return (size_t)cap * 12 * kPipeBufs + (size_t)kPipeCons * 2 * kPipeUsed * 4 +
+           pipe_scratch_bytes(np);
+}
 constexpr unsigned long long kPipeWaitNs = 2000000000ull;
 
 __device__ __forceinline__ void pipe_bar_init(uint64_t* bar, uint32_t count) {
@@ -2072,31 +2362,29 @@ __device__ __forceinline__ bool pipe_bar_wait(uint64_t* bar, uint32_t parity,
 }
 
 template <bool SPARSE, bool MODIFIED>
-__global__ void pair_kernel_pipe(PairParams P) {
+__global__ void __maxnreg__(80)
+pair_kernel_pipe(PairParams P) {
     if (*P.bad) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // two candidate buffers, then the consumer's used-peak bitmaps
     unsigned long long* okey0 = reinterpret_cast<unsigned long long*>(smem_raw);
-    uint32_t* cgen0 = reinterpret_cast<uint32_t*>(okey0 + 2 * P.cap);
-    uint32_t* used_r = cgen0 + 2 * P.cap;  // 2048 words: 65536 peaks
-    uint32_t* used_q = used_r + 2048;
-    // the producers' sort scratch: one 64-bit word per candidate slot, and one
-    // more per eight (the padded layout of the sorted words)
-    unsigned long long* scratch = reinterpret_cast<unsigned long long*>(used_q + 2048);
+    uint32_t* cgen0 = reinterpret_cast<uint32_t*>(okey0 + kPipeBufs * P.cap);
+    uint32_t* used0 = cgen0 + kPipeBufs * P.cap;
+    void* scratch = used0 + kPipeCons * 2 * kPipeUsed;
     __shared__ int s_scan[32];
-    __shared__ int s_flag;
+    __shared__ uint16_t s_queue[kPipeCons][kQueued];
+    __shared__ int s_flags[kFixPasses + 1];
     __shared__ unsigned long long s_item;
-    __shared__ __align__(8) uint64_t s_full[2], s_empty[2];
-    __shared__ long long s_ri[2], s_qi[2];
-    __shared__ int s_total[2];  // candidates generated; -1: no more pairs
-    __shared__ int s_go;        // producers: 1 to continue
+    __shared__ __align__(8) uint64_t s_full[kPipeBufs], s_empty[kPipeBufs];
+    __shared__ long long s_ri[kPipeBufs], s_qi[kPipeBufs];
+    __shared__ int s_total[kPipeBufs];  // candidates generated; -1: no more pairs
+    __shared__ int s_go;                // producers: 1 to continue
     __shared__ volatile int s_stop;
 
     const int tid = threadIdx.x;
-    const int np = (int)blockDim.x - 32;  // producer threads
+    const int np = (int)blockDim.x - 32 * kPipeCons;  // producer threads
     const bool producer = tid < np;
     if (tid == 0) {
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kPipeBufs; ++b) {
             pipe_bar_init(&s_full[b], (uint32_t)np);
             pipe_bar_init(&s_empty[b], 1u);
         }
@@ -2108,9 +2396,11 @@ __global__ void pair_kernel_pipe(PairParams P) {
 
     if (producer) {
         const GroupSync sync{np};
+        const GenScratch gen = gen_scratch(scratch, np, kPipeCache);
         int b = 0;
         uint32_t ph = 0;  // parity of buffer b's current use
-        for (int64_t iter = 0;; ++iter) {
+        int ends = 0;     // end marks posted, one for each consumer
+        for (int64_t iter = 0; ends < kPipeCons; ++iter) {
             if (tid == 0) s_item = P.pairs ? atomicAdd(P.work, 1ull)
                                            : (unsigned long long)(blockIdx.x + iter * gridDim.x);
             sync();
@@ -2121,7 +2411,7 @@ __global__ void pair_kernel_pipe(PairParams P) {
                 sync();  // s_item is rewritten by the next fetch
                 continue;
             }
-            // buffer b free (the consumer is done with its previous pair)?
+            // buffer b free (its consumer is done with its previous pair)?
             if (tid == 0) s_go = pipe_bar_wait(&s_empty[b], ph ^ 1u, &s_stop) ? 1 : 0;
             sync();
             if (!s_go) {
@@ -2135,7 +2425,7 @@ __global__ void pair_kernel_pipe(PairParams P) {
             uint32_t* cgen = cgen0 + (size_t)b * P.cap;
             int total = -1;
             if (more) {
-                total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, np, tid, s_scan, sync);
+                total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, np, tid, s_scan, gen, sync);
                 const int n = min(total, P.match_limit);
                 if (n > 0) {
                     int m = 1;
@@ -2143,9 +2433,13 @@ __global__ void pair_kernel_pipe(PairParams P) {
                     // one word per candidate when the pair fills the register
                     // sort; the (key, gen) pairs themselves otherwise
                     if (!(m == 8 * np &&
-                          sort8_by_word(okey, cgen, scratch, &s_flag, n, m, np, tid, sync)))
+                          (sort8_by_float(okey, cgen, scratch, s_flags, n, m, np, tid, sync) ||
+                           sort8_by_word(okey, cgen, reinterpret_cast<unsigned long long*>(scratch),
+                                         s_flags, n, m, np, tid, sync))))
                         sort_pair(okey, cgen, n, m, np, tid, sync);
                 }
+            } else {
+                ++ends;
             }
             if (tid == 0) {
                 s_ri[b] = ri;
@@ -2154,18 +2448,18 @@ __global__ void pair_kernel_pipe(PairParams P) {
             }
             sync();
             pipe_bar_arrive(&s_full[b]);
-            if (!more) break;
-            if (++b == 2) {
+            if (++b == kPipeBufs) {
                 b = 0;
                 ph ^= 1u;
             }
         }
     } else if (!P.test_stall) {
-        // consumer warp
-        const int lane = tid & 31;
-        int b = 0;
-        uint32_t ph = 0;
-        for (;;) {
+        // consumer warp w: every kPipeCons-th buffer use, from use w on
+        const int lane = tid & 31, w = (tid - np) >> 5;
+        uint32_t* used_r = used0 + w * 2 * kPipeUsed;
+        for (int use = w;; use += kPipeCons) {
+            const int b = use % kPipeBufs;
+            const uint32_t ph = (uint32_t)(use / kPipeBufs) & 1u;
             int ok = 0;
             if (lane == 0) ok = pipe_bar_wait(&s_full[b], ph, &s_stop) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -2185,20 +2479,22 @@ __global__ void pair_kernel_pipe(PairParams P) {
             if (n > 0) {
                 const int nr = (int)(P.R.off[ri + 1] - P.R.off[ri]);
                 const int nq = (int)(P.Q.off[qi + 1] - P.Q.off[qi]);
-                for (int i = lane; i < (nr + 31) / 32; i += 32) used_r[i] = 0u;
-                for (int i = lane; i < (nq + 31) / 32; i += 32) used_q[i] = 0u;
+                const bool fits = max(nr, nq) <= 32 * kPipeUsed;
+                uint32_t* used_q = fits ? used_r + kPipeUsed : nullptr;
+                if (fits) {
+                    for (int i = lane; i < (nr + 31) / 32; i += 32) used_r[i] = 0u;
+                    for (int i = lane; i < (nq + 31) / 32; i += 32) used_q[i] = 0u;
+                } else {
+                    for (int i = lane; i < (n + 31) / 32; i += 32) used_r[i] = 0u;
+                }
                 __syncwarp();
                 greedy_pair<MODIFIED>(okey0 + (size_t)b * P.cap, cgen0 + (size_t)b * P.cap,
-                                      used_r, used_q, n, score, matches);
+                                      used_r, used_q, s_queue[w], n, score, matches);
             }
             __syncwarp();
             if (lane == 0) {
                 pipe_bar_arrive(&s_empty[b]);
                 write_pair<SPARSE>(P, ri, qi, n, score, matches, total >= P.match_limit);
-            }
-            if (++b == 2) {
-                b = 0;
-                ph ^= 1u;
             }
         }
     }
@@ -2365,7 +2661,7 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
                   "(%lld != %lld)", (long long)args.ref.n, (long long)args.qry.n);
         return CMS_ERR_INVALID;
     }
-    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4;
+    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(p.pair_threads, 0);
     if (pair_smem > ctx->smem_optin) {
         set_error("cms_cosine_greedy: match_limit %d needs %zu B shared memory (> %zu)",
                   args.match_limit, pair_smem, ctx->smem_optin);
@@ -2411,7 +2707,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
                    const SparseOut* sparse, const Plan& p, cudaStream_t s) {
     int rc = CMS_OK;
     const int sym = p.sym;
-    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4;
+    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(p.pair_threads, 0);
     const int64_t nR = args.ref.n, nQ = args.qry.n;
     const size_t gpool_warps = (size_t)ctx->sm_count * 64;
     const size_t gpool_bytes = gpool_warps * (size_t)kGPool * 16;
@@ -2493,17 +2789,16 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     pair_blocks_per_sm = std::max(1, pair_blocks_per_sm);
     const int pair_grid = ctx->sm_count * pair_blocks_per_sm;
 
-    if (p.mode == 2 &&
-        pair_smem + (size_t)p.cap * 12 + (size_t)p.pair_threads * 72 <= ctx->smem_optin) {
+    const size_t pipe_smem = pipe_smem_bytes(p.cap, p.pair_threads);
+    if (p.mode == 2 && pipe_smem <= ctx->smem_optin &&
+        p.cap / 32 <= 2 * kPipeUsed) {  // the accepted bitmap of spectra past kPipeUsed
         // whole matrix: the pipelined pair kernel (pair_threads producers
-        // plus a consumer warp, two candidate buffers)
+        // plus the consumer warps)
         void (*pipe_k)(PairParams) =
             sparse ? (args.modified ? pair_kernel_pipe<true, true> : pair_kernel_pipe<true, false>)
                    : (args.modified ? pair_kernel_pipe<false, true>
                                     : pair_kernel_pipe<false, false>);
-        // two candidate buffers and the sort's word scratch (8 per producer)
-        const size_t pipe_smem = pair_smem + (size_t)p.cap * 12 + (size_t)p.pair_threads * 72;
-        const int pipe_threads = p.pair_threads + 32;
+        const int pipe_threads = p.pair_threads + 32 * kPipeCons;
         pp.test_stall = test_stall("pair");
         if ((rc = set_func_smem(pipe_k, pipe_smem))) return rc;
         int per_sm = 1;
@@ -3041,7 +3336,8 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     pp.err = err;
     pp.bad = bad;
     const int pair_threads = 128;
-    const size_t pair_smem = (size_t)cap * 12 + 2 * 2048 * 4;
+    const size_t pair_smem =
+        (size_t)cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(pair_threads, 0);
     if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
     int per_sm = 1;
     CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<false, false>,
@@ -3215,7 +3511,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     if (n_q == 0) return CMS_OK;
 
     const int cap = next_pow2(std::max(2, lib->match_limit));
-    const size_t pair_smem = (size_t)cap * 12 + 2 * 2048 * 4;
+    const size_t pair_smem = (size_t)cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(128, 0);
     if (pair_smem > ctx->smem_optin) {
         set_error("cms_library_search: match_limit too large for shared memory");
         return CMS_ERR_UNSUPPORTED;

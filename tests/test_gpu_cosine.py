@@ -331,3 +331,45 @@ def test_large_sampled(cuda_device):
     np.testing.assert_array_equal(a[2][pr, pq], o)
     np.testing.assert_array_equal(a[1][pr, pq], m)
     np.testing.assert_array_equal(a[0][pr, pq].view(np.uint32), s.view(np.uint32))
+
+
+@pytest.mark.parametrize("scale", ["plain", "ties", "wide", "tiny"])
+def test_pair_pipeline_sort_paths(cuda_device, scale):
+    """The pipelined pair kernel's sort through float32 words and what it falls back to:
+    ordinary keys, many equal keys, keys that differ only below float32, keys below
+    float32's range; truncated candidate lists of several sizes."""
+    from cudams import synthetic
+    from cudams.packing import PackedSpectra
+
+    def weights(s, seed):
+        rng = np.random.default_rng(seed)
+        b = s.b.copy()
+        if scale == "ties":
+            b = np.round(rng.random(b.shape[0]) * 4 + 1)
+        elif scale == "wide":
+            b = 1.0 + rng.integers(0, 1 << 20, b.shape[0]) * 2.0 ** -45
+        elif scale == "tiny":
+            b = b * 2.0 ** -90
+        return PackedSpectra(s.mz, None if scale != "plain" else s.a, b, s.offsets,
+                             s.mz_power, s.intensity_power, s.n_max_peaks)
+
+    ref = weights(synthetic.clustered_spectra(9, seed=91), 1)
+    qry = weights(synthetic.clustered_spectra(11, seed=92), 2)
+    for limit in (512, 1000, 1024, 2048):
+        want = oracle.cosine_greedy(ref, qry, 0.05, 0.0, limit)
+        assert_same(gpu_dense(ref, qry, P(0.05, limit, 2048), {"mode": 2}), want, f"{scale} {limit}")
+
+
+def test_pair_pipeline_long_spectra(cuda_device):
+    """Spectra with more peaks than the used-peak bitmaps of the pipelined kernel."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(93)
+    def make(lens, seed):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(100.0, 130.0, k)) for k in lens])
+        return pack_csr(mz.astype(np.float32), rng.random(off[-1]).astype(np.float32) + 0.01, off, None)
+    ref, qry = make([8192, 8193, 20000, 3], 1), make([9000, 8192, 50], 2)
+    for limit in (1024, 4096):
+        want = oracle.cosine_greedy(ref, qry, 0.01, 0.0, limit)
+        assert_same(gpu_dense(ref, qry, P(0.01, limit, 65535), {"mode": 2}), want, f"{limit}")
