@@ -39,57 +39,99 @@ struct FpParams {
     int test_stall;
 };
 
-// Branch-free IEEE float32 division and square root for the operands the
-// measures produce.  Both follow the published Newton-Raphson/FMA schemes
-// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// Branch-free IEEE float32 arithmetic for the operands the measures produce, two
+// elements to an instruction (Blackwell's packed float32 operations; each half
+// is rounded like the scalar one).  It follows the published Newton-Raphson/FMA
+// schemes (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al.,
 // Handbook of Floating-Point Arithmetic, 2nd ed., 2018, sections 4.7-4.8):
-// the hardware approximation, one Newton step, and one FMA correction of the
-// result.  They carry no special-case branch, so the 32 elements of a lane's
-// chunk interleave freely.  Correct rounding is established by exhaustive
-// comparison with CUDA's __fdiv_rn / __fsqrt_rn / __frcp_rn on the device
-// (cms_fingerprint_arith_check) over every operand that can occur: n / d for
-// integers 0 <= n <= d <= 65536 (Jaccard, Dice: 32768-bit fingerprints at
-// most), sqrt(p) for every float p in [1, 2^30] (p = a * b rounded), the
-// reciprocal of every such sqrt(p) (which makes the quotient correctly
-// rounded for every numerator, by Markstein's theorem), and every cosine
-// triple of fingerprints up to 2048 bits.  d = 0 or p = 0 give NaN (0/0
-// only), which the measure maps to 0.
-__device__ __forceinline__ float rcp_fp(float d) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-    return __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
+//   n / d, integers 0 <= n <= d <= 65536 (Jaccard, Dice: 32768-bit fingerprints at
+//     most): the hardware reciprocal y, q = n y, and one correction q + (n - q d) y,
+//     accurate to about 2^-45 before its rounding.  A quotient of such integers is
+//     at least 2^-42 of itself away from any rounding boundary, so that is enough
+//     and the reciprocal needs no Newton step.
+//   n / sqrt(p): the hardware reciprocal root, one Newton step and one correction
+//     give the correctly rounded root, its hardware reciprocal and one Newton step
+//     the root's correctly rounded reciprocal, which by Markstein's theorem makes
+//     the corrected quotient correctly rounded for every numerator.
+// Correct rounding is established by exhaustive comparison with CUDA's
+// __fdiv_rn / __fsqrt_rn / __frcp_rn on the device (cms_fingerprint_arith_check)
+// over every operand that can occur: n / d as above, sqrt(p) and the reciprocal
+// of every such sqrt(p) for every float p in [1, 2^30] (p = a * b rounded), and
+// every cosine triple of fingerprints up to 2048 bits.  A denominator of 0 (two
+// empty fingerprints) gives NaN, which the measure maps to 0.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
-__device__ __forceinline__ float div_fp(float n, float d) {
-    const float y = rcp_fp(d);
-    const float q = __fmul_rn(n, y);
-    return __fmaf_rn(__fmaf_rn(-q, d, n), y, q);
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "mul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
-__device__ __forceinline__ float sqrt_fp(float p) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p));
-    float g = __fmul_rn(p, r), h = __fmul_rn(0.5f, r);
-    const float e = __fmaf_rn(-g, h, 0.5f);
-    g = __fmaf_rn(g, e, g);
-    h = __fmaf_rn(h, e, h);
-    return __fmaf_rn(__fmaf_rn(-g, g, p), h, g);
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "mov.b64 z, {%6, %7};\n\tfma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 rcp2_approx(float2 d) {
+    float2 y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(d.y));
+    return y;
+}
+// n / d, given -d too
+__device__ __forceinline__ float2 div2_int(float2 n, float2 d, float2 minus_d) {
+    const float2 y = rcp2_approx(d);
+    const float2 q = mul2(n, y);
+    return fma2(fma2(q, minus_d, n), y, q);
+}
+// sqrt(p) and 1 / sqrt(p), both correctly rounded (the latter of the rounded root)
+__device__ __forceinline__ void root2(float2 p, float2& root, float2& rcp) {
+    float2 r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(p.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(p.y));
+    const float2 g = mul2(p, r);
+    const float2 e = fma2(g, mul2(r, both(-0.5f)), both(0.5f));
+    const float2 g1 = fma2(g, e, g), y = fma2(r, e, r);  // sqrt(p), 1 / sqrt(p)
+    root = fma2(fma2(g1, mul2(g1, both(-1.0f)), p), mul2(y, both(0.5f)), g1);
+    // (from the root's own hardware reciprocal: y above, refined, stays one unit off
+    // where the root's mantissa is all ones)
+    const float2 z = rcp2_approx(root);
+    rcp = fma2(fma2(mul2(root, both(-1.0f)), z, both(1.0f)), z, z);
+}
+__device__ __forceinline__ float2 div2_root(float2 n, float2 p) {
+    float2 root, y;
+    root2(p, root, y);
+    const float2 q = mul2(n, y);
+    return fma2(fma2(q, mul2(root, both(-1.0f)), n), y, q);
 }
 
-// The measure from the intersection count fi and the row bit counts fa, fb
-// (all exact integers in float32), in the reference's order of operations.
-// Only 0/0 is NaN here (fi > 0 implies a nonzero denominator), and fmaxf maps
-// it to 0 while keeping every other value, which is >= 0.
+// The measure of two elements from the intersection counts fi and the row bit
+// counts fa, fb (all exact integers in float32), in the reference's order of
+// operations; NaN where both rows are empty.
 template <int MEASURE>
-__device__ __forceinline__ float measure_of(float fi, float fa, float fb) {
-    float v;
+__device__ __forceinline__ float2 measure_of(float2 fi, float2 fa, float2 fb) {
     if (MEASURE == CMS_FP_JACCARD) {
-        v = div_fp(fi, __fsub_rn(__fadd_rn(fa, fb), fi));
+        const float2 s = add2(fa, fb);
+        return div2_int(fi, fma2(fi, both(-1.0f), s), fma2(s, both(-1.0f), fi));
     } else if (MEASURE == CMS_FP_DICE) {
-        v = __fmul_rn(2.0f, div_fp(fi, __fadd_rn(fa, fb)));
+        const float2 s = add2(fa, fb);
+        return mul2(both(2.0f), div2_int(fi, s, mul2(s, both(-1.0f))));
     } else {
-        v = div_fp(fi, sqrt_fp(__fmul_rn(fa, fb)));
+        return div2_root(fi, mul2(fa, fb));
     }
-    return fmaxf(v, 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -97,31 +139,32 @@ __device__ __forceinline__ float measure_of(float fi, float fa, float fb) {
 // ---------------------------------------------------------------------------
 // The bit-packed rows are expanded on the fly, straight into the
 // shared-memory operand stages (no expanded copy in global memory), to packed
-// 4-bit floats (E2M1) of value 0 or 1: nibble 0x2 is 1.0.  Every block scale
-// factor is 1.0 (E8M0 0x7F), so a dot product over K = n_words * 32 is the
-// intersection count, exact in the float32 accumulator (counts <= 32768 are
-// integers far below 2^24).  The K order inside a 32-bit word is permuted by
-// the expansion -- nibble t of output word v_s holds bit 4t + s -- identically
-// for both operands, which leaves every dot product unchanged.  Against 0/1
+// 4-bit floats (E2M1), whose products are 1 where both bits are set.  Every
+// block scale factor is 1.0 (E8M0 0x7F), so a dot product over K = n_words * 32
+// is the intersection count, exact in the float32 accumulator (counts <= 32768
+// are integers far below 2^24).  The K order inside a 32-bit word is permuted by
+// the expansion identically for both operands, which leaves every dot product
+// unchanged.  Against 0/1
 // bytes (kind::i8) this halves the expansion work, the shared-memory operand
 // bytes and the MMA instructions per K bit.
 //
 // One persistent CTA per SM, warp-specialised:
-//   warps 0-7   epilogue: TMEM -> registers (tcgen05.ld 32x32b), measure in
-//               IEEE float32, 32 x 32 chunks staged in shared memory and
-//               written by 2-D tensor stores.  Warps w and w+4 share TMEM
-//               lanes 32*(w%4)..+31 (rows) and take alternate 32-column
-//               chunks of the 224 columns.
-//   warps 8-11  producers: per 256-bit K block, take the 32 bytes of each of
-//               the tile's 128 reference and 224 query rows from the ring,
-//               expand them to 128 bytes each in the canonical K-major
-//               SWIZZLE_128B layout, make the writes visible to the tensor
-//               core (fence.proxy.async), and count the rows' bits (popcounts
-//               of the whole row per tile).
-//   warp 12     MMA issuer: one thread issues 4 x tcgen05.mma (M=128, N=224,
+//   warps 0-11  epilogue: TMEM -> registers (tcgen05.ld 32x32b, 16 columns
+//               ahead of their use), measure in IEEE float32 two elements an
+//               instruction, 32 x 32 chunks staged in shared memory and written
+//               by 2-D tensor stores.  Warps w, w+4 and w+8 share TMEM lanes
+//               32*(w%4)..+31 (rows) and take every third 32-column chunk of
+//               the 224 columns.
+//   warps 12-22 producers: per 256-bit K block, take the 32 bytes of each of
+//               the tile's 128 reference and 224 query rows (a row a thread)
+//               from the ring, expand them to 128 bytes each in the canonical
+//               K-major SWIZZLE_128B layout, make the writes visible to the
+//               tensor core (fence.proxy.async), and count the rows' bits
+//               (popcounts of the whole row per tile).
+//   warp 23     MMA issuer: one thread issues 4 x tcgen05.mma (M=128, N=224,
 //               K=64) per stage and commits stage release / accumulator ready.
-//   warp 13     loader: one thread brings each K block of the tile's packed
-//               rows into a 4-deep shared-memory ring with two 2-D tensor
+//   warp 24     loader: one thread brings each K block of the tile's packed
+//               rows into a 3-deep shared-memory ring with two 2-D tensor
 //               loads (4 KB + 7 KB), so that the producers' reads are
 //               shared-memory reads instead of 16-byte global loads from 352
 //               rows 256 bytes apart.  When the rows do not meet the
@@ -133,6 +176,13 @@ __device__ __forceinline__ float measure_of(float fi, float fa, float fb) {
 // with 0x7F bytes makes every factor 1.0 whatever byte of it an MMA reads.  Every mbarrier wait is bounded in
 // time; on expiry the kernel sets an error bit, every role stops, and TMEM is
 // released before exit.
+//
+// Bound by instruction issue (67% of the slots; tensor pipe 30%, shared-memory data
+// path 56%, output write 30% of the copy rate at 2048 bits).  60000 x 60000:
+//   2048 bits Jaccard 6.9 -> 5.6 ms, cosine 7.05 -> 6.3; 1024 bits 4.5 -> 4.1;
+//   59999 columns 25.9 -> 7.9 ms
+// from four producer and eight epilogue warps, scalar arithmetic with a Newton step
+// more per division, and stores lane by lane where rows are not 16-byte aligned.
 namespace umma {
 
 constexpr int kBM = 128;           // reference rows per tile (TMEM lanes)
@@ -146,15 +196,21 @@ constexpr int kStages = 3;
 constexpr int kABytes = kBM * kBKBytes;  // 16 KB
 constexpr int kBBytes = kBN * kBKBytes;  // 28 KB
 constexpr int kStageBytes = kABytes + kBBytes;
-constexpr int kEpiWarps = 8;      // a multiple of 4 (one set per TMEM lane quarter)
+constexpr int kEpiWarps = 12;      // a multiple of 4 (one set per TMEM lane quarter)
 constexpr int kEpiSets = kEpiWarps / 4;
-constexpr int kProdWarps = 4;
+// with four producer warps (one a scheduler) their own dependent instructions set
+// the time of a tile, 7.0 ms for 60000 x 60000 at 2048 bits; eleven rows' worth of
+// warps give every thread exactly one of the 352 operand rows (5.6 ms; eight: 6.8)
+constexpr int kProdWarps = 11;
 constexpr int kMmaWarp = kEpiWarps + kProdWarps;
 constexpr int kLoadWarp = kMmaWarp + 1;
 constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
 constexpr int kProdThreads = kProdWarps * 32;
+constexpr int kRows = kBM + kBN;  // operand rows of a tile
+constexpr int kProdRows = (kRows + kProdThreads - 1) / kProdThreads;
 constexpr int kTmemCols = 512;
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bounded waits: 2 s
+constexpr uint32_t kWaitHintNs = 100000;  // longest sleep of one barrier poll
 
 // shared-memory layout (offsets from a 1024-byte aligned base)
 constexpr int kOffStages = 0;
@@ -165,7 +221,7 @@ constexpr int kOffStg = kStages * kStageBytes;
 // ring of packed K blocks brought by 2-D tensor loads: kBM + kBN rows of
 // kBKWords words (32 bytes) each, row-major, 32-byte swizzle (the 16-byte
 // halves of row r swapped when r & 4)
-constexpr int kIn = 4;
+constexpr int kIn = 3;
 constexpr int kInABytes = kBM * kBKWords * 4;  // 4 KB
 constexpr int kInBytes = (kBM + kBN) * kBKWords * 4;  // 11 KB
 constexpr int kOffIn = kOffStg + kEpiWarps * kStgBytes;
@@ -208,10 +264,10 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
         : "memory");
     return ok != 0;
 }
@@ -271,37 +327,27 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
             smem_u32(bar))
         : "memory");
 }
-// Load 32 TMEM columns of this warp's 32 lanes (lane i: row i, r[j]: column
+// Load 16 TMEM columns of this warp's 32 lanes (lane i: row i, r[j]: column
 // j) without waiting; tmem_wait_ld completes it.  The wait names the
 // destination registers as read-write operands, so the compiler can neither
 // read nor move them before the data has arrived, and the load overlaps
 // whatever the warp does in between.
-__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
                    "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
-                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]),
-                   "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
-                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
-                   "+r"(r[30]), "+r"(r[31])
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                  :
                  : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    tmem_ld32_async(taddr, r);
-    tmem_wait_ld(r);
 }
 
 // 2-D tensor store of one staged chunk (box 32 x 32 floats at column x, row
@@ -379,19 +425,32 @@ __device__ __forceinline__ int popc_bits(const Bits& b) {
            __popc(b.hi.y) + __popc(b.hi.z) + __popc(b.hi.w);
 }
 
-// Expand one row's 256 bits into 128 bytes of E2M1 nibbles (0x2 = 1.0 where
-// the bit is set) at row r of an operand stage (SWIZZLE_128B: 16-byte chunk c
-// of row r sits at chunk c ^ (r % 8)).  Word q goes to chunk q; its output
-// word s holds bits 4t + s at bit 1 of nibble t.
+// Expand one row's 256 bits into 128 bytes of E2M1 nibbles at row r of the operand
+// stage (SWIZZLE_128B: 16-byte chunk c of row r sits at chunk c ^ (r % 8)).  Word
+// q goes to chunk q, its bits 4t + s to output word s.  A bit may stay where it
+// is in its nibble, as 0.5, 1 or 2, if the other operand's is such that the
+// product is 1, and may move to the next nibble if the other's does, so one or two
+// rotations and four masks do (shifting each plane to bit 1 took three shifts):
+//   plane      reference          query
+//   s = 0      0.5 (in place)     2.0 (rotated by 2)
+//   s = 1      1.0 (in place)     1.0 (in place)
+//   s = 2      2.0 (rotated by 4) 0.5 (rotated by 2: the next nibble's bit 0)
+//   s = 3      1.0 (rotated by 2: the next nibble's bit 1, both)
+template <bool QUERY>
 __device__ __forceinline__ void expand_row(unsigned char* stage, int r, const Bits& bits) {
     unsigned char* row = stage + (r >> 3) * 1024 + (r & 7) * 128;
     const uint32_t w[8] = {bits.lo.x, bits.lo.y, bits.lo.z, bits.lo.w,
                            bits.hi.x, bits.hi.y, bits.hi.z, bits.hi.w};
+    const uint32_t half = 0x11111111u, one = 0x22222222u, two = 0x44444444u;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const uint32_t m = 0x22222222u;
-        *reinterpret_cast<uint4*>(row + ((q ^ (r & 7)) << 4)) =
-            make_uint4((w[q] << 1) & m, w[q] & m, (w[q] >> 1) & m, (w[q] >> 2) & m);
+        const uint32_t w2 = __funnelshift_l(w[q], w[q], 2);
+        uint4 v;
+        if (QUERY)
+            v = make_uint4(w2 & two, w[q] & one, w2 & half, w2 & one);
+        else
+            v = make_uint4(w[q] & half, w[q] & one, __funnelshift_l(w[q], w[q], 4) & two, w2 & one);
+        *reinterpret_cast<uint4*>(row + ((q ^ (r & 7)) << 4)) = v;
     }
 }
 
@@ -461,7 +520,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kProdWarps) {
         // ------------------------------ producers ------------------------------
-        const int pt = threadIdx.x - kEpiWarps * 32;  // 0..127
+        const int pt = threadIdx.x - kEpiWarps * 32;  // 0..kProdThreads - 1
         const bool vec = (P.n_words % kBKWords) == 0 &&
                          (reinterpret_cast<uintptr_t>(P.r) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(P.q) & 15) == 0;
@@ -475,20 +534,24 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int acc = (int)(it & 1);
             const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
             ++it;
-            const int64_t ra = (int64_t)tm * kBM + pt;
-            // query rows pt and (for pt < kBN - 128) pt + 128 of the tile
-            const bool two_b = pt + 128 < kBN;
-            const int64_t qb0 = (int64_t)tn * kBN + pt;
-            const int64_t qb1 = two_b ? qb0 + 128 : P.n_q;  // past the end: zero bits
-            int ca = 0, cb0 = 0, cb1 = 0;
-            Bits xa{}, xb0{}, xb1{};
-            if (!use_in) {
-                xa = load_bits(P.r, ra, P.n_r, P.n_words, 0, vec);
-                xb0 = load_bits(P.q, qb0, P.n_q, P.n_words, 0, vec);
-                xb1 = load_bits(P.q, qb1, P.n_q, P.n_words, 0, vec);
-            }
+            // operand rows pt, pt + kProdThreads, ...: the reference rows, then the
+            // query rows of the tile
+            int cnt[kProdRows];
+            Bits x[kProdRows];
+#pragma unroll
+            for (int u = 0; u < kProdRows; ++u) cnt[u] = 0;
+            auto own_load = [&](int kb) {
+#pragma unroll
+                for (int u = 0; u < kProdRows; ++u) {
+                    const int row = pt + u * kProdThreads;
+                    x[u] = row < kBM ? load_bits(P.r, (int64_t)tm * kBM + row, P.n_r, P.n_words, kb, vec)
+                                     : load_bits(P.q, row < kRows ? (int64_t)tn * kBN + row - kBM : P.n_q,
+                                                 P.n_q, P.n_words, kb, vec);
+                }
+            };
+            if (!use_in) own_load(0);
             for (int kb = 0; kb < G.kb; ++kb) {
-                Bits a = xa, b0 = xb0, b1 = xb1;
+                Bits y[kProdRows];
                 if (use_in) {  // this block's rows from the ring
                     if (!mbar_wait(&in_full[islot], iph, abort_flag)) {
                         ok = false;
@@ -496,31 +559,36 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     const uint4* in = reinterpret_cast<const uint4*>(sm + kOffIn + islot * kInBytes);
                     // 32-byte swizzle: the two 16-byte halves of row r are
-                    // swapped when bit 2 of r is set (the same for all three
-                    // rows of this thread), so that eight lanes read eight
-                    // different bank groups
+                    // swapped when bit 2 of r is set (the same for all rows of
+                    // this thread), so that eight lanes read eight different
+                    // bank groups
                     const int sw = (pt >> 2) & 1;
-                    a = Bits{in[2 * pt + sw], in[2 * pt + (sw ^ 1)]};
-                    b0 = Bits{in[2 * (kBM + pt) + sw], in[2 * (kBM + pt) + (sw ^ 1)]};
-                    if (two_b)
-                        b1 = Bits{in[2 * (kBM + pt + 128) + sw], in[2 * (kBM + pt + 128) + (sw ^ 1)]};
-                } else if (kb + 1 < G.kb) {  // next block's bits load while this one expands
-                    xa = load_bits(P.r, ra, P.n_r, P.n_words, kb + 1, vec);
-                    xb0 = load_bits(P.q, qb0, P.n_q, P.n_words, kb + 1, vec);
-                    xb1 = load_bits(P.q, qb1, P.n_q, P.n_words, kb + 1, vec);
+#pragma unroll
+                    for (int u = 0; u < kProdRows; ++u) {
+                        const int row = pt + u * kProdThreads;
+                        if (row < kRows) y[u] = Bits{in[2 * row + sw], in[2 * row + (sw ^ 1)]};
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kProdRows; ++u) y[u] = x[u];
+                    if (kb + 1 < G.kb) own_load(kb + 1);  // loads while this block expands
                 }
                 if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) {
                     ok = false;
                     break;
                 }
                 unsigned char* sa = sm + kOffStages + stage * kStageBytes;
-                unsigned char* sb = sa + kABytes;
-                expand_row(sa, pt, a);
-                expand_row(sb, pt, b0);
-                if (two_b) expand_row(sb, pt + 128, b1);
-                ca += popc_bits(a);
-                cb0 += popc_bits(b0);
-                cb1 += popc_bits(b1);
+#pragma unroll
+                for (int u = 0; u < kProdRows; ++u) {
+                    const int row = pt + u * kProdThreads;
+                    if (row < kRows) {  // reference and query rows lie behind one another
+                        if (row < kBM)
+                            expand_row<false>(sa, row, y[u]);
+                        else
+                            expand_row<true>(sa, row, y[u]);
+                        cnt[u] += popc_bits(y[u]);
+                    }
+                }
                 fence_proxy_async_smem();
                 mbar_arrive(&full[stage]);
                 if (use_in) {
@@ -543,12 +611,19 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) break;
             // the tile's row popcounts (-1: no fingerprint) for its epilogue
             if (!mbar_wait(&pempty[acc], acc_phase ^ 1u, abort_flag)) break;
-            const bool va = ra < P.n_r && (P.r_valid ? P.r_valid[ra] != 0 : true);
-            const bool vb0 = qb0 < P.n_q && (P.q_valid ? P.q_valid[qb0] != 0 : true);
-            const bool vb1 = qb1 < P.n_q && (P.q_valid ? P.q_valid[qb1] != 0 : true);
-            pa[acc * kBM + pt] = va ? (float)ca : -1.0f;
-            pb[acc * kBN + pt] = vb0 ? (float)cb0 : -1.0f;
-            if (two_b) pb[acc * kBN + pt + 128] = vb1 ? (float)cb1 : -1.0f;
+#pragma unroll
+            for (int u = 0; u < kProdRows; ++u) {
+                const int row = pt + u * kProdThreads;
+                if (row < kBM) {
+                    const int64_t i = (int64_t)tm * kBM + row;
+                    const bool v = i < P.n_r && (P.r_valid ? P.r_valid[i] != 0 : true);
+                    pa[acc * kBM + row] = v ? (float)cnt[u] : -1.0f;
+                } else if (row < kRows) {
+                    const int64_t i = (int64_t)tn * kBN + row - kBM;
+                    const bool v = i < P.n_q && (P.q_valid ? P.q_valid[i] != 0 : true);
+                    pb[acc * kBN + row - kBM] = v ? (float)cnt[u] : -1.0f;
+                }
+            }
             mbar_arrive(&pfull[acc]);
         }
     } else if (warp == kLoadWarp) {
@@ -634,7 +709,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ------------------------------ epilogue ------------------------------
         const int quarter = warp & 3;        // TMEM lanes 32*quarter .. +31
         const int set = warp >> 2;           // which of the kEpiSets warps of this quarter
-        const bool vec_out = (P.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(P.out) & 15) == 0;
         unsigned char* stg = sm + kOffStg + warp * kStgBytes;
         int64_t it = 0;
         for (int64_t t = blockIdx.x; t < G.n_tiles; t += gridDim.x) {
@@ -649,99 +723,94 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(&pfull[acc], acc_phase, abort_flag))) break;
             const int row_l = quarter * 32 + lane;
             const float fa = pa[acc * kBM + row_l];
-            const int64_t gr = (int64_t)tm * kBM + row_l;  // this lane's output row
-            float* orow = P.out + gr * P.ld;
             // the quarter's warps take every kEpiSets-th 32-column chunk,
             // starting one further on each tile, so that the odd chunk of
             // the 224 columns goes to each warp in turn
-            // chunk c's accumulator columns are read (into vn) while chunk
-            // c - kEpiSets is computed and stored
-            uint32_t vn[32];
+            // each half chunk's 16 accumulator columns are read (into vn) while the
+            // half before it is computed
+            uint32_t vn[16];
             const uint32_t tbase =
                 tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kAccStride);
             const int c0 = (int)((set + it) % kEpiSets);
             __syncwarp();
-            if (c0 < kBN / 32) tmem_ld32(tbase + (uint32_t)(c0 * 32), vn);
+            if (c0 < kBN / 32) tmem_ld16_async(tbase + (uint32_t)(c0 * 32), vn);
             for (int c = c0; c < kBN / 32; c += kEpiSets) {
                 const int col_l = c * 32;  // first column of this chunk in the tile
                 const int64_t gc0 = (int64_t)tn * kBN + col_l;
-                uint32_t v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = vn[j];
-                __syncwarp();
-                if (c + kEpiSets < kBN / 32)
-                    tmem_ld32_async(tbase + (uint32_t)((c + kEpiSets) * 32), vn);
                 const float* pbc = pb + acc * kBN + col_l;
-                // every row and column of the chunk has a fingerprint: no
-                // per-element fill test
-                const bool whole = __all_sync(0xFFFFFFFFu, fa >= 0.0f && pbc[lane] >= 0.0f);
-                // a chunk inside the tensor map's columns is stored by the
-                // warp (rows past the end hold the fill value and are clipped
-                // by the store); the others lane by lane
+                // every row and column of the chunk has a fingerprint with a bit set:
+                // no per-element test
+                const bool whole = __all_sync(0xFFFFFFFFu, fa > 0.0f && pbc[lane] > 0.0f);
+                // a chunk inside the tensor map's columns is stored by one
+                // lane's tensor store (rows past the end hold the fill value and
+                // are clipped by the store); the others by the warp
                 const bool tma_chunk = use_map && gc0 + 32 <= (P.n_q & ~int64_t(3));
-                const bool live = tma_chunk ? (int64_t)tm * kBM + quarter * 32 < P.n_r
-                                            : (gr < P.n_r && gc0 < P.n_q);
-                if (live) {
-                    float o[32];
-                    const float4* pbv = reinterpret_cast<const float4*>(pbc);
-                    if (whole) {
+                const bool live = (int64_t)tm * kBM + quarter * 32 < P.n_r && gc0 < P.n_q;
+                // the previous chunk has left stg
+                if (live && use_map && lane == 0) tma_store_wait_read();
 #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            const float4 b4 = pbv[j4];
-                            const float fb[4] = {b4.x, b4.y, b4.z, b4.w};
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t v[16];
+                    tmem_wait_ld(vn);
 #pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                o[4 * j4 + u] =
-                                    measure_of<MEASURE>(__uint_as_float(v[4 * j4 + u]), fa, fb[u]);
+                    for (int j = 0; j < 16; ++j) v[j] = vn[j];
+                    __syncwarp();
+                    if (h == 0)
+                        tmem_ld16_async(tbase + (uint32_t)(col_l + 16), vn);
+                    else if (c + kEpiSets < kBN / 32)
+                        tmem_ld16_async(tbase + (uint32_t)((c + kEpiSets) * 32), vn);
+                    if (!live) continue;
+                    const float4* pbv = reinterpret_cast<const float4*>(pbc) + 4 * h;
+#pragma unroll
+                    for (int j4 = 0; j4 < 4; ++j4) {
+                        const float4 b4 = pbv[j4];
+                        float2 o0 = measure_of<MEASURE>(make_float2(__uint_as_float(v[4 * j4]),
+                                                                    __uint_as_float(v[4 * j4 + 1])),
+                                                        both(fa), make_float2(b4.x, b4.y));
+                        float2 o1 = measure_of<MEASURE>(make_float2(__uint_as_float(v[4 * j4 + 2]),
+                                                                    __uint_as_float(v[4 * j4 + 3])),
+                                                        both(fa), make_float2(b4.z, b4.w));
+                        if (!whole) {  // empty (0 / 0 is 0) or missing fingerprints
+                            auto fix = [&](float x, float b) {
+                                return fa >= 0.0f && b >= 0.0f ? fmaxf(x, 0.0f) : P.fill;
+                            };
+                            o0 = make_float2(fix(o0.x, b4.x), fix(o0.y, b4.y));
+                            o1 = make_float2(fix(o1.x, b4.z), fix(o1.y, b4.w));
                         }
-                    } else {
-#pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            const float4 b4 = pbv[j4];
-                            const float fb[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const int j = 4 * j4 + u;
-                                o[j] = (fa >= 0.0f && fb[u] >= 0.0f)
-                                           ? measure_of<MEASURE>(__uint_as_float(v[j]), fa, fb[u])
-                                           : P.fill;
-                            }
-                        }
-                    }
-                    // with the output's tensor map: the warp stages its 32 x 32
-                    // chunk and one lane stores it (under sym, elements below
-                    // the diagonal are rewritten by the mirror pass anyway).
-                    // Else a lane writes 32 consecutive floats of its row:
-                    // eight 16-byte streaming stores when the chunk is whole,
-                    // aligned and (under sym) on or above the diagonal, else
-                    // one by one.
-                    if (tma_chunk) {
-                        if (lane == 0) tma_store_wait_read();  // the previous chunk left stg
-                        __syncwarp();
-#pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4)
-                            *reinterpret_cast<float4*>(stg + lane * 128 + ((j4 ^ (lane & 7)) << 4)) =
-                                make_float4(o[4 * j4], o[4 * j4 + 1], o[4 * j4 + 2], o[4 * j4 + 3]);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0)
-                            tma_store_2d(&out_map, smem_u32(stg), (int)gc0,
-                                         (int)((int64_t)tm * kBM + quarter * 32));
-                    } else if (vec_out && gc0 + 32 <= P.n_q && !(P.sym && gr > gc0)) {
-#pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4)
-                            __stcs(reinterpret_cast<float4*>(orow + gc0) + j4,
-                                   make_float4(o[4 * j4], o[4 * j4 + 1], o[4 * j4 + 2],
-                                               o[4 * j4 + 3]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const int64_t gc = gc0 + j;
-                            if (gc < P.n_q && !(P.sym && gr > gc)) __stcs(orow + gc, o[j]);
-                        }
+                        *reinterpret_cast<float4*>(
+                            stg + lane * 128 + (((4 * h + j4) ^ (lane & 7)) << 4)) =
+                            make_float4(o0.x, o0.y, o1.x, o1.y);
                     }
                 }
-                tmem_wait_ld(vn);
+                // the warp's 32 x 32 chunk is staged; with the output's tensor map
+                // one lane stores it (under sym, elements below the diagonal are
+                // rewritten by the mirror pass anyway), else (rows not 16-byte
+                // aligned, or the last columns) the warp does, 128 consecutive
+                // bytes of a row at a time
+                if (!live) continue;
+                if (tma_chunk) {
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0)
+                        tma_store_2d(&out_map, smem_u32(stg), (int)gc0,
+                                     (int)((int64_t)tm * kBM + quarter * 32));
+                } else {
+                    __syncwarp();
+                    const int64_t row0 = (int64_t)tm * kBM + quarter * 32;
+                    const int rows = (int)min((int64_t)32, P.n_r - row0);
+                    const int64_t gc = gc0 + lane;
+                    float* po = P.out + row0 * P.ld + gc;
+                    if (gc < P.n_q) {
+#pragma unroll 4
+                        for (int r = 0; r < rows; ++r, po += P.ld) {
+                            if (P.sym && row0 + r > gc) continue;
+                            __stcs(po, *reinterpret_cast<const float*>(
+                                           stg + r * 128 + ((((lane >> 2) ^ (r & 7)) << 4) |
+                                                            ((lane & 3) << 2))));
+                        }
+                    }
+                    __syncwarp();
+                }
             }
             __syncwarp();
             tc_fence_before();
@@ -940,8 +1009,11 @@ __global__ void arith_div_check(unsigned long long* bad) {  // n / d, 0 <= n <= 
     if (d > 65536) return;
     const float fd = (float)d;
     unsigned long long b = 0;
-    for (int n = 0; n <= d; ++n)
-        b += __float_as_uint(div_fp((float)n, fd)) != __float_as_uint(__fdiv_rn((float)n, fd));
+    for (int n = 0; n <= d; n += 2) {  // the second half of the last pair may be d + 1
+        const float2 q = div2_int(make_float2((float)n, (float)(n + 1)), both(fd), both(-fd));
+        b += __float_as_uint(q.x) != __float_as_uint(__fdiv_rn((float)n, fd));
+        if (n + 1 <= d) b += __float_as_uint(q.y) != __float_as_uint(__fdiv_rn((float)(n + 1), fd));
+    }
     if (b) atomicAdd(bad, b);
 }
 __global__ void arith_sqrt_check(unsigned long long* bad_sqrt, unsigned long long* bad_rcp) {
@@ -950,15 +1022,18 @@ __global__ void arith_sqrt_check(unsigned long long* bad_sqrt, unsigned long lon
     for (uint32_t u = lo + blockIdx.x * blockDim.x + threadIdx.x; u <= hi;
          u += gridDim.x * blockDim.x) {
         const float p = __uint_as_float(u), root = __fsqrt_rn(p);
-        bs += __float_as_uint(sqrt_fp(p)) != __float_as_uint(root);
-        br += __float_as_uint(rcp_fp(root)) != __float_as_uint(__frcp_rn(root));
+        float2 g, y;
+        root2(make_float2(p, 1.0f), g, y);
+        bs += __float_as_uint(g.x) != __float_as_uint(root);
+        br += __float_as_uint(y.x) != __float_as_uint(__frcp_rn(root));
     }
     if (bs) atomicAdd(bad_sqrt, bs);
     if (br) atomicAdd(bad_rcp, br);
 }
 __device__ __forceinline__ unsigned long long cosine_mismatch(int i, int a, int b) {
     const float p = __fmul_rn((float)a, (float)b), fi = (float)i;
-    return __float_as_uint(div_fp(fi, sqrt_fp(p))) != __float_as_uint(__fdiv_rn(fi, __fsqrt_rn(p)));
+    return __float_as_uint(div2_root(make_float2(fi, 0.0f), make_float2(p, 1.0f)).x) !=
+           __float_as_uint(__fdiv_rn(fi, __fsqrt_rn(p)));
 }
 __global__ void arith_cos_check(unsigned long long* bad) {  // a, b <= 2048, every i <= min(a, b)
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
