@@ -373,3 +373,29 @@ def test_pair_pipeline_long_spectra(cuda_device):
     for limit in (1024, 4096):
         want = oracle.cosine_greedy(ref, qry, 0.01, 0.0, limit)
         assert_same(gpu_dense(ref, qry, P(0.01, limit, 65535), {"mode": 2}), want, f"{limit}")
+
+
+@pytest.mark.parametrize("weights", ["plain", "ties", "close"])
+def test_run_lengths(cuda_device, weights):
+    """Pairs with every number of candidates at which the join's way of resolving them changes
+    (4/5, 8/9, 16/17, 32/33), all in one window or each peak with a few of its own; keys
+    distinct, equal, and equal once rounded to float32."""
+    from cudams.packing import PackedSpectra
+
+    rng = np.random.default_rng(95)
+
+    def make(lens, spacing):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([100.0 + spacing * np.arange(k) for k in lens]).astype(np.float32)
+        b = {"plain": rng.random(off[-1]) + 0.01, "ties": np.round(rng.random(off[-1]) * 2 + 1),
+             "close": 1.0 + rng.integers(0, 1 << 20, off[-1]) * 2.0 ** -45}[weights]
+        return PackedSpectra(mz, None, b, off, 0.0, 1.0, 64)
+
+    for spacing in (0.001, 0.03):
+        ref = make(list(range(1, 9)) * 6 + [12], spacing)
+        qry = make([1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 15, 16, 17, 31, 32, 33] * 5, spacing)
+        want = oracle.cosine_greedy(ref, qry, 0.05, 0.0, 2048)
+        for cfg in ({"mode": 1, "tile_spectra": 64}, {"mode": 1, "tile_spectra": 4096}):
+            assert_same(gpu_dense(ref, qry, P(0.05, 2048), cfg), want, f"{spacing} {cfg}")
+        want = oracle.cosine_greedy(qry, ref, 0.05, 0.0, 2048)
+        assert_same(gpu_dense(qry, ref, P(0.05, 2048), {"mode": 1}), want, f"{spacing} swapped")
