@@ -7,11 +7,12 @@
 // ordered differs.
 //
 // Pipeline of one call (all on one stream, no host synchronisation):
-//   1. prep_kernel       both sets: offsets sane, spectra <= CMS_MAX_PEAKS
+//   1. prep_kernel       both sets in one launch: offsets sane, spectra <= CMS_MAX_PEAKS
 //                        (else every later kernel exits at once and the error
 //                        word is set); sqrt(sum (a*b)^2) per spectrum,
 //                        sequential float64; the reference spectra's length
-//                        classes and the query peaks' bucket counts
+//                        classes and the query peaks' bucket counts;
+//      probe_kernel      per reference peak its window and buckets
 //   2. order_scatter     reference spectra ordered by peak count, largest
 //                        first (log2 length classes), for load balance
 //   3. index kernels     query spectra are cut into tiles of tile_spectra;
@@ -30,7 +31,7 @@
 //                        memory, extended in global memory).  Each query's
 //                        run is then resolved greedily: 1-4 candidates in
 //                        closed form by one lane, 5-8 by an 8-lane segment,
-//                        9-32 by the warp.
+//                        9-16 by half a warp, 17-32 by the warp.
 //                        The sweep is load-balanced: a chunk's window entries
 //                        are expanded 32 at a time over the warp, and each
 //                        query's candidates are chained through a per-warp
@@ -241,37 +242,63 @@ struct PrepSide {
     uint32_t* cls_count;  // spectra per length class (null: not wanted)
     uint32_t* cnt;        // peaks per (tile, bucket) of the m/z index (null: not wanted)
     uint32_t* cnt2;       // the same of the neutral-loss index (null: not wanted)
-    Probe* probe;         // per peak, for the sweeping side (null: not wanted)
     double* w;            // per peak a * b (null: not wanted)
-    uint2* probe2;        // per peak, its shifted window's buckets (null: not wanted)
-    double tol, shift;    // of the windows
-    int is_ref;           // the sweeping side is the reference side
 };
 
-// The windows and buckets of one sweeping peak.
-__device__ void make_probe(const PrepSide& P, const IndexGeom& g, int64_t s, int64_t k,
-                           uint32_t* err) {
-    const float mz = P.S.mz[k];
-    Probe p{1.0f, 0.0f, kNoBucket, 0u};
-    float L, H;
-    const bool ok = !P.is_ref        ? Window<false, false>::bounds(mz, P.tol, P.shift, L, H)
-                    : P.shift == 0.0 ? Window<true, true>::bounds(mz, P.tol, P.shift, L, H)
-                                     : Window<true, false>::bounds(mz, P.tol, P.shift, L, H);
-    if (ok) {
-        const uint2 b = bucket_range(L, H, g);
-        p = Probe{L, H, b.x, b.y};
-    } else {
-        atomicOr(err, kErrBadOffsets);
-    }
-    *reinterpret_cast<uint4*>(&P.probe[k]) =
-        make_uint4(__float_as_uint(p.lo), __float_as_uint(p.hi), p.bl, p.bh);
-    if (P.probe2) {
-        uint2 b = make_uint2(kNoBucket, 0u);
-        if (nl_window(mz, P.S.prec[s], P.tol, L, H))
-            b = bucket_range(L, H, g);
-        else
+// The sides of a call in one launch: its first blocks0 blocks take side 0.
+struct PrepSides {
+    PrepSide side[2];
+    int blocks0;
+};
+
+struct ProbeArgs {
+    SpecSet S;          // the sweeping side
+    Probe* probe;       // per peak
+    uint2* probe2;      // per peak, its shifted window's buckets (null: not wanted)
+    double tol, shift;  // of the windows
+    int is_ref;         // the sweeping side is the reference side
+};
+
+// The windows and buckets of every sweeping peak, a thread a peak.  In a launch
+// of its own: warps of the kernel below, a few spectra each, took 20 us for
+// them at 1024 spectra and 25 at 20000 (4 and 10 here).
+constexpr int kProbeThreads = 256;
+__global__ void __launch_bounds__(kProbeThreads)
+probe_kernel(ProbeArgs P, IndexGeom g, const uint32_t* bad, uint32_t* err) {
+    if (*bad) return;
+    const int64_t first = P.S.off[0], last = P.S.off[P.S.n];
+    const int64_t step = (int64_t)gridDim.x * kProbeThreads;
+    for (int64_t k = first + (int64_t)blockIdx.x * kProbeThreads + threadIdx.x; k < last; k += step) {
+        const float mz = P.S.mz[k];
+        Probe p{1.0f, 0.0f, kNoBucket, 0u};
+        float L, H;
+        const bool ok = !P.is_ref        ? Window<false, false>::bounds(mz, P.tol, P.shift, L, H)
+                        : P.shift == 0.0 ? Window<true, true>::bounds(mz, P.tol, P.shift, L, H)
+                                         : Window<true, false>::bounds(mz, P.tol, P.shift, L, H);
+        if (ok) {
+            const uint2 b = bucket_range(L, H, g);
+            p = Probe{L, H, b.x, b.y};
+        } else {
             atomicOr(err, kErrBadOffsets);
-        P.probe2[k] = b;
+        }
+        *reinterpret_cast<uint4*>(&P.probe[k]) =
+            make_uint4(__float_as_uint(p.lo), __float_as_uint(p.hi), p.bl, p.bh);
+        if (P.probe2) {
+            int64_t s = 0, e = P.S.n;  // the spectrum: off[s] <= k < off[e]
+            while (e - s > 1) {
+                const int64_t m = s + (e - s) / 2;
+                if (P.S.off[m] <= k)
+                    s = m;
+                else
+                    e = m;
+            }
+            uint2 b = make_uint2(kNoBucket, 0u);
+            if (nl_window(mz, P.S.prec[s], P.tol, L, H))
+                b = bucket_range(L, H, g);
+            else
+                atomicOr(err, kErrBadOffsets);
+            P.probe2[k] = b;
+        }
     }
 }
 
@@ -280,28 +307,36 @@ __device__ void make_probe(const PrepSide& P, const IndexGeom& g, int64_t s, int
 // the call; such a spectrum is skipped here.
 //
 // A norm is one float64 sum in peak order, a serial chain, so a warp takes
-// kPrepSpectra spectra at once: their peaks come 32 at a time with coalesced
-// loads through a shared-memory tile, and lane j adds up spectrum j while the
-// next 32 peaks of each are in flight.  One thread a spectrum, reading its
-// peaks one after the other, took 24 us for 1024 spectra of up to 200 peaks,
-// 84 us for 50000 of up to 1000 and 445 us for 900 of up to 2000, for each
-// side; this takes 10, 52 and 60 us (17 and 84 us with the bucket counts, which
-// took 7 and 47 us in a launch of their own).
-constexpr int kPrepSpectra = 8;
+// kPrepSpectra spectra at once: their peaks come 32 * kPrepPeaks at a time with
+// coalesced loads through a shared-memory tile, and lane j adds up spectrum j
+// while the next peaks of each are in flight.  One thread a spectrum, reading
+// its peaks one after the other, took 24 us for 1024 spectra of up to 200
+// peaks, 84 us for 50000 of up to 1000 and 445 us for 900 of up to 2000.  What
+// is left is the time of a round of loads, and how many rounds a long spectrum
+// has: both sides of 1024 uniform spectra 9 us, of 12288 lognormal ones 49 us,
+// with the bucket counts; eight spectra of 32 peaks a round 18 and 66, four of
+// 128 12 and 62, one of 256 8 and 62.
+constexpr int kPrepSpectra = 2;
+constexpr int kPrepPeaks = 4;  // of a spectrum, per lane and round
 constexpr int kPrepThreads = 128;
 __global__ void __launch_bounds__(kPrepThreads)
-prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks) {
-    __shared__ double s_tile[kPrepThreads / 32][kPrepSpectra][33];
+prep_kernel(const __grid_constant__ PrepSides sides, IndexGeom g, uint32_t* bad, uint32_t* err,
+            int max_peaks) {
+    const bool second = (int)blockIdx.x >= sides.blocks0;
+    const PrepSide& P = sides.side[second];
+    const int block = (int)blockIdx.x - (second ? sides.blocks0 : 0);
+    const int blocks = second ? (int)gridDim.x - sides.blocks0 : sides.blocks0;
+    __shared__ double s_tile[kPrepThreads / 32][kPrepSpectra][32 * kPrepPeaks + 1];
     __shared__ uint32_t s_cls[kOrderClasses];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
-    double(*tile)[33] = s_tile[wid];
+    double(*tile)[32 * kPrepPeaks + 1] = s_tile[wid];
     if (threadIdx.x < kOrderClasses) s_cls[threadIdx.x] = 0u;
     __syncthreads();
     const unsigned mask = (unsigned)(g.nb - 1);
-    const int64_t warps = (int64_t)gridDim.x * (kPrepThreads / 32);
+    const int64_t warps = (int64_t)blocks * (kPrepThreads / 32);
     const int64_t n = P.S.n;
-    for (int64_t s0 = ((int64_t)blockIdx.x * (kPrepThreads / 32) + wid) * kPrepSpectra; s0 < n;
+    for (int64_t s0 = ((int64_t)block * (kPrepThreads / 32) + wid) * kPrepSpectra; s0 < n;
          s0 += warps * kPrepSpectra) {
         int64_t lo = 0;
         int len = 0;
@@ -322,56 +357,60 @@ prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks
         }
         const int longest = __reduce_max_sync(full, len);
         // the loads of all spectra are issued before the first is used
-        double v[kPrepSpectra], w[kPrepSpectra];
-        float z[kPrepSpectra];
-        auto load = [&](int c) {
+        constexpr int kRound = 32 * kPrepPeaks, kAll = kPrepSpectra * kPrepPeaks;
+        double v[kAll], w[kAll];
+        float z[kAll];
+        auto each = [&](int c, auto&& f) {  // (index, spectrum, offset in it, in it?)
 #pragma unroll
-            for (int j = 0; j < kPrepSpectra; ++j) {
-                const int64_t k = __shfl_sync(full, lo, j) + c + lane;
-                const bool in = c + lane < __shfl_sync(full, len, j);
-                v[j] = in ? P.S.b[k] : 0.0;
-                w[j] = (in && P.S.a) ? P.S.a[k] : 1.0;
-                z[j] = (in && P.cnt) ? P.S.mz[k] : 0.f;
+            for (int i = 0; i < kAll; ++i) {
+                const int j = i / kPrepPeaks, o = c + 32 * (i % kPrepPeaks) + lane;
+                f(i, j, o, o < __shfl_sync(full, len, j));
             }
+        };
+        auto load = [&](int c) {
+            each(c, [&](int i, int j, int o, bool in) {
+                const int64_t k = __shfl_sync(full, lo, j) + o;
+                v[i] = in ? P.S.b[k] : 0.0;
+                w[i] = (in && P.S.a) ? P.S.a[k] : 1.0;
+                z[i] = (in && P.cnt) ? P.S.mz[k] : 0.f;
+            });
         };
         auto weights = [&](int c) {
             if (!P.w) return;
-#pragma unroll
-            for (int j = 0; j < kPrepSpectra; ++j) {
-                const int64_t k = __shfl_sync(full, lo, j) + c + lane;
-                if (c + lane < __shfl_sync(full, len, j)) P.w[k] = __dmul_rn(w[j], v[j]);
-            }
+            each(c, [&](int i, int j, int o, bool in) {
+                const int64_t k = __shfl_sync(full, lo, j) + o;
+                if (in) P.w[k] = __dmul_rn(w[i], v[i]);
+            });
         };
         auto count = [&](int c) {
             if (!P.cnt) return;
-#pragma unroll
-            for (int j = 0; j < kPrepSpectra; ++j) {
-                if (c + lane >= __shfl_sync(full, len, j)) continue;
+            each(c, [&](int i, int j, int, bool in) {
+                if (!in) return;
                 const int64_t t = (s0 + j) / g.tile * (int64_t)g.nb;
-                atomicAdd(&P.cnt[t + ((unsigned)bucket_of(z[j], g.inv_w) & mask)], 1u);
+                atomicAdd(&P.cnt[t + ((unsigned)bucket_of(z[i], g.inv_w) & mask)], 1u);
                 if (P.cnt2) {
-                    const float d = loss_value(z[j], P.S.prec[s0 + j]);
+                    const float d = loss_value(z[i], P.S.prec[s0 + j]);
                     atomicAdd(&P.cnt2[t + ((unsigned)bucket_of(d, g.inv_w) & mask)], 1u);
                 }
-            }
+            });
         };
         double acc = 0.0;
         load(0);
-        for (int c = 0; c < longest; c += 32) {
+        for (int c = 0; c < longest; c += kRound) {
             __syncwarp();
 #pragma unroll
-            for (int j = 0; j < kPrepSpectra; ++j) {
-                const double x = __dmul_rn(w[j], v[j]);
-                tile[j][lane] = __dmul_rn(x, x);
+            for (int i = 0; i < kAll; ++i) {
+                const double x = __dmul_rn(w[i], v[i]);
+                tile[i / kPrepPeaks][32 * (i % kPrepPeaks) + lane] = __dmul_rn(x, x);
             }
             count(c);
             weights(c);
             __syncwarp();
-            if (c + 32 < longest) load(c + 32);
+            if (c + kRound < longest) load(c + kRound);
             // past a spectrum's end the tile holds +0.0, which leaves the sum as it is
             if (lane < kPrepSpectra) {
-#pragma unroll 8
-                for (int k = 0; k < 32; ++k) acc = __dadd_rn(acc, tile[lane][k]);
+#pragma unroll 16
+                for (int k = 0; k < kRound; ++k) acc = __dadd_rn(acc, tile[lane][k]);
             }
         }
         if (lane < kPrepSpectra && s0 + lane < n) {
@@ -379,13 +418,6 @@ prep_kernel(PrepSide P, IndexGeom g, uint32_t* bad, uint32_t* err, int max_peaks
             P.sn[s0 + lane] = sn;
             if (P.rn) P.rn[s0 + lane] = recip_norm(sn);
         }
-        if (P.probe)
-#pragma unroll 1
-            for (int j = 0; j < kPrepSpectra; ++j) {
-                const int64_t lj = __shfl_sync(full, lo, j);
-                const int nj = __shfl_sync(full, len, j);
-                for (int i = lane; i < nj; i += 32) make_probe(P, g, s0 + j, lj + i, err);
-            }
         __syncwarp();
     }
     __syncthreads();
@@ -2590,6 +2622,18 @@ int blocks_for(int64_t n, int per, int sms) {
 constexpr int kPrepPerBlock = kPrepSpectra * (kPrepThreads / 32);
 constexpr int kScatterThreads = 256;  // index scatter: a warp per spectrum
 
+// Prepare one or two spectrum sets (the second may be empty) in one launch.
+void launch_prep(const PrepSide& p0, const PrepSide& p1, const IndexGeom& g, uint32_t* bad,
+                 uint32_t* err, int max_peaks, int sms, cudaStream_t s) {
+    const PrepSides sides{{p0, p1}, blocks_for(p0.S.n, kPrepPerBlock, sms)};
+    const int blocks1 = p1.S.n > 0 ? blocks_for(p1.S.n, kPrepPerBlock, sms) : 0;
+    prep_kernel<<<sides.blocks0 + blocks1, kPrepThreads, 0, s>>>(sides, g, bad, err, max_peaks);
+}
+void launch_probe(const ProbeArgs& p, const IndexGeom& g, const uint32_t* bad, uint32_t* err, int sms,
+                  cudaStream_t s) {
+    probe_kernel<<<blocks_for(p.S.n_peaks, kProbeThreads, sms), kProbeThreads, 0, s>>>(p, g, bad, err);
+}
+
 // Launch the join.  Persistent (waves == 0): one resident CTA per slot, each
 // warp pulling work until none is left; CTA b owns global-pool slices
 // 8b..8b+7, so the grid may not exceed the resident CTAs.  Bounded
@@ -2731,15 +2775,14 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     const IndexGeom g{p.tile, p.n_tiles, p.nb, 1.0 / p.width};
     const int sms = ctx->sm_count;
     {
-        StageScope sc(ctx, 0, 2, s);
+        StageScope sc(ctx, 0, idx ? 2 : 1, s);
         const int max_peaks = args.modified ? kModifiedMaxPeaks : CMS_MAX_PEAKS;
-        const PrepSide pr{args.ref, snR,   nullptr, idx ? cls_count : nullptr, nullptr, nullptr,
-                          probe,    wR,    probe2, args.tol, args.shift, 1};
-        const PrepSide pq{args.qry, snQ, rnQ, nullptr, cur, cur2};
-        prep_kernel<<<blocks_for(nR, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-            pr, g, bad, ctx->err_word, max_peaks);
-        prep_kernel<<<blocks_for(nQ, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-            pq, g, bad, ctx->err_word, max_peaks);
+        launch_prep(PrepSide{args.ref, snR, nullptr, idx ? cls_count : nullptr, nullptr, nullptr, wR},
+                    PrepSide{args.qry, snQ, rnQ, nullptr, cur, cur2}, g, bad, ctx->err_word,
+                    max_peaks, sms, s);
+        if (idx)
+            launch_probe(ProbeArgs{args.ref, probe, probe2, args.tol, args.shift, 1}, g, bad,
+                         ctx->err_word, sms, s);
     }
     CMS_CUDA_TRY(cudaGetLastError());
 
@@ -3302,10 +3345,8 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     CMS_CUDA_TRY(cudaGetDevice(&dev));
     CMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const IndexGeom none{1, 1, 1, 1.0};
-    prep_kernel<<<blocks_for(n_ref, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-        PrepSide{args.ref, snR}, none, bad, err, CMS_MAX_PEAKS);
-    prep_kernel<<<blocks_for(n_q, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-        PrepSide{args.qry, snQ}, none, bad, err, CMS_MAX_PEAKS);
+    launch_prep(PrepSide{args.ref, snR}, PrepSide{args.qry, snQ}, none, bad, err, CMS_MAX_PEAKS, sms,
+                s);
     CMS_CUDA_TRY(cudaGetLastError());
 
     PairParams pp{};
@@ -3436,9 +3477,8 @@ extern "C" int cms_library_create(cms_ctx* ctx, const float* mz, const double* a
     if (e == cudaSuccess) e = cudaMemsetAsync(cur, 0, sizeof(uint32_t) * n_cur, s);
     if (e == cudaSuccess) {
         const int sms = ctx->sm_count;
-        prep_kernel<<<blocks_for(n, kPrepPerBlock, sms), kPrepThreads, 0, s>>>(
-            PrepSide{L->spec, L->sn, L->rn, nullptr, cur}, L->g, L->bad, ctx->err_word,
-            CMS_MAX_PEAKS);
+        launch_prep(PrepSide{L->spec, L->sn, L->rn, nullptr, cur}, PrepSide{}, L->g, L->bad,
+                    ctx->err_word, CMS_MAX_PEAKS, sms, s);
         index_sums_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, cur + n_cur, L->bad);
         index_scan_kernel<<<n_chunks, kScanThreads, 0, s>>>(L->g, cur, L->tab, cur + n_cur, L->bad);
         index_scatter_kernel<false><<<blocks_for(n, kScatterThreads / 32, sms), kScatterThreads, 0,
@@ -3540,12 +3580,11 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
 
     {
-        StageScope sc(ctx, 0, 1, s);
-        prep_kernel<<<blocks_for(n_q, kPrepPerBlock, ctx->sm_count), kPrepThreads, 0, s>>>(
-            PrepSide{Q, snQ, nullptr, cls_count, nullptr, nullptr, probe, nullptr, nullptr,
-                     lib->tol, lib->shift, 0},
-            lib->g, bad, ctx->err_word,
-            CMS_MAX_PEAKS);
+        StageScope sc(ctx, 0, 2, s);
+        launch_prep(PrepSide{Q, snQ, nullptr, cls_count}, PrepSide{}, lib->g, bad, ctx->err_word,
+                    CMS_MAX_PEAKS, ctx->sm_count, s);
+        launch_probe(ProbeArgs{Q, probe, nullptr, lib->tol, lib->shift, 0}, lib->g, bad,
+                     ctx->err_word, ctx->sm_count, s);
     }
     {
         StageScope sc(ctx, 1, 1, s);

@@ -399,3 +399,25 @@ def test_run_lengths(cuda_device, weights):
             assert_same(gpu_dense(ref, qry, P(0.05, 2048), cfg), want, f"{spacing} {cfg}")
         want = oracle.cosine_greedy(qry, ref, 0.05, 0.0, 2048)
         assert_same(gpu_dense(qry, ref, P(0.05, 2048), {"mode": 1}), want, f"{spacing} swapped")
+
+
+@pytest.mark.parametrize("n", [1, 2, 7])
+def test_preparation_rounds(cuda_device, n):
+    """Norms, weights and windows of spectra that end at, before and after a round of the
+    preparation's loads, for one, two and an odd number of them a side."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(96)
+    lens = np.array([129, 0, 128, 1, 127, 256, 1000])
+
+    def make(lens):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(50.0, 150.0, k)) for k in lens])
+        inten = rng.random(off[-1]) + 0.01
+        return pack_csr(mz.astype(np.float32), inten.astype(np.float32), off, None, mz_power=1.0,
+                        intensity_power=0.5)
+
+    ref, qry = make(lens[:n]), make(np.roll(lens, 3)[:n])
+    want = oracle.cosine_greedy(ref, qry, 0.02, 0.0, 4096)
+    for cfg in ({"mode": 1, "tile_spectra": 32}, {"mode": 2}):
+        assert_same(gpu_dense(ref, qry, P(0.02, 4096), cfg), want, f"{n} {cfg}")
