@@ -63,7 +63,6 @@ namespace {
 
 constexpr int kJoinWarps = 8;
 constexpr int kJoinThreads = kJoinWarps * 32;
-constexpr int kPool = 256;        // candidate pool entries per warp
 constexpr int kMidRun = 8;        // runs up to this length are resolved four per warp step
 constexpr int kMaxTile = 4096;    // max query spectra per tile
 constexpr int kOrderClasses = 17; // log2 length classes (0..16)
@@ -696,7 +695,8 @@ struct JoinParams {
     // tuner's measured candidate-pool split); 0: init_width_scale decides
     int width_by_class[kOrderClasses];
     int warp_smem_bytes;     // per-warp slice of dynamic shared memory
-    int pool_max;            // candidates a sweep may hold: kPoolMax, or kPool without gpool
+    int pool_smem;           // candidates of the pool in shared memory (join_pool)
+    int pool_max;            // candidates a sweep may hold: kPoolMax, or pool_smem without gpool
     int max_fetch;           // work items per warp before it exits (0: no limit)
     unsigned char* gpool;    // global pool extension, kGPool * 16 bytes per warp (or null)
     // bounded launches: a CTA claims one of n_slots global-pool slices (a bit
@@ -720,7 +720,8 @@ constexpr int kIlpR = 2;
 constexpr int kSearchWaves = 4;            // waves of short-lived CTAs per library search
 constexpr int kSlotWords = 64;             // slot bitmap words of a bounded join launch
 constexpr int kPoolMax = 4096;             // candidates per sweep: smem pool + global extension
-constexpr int kGPool = kPoolMax - kPool;   // global extension entries per warp
+constexpr int kPoolMin = 128;              // of them at least in shared memory (join_pool)
+constexpr int kGPool = kPoolMax - kPoolMin;  // global extension entries per warp
 static_assert(kPoolMax <= 4096, "pool slots are packed into 12 bits");
 static_assert(kMaxTile <= 4096, "query indices within a range are packed into 12 bits");
 
@@ -738,15 +739,16 @@ constexpr uint32_t kHasNext = 1u << 24;
 __device__ __forceinline__ int meta_query(uint32_t m) { return (int)(m & 0xFFFu); }
 __device__ __forceinline__ int meta_next(uint32_t m) { return (int)((m >> 12) & 0xFFFu); }
 
-// A warp's candidate pool: the first kPool entries live in shared memory, the
+// A warp's candidate pool: the first n_smem entries live in shared memory, the
 // rest in a per-warp slice of global scratch (L2-resident), so that a large
 // reference spectrum is swept once even when it has thousands of candidates
 // in a tile.  Slots are indices into the concatenation; an access is one
-// 16-byte generic load or store (gbase points kPool entries before the slice).
+// 16-byte generic load or store (gbase points n_smem entries before the slice).
 struct Pool {
     PoolEntry* sbase;
     PoolEntry* gbase;
-    __device__ __forceinline__ PoolEntry* at(int i) const { return (i < kPool ? sbase : gbase) + i; }
+    int n_smem;
+    __device__ __forceinline__ PoolEntry* at(int i) const { return (i < n_smem ? sbase : gbase) + i; }
     __device__ __forceinline__ PoolEntry get(int i) const {
         const uint4 v = *reinterpret_cast<const uint4*>(at(i));
         return PoolEntry{__hiloint2double((int)v.y, (int)v.x), v.z, v.w};
@@ -760,10 +762,6 @@ struct Pool {
 
 // Per-warp shared-memory slice (offsets in bytes; the head table's length
 // depends on the tile size, so the slice size is computed at launch).
-//   pool  PoolEntry [kPool]
-//   head  uint16 [tile]      one per query of the range: (epoch << 12) | slot of
-//                            its last candidate; a head of another epoch means
-//                            "no candidate yet"
 //   rec   uint4 [32]         sweep: the chunk's peaks with window entries, in order:
 //                            stream offset, window, lane.  Resolution: uint16 queue
 //                            of chain heads with two or more candidates
@@ -772,15 +770,33 @@ struct Pool {
 //   runs  uint32 [kLongRuns] runs of five or more candidates queued for the warp:
 //                            slot of the chain head | length << 12; runs of at
 //                            most kMidRun from the front, longer ones from the back
-//   lists uint16 [kLists]    slots of the long runs being resolved: 32 of up to 8
-//                            candidates or 16 of up to 32
+//   lists uint16 [kLists]    slots of the long runs being resolved: 32 of up to
+//                            8 candidates or 8 of up to 32
 //   t0    uint64             %globaltimer at the current item's start (trace only)
+//   head  uint16 [tile]      one per query of the range: (epoch << 12) | slot of
+//                            its last candidate; a head of another epoch means
+//                            "no candidate yet"
+//   pool  PoolEntry [join_pool(tile)]
 constexpr int kLongRuns = 64;
-constexpr int kLists = 512;
+constexpr int kLists = 256;
 constexpr int kQueue = 256;
 __host__ __device__ constexpr int head_bytes(int tile) { return (2 * tile + 15) & ~15; }
+constexpr int kSliceFixed = 16 * 32 + 8 * 32 + 4 * kLongRuns + 2 * kLists + 16;
+// Pool entries in shared memory, between kPoolMin and kPoolMost: as many as
+// leave the L1 cache its share when three CTAs are resident.  Above kSliceTarget
+// bytes a warp the next larger carve-out of shared memory is taken, which
+// costs about 32 KB of L1, where the bucket table's and the tile stream's
+// sectors hit: 50000 x 50000 lognormal spectra in tiles of 1792 take 9.6 ms
+// with 8208 bytes a warp, 8.9 ms with 8112 (186 entries) and 8.95 ms with 7800.
+// More than 256 entries gain nothing where the tiles are small.
+constexpr int kPoolMost = 256;
+constexpr int kSliceTarget = 8112;
+__host__ __device__ constexpr int join_pool(int tile) {
+    const int fit = (kSliceTarget - kSliceFixed - head_bytes(tile)) / 16;
+    return fit < kPoolMin ? kPoolMin : fit > kPoolMost ? kPoolMost : fit;
+}
 __host__ __device__ constexpr int warp_slice_bytes(int tile) {
-    return 16 * kPool + head_bytes(tile) + 16 * 32 + 8 * 32 + 4 * kLongRuns + 2 * kLists + 16;
+    return kSliceFixed + head_bytes(tile) + 16 * join_pool(tile);
 }
 
 // Reference peak of a candidate's generation word.  Modified cosine marks
@@ -831,13 +847,13 @@ join_kernel(JoinParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int hb = head_bytes(P.g.tile);
     unsigned char* slice = smem_raw + (size_t)(threadIdx.x >> 5) * P.warp_smem_bytes;
-    uint16_t* head = reinterpret_cast<uint16_t*>(slice + 16 * kPool);
-    uint4* s_rec = reinterpret_cast<uint4*>(slice + 16 * kPool + hb);
+    uint4* s_rec = reinterpret_cast<uint4*>(slice);
     uint16_t* queue = reinterpret_cast<uint16_t*>(s_rec);
-    double* s_wa = reinterpret_cast<double*>(slice + 16 * kPool + hb + 16 * 32);
-    uint32_t* long_runs = reinterpret_cast<uint32_t*>(slice + 16 * kPool + hb + 24 * 32);
+    double* s_wa = reinterpret_cast<double*>(slice + 16 * 32);
+    uint32_t* long_runs = reinterpret_cast<uint32_t*>(slice + 24 * 32);
     uint16_t* lists = reinterpret_cast<uint16_t*>(long_runs + kLongRuns);
     unsigned long long* s_t0 = reinterpret_cast<unsigned long long*>(lists + kLists);
+    uint16_t* head = reinterpret_cast<uint16_t*>(slice + kSliceFixed);
     // Global-pool slice of this CTA: blockIdx.x, or under bounded launches a
     // slice claimed from the slot bitmap (at most n_slots CTAs are resident at
     // once, so one is free; if a release has not landed yet the CTA runs with
@@ -870,13 +886,14 @@ join_kernel(JoinParams P) {
         __syncthreads();
         pslot = s_slot;
     }
-    const int pool_max = (P.gpool && pslot >= 0) ? P.pool_max : kPool;
+    const int pool_max = (P.gpool && pslot >= 0) ? P.pool_max : P.pool_smem;
     Pool pool;
-    pool.sbase = reinterpret_cast<PoolEntry*>(slice);
+    pool.n_smem = P.pool_smem;
+    pool.sbase = reinterpret_cast<PoolEntry*>(slice + kSliceFixed + hb);
     pool.gbase = pool.sbase;
     if (P.gpool && pslot >= 0)
         pool.gbase = reinterpret_cast<PoolEntry*>(P.gpool) +
-                     ((size_t)pslot * kJoinWarps + (threadIdx.x >> 5)) * (size_t)kGPool - kPool;
+                     ((size_t)pslot * kJoinWarps + (threadIdx.x >> 5)) * (size_t)kGPool - P.pool_smem;
 
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -1352,7 +1369,7 @@ join_kernel(JoinParams P) {
                         // Runs of 5..8 candidates are resolved four at a time on 8-lane segments,
                         // of 9..16 two at a time, longer ones by the whole warp; more than 32
                         // candidates, or match_limit, go to the pair kernel.  Their chains are
-                        // walked first, a lane a run and 32 (16 long) runs at a time, which leaves
+                        // walked first, a lane a run and 32 (8 longer) runs at a time, which leaves
                         // the slots of run i at lists[i + stride * j].  A walk per resolved run was
                         // a chain of up to 32 dependent reads each, and all pairs of a run were
                         // compared as float64 keys with their generation words: 8.83 -> 6.32 ms
@@ -1361,7 +1378,7 @@ join_kernel(JoinParams P) {
 #pragma unroll 1
                         for (int r0 = 0; r0 < n_mid + n_big;) {
                             const bool mid = r0 < n_mid;
-                            const int stride = mid ? 32 : 16;
+                            const int stride = mid ? kLists / kMidRun : kLists / 32;
                             const int cnt = min(stride, (mid ? n_mid : n_mid + n_big) - r0);
                             int Lw = 0;  // length of the run this lane walked
                             if (lane < cnt) {
@@ -2664,7 +2681,7 @@ int launch_join(cms_ctx* ctx, JoinParams jp, size_t smem, size_t gpool_warps, in
         if (!jp.slots) jp.gpool = nullptr;
         jp.n_slots = (int)std::min<int64_t>(resident, (int64_t)(gpool_warps / kJoinWarps));
         if (jp.n_slots <= 0) jp.gpool = nullptr;
-        if (!jp.gpool) jp.pool_max = kPool;
+        if (!jp.gpool) jp.pool_max = jp.pool_smem;
     } else {
         jp.max_fetch = 0;
         jp.slots = nullptr;
@@ -2918,6 +2935,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         jp.init_width_scale = (float)(0.5 * kPoolMax / lambda);
     }
     jp.warp_smem_bytes = warp_slice_bytes(p.tile);
+    jp.pool_smem = join_pool(p.tile);
     jp.pool_max = kPoolMax;
     jp.max_fetch = 0;
     jp.gpool = gpool;
@@ -3614,6 +3632,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     // A search runs as kSearchWaves waves of short-lived CTAs (an equal share
     // of fetches per warp) so that searches on other streams interleave with
     // it on the device; each CTA claims a global-pool slice while it lives.
+    jp.pool_smem = join_pool(lib->g.tile);
     jp.pool_max = kPoolMax;
     jp.gpool = gpool;
     jp.slots = slots;

@@ -5,7 +5,7 @@ Two decisions matter for cms_cosine_greedy:
     pair kernel over the whole matrix (mode 2) when nearly every pair has
     hundreds (dense, overflow-heavy spectra);
   * tile_spectra: the join keeps every candidate of (reference, query tile)
-    in a 256-entry shared-memory pool, so the tile must be small enough that
+    in a shared-memory pool of 128 to 256, so the tile must be small enough that
     the pool rarely overflows, and large enough that the bucket lookups per
     reference peak are amortised over many queries.
 
@@ -120,9 +120,11 @@ TARGET_ITEMS = 100_000
 # time per pair falls from 7.75 ps at ~130 candidates per item (1312 queries)
 # to 7.09 ps at ~200 (2048); below ~75 the per-peak bucket lookups dominate
 CANDIDATES_PER_ITEM = 200.0
-# largest automatic tile: the join's per-warp query counters grow with the
-# tile, and above ~2300 queries three CTAs no longer fit an SM
-MAX_AUTO_TILE = 2048
+# largest automatic tile: the join's per-warp query heads grow with the tile and
+# take the place of its candidate pool in shared memory.  50000 x 50000
+# lognormal spectra: 8.96 ms with tiles of 1536, 8.9 ms with 1696 and 1856,
+# 9.2 ms with 2048; searches differ by less than their runs do
+MAX_AUTO_TILE = 1792
 
 
 def heuristic_config(stats: WorkloadStats, n_q: int, n_ref: int = 1 << 30) -> dict:
