@@ -41,8 +41,8 @@
 //                        stores just before, and each run stores its result
 //                        over its zeros.  Pairs with longer runs (or >=
 //                        match_limit candidates) go to a spill list.
-//   5. pair_kernel       one CTA per spilled pair (or per pair of the whole
-//                        matrix in mode 2): exact generation-order sweep with
+//   5. pair_kernel       a CTA per heavy spilled pair (or per pair of the whole
+//                        matrix in mode 2), a warp per light one: exact generation-order sweep with
 //                        match_limit truncation, bitonic sort of (key, gen)
 //                        (in registers when there are eight candidates a
 //                        thread, else in shared memory), warp greedy with
@@ -653,16 +653,26 @@ struct TraceOut {
     unsigned int tag;
 };
 
+// Pairs for the pair kernel, which works on them by size: heavy ones from the
+// front of the list, light ones from its back.
+// A pair with a longer spectrum than this is heavy: a warp alone would be the last
+// one running.  (128, 256, 512 and 1024 peaks: 209, 180, 211 and 285 us for 12345
+// symmetric spectra, 124, 113, 174 and 270 for sparse 20000 x 20000, 340, 297, 243
+// and 223 for modified cosine of 9001 x 11003.)
+constexpr int kHeavyPeaks = 256;
 struct SpillList {
-    int2* pairs;  // (reference, query)
-    unsigned int* count;
+    int2* pairs;                // (reference, query)
+    unsigned long long* count;  // heavy pairs | light pairs << 32
     unsigned int cap;
 };
 
-__device__ __forceinline__ void spill_push(const SpillList& sl, int r, int q, uint32_t* err) {
-    const unsigned int pos = atomicAdd(sl.count, 1u);
-    if (pos < sl.cap)
-        sl.pairs[pos] = make_int2(r, q);
+__device__ __forceinline__ void spill_push(const SpillList& sl, int r, int q, int64_t longest,
+                                           uint32_t* err) {
+    const bool heavy = longest > kHeavyPeaks;
+    const unsigned long long n = atomicAdd(sl.count, heavy ? 1ull : 1ull << 32);
+    const unsigned int front = (unsigned int)n, back = (unsigned int)(n >> 32);
+    if ((unsigned long long)front + back < sl.cap)
+        sl.pairs[heavy ? front : sl.cap - 1 - back] = make_int2(r, q);
     else
         atomicOr(err, kErrSpillOverrun);
 }
@@ -963,7 +973,9 @@ join_kernel(JoinParams P) {
         };
         // a run for the pair kernel (its dense cells marked until then)
         auto spill_run = [&](int q) {
-            spill_push(P.spill, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a, P.err);
+            const int64_t nq = P.B.off[b_begin + q + 1] - P.B.off[b_begin + q];
+            spill_push(P.spill, A_IS_REF ? a : b_begin + q, A_IS_REF ? b_begin + q : a,
+                       max((int64_t)na, nq), P.err);
             if (!SPARSE) {
                 __stcs(P.dense.score + row() + q, __int_as_float(0x7fc00000));
                 __stcs(P.dense.matches + row() + q, -1);
@@ -1529,7 +1541,7 @@ join_kernel(JoinParams P) {
 }
 
 // ---------------------------------------------------------------------------
-// 5. pair kernel: one CTA per pair
+// 5. pair kernel: a CTA or a warp per pair
 // ---------------------------------------------------------------------------
 struct PairParams {
     SpecSet R;
@@ -1540,9 +1552,10 @@ struct PairParams {
     double shift;
     int match_limit;
     int cap;  // power of two >= match_limit
+    int cache;  // pair_kernel: query m/z values kept in shared memory (pair_cache)
     // work: either the spill list (pairs != nullptr) or every pair of R x Q
     const int2* pairs;
-    const unsigned int* n_pairs;
+    const unsigned long long* n_pairs;  // SpillList::count
     unsigned int pairs_cap;
     unsigned long long* work;
     DenseOut dense;
@@ -1591,6 +1604,9 @@ __device__ __forceinline__ void sort8_local(Cand (&c)[8], int base, int kk) {
 // barrier 1.
 struct BlockSync {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+struct WarpSync {
+    __device__ __forceinline__ void operator()() const { __syncwarp(); }
 };
 struct GroupSync {
     int n;  // participating threads (a multiple of 32)
@@ -1683,10 +1699,10 @@ __device__ __forceinline__ GenScratch gen_scratch(void* p, int threads, int cach
     return g;
 }
 
-// Candidates of pair (ri, qi) in generation order, truncated at match_limit,
+// Candidates of pair (ri, qi) in generation order, truncated at `limit`,
 // into okey/cgen, by nt threads (tid 0..nt-1, whole warps) with barrier
 // `sync`; s_scan holds one int per warp.  Returns the number generated
-// before truncation stopped it (>= match_limit means overflow).
+// before truncation stopped it (>= limit: there may be more).
 //
 // A thread takes a reference peak and finds its window by binary search, in a
 // shared-memory copy of the query's m/z where it fits (eleven dependent reads:
@@ -1695,8 +1711,8 @@ __device__ __forceinline__ GenScratch gen_scratch(void* p, int threads, int cach
 // independent and no thread waits for one with more candidates.
 template <bool MODIFIED, typename Sync>
 __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned long long* okey,
-                        uint32_t* cgen, int nt, int tid, int* s_scan, const GenScratch& G,
-                        Sync sync) {
+                        uint32_t* cgen, int limit, int nt, int tid, int* s_scan,
+                        const GenScratch& G, Sync sync) {
     const int lane = tid & 31, wid = tid >> 5, nwarps = nt >> 5;
     const unsigned full = 0xffffffffu;
     const int64_t r0 = P.R.off[ri], q0 = P.Q.off[qi];
@@ -1782,7 +1798,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                 if (w < wid) first += x;
                 chunk_total += x;
             }
-            const int take = min(chunk_total, P.match_limit - total);
+            const int take = min(chunk_total, limit - total);
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
                 uint32_t gen = ((uint32_t)pass << 31) |
@@ -1815,7 +1831,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                 }
             }
             total += chunk_total;
-            if (total >= P.match_limit) overflow = true;
+            if (total >= limit) overflow = true;
             sync();
         }
     }
@@ -2287,51 +2303,150 @@ __device__ __forceinline__ bool pair_of(const PairParams& P, int64_t item, int64
     return !(P.sym && ri > qi);
 }
 
+constexpr int kUsedWords = 256;  // words of each used-peak bitmap: spectra of up to 8192 peaks
+constexpr int kPairCache = 1024;  // query m/z values pair_kernel keeps in shared memory
+constexpr int kPairSlice = 512;   // candidates a warp takes on alone, at most
+constexpr int kDeferred = 64;     // pairs with more that a CTA collects
+
+// Shared memory of pair_kernel: candidates, used-peak bitmaps (or the bitmap of
+// accepted candidates, for spectra with more peaks), gen_pair's scratch, the
+// warps' greedy queues.
+__host__ __device__ constexpr int pair_used_words(int cap) {
+    return cap / 32 > 2 * kUsedWords ? cap / 32 : 2 * kUsedWords;
+}
+constexpr size_t pair_smem_bytes(int cap, int threads, int cache) {
+    return (size_t)cap * 12 + (size_t)pair_used_words(cap) * 4 + gen_scratch_bytes(threads, cache) +
+           (size_t)threads / 32 * kQueued * sizeof(uint16_t);
+}
+// the query's m/z are kept where they fit
+constexpr int pair_cache(int cap, int threads, size_t optin) {
+    return pair_smem_bytes(cap, threads, kPairCache) <= optin ? kPairCache : 0;
+}
+
+// Pairs of the spill list (or of the whole matrix, where the pipelined kernel
+// below does not fit).  Most spilled pairs have somewhat more candidates than the
+// join resolves; a CTA spent 15 us on each, most of it at barriers and behind
+// the one greedy warp.  So CTAs take only the heavy pairs, first, and then every
+// warp takes light ones of its own into a share of the candidate buffer; a pair
+// with more candidates than that holds (512 of 2048) is left to the CTA.  With
+// the bitmaps cut to 8192 peaks, 1024 query m/z in shared memory and 80
+// registers six CTAs fit an SM (five before): the pairs of 12345 symmetric spectra
+// take 180 us (305 before), of sparse 20000 x 20000 113 (216), of modified cosine
+// 297 (421).  What is left is the longest heavy pairs.
 template <bool SPARSE, bool MODIFIED>
-__global__ void pair_kernel(PairParams P) {
+__global__ void __maxnreg__(80) pair_kernel(PairParams P) {
     if (*P.bad) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned long long* okey = reinterpret_cast<unsigned long long*>(smem_raw);
     uint32_t* cgen = reinterpret_cast<uint32_t*>(okey + P.cap);
-    uint32_t* used_r = cgen + P.cap;          // 2048 words: 65536 peaks
-    uint32_t* used_q = used_r + 2048;
-    const GenScratch gen = gen_scratch(used_q + 2048, blockDim.x, 0);
+    uint32_t* used = cgen + P.cap;
+    const int used_words = pair_used_words(P.cap);
+    const GenScratch gen = gen_scratch(used + used_words, blockDim.x, P.cache);
+    uint16_t* queues = reinterpret_cast<uint16_t*>(gen.qmz + P.cache);
     __shared__ int s_scan[32];
-    __shared__ uint16_t s_queue[kQueued];
-    __shared__ unsigned long long s_item;
+    __shared__ int s_deferred[kDeferred];
+    __shared__ int s_n_deferred, s_done;
 
-    const int tid = threadIdx.x, wid = tid >> 5;
-    const int64_t n_items = P.pairs ? (int64_t)min(*P.n_pairs, P.pairs_cap) : P.R.n * P.Q.n;
-    const BlockSync sync;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    // an overrun list (an error that is reported) has gaps: nothing of it is read
+    const unsigned long long count = P.pairs ? *P.n_pairs : 0ull;
+    const unsigned int front = (unsigned int)count, back = (unsigned int)(count >> 32);
+    const bool sound = (unsigned long long)front + back <= P.pairs_cap;
+    const int64_t n_heavy = !P.pairs ? P.R.n * P.Q.n : sound ? front : 0;
+    const int64_t n_light = sound ? back : 0;
+    // a warp's share: a power of two (the sorts pad to one)
+    int slice = kPairSlice;
+    while (slice * nw > P.cap) slice >>= 1;
+    const int share = used_words / nw;
 
-    for (int64_t iter = 0;; ++iter) {
-        // spill list: dynamic (pairs differ widely in cost); whole matrix:
-        // static stride (uniform pairs, no contention on one counter)
-        __syncthreads();
-        if (tid == 0) s_item = P.pairs ? atomicAdd(P.work, 1ull)
-                                       : (unsigned long long)(blockIdx.x + iter * gridDim.x);
-        __syncthreads();
-        const int64_t item = (int64_t)s_item;
-        if (item >= n_items) break;
-        int64_t ri, qi;
-        if (!pair_of(P, item, ri, qi)) continue;
-        const int total =
-            gen_pair<MODIFIED>(P, ri, qi, okey, cgen, blockDim.x, tid, s_scan, gen, sync);
+    // candidates, order, greedy and output of a pair, by nt threads; false if
+    // it has as many candidates as `limit` below match_limit
+    auto resolve = [&](int64_t ri, int64_t qi, int limit, unsigned long long* k, uint32_t* g,
+                       uint32_t* used_r, int words, const GenScratch& G, int nt, int t, int* scan,
+                       uint16_t* queue, auto sync) {
+        const int total = gen_pair<MODIFIED>(P, ri, qi, k, g, limit, nt, t, scan, G, sync);
+        if (total >= limit && limit < P.match_limit) return false;
         const int n = min(total, P.match_limit);
         double score = 0.0;
         int matches = 0;
         if (n > 0) {
             const int nr = (int)(P.R.off[ri + 1] - P.R.off[ri]);
             const int nq = (int)(P.Q.off[qi + 1] - P.Q.off[qi]);
-            for (int i = tid; i < (nr + 31) / 32; i += blockDim.x) used_r[i] = 0u;
-            for (int i = tid; i < (nq + 31) / 32; i += blockDim.x) used_q[i] = 0u;
+            uint32_t* used_q = max(nr, nq) <= 16 * words ? used_r + words / 2 : nullptr;
+            const int words_r = ((used_q ? nr : n) + 31) / 32, words_q = used_q ? (nq + 31) / 32 : 0;
+            for (int i = t; i < words_r; i += nt) used_r[i] = 0u;
+            for (int i = t; i < words_q; i += nt) used_q[i] = 0u;
             int m = 1;
             while (m < n) m <<= 1;
-            sort_pair(okey, cgen, n, m, blockDim.x, tid, sync);
-            if (wid == 0)
-                greedy_pair<MODIFIED>(okey, cgen, used_r, used_q, s_queue, n, score, matches);
+            sort_pair(k, g, n, m, nt, t, sync);
+            if (t < 32) greedy_pair<MODIFIED>(k, g, used_r, used_q, queue, n, score, matches);
         }
-        if (tid == 0) write_pair<SPARSE>(P, ri, qi, n, score, matches, total >= P.match_limit);
+        if (t == 0) write_pair<SPARSE>(P, ri, qi, n, score, matches, total >= P.match_limit);
+        sync();
+        return true;
+    };
+
+    auto whole = [&](int64_t item) {
+        int64_t ri, qi;
+        if (pair_of(P, item, ri, qi))
+            resolve(ri, qi, P.match_limit, okey, cgen, used, used_words, gen, blockDim.x, tid, s_scan,
+                    queues, BlockSync{});
+    };
+    __shared__ unsigned long long s_item;
+    int n_whole = 0;
+    // One loop for the three sources of pairs that the CTA takes as a whole, so
+    // that their code is there once: the whole matrix at a static stride, the
+    // heavy pairs one by one, those deferred by the warps.
+    bool heavy = true, done = false;
+    if (tid == 0) s_n_deferred = s_done = 0;
+    for (int64_t iter = 0;; ++iter) {
+        int64_t item = -1;
+        if (heavy) {
+            item = blockIdx.x + iter * gridDim.x;
+            if (P.pairs) {
+                __syncthreads();
+                if (tid == 0) s_item = atomicAdd(P.work, 1ull);
+                __syncthreads();
+                item = (int64_t)s_item;
+            }
+            heavy = item < n_heavy;
+            if (!heavy) item = -1;
+        }
+        if (!heavy) {
+            if (!P.pairs) break;
+            if (n_whole == 0) {
+                if (done) break;
+                const GenScratch G{gen.w + kGenPeaks * 32 * wid, gen.qmz + P.cache / nw * wid,
+                                   P.cache / nw};
+                for (;;) {
+                    int i = -1;
+                    if (lane == 0 && *(volatile int*)&s_n_deferred <= kDeferred - nw) {
+                        const unsigned long long k = atomicAdd(P.work + 1, 1ull);
+                        if ((int64_t)k < n_light)
+                            i = (int)(P.pairs_cap - 1 - (unsigned int)k);
+                        else
+                            s_done = 1;
+                    }
+                    i = __shfl_sync(0xffffffffu, i, 0);
+                    if (i < 0) break;
+                    const int2 pr = P.pairs[i];
+                    if (!resolve(pr.x, pr.y, min(slice, P.match_limit), okey + slice * wid,
+                                 cgen + slice * wid, used + share * wid, share, G, 32, lane,
+                                 s_scan + wid, queues + kQueued * wid, WarpSync{}) &&
+                        lane == 0)
+                        s_deferred[atomicAdd(&s_n_deferred, 1)] = i;
+                }
+                __syncthreads();
+                n_whole = s_n_deferred;
+                done = s_done;
+                __syncthreads();  // read by all before either is written again
+                if (tid == 0) s_n_deferred = 0;
+                if (n_whole == 0) continue;
+            }
+            item = s_deferred[--n_whole];
+        }
+        whole(item);
+        if (!heavy) __syncthreads();
     }
 }
 
@@ -2357,16 +2472,15 @@ __global__ void pair_kernel(PairParams P) {
 // instructions at 57% issue.
 constexpr int kPipeBufs = 3;
 constexpr int kPipeCons = 2;
-constexpr int kPipeUsed = 256;   // words of each used-peak bitmap: spectra of up to 8192 peaks
-constexpr int kPipeCache = 2048; // query m/z values kept in shared memory while generating
+constexpr int kGenCache = 2048; // query m/z values kept in shared memory while generating
 // shared memory of np producer threads and buffers of cap candidates; the
 // scratch serves gen_pair, then the sorts (a 64-bit word per candidate and one
 // more per eight: 72 bytes a thread)
 constexpr size_t pipe_scratch_bytes(int np) {
-    return std::max<size_t>(gen_scratch_bytes(np, kPipeCache), (size_t)np * 72);
+    return std::max<size_t>(gen_scratch_bytes(np, kGenCache), (size_t)np * 72);
 }
 constexpr size_t pipe_smem_bytes(int cap, int np) {
-    return (size_t)cap * 12 * kPipeBufs + (size_t)kPipeCons * 2 * kPipeUsed * 4 +
+    return (size_t)cap * 12 * kPipeBufs + (size_t)kPipeCons * 2 * kUsedWords * 4 +
            pipe_scratch_bytes(np);
 }
 constexpr unsigned long long kPipeWaitNs = 2000000000ull;
@@ -2410,7 +2524,7 @@ pair_kernel_pipe(PairParams P) {
     unsigned long long* okey0 = reinterpret_cast<unsigned long long*>(smem_raw);
     uint32_t* cgen0 = reinterpret_cast<uint32_t*>(okey0 + kPipeBufs * P.cap);
     uint32_t* used0 = cgen0 + kPipeBufs * P.cap;
-    void* scratch = used0 + kPipeCons * 2 * kPipeUsed;
+    void* scratch = used0 + kPipeCons * 2 * kUsedWords;
     __shared__ int s_scan[32];
     __shared__ uint16_t s_queue[kPipeCons][kQueued];
     __shared__ int s_flags[kFixPasses + 1];
@@ -2433,17 +2547,16 @@ pair_kernel_pipe(PairParams P) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const int64_t n_items = P.pairs ? (int64_t)min(*P.n_pairs, P.pairs_cap) : P.R.n * P.Q.n;
+    const int64_t n_items = P.R.n * P.Q.n;
 
     if (producer) {
         const GroupSync sync{np};
-        const GenScratch gen = gen_scratch(scratch, np, kPipeCache);
+        const GenScratch gen = gen_scratch(scratch, np, kGenCache);
         int b = 0;
         uint32_t ph = 0;  // parity of buffer b's current use
         int ends = 0;     // end marks posted, one for each consumer
         for (int64_t iter = 0; ends < kPipeCons; ++iter) {
-            if (tid == 0) s_item = P.pairs ? atomicAdd(P.work, 1ull)
-                                           : (unsigned long long)(blockIdx.x + iter * gridDim.x);
+            if (tid == 0) s_item = (unsigned long long)(blockIdx.x + iter * gridDim.x);
             sync();
             const int64_t item = (int64_t)s_item;
             int64_t ri = 0, qi = 0;
@@ -2466,7 +2579,8 @@ pair_kernel_pipe(PairParams P) {
             uint32_t* cgen = cgen0 + (size_t)b * P.cap;
             int total = -1;
             if (more) {
-                total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, np, tid, s_scan, gen, sync);
+                total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, P.match_limit, np, tid, s_scan, gen,
+                                           sync);
                 const int n = min(total, P.match_limit);
                 if (n > 0) {
                     int m = 1;
@@ -2497,7 +2611,7 @@ pair_kernel_pipe(PairParams P) {
     } else if (!P.test_stall) {
         // consumer warp w: every kPipeCons-th buffer use, from use w on
         const int lane = tid & 31, w = (tid - np) >> 5;
-        uint32_t* used_r = used0 + w * 2 * kPipeUsed;
+        uint32_t* used_r = used0 + w * 2 * kUsedWords;
         for (int use = w;; use += kPipeCons) {
             const int b = use % kPipeBufs;
             const uint32_t ph = (uint32_t)(use / kPipeBufs) & 1u;
@@ -2520,8 +2634,8 @@ pair_kernel_pipe(PairParams P) {
             if (n > 0) {
                 const int nr = (int)(P.R.off[ri + 1] - P.R.off[ri]);
                 const int nq = (int)(P.Q.off[qi + 1] - P.Q.off[qi]);
-                const bool fits = max(nr, nq) <= 32 * kPipeUsed;
-                uint32_t* used_q = fits ? used_r + kPipeUsed : nullptr;
+                const bool fits = max(nr, nq) <= 32 * kUsedWords;
+                uint32_t* used_q = fits ? used_r + kUsedWords : nullptr;
                 if (fits) {
                     for (int i = lane; i < (nr + 31) / 32; i += 32) used_r[i] = 0u;
                     for (int i = lane; i < (nq + 31) / 32; i += 32) used_q[i] = 0u;
@@ -2714,7 +2828,7 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
                   "(%lld != %lld)", (long long)args.ref.n, (long long)args.qry.n);
         return CMS_ERR_INVALID;
     }
-    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(p.pair_threads, 0);
+    const size_t pair_smem = pair_smem_bytes(p.cap, p.pair_threads, 0);
     if (pair_smem > ctx->smem_optin) {
         set_error("cms_cosine_greedy: match_limit %d needs %zu B shared memory (> %zu)",
                   args.match_limit, pair_smem, ctx->smem_optin);
@@ -2760,7 +2874,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
                    const SparseOut* sparse, const Plan& p, cudaStream_t s) {
     int rc = CMS_OK;
     const int sym = p.sym;
-    const size_t pair_smem = (size_t)p.cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(p.pair_threads, 0);
+    const int cache = pair_cache(p.cap, p.pair_threads, ctx->smem_optin);
+    const size_t pair_smem = pair_smem_bytes(p.cap, p.pair_threads, cache);
     const int64_t nR = args.ref.n, nQ = args.qry.n;
     const size_t gpool_warps = (size_t)ctx->sm_count * 64;
     const size_t gpool_bytes = gpool_warps * (size_t)kGPool * 16;
@@ -2769,7 +2884,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     uint32_t* bad = reinterpret_cast<uint32_t*>(small);            // word 0
     uint32_t* cls_count = reinterpret_cast<uint32_t*>(small + 1);  // 17 words
     uint32_t* cls_cursor = reinterpret_cast<uint32_t*>(small + 10);  // 17 words
-    unsigned int* spill_count = reinterpret_cast<unsigned int*>(small + 20);
+    unsigned long long* spill_count = reinterpret_cast<unsigned long long*>(small + 20);
     unsigned long long* work_join = reinterpret_cast<unsigned long long*>(small + 21);
     unsigned long long* work_pair = reinterpret_cast<unsigned long long*>(small + 22);
     // the bucket counts lie behind the counters: one memset clears both
@@ -2814,6 +2929,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     pp.shift = args.shift;
     pp.match_limit = args.match_limit;
     pp.cap = p.cap;
+    pp.cache = cache;
     pp.pairs = nullptr;
     pp.n_pairs = nullptr;
     pp.pairs_cap = 0;
@@ -2843,7 +2959,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
 
     const size_t pipe_smem = pipe_smem_bytes(p.cap, p.pair_threads);
     if (p.mode == 2 && pipe_smem <= ctx->smem_optin &&
-        p.cap / 32 <= 2 * kPipeUsed) {  // the accepted bitmap of spectra past kPipeUsed
+        p.cap / 32 <= 2 * kUsedWords) {  // the accepted bitmap of spectra past kUsedWords
         // whole matrix: the pipelined pair kernel (pair_threads producers
         // plus the consumer warps)
         void (*pipe_k)(PairParams) =
@@ -3387,8 +3503,7 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     pp.err = err;
     pp.bad = bad;
     const int pair_threads = 128;
-    const size_t pair_smem =
-        (size_t)cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(pair_threads, 0);
+    const size_t pair_smem = pair_smem_bytes(cap, pair_threads, 0);
     if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
     int per_sm = 1;
     CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<false, false>,
@@ -3561,7 +3676,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     if (n_q == 0) return CMS_OK;
 
     const int cap = next_pow2(std::max(2, lib->match_limit));
-    const size_t pair_smem = (size_t)cap * 12 + 2 * 2048 * 4 + gen_scratch_bytes(128, 0);
+    const int cache = pair_cache(cap, 128, ctx->smem_optin);
+    const size_t pair_smem = pair_smem_bytes(cap, 128, cache);
     if (pair_smem > ctx->smem_optin) {
         set_error("cms_library_search: match_limit too large for shared memory");
         return CMS_ERR_UNSUPPORTED;
@@ -3586,7 +3702,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     uint32_t* bad = reinterpret_cast<uint32_t*>(small);
     uint32_t* cls_count = reinterpret_cast<uint32_t*>(small + 1);
     uint32_t* cls_cursor = reinterpret_cast<uint32_t*>(small + 10);
-    unsigned int* spill_count = reinterpret_cast<unsigned int*>(small + 20);
+    unsigned long long* spill_count = reinterpret_cast<unsigned long long*>(small + 20);
     unsigned long long* work_join = reinterpret_cast<unsigned long long*>(small + 21);
     unsigned long long* work_pair = reinterpret_cast<unsigned long long*>(small + 22);
     uint32_t* slots = bp.take<uint32_t>(kSlotWords);  // cleared with the counters before it
@@ -3664,6 +3780,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     pp.shift = lib->shift;
     pp.match_limit = lib->match_limit;
     pp.cap = cap;
+    pp.cache = cache;
     pp.pairs = spill;
     pp.n_pairs = spill_count;
     pp.pairs_cap = spill_cap;

@@ -421,3 +421,26 @@ def test_preparation_rounds(cuda_device, n):
     want = oracle.cosine_greedy(ref, qry, 0.02, 0.0, 4096)
     for cfg in ({"mode": 1, "tile_spectra": 32}, {"mode": 2}):
         assert_same(gpu_dense(ref, qry, P(0.02, 4096), cfg), want, f"{n} {cfg}")
+
+
+@pytest.mark.parametrize("ml", [1, 40, 512, 520, 2048, 16384])
+def test_spilled_pairs(cuda_device, ml):
+    """Pairs the join leaves to the pair kernel, around the number of candidates up to which a
+    warp takes one alone (512, or a share of small match limits), and with more peaks than its
+    share of the used-peak bitmaps holds (2048)."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(97)
+
+    def make(lens, spacing):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([100.0 + s * np.arange(k) for k, s in zip(lens, spacing)])
+        inten = rng.integers(1, 50, off[-1])
+        return pack_csr(mz.astype(np.float32), inten.astype(np.float32), off, None)
+
+    ref = make([16, 5, 32, 2100, 33, 60], [0.001, 0.001, 0.001, 0.004, 0.001, 0.03])
+    qry = make([31, 32, 33, 2047, 2049, 64, 7, 300], [0.001, 0.001, 0.001, 0.005, 0.005, 0.02, 0.001, 0.001])
+    want = oracle.cosine_greedy(ref, qry, 0.05, 0.0, ml)
+    for cfg in ({"mode": 1, "tile_spectra": 32}, {"mode": 1, "tile_spectra": 32, "pair_threads": 512},
+                {"mode": 1, "tile_spectra": 32, "pair_threads": 96}):
+        assert_same(gpu_dense(ref, qry, P(0.05, ml, 65535), cfg), want, f"{cfg}")
