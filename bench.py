@@ -57,13 +57,13 @@ WORKLOAD = ("batched greedy cosine 100k x 100k, lognormal peaks (median 60, sigm
             "clip 5-1000), m/z U(50,2000), tol 0.01, powers (0,1), match_limit 4096")
 BYTES_PER_PAIR = 9
 # DRAM bytes per pair of join_kernel (read + write), from an ncu capture of the
-# 20k x 20k case of this workload (profiles/join_kernel_batched_cosine_20k.txt);
+# 20000 x 20480 case of this workload (profiles/join_kernel_batched_cosine_20k.txt);
 # traffic grows with pairs, so a full launch is scaled by its pair count.
-JOIN_TRAFFIC_BYTES_PER_PAIR = 11.37
+JOIN_TRAFFIC_BYTES_PER_PAIR = 11.48
 # issue activity and the long-scoreboard share of stalls in the same capture
 # (quoted, not measured by a bench run)
-JOIN_PROFILE = "profiles/join_kernel_batched_cosine_20k.txt (20k x 20k capture)"
-JOIN_PROFILE_FIGURES = {"issue_active_pct": 38.5, "long_scoreboard_stall_pct": 40.0}
+JOIN_PROFILE = "profiles/join_kernel_batched_cosine_20k.txt (20000 x 20480 capture)"
+JOIN_PROFILE_FIGURES = {"issue_active_pct": 43.7, "long_scoreboard_stall_pct": 54.0}
 
 
 def parse():
@@ -412,7 +412,7 @@ def run_ours(args, world, rank, local):
     roofline = {"bound": "hbm", "kernel": "join_kernel", "achieved": achieved, "peak": hbm,
                 "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": JOIN_TRAFFIC_BYTES_PER_PAIR * pairs_per_launch,
-                "traffic_source": "ncu dram bytes of a 20k x 20k capture, scaled by pairs",
+                "traffic_source": "ncu dram bytes of a 20000 x 20480 capture, scaled by pairs",
                 "peak_source": f"{peak_kind} hbm_gbs (copy)",
                 "algorithmic_bytes_per_launch": alg_bytes, "launch_ms": join_ms,
                 "stage_ms_per_step": {n: float(v) / args.steps for n, v in zip(names, stage_ms)},

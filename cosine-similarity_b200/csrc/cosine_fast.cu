@@ -845,7 +845,7 @@ __device__ __forceinline__ float cosine_of(double score, double rr, double rq, c
 // buckets come ready-made per sweeping peak, item descriptors in order, a
 // pool entry is one 16-byte access, and owners of one candidate do not wait
 // for the code of longer runs (50000 x 50000: 11.45 ms with all of that done
-// per item, 9.6 ms now).  The code is kept short, 45 KB instead of 126 KB:
+// per item, 9.6 ms after; 8.5 ms with the L1 cache that join_pool leaves).  The code is kept short, 45 KB instead of 126 KB:
 // modified cosine 13.2 -> 8.8 ms and 1024 x 1024 328 -> 272 us together with
 // the comparison instead of the sorting of long runs.  Four CTAs at 64
 // registers spill: 1024 x 1024 +13%, search of 1000 +10%, modified +6%.
