@@ -840,13 +840,13 @@ __device__ __forceinline__ float cosine_of(double score, double rr, double rq, c
 
 // Bound by instruction issue and latency together (about 13 cycles between a
 // warp's instructions at six warps a scheduler), not by memory: 50000 x 50000
-// lognormal spectra, dense, move 11.4 B a pair at a quarter of the copy rate.
+// lognormal spectra, dense, move 11.5 B a pair at half the copy rate.
 // So what counts is the length of an item's instruction chain: windows and
 // buckets come ready-made per sweeping peak, item descriptors in order, a
 // pool entry is one 16-byte access, and owners of one candidate do not wait
 // for the code of longer runs (50000 x 50000: 11.45 ms with all of that done
-// per item, 9.6 ms after; 8.5 ms with the L1 cache that join_pool leaves).  The code is kept short, 45 KB instead of 126 KB:
-// modified cosine 13.2 -> 8.8 ms and 1024 x 1024 328 -> 272 us together with
+// per item, 9.6 ms after; 8.5 ms with the L1 cache that join_pool leaves).
+// The code is kept short, 45 KB instead of 126 KB: modified cosine 13.2 -> 8.8 ms and 1024 x 1024 328 -> 272 us together with
 // the comparison instead of the sorting of long runs.  Four CTAs at 64
 // registers spill: 1024 x 1024 +13%, search of 1000 +10%, modified +6%.
 // Three CTAs (24 warps) per SM: up to 80 registers a thread.

@@ -115,11 +115,12 @@ def workload_stats(ref: PackedSpectra, qry: PackedSpectra, tolerance: float,
 # resident warp of the join kernel (148 SMs x 24 warps), so that small
 # problems still fill the GPU and the last items do not leave it idle
 TARGET_ITEMS = 100_000
-# expected candidates per work item: measured on B200 with lognormal spectra
-# (tol 0.01, ~0.1 candidates per pair, 100k x 100k, whole query tiles) the
-# time per pair falls from 7.75 ps at ~130 candidates per item (1312 queries)
-# to 7.09 ps at ~200 (2048); below ~75 the per-peak bucket lookups dominate
-CANDIDATES_PER_ITEM = 200.0
+# expected candidates per work item: about what the join's shared pool holds beside
+# the heads of the tile.  Lognormal spectra, tol 0.01, ~0.1 candidates per pair,
+# 50000 x 50000: 8.9 ms at 168 to 184 (tiles of 1696 and 1856 queries), 9.0 at
+# 152, 9.1 at 133, 9.2 at 203; 12345 symmetric ones, 0.2 per pair: 1.35 ms at
+# 146, 1.38 at 206, 1.49 at 106
+CANDIDATES_PER_ITEM = 176.0
 # largest automatic tile: the join's per-warp query heads grow with the tile and
 # take the place of its candidate pool in shared memory.  50000 x 50000
 # lognormal spectra: 8.96 ms with tiles of 1536, 8.9 ms with 1696 and 1856,
