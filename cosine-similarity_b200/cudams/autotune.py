@@ -44,7 +44,7 @@ from .packing import PackedSpectra
 POOL = 256
 DENSE_CANDIDATES = 48.0  # mean candidates per pair above which mode 2 is used
 # up to this many pairs (two or three for each resident CTA of the pair kernel)
-# mode 2 is used without looking at the spectra, on B200 with tolerance 0.1:
+# of ordinary values mode 2 is used without an estimate, on B200 with tolerance 0.1:
 # one pair of 100-peak spectra 29 us (join 54), 24 x 24 37 us (97), 40 x 40 52 us
 # (103), 60 x 60 75 us (104); 24 x 24 heavy-tailed 49 us (118).  The estimate alone
 # took 4.3 ms of host time a call.
@@ -300,9 +300,33 @@ def measure(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: flo
     return _default.measure(ref, qry, tolerance, shift, match_limit, device, gpu, **kw)
 
 
+def _ordinary(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: float,
+              precursors=()) -> bool:
+    """Whether both modes of the kernels are sure to treat every value alike.  They
+    differ, in the candidates they take or in whether they report an error, where a
+    value is not finite, where a product of weights overflows or is a negative zero,
+    and where a window ends next to zero under a shift (float32 m/z are then much
+    finer than the float64 sums they are compared in)."""
+    def plain(x, limit):
+        return x is None or not x.size or (not np.signbit(x).any() and bool(x.max() < limit))
+
+    for s in (ref, qry):
+        if not (plain(s.mz, 1e30) and plain(s.a, 1e70) and plain(s.b, 1e70)):
+            return False
+    if not all(bool((np.abs(p) < 1e30).all()) for p in precursors):
+        return False
+    if not (tolerance < 1e30 and abs(shift) < 1e30):
+        return False
+    if shift and ref.mz.size:
+        ends = np.abs(np.abs(ref.mz.astype(np.float64) - shift) - tolerance)
+        return bool(ends.min() > 1e-7 * (abs(shift) + float(ref.mz.max()) + 1.0))
+    return True
+
+
 def choose_config(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: float = 0.0,
-                  gpu: str = "B200") -> dict:
-    if ref.n * qry.n <= FEW_PAIRS:
+                  gpu: str = "B200", precursors=()) -> dict:
+    """precursors: both sides' precursor m/z where the scores depend on them."""
+    if ref.n * qry.n <= FEW_PAIRS and _ordinary(ref, qry, tolerance, shift, precursors):
         return {"mode": 2}
     # the 99th percentile takes no part in the choice: no pair sample
     stats = workload_stats(ref, qry, tolerance, shift, n_pairs=0)

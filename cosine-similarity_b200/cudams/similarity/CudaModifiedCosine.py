@@ -76,10 +76,10 @@ class CudaModifiedCosine(CudaCosineGreedy):
             return self.pack(packed), prec
         return self.pack(spectra), precursors_of(spectra)
 
-    def _config_for(self, ref: PackedSpectra, qry: PackedSpectra) -> dict:
+    def _config_for(self, ref: PackedSpectra, qry: PackedSpectra, precursors=()) -> dict:
         if self.config is not None:
             return dict(self.config)
-        cfg = autotune.choose_config(ref, qry, float(self.tolerance), 0.0)
+        cfg = autotune.choose_config(ref, qry, float(self.tolerance), 0.0, precursors=precursors)
         if cfg.get("cand_per_pair"):  # the shifted pass adds about as many again
             cfg["cand_per_pair"] = 2.0 * cfg["cand_per_pair"]
             cfg["tile_spectra"] = max(32, (cfg.get("tile_spectra", 64) // 2 + 31) // 32 * 32)
@@ -96,7 +96,7 @@ class CudaModifiedCosine(CudaCosineGreedy):
         self.kernel_time = 0.0
         if R == 0 or Q == 0:
             return score, matches, overflow
-        cfg = self._config_for(ref, qry)
+        cfg = self._config_for(ref, qry, (rprec, qprec))
         rows = self._row_block(R, Q, dev)
         stream = torch.cuda.current_stream(dev)
         one_block = rows >= R
@@ -168,7 +168,7 @@ class CudaModifiedCosine(CudaCosineGreedy):
             s, m, o = score[r, q], matches[r, q], overflow[r, q]
         else:
             dev = self._torch_device()
-            cfg = self._config_for(ref, qry)
+            cfg = self._config_for(ref, qry, (rprec, qprec))
             if symmetric:
                 cfg = dict(cfg, symmetric=1)
             stream = torch.cuda.current_stream(dev)

@@ -137,3 +137,29 @@ def test_rejects_over_32767_peaks(cuda_device):
     with pytest.raises(_native.NativeError, match="32767"):
         kernels.modified_cosine_dense(big.to_device(dev), p, big.to_device(dev), p, 0.1, 2048,
                                       check_errors=True)
+
+
+@pytest.mark.parametrize("side,value", [("q", np.nan), ("q", np.inf), ("q", -np.inf),
+                                        ("r", np.nan), ("r", np.inf)])
+def test_unusual_precursor_answers_do_not_depend_on_the_call_size(cuda_device, side, value):
+    """A pair's result (or the call's error) with a precursor that is not finite is the
+    same in a call small enough for the whole-matrix pair kernel and in a larger one."""
+    from cudams import autotune, synthetic
+    from cudams._native import NativeError
+    from cudams.similarity import CudaModifiedCosine
+
+    ref, qry = synthetic.uniform_spectra(41, seed=51), synthetic.uniform_spectra(40, seed=52)
+    rng = np.random.default_rng(53)
+    rp, qp = rng.uniform(300, 900, 41), rng.uniform(300, 900, 40)
+    (rp if side == "r" else qp)[3] = value
+    assert 40 * 40 <= autotune.FEW_PAIRS < 41 * 40
+    sim = CudaModifiedCosine(tolerance=0.1)
+    calls = [lambda n=n: sim.matrix((ref.subset(0, n), rp[:n]), (qry, qp)) for n in (40, 41)]
+    if side == "r":
+        for call in calls:
+            with pytest.raises(NativeError):
+                call()
+        return
+    small, large = (call()[:40] for call in calls)
+    for name in ("score", "matches", "overflow"):
+        np.testing.assert_array_equal(small[name], large[name])

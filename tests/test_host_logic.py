@@ -109,3 +109,44 @@ def test_take_selects_spectra():
                                       P.mz[P.offsets[i]:P.offsets[i + 1]])
         np.testing.assert_array_equal(T.b[T.offsets[k]:T.offsets[k + 1]],
                                       P.b[P.offsets[i]:P.offsets[i + 1]])
+
+
+def test_few_pairs_of_unusual_values_take_the_ordinary_route(tmp_path, monkeypatch):
+    """Small calls go straight to the pair kernel only where both kernels are sure to
+    give the same answer: not with a precursor, weight or m/z that is not finite (or
+    a negative zero, or a window that ends at zero), on either side."""
+    from cudams import autotune
+    from cudams.packing import PackedSpectra
+
+    monkeypatch.setattr(autotune, "_default", autotune.Tuner(str(tmp_path / "none.json")))
+    rng = np.random.default_rng(0)
+
+    def spectra(mz_at=None, a_at=None, b_at=None):
+        off = np.arange(0, 41, 10)
+        mz = np.sort(rng.uniform(100, 500, (4, 10))).ravel().astype(np.float32)
+        a, b = mz.astype(np.float64), rng.random(40) + 0.1
+        for x, v in ((mz, mz_at), (a, a_at), (b, b_at)):
+            if v is not None:
+                x[7] = v
+        return PackedSpectra(mz, a, b, off, 1.0, 1.0, 1024)
+
+    plain, prec = spectra(), rng.uniform(200, 600, 4)
+    choose = lambda r, q, shift=0.0, p=(): autotune.choose_config(r, q, 0.1, shift, precursors=p)  # noqa: E731
+    assert choose(plain, plain) == {"mode": 2}
+    assert choose(plain, plain, -250.0, (prec, prec)) == {"mode": 2}
+    empty = plain.subset(0, 0)
+    assert choose(empty, plain, 17.0, (prec[:0], prec)) == {"mode": 2}
+    for value in (np.nan, np.inf, -np.inf, 1e300):
+        odd = prec.copy()
+        odd[2] = value
+        assert choose(plain, plain, 0.0, (odd, prec))["mode"] == 1
+        assert choose(plain, plain, 0.0, (prec, odd))["mode"] == 1
+    for value in (np.nan, np.inf, -0.0, -1.0, 1e200):
+        for at in ("a_at", "b_at"):
+            odd = spectra(**{at: value})
+            assert choose(odd, plain)["mode"] == 1 and choose(plain, odd)["mode"] == 1
+    for value in (np.nan, np.inf):
+        with np.errstate(all="ignore"):
+            odd = spectra(mz_at=value)
+            assert choose(odd, plain)["mode"] == 1 and choose(plain, odd)["mode"] == 1
+    assert choose(plain, plain, float(plain.mz[5]) + 0.1)["mode"] == 1
