@@ -26,7 +26,8 @@ sub-range swept per candidate-pool fill (cms_cosine_config.width_by_class:
 narrower ranges keep a large spectrum's candidates in the shared-memory
 pool, wider ones amortise its bucket lookups over more queries).  The
 winners are recorded per workload key in an on-disk cache (JSON,
-`Tuner.record`) that `choose_config` consults first.
+`Tuner.record`) that `choose_config` consults first.  Without a record, calls
+of few pairs take mode 2 whatever the estimate (`FEW_PAIRS`).
 """
 from __future__ import annotations
 
@@ -165,15 +166,23 @@ class Tuner:
                 self._cache = {}
         return self._cache
 
-    def lookup(self, stats: WorkloadStats, gpu: str, n_q: int, n_ref: int = 1 << 30) -> dict:
+    def has_records(self) -> bool:
+        with self._lock:
+            return bool(self._load())
+
+    def recorded(self, stats: WorkloadStats, gpu: str, n_q: int) -> Optional[dict]:
+        """The measured choice for this workload, if there is one."""
         with self._lock:
             hit = self._load().get(self.key(stats, gpu))
-        if hit:
-            cfg = dict(hit)
-            if cfg.get("tile_spectra"):
-                cfg["tile_spectra"] = min(cfg["tile_spectra"], max(32, n_q))
-            return cfg
-        return heuristic_config(stats, n_q, n_ref)
+        if not hit:
+            return None
+        cfg = dict(hit)
+        if cfg.get("tile_spectra"):
+            cfg["tile_spectra"] = min(cfg["tile_spectra"], max(32, n_q))
+        return cfg
+
+    def lookup(self, stats: WorkloadStats, gpu: str, n_q: int, n_ref: int = 1 << 30) -> dict:
+        return self.recorded(stats, gpu, n_q) or heuristic_config(stats, n_q, n_ref)
 
     def record(self, stats: WorkloadStats, gpu: str, config: dict) -> None:
         with self._lock:
@@ -326,8 +335,11 @@ def _ordinary(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: f
 def choose_config(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: float = 0.0,
                   gpu: str = "B200", precursors=()) -> dict:
     """precursors: both sides' precursor m/z where the scores depend on them."""
-    if ref.n * qry.n <= FEW_PAIRS and _ordinary(ref, qry, tolerance, shift, precursors):
+    few = ref.n * qry.n <= FEW_PAIRS and _ordinary(ref, qry, tolerance, shift, precursors)
+    if few and not _default.has_records():
         return {"mode": 2}
     # the 99th percentile takes no part in the choice: no pair sample
     stats = workload_stats(ref, qry, tolerance, shift, n_pairs=0)
+    if few:
+        return _default.recorded(stats, gpu, qry.n) or {"mode": 2}
     return _default.lookup(stats, gpu, qry.n, ref.n)

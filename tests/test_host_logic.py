@@ -150,3 +150,16 @@ def test_few_pairs_of_unusual_values_take_the_ordinary_route(tmp_path, monkeypat
             odd = spectra(mz_at=value)
             assert choose(odd, plain)["mode"] == 1 and choose(plain, odd)["mode"] == 1
     assert choose(plain, plain, float(plain.mz[5]) + 0.1)["mode"] == 1
+
+
+def test_recorded_choices_hold_for_few_pairs_too(tmp_path, monkeypatch):
+    from cudams import autotune, synthetic
+
+    tuner = autotune.Tuner(str(tmp_path / "tune.json"))
+    monkeypatch.setattr(autotune, "_default", tuner)
+    small, other = synthetic.uniform_spectra(20, seed=1), synthetic.clustered_spectra(4, seed=2)
+    assert autotune.choose_config(small, small, 0.1) == {"mode": 2}
+    cfg = {"mode": 1, "tile_spectra": 777, "cand_per_pair": 1.5}
+    tuner.record(autotune.workload_stats(small, small, 0.1), "B200", cfg)
+    assert autotune.choose_config(small, small, 0.1) == dict(cfg, tile_spectra=32)
+    assert autotune.choose_config(other, other, 0.1) == {"mode": 2}
