@@ -1749,11 +1749,17 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                 if (p1 < nr) {
                     const double mz1 = (double)mz[u];
                     // the window as float32 bounds of the query's m/z (exact, see
-                    // Window): first p2 at or above, then on to the last one inside
+                    // Window): first p2 at or above, then on to the last one inside.
+                    // (With a shift the search for the lower bound may end early next
+                    // to zero, where float32 is finer than the float64 sums.)
                     float wl, wh;
-                    const bool ok = shift == 0.0
-                                        ? Window<true, true>::bounds(mz[u], P.tol, shift, wl, wh)
-                                        : Window<true, false>::bounds(mz[u], P.tol, shift, wl, wh);
+                    const bool ok =
+                        shift == 0.0
+                            ? Window<true, true>::bounds(mz[u], P.tol, shift, wl, wh)
+                            : Window<true, false>::bounds(mz[u], P.tol, shift, wl, wh) &&
+                                  !Window<true, false>::not_below(nextafterf(wl, -INFINITY),
+                                                                  __dsub_rn(mz1, P.tol), 0.0, P.tol,
+                                                                  shift);
                     int L = 0, H = nq;
                     if (ok) {
                         while (L < H) {
@@ -1764,8 +1770,8 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                                 H = M;
                         }
                         start[u] = L;
-                        while (L < nq && qmz[L] <= wh) ++L;
-                    } else {  // not finite: as the definition tests it
+                        while (L < nq && !(qmz[L] > wh)) ++L;
+                    } else {  // no such bounds: as the definition tests it
                         const double lo = __dsub_rn(mz1, P.tol), hi = __dadd_rn(mz1, P.tol);
                         while (L < H) {
                             const int M = (L + H) >> 1;

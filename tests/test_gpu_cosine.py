@@ -444,3 +444,30 @@ def test_spilled_pairs(cuda_device, ml):
     for cfg in ({"mode": 1, "tile_spectra": 32}, {"mode": 1, "tile_spectra": 32, "pair_threads": 512},
                 {"mode": 1, "tile_spectra": 32, "pair_threads": 96}):
         assert_same(gpu_dense(ref, qry, P(0.05, ml, 65535), cfg), want, f"{cfg}")
+
+
+@pytest.mark.parametrize("pair_threads", [64, 128])
+def test_pair_kernel_windows_as_defined(cuda_device, pair_threads):
+    """m/z that are NaN (every window's last candidate) or next to zero under a shift that
+    ends a window there: the candidates the float64 comparisons define."""
+    from cudams.packing import pack_csr
+
+    def pack(spectra):
+        off = np.concatenate([[0], np.cumsum([len(s) for s in spectra])])
+        mz = np.concatenate(spectra).astype(np.float32)
+        inten = np.random.default_rng(len(spectra)).random(off[-1]).astype(np.float32) + 0.5
+        return pack_csr(mz, inten, off, None, check=False)
+
+    ref = pack([[100.0, 120.0, 300.0], [99.75, 100.0], [700.0]])
+    qry = pack([[100.05, 119.95, np.nan], [299.95, np.nan, np.nan], [700.0], [np.nan]])
+    cfg = {"mode": 2, "pair_threads": pair_threads}
+    want = oracle.cosine_greedy(ref, qry, 0.1, 0.0, 64)
+    assert want[1][0, 0] == 3 and want[1][0, 3] == 1
+    assert_same(gpu_dense(ref, qry, P(0.1, 64), cfg), want, "nan")
+    # lower end of the first peak's window one float64 step above zero
+    near = pack([[0.0, 5e-15, 7.5e-15, 1e-14, 1.3e-14, 0.1, 0.2], [-1e-20, 1e-20]]
+                + [[x] for x in (0.0, 5e-15, 7.5e-15, 1e-14, 1.3e-14)])
+    for shift in (float(np.nextafter(100.0 - 0.1, 0.0)), 100.0 - 0.1, 100.0 + 0.1,
+                  float(np.nextafter(100.0 + 0.1, 0.0))):
+        want = oracle.cosine_greedy(ref, near, 0.1, shift, 64)
+        assert_same(gpu_dense(ref, near, P(0.1, 64, shift=shift), cfg), want, f"{shift}")
