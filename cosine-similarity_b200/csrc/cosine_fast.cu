@@ -54,6 +54,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "cms_internal.cuh"
@@ -248,7 +249,9 @@ struct PrepSide {
 struct PrepSides {
     PrepSide side[2];
     int blocks0;
+    uint32_t* any_long;  // set to 1 by a spectrum of more than kLongPeaks peaks (null: not wanted)
 };
+constexpr int kLongPeaks = 8192;  // longer spectra have no used-peak bitmaps in shared memory
 
 struct ProbeArgs {
     SpecSet S;          // the sweeping side
@@ -352,6 +355,7 @@ prep_kernel(const __grid_constant__ PrepSides sides, IndexGeom g, uint32_t* bad,
             } else {
                 len = (int)(hi - lo);
                 if (P.cls_count) atomicAdd(&s_cls[length_class(len)], 1u);
+                if (sides.any_long && len > kLongPeaks) *sides.any_long = 1u;
             }
         }
         const int longest = __reduce_max_sync(full, len);
@@ -1553,6 +1557,12 @@ struct PairParams {
     int match_limit;
     int cap;  // power of two >= match_limit
     int cache;  // pair_kernel: query m/z values kept in shared memory (pair_cache)
+    int used_words;       // pair_kernel: words of each used-peak bitmap in shared memory
+    uint32_t* long_bits;  // bitmaps of pairs with more peaks, kLongWords a greedy warp (or null)
+    // launches for either kind of call (null: always run): the kernel returns
+    // unless *gate == gate_value
+    const uint32_t* gate;
+    uint32_t gate_value;
     // work: either the spill list (pairs != nullptr) or every pair of R x Q
     const int2* pairs;
     const unsigned long long* n_pairs;  // SpillList::count
@@ -2169,9 +2179,8 @@ __device__ void sort_pair(unsigned long long* okey, uint32_t* cgen, int n, int m
 constexpr int kFill = 2;                    // chunks of 32 candidates looked at together
 constexpr int kQueued = 32 * (kFill + 1);  // at most 31 waiting, plus one look's candidates
 // Greedy by one warp over the sorted candidates.  used_r / used_q, zeroed for
-// the pair's peaks, hold the peaks taken; or, used_q null, used_r is a bitmap over
-// the candidates (n bits, zeroed) of those accepted, and a candidate is compared
-// with each of them (spectra with more peaks than the bitmaps hold).
+// the pair's peaks, hold the peaks taken, in shared memory or (GLOBAL) in device
+// memory.
 //
 // Most candidates have a taken peak when their turn comes, so the live ones are
 // first queued (their positions, in order; `queue` holds kQueued) and resolved 32 at a
@@ -2181,23 +2190,20 @@ constexpr int kQueued = 32 * (kFill + 1);  // at most 31 waiting, plus one look'
 // decided (the lowest undecided lane always can, so this ends; usually after two
 // or three rounds).  Accepted keys are summed in sorted order, as the sequential
 // greedy; every lane ends with the same score and match count.
-template <bool MODIFIED>
-__device__ void greedy_pair(unsigned long long* okey, const uint32_t* cgen, uint32_t* used_r,
-                            uint32_t* used_q, uint16_t* queue, int n, double& score,
-                            int& matches) {
+template <bool MODIFIED, bool GLOBAL>
+__device__ __forceinline__ void greedy_pair(unsigned long long* okey, const uint32_t* cgen,
+                                            uint32_t* used_r, uint32_t* used_q, uint16_t* queue,
+                                            int n, double& score, int& matches) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    // from device memory past the L1 cache, which other multiprocessors' and
+    // earlier pairs' writes do not reach
+    auto word = [](const uint32_t* p) { return GLOBAL ? __ldcg(p) : *p; };
     auto free_peaks = [&](uint32_t g) {
         const int p1 = (int)gen_p1<MODIFIED>(g), p2 = (int)(g & 0xFFFFu);
-        if (used_q)
-            return (((used_r[p1 >> 5] >> (p1 & 31)) | (used_q[p2 >> 5] >> (p2 & 31))) & 1u) == 0u;
-        for (int w = 0; w < (n + 31) / 32; ++w)
-            for (unsigned m = used_r[w]; m; m &= m - 1u) {
-                const uint32_t o = cgen[32 * w + __ffs(m) - 1];
-                if ((int)gen_p1<MODIFIED>(o) == p1 || (int)(o & 0xFFFFu) == p2) return false;
-            }
-        return true;
+        return (((word(used_r + (p1 >> 5)) >> (p1 & 31)) | (word(used_q + (p2 >> 5)) >> (p2 & 31))) &
+                1u) == 0u;
     };
     int queued = 0, c = 0;
 #pragma unroll 1
@@ -2244,12 +2250,8 @@ __device__ void greedy_pair(unsigned long long* okey, const uint32_t* cgen, uint
             acc = __ballot_sync(full, my_acc);
         }
         if ((acc >> lane) & 1u) {
-            if (used_q) {
-                atomicOr(&used_r[p1 >> 5], 1u << (p1 & 31));
-                atomicOr(&used_q[p2 >> 5], 1u << (p2 & 31));
-            } else {
-                atomicOr(&used_r[pos >> 5], 1u << (pos & 31));
-            }
+            atomicOr(&used_r[p1 >> 5], 1u << (p1 & 31));
+            atomicOr(&used_q[p2 >> 5], 1u << (p2 & 31));
         }
         // accepted keys, in order, over the keys of resolved candidates (there are
         // at least as many of those, all before the first one queued)
@@ -2273,6 +2275,35 @@ __device__ void greedy_pair(unsigned long long* okey, const uint32_t* cgen, uint
 #pragma unroll 8
     for (int i = 0; i < matches; ++i)
         score = __dadd_rn(score, __longlong_as_double((long long)okey[i]));
+}
+
+// Spectra of up to 8192 peaks have their bitmaps in shared memory; bitmaps for
+// every peak index there (16 KB a greedy warp) would halve the resident CTAs.
+// Longer ones have theirs in device memory, which the L2 cache holds: 64 pairs of
+// 20000 peaks with a candidate each take 0.34 ms at match_limit 2048 and 1.27 ms at
+// 16384 (of 8190 peaks 0.20 and 0.52; without bitmaps, each candidate compared
+// with every accepted one, 8.9 and 567 ms).  Out of line: the callers' registers
+// are for the ordinary case.
+constexpr int kUsedWords = kLongPeaks / 32;  // words of each bitmap in shared memory
+constexpr int kFullWords = 2048;  // words that hold every peak index
+constexpr int kLongWords = 2 * kFullWords;
+// greedy warps a multiprocessor with bitmaps in device memory: at 80 registers 25
+// warps fit, of which at most every second is one
+constexpr int kLongWarps = 12;
+struct Greedy {
+    double score;
+    int matches;
+};
+template <bool MODIFIED>
+__device__ __noinline__ Greedy greedy_long(unsigned long long* okey, const uint32_t* cgen,
+                                           uint32_t* bits, uint16_t* queue, int n) {
+    Greedy r{0.0, 0};
+    greedy_pair<MODIFIED, true>(okey, cgen, bits, bits + kFullWords, queue, n, r.score, r.matches);
+    return r;
+}
+inline bool may_be_long(const SpecSet& s) { return s.n_peaks > 32 * kUsedWords; }
+constexpr size_t long_bits_bytes(int sms) {
+    return (size_t)sms * kLongWarps * kLongWords * sizeof(uint32_t);
 }
 
 // The pair's outputs (dense, or a sparse hit above the threshold).
@@ -2309,21 +2340,19 @@ __device__ __forceinline__ bool pair_of(const PairParams& P, int64_t item, int64
     return !(P.sym && ri > qi);
 }
 
-constexpr int kUsedWords = 256;  // words of each used-peak bitmap: spectra of up to 8192 peaks
 constexpr int kPairCache = 1024;  // query m/z values pair_kernel keeps in shared memory
 constexpr int kPairSlice = 512;   // candidates a warp takes on alone, at most
 constexpr int kDeferred = 64;     // pairs with more that a CTA collects
 
-// Shared memory of pair_kernel: candidates, used-peak bitmaps (or the bitmap of
-// accepted candidates, for spectra with more peaks), gen_pair's scratch, the
-// warps' greedy queues.
-__host__ __device__ constexpr int pair_used_words(int cap) {
-    return cap / 32 > 2 * kUsedWords ? cap / 32 : 2 * kUsedWords;
-}
-constexpr size_t pair_smem_bytes(int cap, int threads, int cache) {
-    return (size_t)cap * 12 + (size_t)pair_used_words(cap) * 4 + gen_scratch_bytes(threads, cache) +
+// Shared memory of pair_kernel: candidates, used-peak bitmaps, gen_pair's scratch,
+// the warps' greedy queues.
+constexpr size_t pair_smem_bytes(int cap, int threads, int cache, int used_words = kUsedWords) {
+    return (size_t)cap * 12 + (size_t)used_words * 8 + gen_scratch_bytes(threads, cache) +
            (size_t)threads / 32 * kQueued * sizeof(uint16_t);
 }
+constexpr int kMaxPairWarps = 16;
+static_assert(2 * kUsedWords / kMaxPairWarps / 2 * 32 >= kHeavyPeaks,
+              "a light pair's bitmaps fit every warp's share");
 // the query's m/z are kept where they fit
 constexpr int pair_cache(int cap, int threads, size_t optin) {
     return pair_smem_bytes(cap, threads, kPairCache) <= optin ? kPairCache : 0;
@@ -2335,18 +2364,18 @@ constexpr int pair_cache(int cap, int threads, size_t optin) {
 // the one greedy warp.  So CTAs take only the heavy pairs, first, and then every
 // warp takes light ones of its own into a share of the candidate buffer; a pair
 // with more candidates than that holds (512 of 2048) is left to the CTA.  With
-// the bitmaps cut to 8192 peaks, 1024 query m/z in shared memory and 80
+// the bitmaps of 8192 peaks, 1024 query m/z in shared memory and 80
 // registers six CTAs fit an SM (five before): the pairs of 12345 symmetric spectra
 // take 180 us (305 before), of sparse 20000 x 20000 113 (216), of modified cosine
 // 297 (421).  What is left is the longest heavy pairs.
 template <bool SPARSE, bool MODIFIED>
 __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
-    if (*P.bad) return;
+    if (*P.bad || (P.gate && *P.gate != P.gate_value)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned long long* okey = reinterpret_cast<unsigned long long*>(smem_raw);
     uint32_t* cgen = reinterpret_cast<uint32_t*>(okey + P.cap);
     uint32_t* used = cgen + P.cap;
-    const int used_words = pair_used_words(P.cap);
+    const int used_words = 2 * P.used_words;
     const GenScratch gen = gen_scratch(used + used_words, blockDim.x, P.cache);
     uint16_t* queues = reinterpret_cast<uint16_t*>(gen.qmz + P.cache);
     __shared__ int s_scan[32];
@@ -2378,14 +2407,26 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
         if (n > 0) {
             const int nr = (int)(P.R.off[ri + 1] - P.R.off[ri]);
             const int nq = (int)(P.Q.off[qi + 1] - P.Q.off[qi]);
-            uint32_t* used_q = max(nr, nq) <= 16 * words ? used_r + words / 2 : nullptr;
-            const int words_r = ((used_q ? nr : n) + 31) / 32, words_q = used_q ? (nq + 31) / 32 : 0;
-            for (int i = t; i < words_r; i += nt) used_r[i] = 0u;
-            for (int i = t; i < words_q; i += nt) used_q[i] = 0u;
+            // a warp's pairs are light ones, whose peaks fit its share of the bitmaps
+            constexpr bool kCta = std::is_same<decltype(sync), BlockSync>::value;
+            const bool fits = !kCta || max(nr, nq) <= 32 * (words / 2);
+            uint32_t* const bits_r = fits ? used_r : P.long_bits + (size_t)blockIdx.x * kLongWords;
+            uint32_t* const bits_q = bits_r + (fits ? words / 2 : kFullWords);
+            for (int i = t; i < (nr + 31) / 32; i += nt) bits_r[i] = 0u;
+            for (int i = t; i < (nq + 31) / 32; i += nt) bits_q[i] = 0u;
             int m = 1;
             while (m < n) m <<= 1;
             sort_pair(k, g, n, m, nt, t, sync);
-            if (t < 32) greedy_pair<MODIFIED>(k, g, used_r, used_q, queue, n, score, matches);
+            if (t < 32) {
+                if (fits) {
+                    greedy_pair<MODIFIED, false>(k, g, used_r, used_r + words / 2, queue, n, score,
+                                                 matches);
+                } else {
+                    const Greedy r = greedy_long<MODIFIED>(k, g, bits_r, queue, n);
+                    score = r.score;
+                    matches = r.matches;
+                }
+            }
         }
         if (t == 0) write_pair<SPARSE>(P, ri, qi, n, score, matches, total >= P.match_limit);
         sync();
@@ -2641,16 +2682,22 @@ pair_kernel_pipe(PairParams P) {
                 const int nr = (int)(P.R.off[ri + 1] - P.R.off[ri]);
                 const int nq = (int)(P.Q.off[qi + 1] - P.Q.off[qi]);
                 const bool fits = max(nr, nq) <= 32 * kUsedWords;
-                uint32_t* used_q = fits ? used_r + kUsedWords : nullptr;
-                if (fits) {
-                    for (int i = lane; i < (nr + 31) / 32; i += 32) used_r[i] = 0u;
-                    for (int i = lane; i < (nq + 31) / 32; i += 32) used_q[i] = 0u;
-                } else {
-                    for (int i = lane; i < (n + 31) / 32; i += 32) used_r[i] = 0u;
-                }
+                uint32_t* const bits_r =
+                    fits ? used_r : P.long_bits + ((size_t)blockIdx.x * kPipeCons + w) * kLongWords;
+                uint32_t* const bits_q = bits_r + (fits ? kUsedWords : kFullWords);
+                for (int i = lane; i < (nr + 31) / 32; i += 32) bits_r[i] = 0u;
+                for (int i = lane; i < (nq + 31) / 32; i += 32) bits_q[i] = 0u;
                 __syncwarp();
-                greedy_pair<MODIFIED>(okey0 + (size_t)b * P.cap, cgen0 + (size_t)b * P.cap,
-                                      used_r, used_q, s_queue[w], n, score, matches);
+                unsigned long long* okey = okey0 + (size_t)b * P.cap;
+                const uint32_t* cgen = cgen0 + (size_t)b * P.cap;
+                if (fits) {
+                    greedy_pair<MODIFIED, false>(okey, cgen, used_r, used_r + kUsedWords,
+                                                 s_queue[w], n, score, matches);
+                } else {
+                    const Greedy r = greedy_long<MODIFIED>(okey, cgen, bits_r, s_queue[w], n);
+                    score = r.score;
+                    matches = r.matches;
+                }
             }
             __syncwarp();
             if (lane == 0) {
@@ -2761,8 +2808,8 @@ constexpr int kScatterThreads = 256;  // index scatter: a warp per spectrum
 
 // Prepare one or two spectrum sets (the second may be empty) in one launch.
 void launch_prep(const PrepSide& p0, const PrepSide& p1, const IndexGeom& g, uint32_t* bad,
-                 uint32_t* err, int max_peaks, int sms, cudaStream_t s) {
-    const PrepSides sides{{p0, p1}, blocks_for(p0.S.n, kPrepPerBlock, sms)};
+                 uint32_t* err, int max_peaks, int sms, cudaStream_t s, uint32_t* any_long = nullptr) {
+    const PrepSides sides{{p0, p1}, blocks_for(p0.S.n, kPrepPerBlock, sms), any_long};
     const int blocks1 = p1.S.n > 0 ? blocks_for(p1.S.n, kPrepPerBlock, sms) : 0;
     prep_kernel<<<sides.blocks0 + blocks1, kPrepThreads, 0, s>>>(sides, g, bad, err, max_peaks);
 }
@@ -2867,6 +2914,8 @@ int run_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         need += bump_size((size_t)p.spill_cap * sizeof(int2));
         need += bump_size(gpool_bytes);
     }
+    if (may_be_long(args.ref) || may_be_long(args.qry))
+        need += bump_size(long_bits_bytes(ctx->sm_count));
     need += 4096;
     rc = arena_reserve(ctx, ctx->scratch, need, s);
     if (rc) return rc;
@@ -2908,6 +2957,9 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     uint2* probe2 = idx == 2 ? bp.take<uint2>(ref_peaks) : nullptr;
     double* snR = bp.take<double>(nR);
     double* snQ = bp.take<double>(nQ);
+    uint32_t* long_bits = may_be_long(args.ref) || may_be_long(args.qry)
+                              ? bp.take<uint32_t>(long_bits_bytes(ctx->sm_count) / 4)
+                              : nullptr;
     CMS_CUDA_TRY(cudaMemsetAsync(small, 0, zeroed, s));
 
     const IndexGeom g{p.tile, p.n_tiles, p.nb, 1.0 / p.width};
@@ -2936,6 +2988,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     pp.match_limit = args.match_limit;
     pp.cap = p.cap;
     pp.cache = cache;
+    pp.used_words = kUsedWords;
+    pp.long_bits = long_bits;
     pp.pairs = nullptr;
     pp.n_pairs = nullptr;
     pp.pairs_cap = 0;
@@ -2961,11 +3015,10 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pair_blocks_per_sm, pair_k, p.pair_threads,
                                                   pair_smem);
     pair_blocks_per_sm = std::max(1, pair_blocks_per_sm);
-    const int pair_grid = ctx->sm_count * pair_blocks_per_sm;
+    const int pair_grid = ctx->sm_count * std::min(kLongWarps, pair_blocks_per_sm);
 
     const size_t pipe_smem = pipe_smem_bytes(p.cap, p.pair_threads);
-    if (p.mode == 2 && pipe_smem <= ctx->smem_optin &&
-        p.cap / 32 <= 2 * kUsedWords) {  // the accepted bitmap of spectra past kUsedWords
+    if (p.mode == 2 && pipe_smem <= ctx->smem_optin) {
         // whole matrix: the pipelined pair kernel (pair_threads producers
         // plus the consumer warps)
         void (*pipe_k)(PairParams) =
@@ -2978,7 +3031,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pipe_k, pipe_threads, pipe_smem);
         StageScope sc(ctx, 4, 1, s);
-        pipe_k<<<ctx->sm_count * std::max(1, per_sm), pipe_threads, pipe_smem, s>>>(pp);
+        per_sm = std::max(1, std::min(kLongWarps / kPipeCons, per_sm));
+        pipe_k<<<ctx->sm_count * per_sm, pipe_threads, pipe_smem, s>>>(pp);
         CMS_CUDA_TRY(cudaGetLastError());
         return mirror();
     }
@@ -3476,6 +3530,7 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     if (rc) return rc;
     uint32_t* bad = reinterpret_cast<uint32_t*>(base);
     uint32_t* err = reinterpret_cast<uint32_t*>(base + 4);
+    uint32_t* any_long = reinterpret_cast<uint32_t*>(base + 32);
     double* snR = reinterpret_cast<double*>(base + kNoAllocHeader);
     double* snQ = snR + n_ref;
     // the array keeps the previous call's contents: reset the flags
@@ -3486,7 +3541,7 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     CMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const IndexGeom none{1, 1, 1, 1.0};
     launch_prep(PrepSide{args.ref, snR}, PrepSide{args.qry, snQ}, none, bad, err, CMS_MAX_PEAKS, sms,
-                s);
+                s, any_long);
     CMS_CUDA_TRY(cudaGetLastError());
 
     PairParams pp{};
@@ -3504,18 +3559,26 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     pp.n_pairs = nullptr;
     pp.pairs_cap = 0;
     pp.work = reinterpret_cast<unsigned long long*>(base + 8);
+    pp.gate = any_long;
     pp.dense = DenseOut{score, matches, overflow, ld};
     pp.sparse = SparseOut{};
     pp.err = err;
     pp.bad = bad;
     const int pair_threads = 128;
-    const size_t pair_smem = pair_smem_bytes(cap, pair_threads, 0);
-    if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
-    int per_sm = 1;
-    CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<false, false>,
-                                                               pair_threads, pair_smem));
-    pair_kernel<false, false><<<sms * std::max(1, per_sm), pair_threads, pair_smem, s>>>(pp);
-    CMS_CUDA_TRY(cudaGetLastError());
+    // Without scratch for the bitmaps of long spectra, a call that has any (known on
+    // the device only) keeps all of them in shared memory: one of two launches
+    // runs, the other returns at once.
+    for (uint32_t full = 0; full < (may_be_long(args.ref) || may_be_long(args.qry) ? 2u : 1u); ++full) {
+        pp.gate_value = full;
+        pp.used_words = full ? kFullWords : kUsedWords;
+        const size_t pair_smem = pair_smem_bytes(cap, pair_threads, 0, pp.used_words);
+        if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
+        int per_sm = 1;
+        CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, pair_kernel<false, false>, pair_threads, pair_smem));
+        pair_kernel<false, false><<<sms * std::max(1, per_sm), pair_threads, pair_smem, s>>>(pp);
+        CMS_CUDA_TRY(cudaGetLastError());
+    }
     if (device_error)
         CMS_CUDA_TRY(cudaMemcpyAsync(device_error, err, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     return CMS_OK;
@@ -3701,6 +3764,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
                   bump_size((size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(Probe)) +
                   bump_size((size_t)spill_cap * sizeof(int2)) +
                   bump_size(kSlotWords * sizeof(uint32_t)) + bump_size(gpool_bytes) + 4096;
+    const bool maybe_long = may_be_long(Q) || may_be_long(lib->spec);
+    if (maybe_long) need += bump_size(long_bits_bytes(ctx->sm_count));
     int rc = arena_reserve(ctx, ctx->scratch, need, s);
     if (rc) return rc;
     Bump bp{(char*)ctx->scratch.ptr, 0, ctx->scratch.bytes};
@@ -3718,6 +3783,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     Probe* probe = bp.take<Probe>((size_t)std::max<int64_t>(1, n_q_peaks));
     int2* spill = bp.take<int2>(spill_cap);
     unsigned char* gpool = bp.take<unsigned char>(gpool_bytes);
+    uint32_t* long_bits =
+        maybe_long ? bp.take<uint32_t>(long_bits_bytes(ctx->sm_count) / 4) : nullptr;
 
     {
         StageScope sc(ctx, 0, 2, s);
@@ -3787,6 +3854,8 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     pp.match_limit = lib->match_limit;
     pp.cap = cap;
     pp.cache = cache;
+    pp.used_words = kUsedWords;
+    pp.long_bits = long_bits;
     pp.pairs = spill;
     pp.n_pairs = spill_count;
     pp.pairs_cap = spill_cap;
@@ -3801,7 +3870,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<true, false>, 128,
                                                       pair_smem);
-        pair_kernel<true, false><<<std::max(1, std::min(ctx->sm_count * std::max(1, per_sm),
+        pair_kernel<true, false><<<std::max(1, std::min(ctx->sm_count * std::max(1, std::min(kLongWarps, per_sm)),
                                                   (int)std::min<long long>(spill_cap, 1 << 20))),
                             128, pair_smem, s>>>(pp);
     }

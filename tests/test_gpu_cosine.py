@@ -471,3 +471,55 @@ def test_pair_kernel_windows_as_defined(cuda_device, pair_threads):
                   float(np.nextafter(100.0 + 0.1, 0.0))):
         want = oracle.cosine_greedy(ref, near, 0.1, shift, 64)
         assert_same(gpu_dense(ref, near, P(0.1, 64, shift=shift), cfg), want, f"{shift}")
+
+
+def _one_candidate_a_peak(n, peaks, seed):
+    from cudams.packing import pack_csr
+
+    off = np.arange(n + 1) * peaks
+    mz = np.tile(100.0 + 1500.0 / peaks * np.arange(peaks), n)
+    inten = np.random.default_rng(seed).random(off[-1]) + 0.01
+    return pack_csr(mz.astype(np.float32), inten.astype(np.float32), off, None)
+
+
+@pytest.mark.parametrize("ml", [64, 4096, 16384])
+def test_long_spectra_used_peaks(cuda_device, ml):
+    """Spectra at and past the peaks whose bitmaps are in shared memory, with peaks
+    shared by many candidates, through every launch of the pair kernels."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(98)
+
+    def make(lens):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(100.0, 400.0, k)) for k in lens])
+        return pack_csr(mz.astype(np.float32), rng.random(off[-1]).astype(np.float32) + 0.01, off,
+                        None)
+
+    ref, qry = make([8192, 8193, 20000, 40, 32767]), make([20000, 8193, 100, 8192])
+    want = oracle.cosine_greedy(ref, qry, 0.03, 0.0, ml)
+    for cfg in ({"mode": 2}, {"mode": 2, "pair_threads": 64}, {"mode": 1, "tile_spectra": 32}):
+        assert_same(gpu_dense(ref, qry, P(0.03, ml, 65535), cfg), want, f"{cfg}")
+
+
+@pytest.mark.parametrize("ml", [2048, 16384])
+def test_long_spectra_cost(cuda_device, ml):
+    """A pair's time grows with its peaks and candidates, not with their square: 2.5
+    times the peaks (and at 16384 twice the candidates) within eight times the time."""
+    import torch
+
+    from cudams import kernels
+
+    def seconds(peaks):
+        a, b = (_one_candidate_a_peak(8, peaks, s).to_device(cuda_device) for s in (1, 2))
+        best = float("inf")
+        for _ in range(4):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            kernels.cosine_greedy_dense(a, b, 450.0 / peaks, 0.0, ml, config={"mode": 2})
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert seconds(20000) < 8 * seconds(8190)

@@ -163,3 +163,23 @@ def test_unusual_precursor_answers_do_not_depend_on_the_call_size(cuda_device, s
     small, large = (call()[:40] for call in calls)
     for name in ("score", "matches", "overflow"):
         np.testing.assert_array_equal(small[name], large[name])
+
+
+@pytest.mark.parametrize("ml", [512, 16384])
+def test_long_spectra(cuda_device, ml):
+    """Spectra at and past the peaks whose used-peak bitmaps are in shared memory."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(54)
+
+    def make(lens):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(100.0, 400.0, k)) for k in lens])
+        return pack_csr(mz.astype(np.float32), rng.random(off[-1]).astype(np.float32) + 0.01, off,
+                        None)
+
+    ref, qry = make([8193, 200, 32767]), make([8192, 20000])
+    rp, qp = rng.uniform(300, 420, 3), rng.uniform(300, 420, 2)
+    want = oracle.modified_cosine(ref, qry, rp, qp, 0.01, ml)
+    for config in ({"mode": 2}, {"mode": 1, "tile_spectra": 32}):
+        assert_same(_gpu(ref, rp, qry, qp, 0.01, ml, config), want, str(config))

@@ -123,3 +123,22 @@ def test_noalloc_rejects_host_output(cuda_device):
     assert "score must be device memory of the current device" in _native.last_error()
     torch.cuda.synchronize()
     assert (host_score == -5.0).all()
+
+
+def test_long_spectra(cuda_device):
+    """Spectra past the peaks of the small used-peak bitmaps: the launch with full ones."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(99)
+
+    def make(lens):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(100.0, 400.0, k)) for k in lens])
+        return pack_csr(mz.astype(np.float32), rng.random(off[-1]).astype(np.float32) + 0.01, off,
+                        None)
+
+    for lens in ([8192, 30, 8192], [8193, 30, 65535]):
+        r, q = make(lens), make(lens[::-1])
+        got, err = _noalloc(r.to_device(cuda_device), q.to_device(cuda_device), 0.03, 0.0, 4096)
+        assert err == 0
+        assert_same(got, _oracle(r, q, 0.03, 0.0, 4096), f"{lens}")
