@@ -1555,7 +1555,7 @@ struct PairParams {
     double tol;
     double shift;
     int match_limit;
-    int cap;  // power of two >= match_limit
+    int cap;  // candidates a buffer holds: a power of two >= match_limit, or list_cap
     int cache;  // pair_kernel: query m/z values kept in shared memory (pair_cache)
     int used_words;       // pair_kernel: words of each used-peak bitmap in shared memory
     uint32_t* long_bits;  // bitmaps of pairs with more peaks, kLongWords a greedy warp (or null)
@@ -2353,6 +2353,13 @@ constexpr size_t pair_smem_bytes(int cap, int threads, int cache, int used_words
 constexpr int kMaxPairWarps = 16;
 static_assert(2 * kUsedWords / kMaxPairWarps / 2 * 32 >= kHeavyPeaks,
               "a light pair's bitmaps fit every warp's share");
+// Candidates the buffer holds when pair_kernel takes a spill list: a warp's share
+// is as large as match_limit, up to kPairSlice, so that small limits leave no pair
+// to the CTAs for want of room (1500 x 1501 uniform spectra at match_limit 16 and
+// tolerance 0.5, nearly all pairs spilled: 7.2 ms with a share of 4, 3.0 with 16).
+constexpr int list_cap(int cap, int threads) {
+    return std::max(cap, threads / 32 * std::min(kPairSlice, cap));
+}
 // the query's m/z are kept where they fit
 constexpr int pair_cache(int cap, int threads, size_t optin) {
     return pair_smem_bytes(cap, threads, kPairCache) <= optin ? kPairCache : 0;
@@ -2724,7 +2731,8 @@ struct Plan {
     int nb;
     double width;
     int pair_threads;
-    int cap;
+    int cap;       // power of two >= match_limit
+    int pair_cap;  // candidates of pair_kernel's buffer
     unsigned int spill_cap;
     int sym;               // cms_cosine_config.symmetric
     double cand_per_pair;  // cms_cosine_config.cand_per_pair (0: unknown)
@@ -2778,6 +2786,7 @@ int make_plan(const CosineArgs& args, const cms_cosine_config* cfg, bool sparse,
         set_error("cms_cosine_greedy: pair_threads must be a multiple of 32 in [64, 512]");
         return CMS_ERR_INVALID;
     }
+    p.pair_cap = p.mode == 2 ? p.cap : list_cap(p.cap, p.pair_threads);
     const long long pairs = (long long)args.ref.n * (long long)args.qry.n;
     long long sc = std::max<long long>(1 << 20, pairs / 64);
     sc = std::min<long long>(sc, std::min<long long>(pairs, 1LL << 28));
@@ -2929,8 +2938,8 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
                    const SparseOut* sparse, const Plan& p, cudaStream_t s) {
     int rc = CMS_OK;
     const int sym = p.sym;
-    const int cache = pair_cache(p.cap, p.pair_threads, ctx->smem_optin);
-    const size_t pair_smem = pair_smem_bytes(p.cap, p.pair_threads, cache);
+    const int cache = pair_cache(p.pair_cap, p.pair_threads, ctx->smem_optin);
+    const size_t pair_smem = pair_smem_bytes(p.pair_cap, p.pair_threads, cache);
     const int64_t nR = args.ref.n, nQ = args.qry.n;
     const size_t gpool_warps = (size_t)ctx->sm_count * 64;
     const size_t gpool_bytes = gpool_warps * (size_t)kGPool * 16;
@@ -2986,7 +2995,7 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     pp.tol = args.tol;
     pp.shift = args.shift;
     pp.match_limit = args.match_limit;
-    pp.cap = p.cap;
+    pp.cap = p.pair_cap;
     pp.cache = cache;
     pp.used_words = kUsedWords;
     pp.long_bits = long_bits;
@@ -3744,7 +3753,7 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     CMS_CUDA_TRY(cudaMemsetAsync(hit_count, 0, sizeof(int64_t), s));
     if (n_q == 0) return CMS_OK;
 
-    const int cap = next_pow2(std::max(2, lib->match_limit));
+    const int cap = list_cap(next_pow2(std::max(2, lib->match_limit)), 128);
     const int cache = pair_cache(cap, 128, ctx->smem_optin);
     const size_t pair_smem = pair_smem_bytes(cap, 128, cache);
     if (pair_smem > ctx->smem_optin) {

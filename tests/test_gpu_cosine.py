@@ -523,3 +523,69 @@ def test_long_spectra_cost(cuda_device, ml):
         return best
 
     assert seconds(20000) < 8 * seconds(8190)
+
+
+@pytest.mark.parametrize("ml,peaks,pair_threads", [(1, 3, 128), (1, 3, 512), (600, 23, 512)])
+def test_many_deferred_pairs(cuda_device, ml, peaks, pair_threads):
+    """More light pairs than a CTA collects before it works them off, several times over,
+    every one with more candidates than a warp's share of the buffer."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(101)
+    n = 300 if ml == 1 else 200
+
+    def make():
+        off = np.arange(n + 1) * peaks
+        mz = np.tile(100.0 + 0.001 * np.arange(peaks), n)
+        return pack_csr(mz.astype(np.float32), rng.integers(1, 9, off[-1]).astype(np.float32), off,
+                        None)
+
+    ref, qry = make(), make()
+    want = oracle.cosine_greedy(ref, qry, 0.05, 0.0, ml)
+    cfg = {"mode": 1, "tile_spectra": 64, "pair_threads": pair_threads}
+    for _ in range(2):
+        assert_same(gpu_dense(ref, qry, P(0.05, ml), cfg), want, f"{cfg}")
+
+
+@pytest.mark.parametrize("pair_threads", [96, 192, 224, 320, 416, 480])
+def test_light_and_heavy_pairs(cuda_device, pair_threads):
+    """Spilled pairs on both sides of the number of peaks a warp takes, with warps whose
+    share of the used-peak bitmaps is an odd number of words."""
+    from cudams.packing import pack_csr
+
+    rng = np.random.default_rng(102)
+
+    def make(lens):
+        off = np.concatenate([[0], np.cumsum(lens)])
+        mz = np.concatenate([np.sort(rng.uniform(100.0, 130.0, k)) for k in lens])
+        return pack_csr(mz.astype(np.float32), rng.integers(1, 30, off[-1]).astype(np.float32), off,
+                        None)
+
+    ref, qry = make([255, 256, 257, 256, 300, 40]), make([256, 257, 255, 64, 256])
+    for tol in (0.05, 0.2):
+        want = oracle.cosine_greedy(ref, qry, tol, 0.0, 4096)
+        cfg = {"mode": 1, "tile_spectra": 32, "pair_threads": pair_threads}
+        assert_same(gpu_dense(ref, qry, P(tol, 4096), cfg), want, f"{tol} {cfg}")
+
+
+def test_small_match_limit_cost(cuda_device):
+    """Nearly every pair reaches a match limit of 16 and is left to the pair kernel, whose
+    warps take such pairs: the call stays within 2.8 times that with a limit of 512."""
+    import torch
+
+    from cudams import kernels, synthetic
+
+    a, b = (synthetic.uniform_spectra(1500, seed=s).to_device(cuda_device) for s in (1, 2))
+
+    def seconds(ml):
+        best = float("inf")
+        for _ in range(4):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            kernels.cosine_greedy_dense(a, b, 0.5, 0.0, ml, config={"mode": 1, "tile_spectra": 64})
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert seconds(16) < 2.8 * seconds(512)
