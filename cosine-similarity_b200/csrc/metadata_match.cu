@@ -609,12 +609,20 @@ extern "C" int cms_mass_match(const double* ref, int64_t n_ref, const double* q,
         return CMS_ERR_INVALID;
     }
     // Rows a warp takes: 128, so that its columns are loaded once for 64 KB of
-    // output (64: 2% slower, 32: 20%), or fewer where that leaves less than four
-    // units a resident warp.  Ten CTAs per resident one, so that the last wave is
-    // short (one per resident: 572 us instead of 420 for 40000 x 50000 in ppm).
+    // output, or fewer where that leaves less than eight units a multiprocessor, or
+    // a second wave of warps that is nearly empty.  Dalton, cold cache: 40000 x 50000
+    // 410 us with 128 rows, 424 with 64; 16000 x 16384 (4000 units of 128 rows for
+    // 3552 resident warps) 72 us with 128, 66 with 64, 76 with 32; 8000 x 8192 33 us
+    // with 128, 25 with 64, 46 with 8; 4000 x 4096 14 us with 16 or 32, 24 with 4.
+    // Ten CTAs per resident one, so that the last wave is short (one per resident:
+    // 572 us instead of 420 for 40000 x 50000 in ppm).
     const int64_t sms = sm_count_of_current(), col_blocks = (n_q + kMassWarpCols - 1) / kMassWarpCols;
+    const int64_t resident = sms * 24;
     int rows = 128;
-    while (rows > 4 && col_blocks * ((n_ref + rows - 1) / rows) < sms * 24 * 4) rows /= 2;
+    for (; rows > 4; rows /= 2) {
+        const int64_t u = col_blocks * ((n_ref + rows - 1) / rows);
+        if (u >= 2 * resident || (u >= sms * 8 && u <= resident)) break;
+    }
     const int64_t units = col_blocks * ((n_ref + rows - 1) / rows);
     const int per_block = kMassThreads / 32;
     const int grid = (int)std::max<int64_t>(

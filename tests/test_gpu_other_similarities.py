@@ -187,3 +187,30 @@ def test_intersect_mz_tiles(cuda_device, n_q, scaling):
                                       check_errors=True).cpu().numpy()
     want = other.intersect_mz(a, b, scaling)
     np.testing.assert_array_equal(got.view(np.uint64), want.view(np.uint64))
+
+
+def test_mass_match_medium_cost(cuda_device):
+    """A result of 64 MB takes at most 1.6 times a plain fill of it: a warp's columns
+    are loaded for enough rows."""
+    import torch
+
+    from cudams import kernels
+
+    rng = np.random.default_rng(61)
+    r, q = (torch.from_numpy(rng.uniform(100.0, 1000.0, n)).to(_dev()) for n in (8000, 8192))
+    out = torch.empty((8000, 8192), dtype=torch.uint8, device=_dev())
+
+    def ms(f):
+        best = float("inf")
+        for _ in range(8):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(8):
+                f()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    fill = ms(lambda: out.fill_(1))
+    assert ms(lambda: kernels.mass_match_matrix(r, q, 0.1, out=out)) < 1.6 * fill
