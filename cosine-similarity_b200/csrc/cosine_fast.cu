@@ -1743,20 +1743,23 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
         const double shift = (MODIFIED && pass) ? __dsub_rn(P.R.prec[ri], P.Q.prec[qi]) : P.shift;
 #pragma unroll 1
         for (int pc = 0; pc < nr && !overflow; pc += kGenPeaks * nt) {
-            // kGenPeaks consecutive peaks a thread: a pair that overflows is usually
-            // done after one chunk of 256
+            // kGenPeaks consecutive peaks a thread (a pair that overflows is usually
+            // done after one chunk of 256), or one where that is enough: a thread's
+            // peaks are searched for one after the other (300 x 301 uniform spectra,
+            // the whole matrix at match_limit 2048: 1250 us with two, 1070 with one)
+            const int per = nr - pc > nt ? kGenPeaks : 1;
             int start[kGenPeaks], cnt[kGenPeaks], mine = 0;
             float mz[kGenPeaks];
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
-                const int p1 = pc + kGenPeaks * tid + u;
-                mz[u] = p1 < nr ? P.R.mz[r0 + p1] : 0.f;
+                const int p1 = pc + per * tid + u;
+                mz[u] = u < per && p1 < nr ? P.R.mz[r0 + p1] : 0.f;
             }
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
-                const int p1 = pc + kGenPeaks * tid + u;
+                const int p1 = pc + per * tid + u;
                 start[u] = cnt[u] = 0;
-                if (p1 < nr) {
+                if (u < per && p1 < nr) {
                     const double mz1 = (double)mz[u];
                     // the window as float32 bounds of the query's m/z (exact, see
                     // Window): first p2 at or above, then on to the last one inside.
@@ -1795,7 +1798,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                     }
                     cnt[u] = L - start[u];
                     if (cnt[u])
-                        G.w[kGenPeaks * tid + u] = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
+                        G.w[per * tid + u] = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
                 }
                 mine += cnt[u];
             }
@@ -1818,7 +1821,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
                 uint32_t gen = ((uint32_t)pass << 31) |
-                               ((uint32_t)(pc + kGenPeaks * tid + u) << 16) | (uint32_t)start[u];
+                               ((uint32_t)(pc + per * tid + u) << 16) | (uint32_t)start[u];
                 const int last = min(take, first + cnt[u]);
 #pragma unroll 1
                 for (int i = first; i < last; ++i) cgen[total + i] = gen++;
