@@ -3583,7 +3583,8 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
     for (uint32_t full = 0; full < (may_be_long(args.ref) || may_be_long(args.qry) ? 2u : 1u); ++full) {
         pp.gate_value = full;
         pp.used_words = full ? kFullWords : kUsedWords;
-        const size_t pair_smem = pair_smem_bytes(cap, pair_threads, 0, pp.used_words);
+        pp.cache = cap <= 2048 ? kPairCache : 0;  // with 4096 it would cost a resident CTA
+        const size_t pair_smem = pair_smem_bytes(cap, pair_threads, pp.cache, pp.used_words);
         if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
         int per_sm = 1;
         CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
