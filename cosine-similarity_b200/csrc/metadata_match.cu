@@ -25,7 +25,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <mutex>
 
 #include "cms_internal.cuh"
 
@@ -550,46 +549,81 @@ int sm_count_of_current() {
     return sms;
 }
 
-// Stream-ordered workspace from a pool of the library's own, one per device,
-// which keeps up to kKeepBytes between calls (the device's default pool gives
-// everything back at each synchronisation: 0.5 ms a call at 10007 x 9000); what
-// is above is returned to the device when a stream is synchronised.  The pool
-// orders reuse between streams and threads itself.
-constexpr uint64_t kKeepBytes = 128ull << 20;
-constexpr int kMaxDevices = 64;
+// Workspace of one IntersectMz call: entries, bucket counts, bucket table, distinct
+// counts, chunk sums.
+struct IxSpace {
+    uint32_t nb;  // buckets: a power of two >= the query peaks, 2^26 at most
+    int chunks;
+    size_t ent_bytes, bytes;
+};
+IxSpace ix_space(int64_t n_q, int64_t n_q_peaks) {
+    IxSpace w{};
+    w.nb = kScanChunk;
+    while (w.nb < (uint64_t)n_q_peaks && w.nb < (1u << 26)) w.nb <<= 1;
+    w.chunks = (int)(w.nb / kScanChunk);
+    w.ent_bytes = (size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(IxEntry);
+    w.bytes = w.ent_bytes + ((size_t)w.nb * 2 + 1 + (size_t)n_q + (size_t)w.chunks) * 4;
+    return w;
+}
 
-int workspace_alloc(unsigned char** p, size_t bytes, cudaStream_t s) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    int dev = 0;
-    CMS_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) {
-        set_error("device ordinal %d out of range", dev);
-        return CMS_ERR_UNSUPPORTED;
+// What every entry point refuses; `launch` says whether there is anything to do.
+int ix_check(const char* who, const double* ref_mz, const int64_t* ref_off, int64_t n_ref,
+             int64_t n_ref_peaks, const double* q_mz, const int64_t* q_off, int64_t n_q,
+             int64_t n_q_peaks, const double* out, int64_t ld, bool& launch) {
+    launch = false;
+    if (n_ref < 0 || n_q < 0 || n_ref_peaks < 0 || n_q_peaks < 0 || ld < n_q ||
+        n_q > 0xFFFFFFFFll || n_q_peaks > 0x7FFFFFFFll) {
+        set_error("%s: invalid sizes (ld >= n_q, n_q < 2^32, n_q_peaks < 2^31)", who);
+        return CMS_ERR_INVALID;
     }
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!pools[dev]) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.handleTypes = cudaMemHandleTypeNone;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            cudaMemPool_t made;
-            CMS_CUDA_TRY(cudaMemPoolCreate(&made, &props));
-            uint64_t keep = kKeepBytes;
-            const cudaError_t e =
-                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
-            if (e != cudaSuccess) {
-                cudaMemPoolDestroy(made);
-                return cuda_fail(e, "cudaMemPoolSetAttribute");
-            }
-            pools[dev] = made;
-        }
-        pool = pools[dev];
+    if (n_ref == 0 || n_q == 0) return CMS_OK;
+    if (!ref_off || !q_off || !out || (n_ref_peaks > 0 && !ref_mz) || (n_q_peaks > 0 && !q_mz)) {
+        set_error("%s: null pointer", who);
+        return CMS_ERR_INVALID;
     }
-    CMS_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, s));
+    launch = true;
+    return CMS_OK;
+}
+
+// The launches, in a workspace of ix_space(n_q, n_q_peaks).bytes.
+int ix_launch(const double* ref_mz, const int64_t* ref_off, int64_t n_ref, int64_t n_ref_peaks,
+              const double* q_mz, const int64_t* q_off, int64_t n_q, int64_t n_q_peaks,
+              double scaling, double* out, int64_t ld, uint32_t* device_error, unsigned char* ws,
+              cudaStream_t s) {
+    const IxSpace w = ix_space(n_q, n_q_peaks);
+    const uint32_t nb = w.nb;
+    const int sms = sm_count_of_current(), chunks = w.chunks;
+    IxEntry* ent = reinterpret_cast<IxEntry*>(ws);
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(ws + w.ent_bytes);
+    uint32_t* tab = cnt + nb;
+    uint32_t* ub = tab + nb + 1;
+    uint32_t* sums = ub + n_q;
+    // query tile: the queries split evenly over the fewest tiles of at most
+    // kIxMaxTile (six bytes of shared memory a query)
+    const int64_t tiles = (n_q + kIxMaxTile - 1) / kIxMaxTile;
+    const int tile = (int)(((n_q + tiles - 1) / tiles + 7) & ~int64_t(7));
+    const size_t smem = (size_t)tile * 6;
+    // 512 threads for long rows, 256 where a row is soon filled
+    auto* kern = tile > 2048 ? intersect_mz_kernel<512> : intersect_mz_kernel<256>;
+    const int threads = tile > 2048 ? 512 : 256;
+    if (const int rc = raise_func_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
+    CMS_CUDA_TRY(cudaMemsetAsync(cnt, 0, (size_t)nb * 4, s));
+    const int igrid = (int)std::max<int64_t>(
+        1, std::min<int64_t>((n_q * 32 + 255) / 256, (int64_t)sms * 16));
+    ix_index_kernel<false><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt, nullptr,
+                                                 ub, device_error);
+    ix_chunk_sums<<<chunks, kScanThreads, 0, s>>>(cnt, sums);
+    ix_chunk_scan<<<chunks, kScanThreads, 0, s>>>(cnt, tab, sums);
+    ix_index_kernel<true><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt, ent,
+                                                nullptr, nullptr);
+    const int64_t units = n_ref * ((n_q + tile - 1) / tile);
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    per_sm = std::max(1, per_sm);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)sms * per_sm));
+    kern<<<grid, threads, smem, s>>>(ref_mz, ref_off, n_ref, n_ref_peaks, n_q, tab, ent, ub, nb - 1,
+                                     scaling, out, ld, tile, device_error);
+    CMS_CUDA_TRY(cudaGetLastError());
     return CMS_OK;
 }
 
@@ -643,63 +677,45 @@ extern "C" int cms_intersect_mz(const double* ref_mz, const int64_t* ref_off, in
                                 int64_t n_q, int64_t n_q_peaks, double scaling, double* out,
                                 int64_t ld, uint32_t* device_error, void* stream) {
     using namespace cms;
-    if (n_ref < 0 || n_q < 0 || n_ref_peaks < 0 || n_q_peaks < 0 || ld < n_q ||
-        n_q > 0xFFFFFFFFll || n_q_peaks > 0x7FFFFFFFll) {
-        set_error("cms_intersect_mz: invalid sizes (ld >= n_q, n_q < 2^32, n_q_peaks < 2^31)");
-        return CMS_ERR_INVALID;
-    }
-    if (n_ref == 0 || n_q == 0) return CMS_OK;
-    if (!ref_off || !q_off || !out || (n_ref_peaks > 0 && !ref_mz) || (n_q_peaks > 0 && !q_mz)) {
-        set_error("cms_intersect_mz: null pointer");
-        return CMS_ERR_INVALID;
-    }
+    bool launch;
+    int rc = ix_check("cms_intersect_mz", ref_mz, ref_off, n_ref, n_ref_peaks, q_mz, q_off, n_q,
+                      n_q_peaks, out, ld, launch);
+    if (rc || !launch) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    // buckets: a power of two >= the query peaks, 2^26 at most
-    uint32_t nb = kScanChunk;
-    while (nb < (uint64_t)n_q_peaks && nb < (1u << 26)) nb <<= 1;
-    const int sms = sm_count_of_current();
-    const int chunks = (int)(nb / kScanChunk);
-    // one workspace: entries, bucket counts, bucket table, distinct counts, chunk sums
-    const size_t ent_bytes = (size_t)std::max<int64_t>(1, n_q_peaks) * sizeof(IxEntry);
-    const size_t words = (size_t)nb * 2 + 1 + (size_t)n_q + (size_t)chunks;
     unsigned char* ws = nullptr;
-    if (const int rc = workspace_alloc(&ws, ent_bytes + words * 4, s)) return rc;
-    IxEntry* ent = reinterpret_cast<IxEntry*>(ws);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(ws + ent_bytes);
-    uint32_t* tab = cnt + nb;
-    uint32_t* ub = tab + nb + 1;
-    uint32_t* sums = ub + n_q;
-    // query tile: the queries split evenly over the fewest tiles of at most
-    // kIxMaxTile (six bytes of shared memory a query)
-    const int64_t tiles = (n_q + kIxMaxTile - 1) / kIxMaxTile;
-    const int tile = (int)(((n_q + tiles - 1) / tiles + 7) & ~int64_t(7));
-    const size_t smem = (size_t)tile * 6;
-    // 512 threads for long rows, 256 where a row is soon filled
-    auto* kern = tile > 2048 ? intersect_mz_kernel<512> : intersect_mz_kernel<256>;
-    const int threads = tile > 2048 ? 512 : 256;
-    int rc = raise_func_smem(reinterpret_cast<const void*>(kern), smem);
-    cudaError_t e = cudaSuccess;
-    if (!rc) e = cudaMemsetAsync(cnt, 0, (size_t)nb * 4, s);
-    if (!rc && e == cudaSuccess) {
-        const int igrid = (int)std::max<int64_t>(
-            1, std::min<int64_t>((n_q * 32 + 255) / 256, (int64_t)sms * 16));
-        ix_index_kernel<false><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt,
-                                                     nullptr, ub, device_error);
-        ix_chunk_sums<<<chunks, kScanThreads, 0, s>>>(cnt, sums);
-        ix_chunk_scan<<<chunks, kScanThreads, 0, s>>>(cnt, tab, sums);
-        ix_index_kernel<true><<<igrid, 256, 0, s>>>(q_mz, q_off, n_q, n_q_peaks, nb - 1, cnt, ent,
-                                                    nullptr, nullptr);
-        const int64_t units = n_ref * ((n_q + tile - 1) / tile);
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-        per_sm = std::max(1, per_sm);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)sms * per_sm));
-        kern<<<grid, threads, smem, s>>>(ref_mz, ref_off, n_ref, n_ref_peaks, n_q, tab, ent, ub,
-                                         nb - 1, scaling, out, ld, tile, device_error);
-        e = cudaGetLastError();
+    CMS_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&ws), ix_space(n_q, n_q_peaks).bytes, s));
+    rc = ix_launch(ref_mz, ref_off, n_ref, n_ref_peaks, q_mz, q_off, n_q, n_q_peaks, scaling, out, ld,
+                   device_error, ws, s);
+    cudaFreeAsync(ws, s);  // stream-ordered: after the kernels
+    return rc;
+}
+
+extern "C" int cms_intersect_mz_workspace(int64_t n_q, int64_t n_q_peaks, int64_t* bytes) {
+    using namespace cms;
+    if (!bytes || n_q < 0 || n_q_peaks < 0 || n_q > 0xFFFFFFFFll || n_q_peaks > 0x7FFFFFFFll) {
+        set_error("cms_intersect_mz_workspace: invalid sizes (n_q < 2^32, n_q_peaks < 2^31)");
+        return CMS_ERR_INVALID;
     }
-    cudaFreeAsync(ws, s);  // stream-ordered: after the kernels above
-    if (rc) return rc;
-    CMS_CUDA_TRY(e);
+    *bytes = (int64_t)ix_space(n_q, n_q_peaks).bytes;
     return CMS_OK;
+}
+
+extern "C" int cms_intersect_mz_in(const double* ref_mz, const int64_t* ref_off, int64_t n_ref,
+                                   int64_t n_ref_peaks, const double* q_mz, const int64_t* q_off,
+                                   int64_t n_q, int64_t n_q_peaks, double scaling, double* out,
+                                   int64_t ld, uint32_t* device_error, void* workspace,
+                                   int64_t workspace_bytes, void* stream) {
+    using namespace cms;
+    bool launch;
+    const int rc = ix_check("cms_intersect_mz_in", ref_mz, ref_off, n_ref, n_ref_peaks, q_mz, q_off,
+                            n_q, n_q_peaks, out, ld, launch);
+    if (rc || !launch) return rc;
+    const int64_t need = (int64_t)ix_space(n_q, n_q_peaks).bytes;
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) || workspace_bytes < need) {
+        set_error("cms_intersect_mz_in: needs a 16-byte aligned workspace of %lld bytes",
+                  (long long)need);
+        return CMS_ERR_INVALID;
+    }
+    return ix_launch(ref_mz, ref_off, n_ref, n_ref_peaks, q_mz, q_off, n_q, n_q_peaks, scaling, out,
+                     ld, device_error, static_cast<unsigned char*>(workspace), (cudaStream_t)stream);
 }

@@ -88,6 +88,10 @@ SIGNATURES = {
     "cms_mass_match": (c_int, [_p, c_int64, _p, c_int64, c_double, c_int, _p, c_int64, _p]),
     "cms_intersect_mz": (c_int, [
         _p, _p, c_int64, c_int64, _p, _p, c_int64, c_int64, c_double, _p, c_int64, _p, _p]),
+    "cms_intersect_mz_workspace": (c_int, [c_int64, c_int64, POINTER(c_int64)]),
+    "cms_intersect_mz_in": (c_int, [
+        _p, _p, c_int64, c_int64, _p, _p, c_int64, c_int64, c_double, _p, c_int64, _p, _p, c_int64,
+        _p]),
     "cms_fingerprint_symmetric": (c_int, [
         c_int, _p, _p, _p, _p, c_int64, c_int, c_float, _p, c_int64, _p]),
 }

@@ -339,10 +339,21 @@ def intersect_mz_matrix(ref_mz, ref_off, q_mz, q_off, scaling: float = 1.0, *, o
     ref_mz, ref_off = ref_mz.contiguous(), ref_off.contiguous()
     q_mz, q_off = q_mz.contiguous(), q_off.contiguous()
     err = torch.zeros(1, dtype=torch.int32, device=device) if check_errors else None
-    rc = lib.cms_intersect_mz(ptr(ref_mz), ptr(ref_off), n_r, int(ref_mz.shape[0]), ptr(q_mz),
-                              ptr(q_off), n_q, int(q_mz.shape[0]), float(scaling), ptr(out),
-                              int(out.stride(0)), ptr(err), stream_handle(s))
-    check(rc, "cms_intersect_mz")
+    n_qp = int(q_mz.shape[0])
+    size = ctypes.c_int64(0)
+    check(lib.cms_intersect_mz_workspace(max(n_q, 0), n_qp, ctypes.byref(size)),
+          "cms_intersect_mz_workspace")
+    # from torch's allocator, on the stream that uses it
+    if stream is None:
+        work = torch.empty(size.value, dtype=torch.uint8, device=device)
+    else:
+        with torch.cuda.stream(stream):
+            work = torch.empty(size.value, dtype=torch.uint8, device=device)
+    rc = lib.cms_intersect_mz_in(ptr(ref_mz), ptr(ref_off), n_r, int(ref_mz.shape[0]), ptr(q_mz),
+                                 ptr(q_off), n_q, n_qp, float(scaling), ptr(out),
+                                 int(out.stride(0)), ptr(err), ptr(work), size.value,
+                                 stream_handle(s))
+    check(rc, "cms_intersect_mz_in")
     if check_errors:
         s.synchronize()
         bits = int(err.item())

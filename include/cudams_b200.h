@@ -403,12 +403,28 @@ int cms_mass_match(const double* ref, int64_t n_ref, const double* q, int64_t n_
  * spectra (CSR: *_off[n+1] into *_mz, peaks sorted by m/z as matchms keeps
  * them; repeated values count once).  Offsets outside [0, n_*_peaks] set
  * bit 2 of *device_error (device memory, may be NULL) and the spectrum reads
- * as empty.
+ * as empty.  The index of the queries (16 bytes a peak and 8 to 16 more for its
+ * table) is allocated on the stream and freed there before the call returns;
+ * a caller that makes many calls, or whose device memory has an allocator of
+ * its own, passes it to cms_intersect_mz_in instead.
  */
 int cms_intersect_mz(const double* ref_mz, const int64_t* ref_off, int64_t n_ref,
                      int64_t n_ref_peaks, const double* q_mz, const int64_t* q_off, int64_t n_q,
                      int64_t n_q_peaks, double scaling, double* out, int64_t ld,
                      uint32_t* device_error, void* stream);
+
+/*
+ * cms_intersect_mz in the caller's device memory: `workspace`, 16-byte
+ * aligned, of at least the bytes that cms_intersect_mz_workspace gives for the
+ * queries.  It is in use until the launches have run on `stream`; nothing is
+ * kept in it between calls.
+ */
+int cms_intersect_mz_workspace(int64_t n_q, int64_t n_q_peaks, int64_t* bytes);
+int cms_intersect_mz_in(const double* ref_mz, const int64_t* ref_off, int64_t n_ref,
+                        int64_t n_ref_peaks, const double* q_mz, const int64_t* q_off, int64_t n_q,
+                        int64_t n_q_peaks, double scaling, double* out, int64_t ld,
+                        uint32_t* device_error, void* workspace, int64_t workspace_bytes,
+                        void* stream);
 
 #ifdef __cplusplus
 }

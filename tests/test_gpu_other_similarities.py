@@ -214,3 +214,68 @@ def test_mass_match_medium_cost(cuda_device):
 
     fill = ms(lambda: out.fill_(1))
     assert ms(lambda: kernels.mass_match_matrix(r, q, 0.1, out=out)) < 1.6 * fill
+
+
+@pytest.mark.parametrize("entry", ["python", "c"])
+def test_intersect_mz_workspace_is_given_back(cuda_device, entry):
+    """Nothing of a call's index (80 MB here) stays outside torch's allocator."""
+    import torch
+
+    from cudams import _native, kernels
+    from cudams._native import ptr, stream_handle
+
+    rng = np.random.default_rng(71)
+    a = _csr([np.sort(rng.uniform(50.0, 900.0, 40)) for _ in range(3)])
+    off = torch.arange(0, 3_000_001, 3000, dtype=torch.int64, device=_dev())
+    mz = torch.from_numpy(np.sort(rng.uniform(50.0, 900.0, (1000, 3000)), axis=1).ravel()).to(_dev())
+    out = torch.empty((3, 1000), dtype=torch.float64, device=_dev())
+
+    def call(q_mz, q_off):
+        if entry == "python":
+            kernels.intersect_mz_matrix(*a, q_mz, q_off, out=out[:, :q_off.shape[0] - 1])
+            return
+        s = torch.cuda.current_stream(_dev())
+        rc = _native.load().cms_intersect_mz(
+            ptr(a[0]), ptr(a[1]), 3, a[0].shape[0], ptr(q_mz), ptr(q_off), q_off.shape[0] - 1,
+            q_mz.shape[0], 1.0, ptr(out), 1000, ptr(None), stream_handle(s))
+        assert rc == _native.CMS_OK, _native.last_error()
+
+    call(mz[:3000], off[:2])  # the module is loaded
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info(_dev())[0]
+    call(mz, off)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    assert before - torch.cuda.mem_get_info(_dev())[0] < 16 << 20
+
+
+def test_intersect_mz_streams_and_capture(cuda_device):
+    """Calls on a stream of their own, overlapping on two, and captured in a graph."""
+    import torch
+
+    from cudams import kernels
+
+    rng = np.random.default_rng(72)
+    pool = np.round(rng.uniform(50.0, 900.0, 4000), 2)
+    sets = [[np.unique(rng.choice(pool, 60)) for _ in range(n)] for n in (300, 290, 310)]
+    r, q1, q2 = (_csr(s) for s in sets)
+    want = [other.intersect_mz(sets[0], s).view(np.uint64) for s in sets[1:]]
+    streams = [torch.cuda.Stream(_dev()) for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = [kernels.intersect_mz_matrix(*r, *q, stream=s, out=torch.empty(
+            (300, q[1].shape[0] - 1), dtype=torch.float64, device=_dev()))
+            for q, s in zip((q1, q2), streams)]
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g.cpu().numpy().view(np.uint64), w)
+    out = torch.zeros((300, 290), dtype=torch.float64, device=_dev())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kernels.intersect_mz_matrix(*r, *q1, out=out)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want[0])

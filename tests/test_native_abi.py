@@ -94,3 +94,23 @@ def test_pack_mz64():
     assert mz.dtype == np.float64 and off.dtype == np.int64
     np.testing.assert_array_equal(off, [0, 3, 3, 4])
     np.testing.assert_array_equal(mz, [1.0, 2.0, 2.0, 0.5])
+
+
+def test_intersect_mz_workspace_arguments():
+    """cms_intersect_mz_in refuses a workspace that is missing, too small or unaligned."""
+    import ctypes
+
+    from cudams import _native
+
+    lib = _native.load()
+    size = ctypes.c_int64(-1)
+    assert lib.cms_intersect_mz_workspace(5, 10, None) == _native.CMS_ERR_INVALID
+    assert lib.cms_intersect_mz_workspace(-1, 10, ctypes.byref(size)) == _native.CMS_ERR_INVALID
+    assert lib.cms_intersect_mz_workspace(5, 10, ctypes.byref(size)) == _native.CMS_OK
+    assert size.value >= 10 * 16 + 5 * 4
+    p = 0x1000  # never read: the checks come first
+    for work, n in ((None, size.value), (p + 8, size.value), (p, size.value - 1)):
+        rc = lib.cms_intersect_mz_in(p, p, 3, 10, p, p, 5, 10, 1.0, p, 5, None, work, n, None)
+        assert rc == _native.CMS_ERR_INVALID
+    assert lib.cms_intersect_mz_in(None, None, 0, 0, None, None, 5, 0, 1.0, None, 5, None, None, 0,
+                                   None) == _native.CMS_OK
