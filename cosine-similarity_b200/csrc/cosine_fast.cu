@@ -2751,15 +2751,17 @@ int make_plan(const CosineArgs& args, const cms_cosine_config* cfg, bool sparse,
     if (cfg && cfg->tile_spectra > 0) {
         p.tile = cfg->tile_spectra;
     } else {
-        // about 200 expected candidates per work item (reference x tile) when
-        // the caller gives candidates per pair, else 1024 queries; at most one
-        // item per 100000 pairs so that every resident warp gets tens of items
+        // about 176 expected candidates per work item (reference x tile) and at most
+        // 1792 queries when the caller gives candidates per pair, which is what the
+        // pool holds beside the heads of the tile (50000 x 50000 lognormal spectra:
+        // 8.9 ms, 9.2 with tiles of 2048), else 1024 queries; at most one item per
+        // 100000 pairs so that every resident warp gets tens of items
         const long long pairs = (long long)args.ref.n * (long long)args.qry.n;
         long long t = 1024;
         if (cfg && cfg->cand_per_pair > 0.0)
-            t = (long long)std::min(2048.0, 200.0 / cfg->cand_per_pair);
+            t = (long long)std::min(1792.0, 176.0 / cfg->cand_per_pair);
         t = std::min(t, pairs / 100000);
-        t = std::max<long long>(32, std::min<long long>(2048, t));
+        t = std::max<long long>(32, t);
         p.tile = (int)((t + 31) / 32 * 32);
     }
     if (p.tile > kMaxTile) {

@@ -589,3 +589,28 @@ def test_small_match_limit_cost(cuda_device):
         return best
 
     assert seconds(16) < 2.8 * seconds(512)
+
+
+@pytest.mark.parametrize("cand", [0.05, 0.11, 0.6])
+def test_automatic_tiles_agree(cuda_device, cand):
+    """The library's own choice of tile is the one the Python estimate makes (the work
+    items of a call, spectra times tiles, are counted by the trace)."""
+    import torch
+
+    from cudams import _native, autotune, kernels
+    from cudams.packing import pack_csr
+
+    n = 15000
+    one = pack_csr(np.full(n, 100.0, np.float32), np.ones(n, np.float32), np.arange(n + 1), None)
+    other = pack_csr(np.full(n, 200.0, np.float32), np.ones(n, np.float32), np.arange(n + 1), None)
+    tile = autotune.heuristic_config(autotune.WorkloadStats(cand, 0.0, 1.0, 1.0), n, n)["tile_spectra"]
+    rec = torch.zeros((1, 4), dtype=torch.int64, device=cuda_device)
+    count = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    ctx = _native.context(cuda_device.index)
+    ctx.trace_enable(rec, count, 1)
+    try:
+        kernels.cosine_greedy_sparse(one.to_device(cuda_device), other.to_device(cuda_device), 0.1,
+                                     0.0, 64, 0.5, config={"mode": 1, "cand_per_pair": cand})
+    finally:
+        ctx.trace_disable()
+    assert int(count.item()) == n * -(-n // tile)
