@@ -309,6 +309,19 @@ def measure(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: flo
     return _default.measure(ref, qry, tolerance, shift, match_limit, device, gpu, **kw)
 
 
+# 1e30 as float32 and 1e70 as float64, as unsigned integers: the patterns of smaller
+# values from +0 on are below them, those of all others (NaN, negative zero) are not
+_MZ_LIMIT = int(np.float32(1e30).view(np.uint32))
+_WEIGHT_LIMIT = int(np.float64(1e70).view(np.uint64))
+
+
+def _below(x, limit: int) -> bool:
+    if x is None or not x.size:
+        return True
+    bits = x.view(np.uint32 if x.dtype == np.float32 else np.uint64)
+    return int(np.maximum.reduce(bits)) < limit
+
+
 def _ordinary(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: float,
               precursors=()) -> bool:
     """Whether both modes of the kernels are sure to treat every value alike.  They
@@ -316,11 +329,9 @@ def _ordinary(ref: PackedSpectra, qry: PackedSpectra, tolerance: float, shift: f
     value is not finite, where a product of weights overflows or is a negative zero,
     and where a window ends next to zero under a shift (float32 m/z are then much
     finer than the float64 sums they are compared in)."""
-    def plain(x, limit):
-        return x is None or not x.size or (not np.signbit(x).any() and bool(x.max() < limit))
-
     for s in (ref, qry):
-        if not (plain(s.mz, 1e30) and plain(s.a, 1e70) and plain(s.b, 1e70)):
+        if not (_below(s.mz, _MZ_LIMIT) and _below(s.a, _WEIGHT_LIMIT)
+                and _below(s.b, _WEIGHT_LIMIT)):
             return False
     if not all(bool((np.abs(p) < 1e30).all()) for p in precursors):
         return False
