@@ -1719,7 +1719,7 @@ __device__ __forceinline__ GenScratch gen_scratch(void* p, int threads, int cach
 // from L2 they were most of the time).  It writes its candidates' generation
 // words; the keys are then made one rank a thread, so that the weight loads are
 // independent and no thread waits for one with more candidates.
-template <bool MODIFIED, typename Sync>
+template <bool MODIFIED, bool ONE, typename Sync>
 __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned long long* okey,
                         uint32_t* cgen, int limit, int nt, int tid, int* s_scan,
                         const GenScratch& G, Sync sync) {
@@ -1744,22 +1744,25 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
 #pragma unroll 1
         for (int pc = 0; pc < nr && !overflow; pc += kGenPeaks * nt) {
             // kGenPeaks consecutive peaks a thread (a pair that overflows is usually
-            // done after one chunk of 256), or one where that is enough: a thread's
-            // peaks are searched for one after the other (300 x 301 uniform spectra,
-            // the whole matrix at match_limit 2048: 1250 us with two, 1070 with one)
-            const int per = nr - pc > nt ? kGenPeaks : 1;
+            // done after one chunk of 256), or (ONE) one where that is enough: a
+            // thread's peaks are searched for one after the other (300 x 301 uniform
+            // spectra, the whole matrix at match_limit 2048: 1250 us with two, 1070
+            // with one; spilled pairs: 183 us with two, 192 with one for 12345
+            // symmetric spectra, 193 and 189 for modified cosine)
+            const bool one = ONE && nr - pc <= nt;
+            auto peak = [&](int u) { return (one ? tid : kGenPeaks * tid) + u; };  // in the chunk
             int start[kGenPeaks], cnt[kGenPeaks], mine = 0;
             float mz[kGenPeaks];
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
-                const int p1 = pc + per * tid + u;
-                mz[u] = u < per && p1 < nr ? P.R.mz[r0 + p1] : 0.f;
+                const int p1 = pc + peak(u);
+                mz[u] = p1 < nr ? P.R.mz[r0 + p1] : 0.f;
             }
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
-                const int p1 = pc + per * tid + u;
+                const int p1 = pc + peak(u);
                 start[u] = cnt[u] = 0;
-                if (u < per && p1 < nr) {
+                if (p1 < nr && (u == 0 || !one)) {
                     const double mz1 = (double)mz[u];
                     // the window as float32 bounds of the query's m/z (exact, see
                     // Window): first p2 at or above, then on to the last one inside.
@@ -1798,7 +1801,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
                     }
                     cnt[u] = L - start[u];
                     if (cnt[u])
-                        G.w[per * tid + u] = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
+                        G.w[peak(u)] = __dmul_rn(peak_a(P.R.a, r0 + p1), P.R.b[r0 + p1]);
                 }
                 mine += cnt[u];
             }
@@ -1821,7 +1824,7 @@ __device__ int gen_pair(const PairParams& P, int64_t ri, int64_t qi, unsigned lo
 #pragma unroll
             for (int u = 0; u < kGenPeaks; ++u) {
                 uint32_t gen = ((uint32_t)pass << 31) |
-                               ((uint32_t)(pc + per * tid + u) << 16) | (uint32_t)start[u];
+                               ((uint32_t)(pc + peak(u)) << 16) | (uint32_t)start[u];
                 const int last = min(take, first + cnt[u]);
 #pragma unroll 1
                 for (int i = first; i < last; ++i) cgen[total + i] = gen++;
@@ -2368,8 +2371,8 @@ constexpr int pair_cache(int cap, int threads, size_t optin) {
     return pair_smem_bytes(cap, threads, kPairCache) <= optin ? kPairCache : 0;
 }
 
-// Pairs of the spill list (or of the whole matrix, where the pipelined kernel
-// below does not fit).  Most spilled pairs have somewhat more candidates than the
+// Pairs of the spill list (LIST), or of the whole matrix, where the pipelined kernel
+// below does not fit.  Most spilled pairs have somewhat more candidates than the
 // join resolves; a CTA spent 15 us on each, most of it at barriers and behind
 // the one greedy warp.  So CTAs take only the heavy pairs, first, and then every
 // warp takes light ones of its own into a share of the candidate buffer; a pair
@@ -2378,7 +2381,7 @@ constexpr int pair_cache(int cap, int threads, size_t optin) {
 // registers six CTAs fit an SM (five before): the pairs of 12345 symmetric spectra
 // take 180 us (305 before), of sparse 20000 x 20000 113 (216), of modified cosine
 // 297 (421).  What is left is the longest heavy pairs.
-template <bool SPARSE, bool MODIFIED>
+template <bool SPARSE, bool MODIFIED, bool LIST>
 __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
     if (*P.bad || (P.gate && *P.gate != P.gate_value)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2394,10 +2397,11 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
 
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     // an overrun list (an error that is reported) has gaps: nothing of it is read
-    const unsigned long long count = P.pairs ? *P.n_pairs : 0ull;
+    const bool list = LIST && P.pairs;
+    const unsigned long long count = list ? *P.n_pairs : 0ull;
     const unsigned int front = (unsigned int)count, back = (unsigned int)(count >> 32);
     const bool sound = (unsigned long long)front + back <= P.pairs_cap;
-    const int64_t n_heavy = !P.pairs ? P.R.n * P.Q.n : sound ? front : 0;
+    const int64_t n_heavy = !list ? P.R.n * P.Q.n : sound ? front : 0;
     const int64_t n_light = sound ? back : 0;
     // a warp's share: a power of two (the sorts pad to one)
     int slice = kPairSlice;
@@ -2409,7 +2413,7 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
     auto resolve = [&](int64_t ri, int64_t qi, int limit, unsigned long long* k, uint32_t* g,
                        uint32_t* used_r, int words, const GenScratch& G, int nt, int t, int* scan,
                        uint16_t* queue, auto sync) {
-        const int total = gen_pair<MODIFIED>(P, ri, qi, k, g, limit, nt, t, scan, G, sync);
+        const int total = gen_pair<MODIFIED, !LIST>(P, ri, qi, k, g, limit, nt, t, scan, G, sync);
         if (total >= limit && limit < P.match_limit) return false;
         const int n = min(total, P.match_limit);
         double score = 0.0;
@@ -2460,7 +2464,7 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
         int64_t item = -1;
         if (heavy) {
             item = blockIdx.x + iter * gridDim.x;
-            if (P.pairs) {
+            if (list) {
                 __syncthreads();
                 if (tid == 0) s_item = atomicAdd(P.work, 1ull);
                 __syncthreads();
@@ -2470,7 +2474,7 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
             if (!heavy) item = -1;
         }
         if (!heavy) {
-            if (!P.pairs) break;
+            if (!list) break;
             if (n_whole == 0) {
                 if (done) break;
                 const GenScratch G{gen.w + kGenPeaks * 32 * wid, gen.qmz + P.cache / nw * wid,
@@ -2636,7 +2640,7 @@ pair_kernel_pipe(PairParams P) {
             uint32_t* cgen = cgen0 + (size_t)b * P.cap;
             int total = -1;
             if (more) {
-                total = gen_pair<MODIFIED>(P, ri, qi, okey, cgen, P.match_limit, np, tid, s_scan, gen,
+                total = gen_pair<MODIFIED, true>(P, ri, qi, okey, cgen, P.match_limit, np, tid, s_scan, gen,
                                            sync);
                 const int n = min(total, P.match_limit);
                 if (n > 0) {
@@ -3022,8 +3026,13 @@ int enqueue_cosine(cms_ctx* ctx, const CosineArgs& args, const DenseOut* dense,
     };
 
     void (*pair_k)(PairParams) =
-        sparse ? (args.modified ? pair_kernel<true, true> : pair_kernel<true, false>)
-               : (args.modified ? pair_kernel<false, true> : pair_kernel<false, false>);
+        p.mode == 2
+            ? (sparse ? (args.modified ? pair_kernel<true, true, false> : pair_kernel<true, false, false>)
+                      : (args.modified ? pair_kernel<false, true, false>
+                                       : pair_kernel<false, false, false>))
+            : (sparse ? (args.modified ? pair_kernel<true, true, true> : pair_kernel<true, false, true>)
+                      : (args.modified ? pair_kernel<false, true, true>
+                                       : pair_kernel<false, false, true>));
     int pair_blocks_per_sm = 1;
     if ((rc = set_func_smem(pair_k, pair_smem))) return rc;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pair_blocks_per_sm, pair_k, p.pair_threads,
@@ -3587,11 +3596,11 @@ extern "C" int cms_cosine_greedy_noalloc(const float* ref_mz, const double* ref_
         pp.used_words = full ? kFullWords : kUsedWords;
         pp.cache = cap <= 2048 ? kPairCache : 0;  // with 4096 it would cost a resident CTA
         const size_t pair_smem = pair_smem_bytes(cap, pair_threads, pp.cache, pp.used_words);
-        if ((rc = set_func_smem(pair_kernel<false, false>, pair_smem))) return rc;
+        if ((rc = set_func_smem(pair_kernel<false, false, false>, pair_smem))) return rc;
         int per_sm = 1;
         CMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, pair_kernel<false, false>, pair_threads, pair_smem));
-        pair_kernel<false, false><<<sms * std::max(1, per_sm), pair_threads, pair_smem, s>>>(pp);
+            &per_sm, pair_kernel<false, false, false>, pair_threads, pair_smem));
+        pair_kernel<false, false, false><<<sms * std::max(1, per_sm), pair_threads, pair_smem, s>>>(pp);
         CMS_CUDA_TRY(cudaGetLastError());
     }
     if (device_error)
@@ -3881,11 +3890,11 @@ extern "C" int cms_library_search(cms_ctx* ctx, const cms_library* lib, const fl
     pp.bad = bad;
     {
         StageScope sc(ctx, 4, 1, s);
-        if ((rc = set_func_smem(pair_kernel<true, false>, pair_smem))) return rc;
+        if ((rc = set_func_smem(pair_kernel<true, false, true>, pair_smem))) return rc;
         int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<true, false>, 128,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_kernel<true, false, true>, 128,
                                                       pair_smem);
-        pair_kernel<true, false><<<std::max(1, std::min(ctx->sm_count * std::max(1, std::min(kLongWarps, per_sm)),
+        pair_kernel<true, false, true><<<std::max(1, std::min(ctx->sm_count * std::max(1, std::min(kLongWarps, per_sm)),
                                                   (int)std::min<long long>(spill_cap, 1 << 20))),
                             128, pair_smem, s>>>(pp);
     }
