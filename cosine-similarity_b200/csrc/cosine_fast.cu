@@ -2400,7 +2400,7 @@ __global__ void __maxnreg__(80) pair_kernel(PairParams P) {
     const bool list = LIST && P.pairs;
     const unsigned long long count = list ? *P.n_pairs : 0ull;
     const unsigned int front = (unsigned int)count, back = (unsigned int)(count >> 32);
-    const bool sound = (unsigned long long)front + back <= P.pairs_cap;
+    const bool sound = (unsigned long long)front + back <= (list ? P.pairs_cap : 0u);
     const int64_t n_heavy = !list ? P.R.n * P.Q.n : sound ? front : 0;
     const int64_t n_light = sound ? back : 0;
     // a warp's share: a power of two (the sorts pad to one)
