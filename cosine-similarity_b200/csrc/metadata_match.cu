@@ -53,18 +53,19 @@ __device__ __forceinline__ bool mass_ok(double r, double q, double tol, int ppm)
 //   x < out_lo or x > out_hi:  no match;   x > in_lo and x < in_hi:  a match
 // (rounding is monotone, and a float32 strictly above in_lo comes from a q
 // above in_lo); what lies between is tested as the definition says.  Rows the
-// argument does not hold for (r not positive or extreme; a tolerance above 5e5,
-// where the ratio's bound of 2e6 gets near) take every column that way, and so
+// argument does not hold for (r not positive or extreme; a tolerance above
+// kMaxBoundPpm, where the ratio's bound of 2e6 gets near) take every column that way, and so
 // do negative q, whose mean may be negative.  mid and half describe [out_lo,
 // out_hi] once more, rounded outwards far enough that float32(|x - mid|) <= half
 // for every x inside.
+constexpr double kMaxBoundPpm = 5e5;
 struct MassRow {
     float mid, half, out_lo, out_hi;
     float in_lo, in_hi, pad0, pad1;
 };
 __device__ __forceinline__ MassRow mass_row(double r, double tol) {
     MassRow w{0.0f, INFINITY, -INFINITY, INFINITY, INFINITY, -INFINITY, 0.0f, 0.0f};
-    if (!(tol >= 0.0 && tol <= 5e5 && r >= 1e-150 && r <= 1e150)) return w;
+    if (!(tol >= 0.0 && tol <= kMaxBoundPpm && r >= 1e-150 && r <= 1e150)) return w;
     const double h = tol * 0.5e-6, m = r * 4e-15;
     const double lo = r * (1.0 - h) / (1.0 + h), hi = r * (1.0 + h) / (1.0 - h);
     w.out_lo = __double2float_rd(lo - m);
@@ -148,7 +149,12 @@ __device__ __forceinline__ void store_tail(uint8_t* row, int lane, uint32_t mask
 // out.  A few lanes that may have a match are looked at by half a warp each, a
 // column a lane; many at once make their masks themselves.  420 us (49999
 // columns: 487 us, 6030 us with a store per byte).
-template <bool PPM>
+//
+// ppm with a tolerance that the bounds do not cover (above kMaxBoundPpm, negative,
+// NaN): as in Dalton mode, with a division per pair (8000 x 8192: 115 us; with
+// every pair passed over by the bounds 407).
+enum MassKind { kDalton, kPpm, kPpmExact };
+template <MassKind KIND>
 __global__ void __launch_bounds__(kMassThreads, 3)
 mass_match_kernel(const double* __restrict__ ref, int64_t n_ref, const double* __restrict__ q,
                   int64_t n_q, double tol, uint8_t* __restrict__ out, int64_t ld, int rows) {
@@ -167,7 +173,7 @@ mass_match_kernel(const double* __restrict__ ref, int64_t n_ref, const double* _
         const double* rp = ref + rb * rows;
         int left = (int)min((int64_t)rows, n_ref - rb * rows);
         uint8_t* mine = out + rb * rows * ld + c0 + kMassCols * lane;
-        if (!PPM) {
+        if (KIND != kPpm) {
             double v[kMassCols];
 #pragma unroll
             for (int k = 0; k < kMassCols; ++k)
@@ -180,7 +186,7 @@ mass_match_kernel(const double* __restrict__ ref, int64_t n_ref, const double* _
                     uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
                     for (int k = 0; k < kMassCols; ++k)
-                        w[k >> 2] |= (uint32_t)mass_ok(r, v[k], tol, 0) << (8 * (k & 3));
+                        w[k >> 2] |= (uint32_t)mass_ok(r, v[k], tol, KIND == kPpmExact) << (8 * (k & 3));
                     __stcs(reinterpret_cast<uint4*>(mine), make_uint4(w[0], w[1], w[2], w[3]));
                 }
                 continue;
@@ -190,7 +196,7 @@ mass_match_kernel(const double* __restrict__ ref, int64_t n_ref, const double* _
                 uint32_t mask = 0u;
 #pragma unroll
                 for (int k = 0; k < kMassCols; ++k)
-                    if (mass_ok(r, v[k], tol, 0)) mask |= 1u << k;
+                    if (mass_ok(r, v[k], tol, KIND == kPpmExact)) mask |= 1u << k;
                 if (cols == kMassWarpCols)
                     store_masks(mine, lane, mask, 1u);
                 else
@@ -642,32 +648,32 @@ extern "C" int cms_mass_match(const double* ref, int64_t n_ref, const double* q,
         set_error("cms_mass_match: null pointer");
         return CMS_ERR_INVALID;
     }
-    // Rows a warp takes: 128, so that its columns are loaded once for 64 KB of
-    // output, or fewer where that leaves less than eight units a multiprocessor, or
-    // a second wave of warps that is nearly empty.  Dalton, cold cache: 40000 x 50000
-    // 410 us with 128 rows, 424 with 64; 16000 x 16384 (4000 units of 128 rows for
-    // 3552 resident warps) 72 us with 128, 66 with 64, 76 with 32; 8000 x 8192 33 us
-    // with 128, 25 with 64, 46 with 8; 4000 x 4096 14 us with 16 or 32, 24 with 4.
+    // Rows a warp takes: as many as leave twelve units a multiprocessor, because its
+    // columns are loaded once for all of them, but not so that a second wave of warps
+    // is short.  Dalton, cold cache: 8000 x 8192 33 us with 128 rows (1008 units for
+    // 3552 resident warps), 26 with 64, 29 with 32, 45 with 8; 16000 x 16384 72 us with
+    // 128 (4000 units), 66 with 64, 76 with 32; 12000 x 12288 41 us with 128, 47 with
+    // 32; 500 x 100000 25 us with 32, 31 with 64; 40000 x 50000 410 us with 128, 424
+    // with 64, where 20000 x 25000 (7700 units of 128) takes 189 and 175.
     // Ten CTAs per resident one, so that the last wave is short (one per resident:
     // 572 us instead of 420 for 40000 x 50000 in ppm).
     const int64_t sms = sm_count_of_current(), col_blocks = (n_q + kMassWarpCols - 1) / kMassWarpCols;
     const int64_t resident = sms * 24;
+    auto units_of = [&](int r) { return col_blocks * ((n_ref + r - 1) / r); };
     int rows = 128;
     for (; rows > 4; rows /= 2) {
-        const int64_t u = col_blocks * ((n_ref + rows - 1) / rows);
-        if (u >= 2 * resident || (u >= sms * 8 && u <= resident)) break;
+        const int64_t u = units_of(rows);
+        if (u >= (rows == 128 ? 4 : 2) * resident || (u >= sms * 12 && u <= resident)) break;
     }
-    const int64_t units = col_blocks * ((n_ref + rows - 1) / rows);
+    const int64_t units = units_of(rows);
     const int per_block = kMassThreads / 32;
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>((units + per_block - 1) / per_block, sms * 30));
     cudaStream_t s = (cudaStream_t)stream;
-    if (ppm)
-        mass_match_kernel<true><<<grid, kMassThreads, 0, s>>>(ref, n_ref, q, n_q, tolerance, out, ld,
-                                                              rows);
-    else
-        mass_match_kernel<false><<<grid, kMassThreads, 0, s>>>(ref, n_ref, q, n_q, tolerance, out,
-                                                               ld, rows);
+    auto* kern = !ppm ? mass_match_kernel<kDalton>
+                 : tolerance >= 0.0 && tolerance <= kMaxBoundPpm ? mass_match_kernel<kPpm>
+                                                                 : mass_match_kernel<kPpmExact>;
+    kern<<<grid, kMassThreads, 0, s>>>(ref, n_ref, q, n_q, tolerance, out, ld, rows);
     CMS_CUDA_TRY(cudaGetLastError());
     return CMS_OK;
 }

@@ -279,3 +279,45 @@ def test_intersect_mz_streams_and_capture(cuda_device):
         graph.replay()
         torch.cuda.synchronize()
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want[0])
+
+
+def test_mass_match_wide_tolerance_cost(cuda_device):
+    """A ppm tolerance past the float32 bounds costs a division a pair, at most twice
+    what the widest tolerance inside them takes."""
+    import torch
+
+    from cudams import kernels
+
+    rng = np.random.default_rng(62)
+    r, q = (torch.from_numpy(rng.uniform(100.0, 1000.0, n)).to(_dev()) for n in (8000, 8192))
+    out = torch.empty((8000, 8192), dtype=torch.uint8, device=_dev())
+
+    def ms(tolerance):
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            kernels.mass_match_matrix(r, q, tolerance, True, out=out)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert ms(6e5) < 2 * ms(4e5)
+
+
+@pytest.mark.parametrize("tol", [5e5, np.nextafter(5e5, 1e6), 1.9e6, 2e6, 2.1e6, -1.0, np.inf])
+@pytest.mark.parametrize("n_q", [512, 777])
+def test_mass_match_outside_the_bounds(cuda_device, n_q, tol):
+    import torch
+
+    from cudams import kernels
+
+    rng = np.random.default_rng(63)
+    r, q = rng.uniform(-100.0, 1000.0, 70), rng.uniform(-100.0, 1000.0, n_q)
+    q[:3] = [np.nan, np.inf, 0.0]
+    got = kernels.mass_match_matrix(torch.from_numpy(r).to(_dev()),
+                                    torch.from_numpy(q).to(_dev()), tol, True).cpu().numpy()
+    with np.errstate(all="ignore"):
+        want = (np.abs(r[:, None] - q[None, :]) / ((r[:, None] + q[None, :]) / 2) * 1e6) <= tol
+    np.testing.assert_array_equal(got.astype(bool), want)
