@@ -180,7 +180,8 @@ __device__ __forceinline__ float2 measure_of(float2 fi, float2 fa, float2 fb) {
 // Bound by instruction issue (67% of the slots; tensor pipe 30%, shared-memory data
 // path 56%, output write 30% of the copy rate at 2048 bits).  60000 x 60000:
 //   2048 bits Jaccard 6.9 -> 5.6 ms, cosine 7.05 -> 6.3; 1024 bits 4.5 -> 4.1;
-//   59999 columns 25.9 -> 7.9 ms
+//   59999 columns 25.9 -> 7.9 ms (the former gave a ring slot back too early there, see
+//   the producers, and its values were wrong)
 // from four producer and eight epilogue warps, scalar arithmetic with a Newton step
 // more per division, and stores lane by lane where rows are not 16-byte aligned.
 namespace umma {

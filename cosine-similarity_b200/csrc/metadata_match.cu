@@ -34,9 +34,11 @@ namespace {
 constexpr int kMassThreads = 256;
 constexpr int kMassCols = 16;                              // columns per thread
 constexpr int kMassWarpCols = 32 * kMassCols;              // 512
-// Queries per CTA pass: 54 KB of counters and list, four CTAs of 512 threads a
-// multiprocessor (10007 x 9000 in one pass 308 us, in two of 4504 338 us; 12000 x
-// 12000 in two of 6000 486 us, in one of 12000 503 us).
+// Queries per CTA pass.  With the static arrays a CTA of this tile has 63 KB of shared
+// memory and three of 512 threads fit a multiprocessor (four up to some 8100 queries).
+// A row's bucket walk is done once a tile, so fewer tiles are faster as long as three
+// fit: 10007 x 9000 in one pass 308 us, in two of 4504 338 us; 12000 x 12000, where one
+// pass leaves two CTAs, in two of 6000 486 us, in one of 12000 503 us.
 constexpr int kIxMaxTile = 9216;
 
 __device__ __forceinline__ bool mass_ok(double r, double q, double tol, int ppm) {

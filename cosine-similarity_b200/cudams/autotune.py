@@ -42,13 +42,15 @@ import numpy as np
 
 from .packing import PackedSpectra
 
-POOL = 256
 DENSE_CANDIDATES = 48.0  # mean candidates per pair above which mode 2 is used
 # up to this many pairs (two or three for each resident CTA of the pair kernel)
 # of ordinary values mode 2 is used without an estimate, on B200 with tolerance 0.1:
 # one pair of 100-peak spectra 29 us (join 54), 24 x 24 37 us (97), 40 x 40 52 us
-# (103), 60 x 60 75 us (104); 24 x 24 heavy-tailed 49 us (118).  The estimate alone
-# took 4.3 ms of host time a call.
+# (103), 60 x 60 75 us (104); 24 x 24 heavy-tailed 49 us (118).  1600 pairs with their
+# launches, match_limit 2048: of 1 x 1600 and 1600 x 1 spectra 69 and 64 us (join 92 and
+# 76), of 1000 peaks each 141 (245 to 890), 40 x 40 of 5000 peaks 0.34 ms (120).  The
+# join is faster, by 20 us, only with 100 peaks at match_limit 16384.  The estimate
+# alone took 4.3 ms of host time a call, and 16 to 120 for 1000 and 5000 peaks.
 FEW_PAIRS = 1600
 
 
@@ -253,7 +255,7 @@ class Tuner:
             return e0.elapsed_time(e1) / reps
 
         # 1) tile size: the estimate and its neighbours (at most MAX_AUTO_TILE:
-        # larger tiles cost the join a CTA per SM), tiles_per_trial tiles each
+        # larger tiles leave the join's shared pool less room), tiles_per_trial tiles each
         best_tile, best_ns = t0, float("inf")
         for t in tiles:
             n_q = min(qry.n, tiles_per_trial * t)
