@@ -10,9 +10,9 @@ values count once),
 
 in float64 (scaling * |A & B| first, then the division).  The score is
 symmetric bit for bit, so is_symmetric=True computes the full matrix.  The
-device kernel is cms_intersect_mz (csrc/metadata_match.cu); it merges the two
-sorted m/z lists, so the peaks of each spectrum must be sorted by m/z, as
-matchms keeps them.
+device kernels (cms_intersect_mz, csrc/metadata_match.cu) look the references'
+distinct values up in an index of the queries' ones and tell repeats by the peak
+before, so the peaks of each spectrum must be sorted by m/z, as matchms keeps them.
 """
 from __future__ import annotations
 
